@@ -262,6 +262,12 @@ struct WinInfo {
 
 }  // namespace ads
 
+// Elements a run's entry arrays are allocated past their last entry: the search copies
+// them 16 bytes at a time from 16-byte boundaries (15 bytes at 2 bytes an entry).
+namespace ads {
+constexpr int kEntrySlack = 8;
+}
+
 struct AdsDia {
   int device = 0;
   int64_t n_obs = 0;

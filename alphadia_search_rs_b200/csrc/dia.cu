@@ -161,8 +161,10 @@ int build_entries(AdsDia* d, const AdsRawArrays* raw, const std::vector<int32_t>
   vals_a.release();
   tmp.release();
 
-  ADS_TRY(d->cycles.alloc(n_items));
-  ADS_TRY(d->intens.alloc(n_items));
+  if (n_items > 0) {  // (16-byte copies may reach past the last entry)
+    ADS_TRY(d->cycles.alloc(n_items + kEntrySlack));
+    ADS_TRY(d->intens.alloc(n_items + kEntrySlack));
+  }
   DevBuf<uint32_t> counts;
   ADS_TRY(counts.alloc((size_t)(n_slots * stride)));
   ADS_TRY(d->slice_starts.alloc((size_t)(n_slots * stride)));

@@ -787,7 +787,7 @@ __global__ void to_bf16_kernel(int64_t n, const float* __restrict__ in, uint16_t
 int ensure_bf16_intensities(AdsDia* d, cudaStream_t st) {
   std::lock_guard<std::mutex> lk(d->mu);
   if (d->intens_bf16.p || d->n_entries == 0) return ADS_OK;
-  ADS_TRY(d->intens_bf16.alloc((size_t)d->n_entries));
+  ADS_TRY(d->intens_bf16.alloc((size_t)d->n_entries + kEntrySlack));
   to_bf16_kernel<<<1184, 256, 0, st>>>(d->n_entries, d->intens.p, d->intens_bf16.p);
   ADS_LAUNCH_CHECK();
   // searches on other streams may read the copy next
@@ -994,7 +994,7 @@ int enqueue_search(AdsSelection* s, const AdsDia* d, const AdsLib* l, AdsCandida
   sa.h = s->h;
   sa.k_out = k_out;
   sa.gather_mode = s->o.gather_mode;
-  sa.scan_thresh = 4 * 32 * (bf16 ? kPrefetchChunks<true> : kPrefetchChunks<false>);
+  sa.scan_thresh = bf16 ? kScanThreshBf16 : kScanThreshFp32;
   sa.err = c->err_p;
   sa.cand_n = s->cand_n.p;
   sa.cand_score = s->cand_score.p;
@@ -1029,14 +1029,14 @@ int enqueue_search(AdsSelection* s, const AdsDia* d, const AdsLib* l, AdsCandida
     // which packs long-window classes into shared memory better than 8
     bool grow = cmax_b > kSmemMaxCycles;
     int nw = s->o.warps_per_block > 0 ? s->o.warps_per_block : kDefaultWarpsPerBlock;
-    if (!grow && search_smem_bytes(1, S, s->h, (cmax_b + 32 * S - 1) / (32 * S) * 32 * S, false) >
+    if (!grow && search_smem_bytes(1, S, s->h, (cmax_b + 32 * S - 1) / (32 * S) * 32 * S, cmax_b, false) >
                      (size_t)max_smem)
       grow = true;  // a very wide kernel: even one warp's plan exceeds shared memory
     if (grow) S = kGrowLaneCycles;
     nw = std::max(1, std::min(nw, max_warps_per_block(bf16, s->h, grow, s->stats_on)));
     const int ncell_b = (cmax_b + 32 * S - 1) / (32 * S) * 32 * S;
-    while (nw > 1 && search_smem_bytes(nw, S, s->h, ncell_b, grow) > (size_t)max_smem) --nw;
-    const size_t smem = search_smem_bytes(nw, S, s->h, ncell_b, grow);
+    while (nw > 1 && search_smem_bytes(nw, S, s->h, ncell_b, cmax_b, grow) > (size_t)max_smem) --nw;
+    const size_t smem = search_smem_bytes(nw, S, s->h, ncell_b, cmax_b, grow);
     if (smem > (size_t)max_smem)
       return fail(ADS_ERR_INTERNAL, "search kernel plan exceeds shared memory (" +
                                         std::to_string(cmax_b) + " cycles)");
@@ -1054,7 +1054,7 @@ int enqueue_search(AdsSelection* s, const AdsDia* d, const AdsLib* l, AdsCandida
     int64_t blocks = std::min<int64_t>((int64_t)s->num_sms * bps, (P + nw - 1) / nw);
     sa.grow = nullptr;
     if (grow) {
-      const size_t warp_bytes = (size_t)warp_plan(S, s->h, ncell_b).total * 4;
+      const size_t warp_bytes = (size_t)warp_plan(S, s->h, ncell_b, cmax_b).total * 4;
       blocks = grow_blocks(blocks, nw, warp_bytes, (size_t)kGrowBudgetBytes);
       ADS_TRY(s->grow.reserve((size_t)blocks * nw * warp_bytes / 4));
       sa.grow = s->grow.p;
@@ -1625,7 +1625,7 @@ int select_noalloc(const AdsDia* d, const AdsLib* l, const AdsSelectionParams* p
   const int S0 = best_lane_cycles(c_max);
   const bool grow =
       c_max > kSmemMaxCycles ||
-      search_smem_bytes(1, S0, h, (int)((c_max + 32 * S0 - 1) / (32 * S0) * 32 * S0)) > (size_t)max_smem;
+      search_smem_bytes(1, S0, h, (int)((c_max + 32 * S0 - 1) / (32 * S0) * 32 * S0), (int)c_max) > (size_t)max_smem;
   const int S = grow ? kGrowLaneCycles : S0;
   const int ncell = (int)((c_max + 32 * S - 1) / (32 * S) * 32 * S);
   const int k_out = (int)std::max<int64_t>(0, std::min<int64_t>(prm.candidate_count, maxima_cap(ncell)));
@@ -1665,7 +1665,7 @@ int select_noalloc(const AdsDia* d, const AdsLib* l, const AdsSelectionParams* p
   float* taps = h > kMaxHalf ? sc.take<float>(L) : nullptr;  // wide kernels: taps on the device
   // long windows: at least one block of warps' working sets must fit after the rest
   const int nw0 = kDefaultWarpsPerBlock;
-  const size_t grow_warp_bytes = grow ? (size_t)warp_plan(S, h, ncell).total * 4 : 0;
+  const size_t grow_warp_bytes = grow ? (size_t)warp_plan(S, h, ncell, (int)c_max).total * 4 : 0;
   float* grow_sets = nullptr;
   size_t grow_bytes = 0;
   if (grow) {  // the rest of the array, which must hold one block's working sets
@@ -1731,8 +1731,8 @@ int select_noalloc(const AdsDia* d, const AdsLib* l, const AdsSelectionParams* p
   ADS_LAUNCH_CHECK();
 
   int nw = nw0;
-  while (nw > 1 && search_smem_bytes(nw, S, h, ncell, grow) > (size_t)max_smem) --nw;
-  const size_t smem = search_smem_bytes(nw, S, h, ncell, grow);
+  while (nw > 1 && search_smem_bytes(nw, S, h, ncell, (int)c_max, grow) > (size_t)max_smem) --nw;
+  const size_t smem = search_smem_bytes(nw, S, h, ncell, (int)c_max, grow);
   if (smem > (size_t)max_smem)
     return fail(ADS_ERR_INTERNAL, "search kernel plan exceeds shared memory (" +
                                       std::to_string(c_max) + " cycles)");
@@ -1767,7 +1767,7 @@ int select_noalloc(const AdsDia* d, const AdsLib* l, const AdsSelectionParams* p
   sa.c_max = (int)c_max;
   sa.ncell = ncell;
   sa.gather_mode = 0;
-  sa.scan_thresh = 4 * 32 * kPrefetchChunks<false>;
+  sa.scan_thresh = kScanThreshFp32;
   sa.work = work;
   sa.err = flags;
   sa.cand_n = cand_n;

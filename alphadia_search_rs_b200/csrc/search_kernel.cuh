@@ -58,17 +58,20 @@ struct SearchArgs {
   unsigned long long* stats;  // nullable
 };
 
-// CSR entries read per round trip of the scanning gather: 2 x 32 for f32 intensities,
-// 3 x 32 for bfloat16 ones (measured: 64-entry batches are 3.7 % faster than 128 on
-// 3000 x 300 FP32 data with 301-cycle windows; for BF16 storage 96-entry batches are
-// 0.5-1 % faster than 128, 64 and 192 slower).
-template <bool FAST>
-constexpr int kPrefetchChunks = FAST ? 3 : 2;
+// The scanning gather copies up to kStageEntries CSR entries of a (fragment, window)
+// range into the warp's staging area in shared memory, asynchronously and 16 bytes per
+// lane: intensities first, then cycles, each from the 16-byte boundary at or below the
+// range's first entry.
+constexpr int kStageEntries = 128;
+constexpr int kStageCycOff = kStageEntries * 4 + 16;                   // bytes
+constexpr int kStageWords = (kStageCycOff + kStageEntries * 2 + 16) / 4;
+// Bin ranges of more entries than this are binary-searched per bin instead of scanned.
+constexpr int kScanThreshFp32 = 256, kScanThreshBf16 = 384;
 constexpr int kBitOff = 32;         // bitmap bit of cycle c is c + kBitOff (room for -h)
 constexpr int kSmemMaxCycles = 2048;  // longest RT window (cycles) a warp's shared-memory plan
                                       // holds; longer windows run with GROW
-constexpr int kTouchCap = 256;      // cells a row records for clearing; beyond it the row is
-                                    // zeroed whole
+constexpr int kTouchCap = 256;      // accepted cells a row records for clearing; beyond it the
+                                    // row is zeroed whole
 
 __host__ __device__ inline int maxima_cap(int ncell) { return ncell / 4 + 8; }
 
@@ -100,9 +103,12 @@ __host__ __device__ constexpr int floordiv(int a, int b) {
 }
 
 // Per-warp shared-memory plan, in 4-byte words.  The block's ln table (double2 x
-// 256 = 1024 words) and kernel taps (h + 1 words, at least 32) come first.
+// 256 = 1024 words), kernel taps (h + 1 words, at least 32) and the warps' staging
+// areas come first.  `ncell` (passes * 32 * S) sizes the bitmap, which every lane reads;
+// the row and the scores, of which only lanes with an output below c_max touch theirs,
+// are sized by c_max (a 801-cycle class of S = 16 would else hold 1024 cycles).
 struct WarpPlan {
-  int row, tags, bm, scr, score, lst, mval, midx, touched, total;
+  int row, bm, cells, score, lst, mval, midx, total;
   int off;        // stored index of cycle c is c + off (off >= h, a multiple of S)
   int row_words;  // words of the row, a multiple of 4
   int lead;       // bitmap words below bm[0]: a window reaching h cycles before cycle 0
@@ -114,28 +120,27 @@ __host__ __device__ inline int block_header_words(int h) {
   return kLnTableSize * 4 + ((h + 1 + 31) / 32) * 32;
 }
 
-__host__ __device__ inline WarpPlan warp_plan(int S, int h, int ncell) {
+__host__ __device__ inline WarpPlan warp_plan(int S, int h, int ncell, int c_max) {
   WarpPlan w;
+  const int cc = (c_max + S - 1) / S * S;
   w.off = (h + S - 1) / S * S;
-  const int span = ncell + h + w.off + S;  // stored indices [0, span) cover every read
+  const int span = cc + h + w.off + S;  // stored indices [0, span) cover every read
   w.row_words = (span + (span / S + 1) * (row_stride(S) - S) + 3) & ~3;
   int o = 0;
   w.row = o;
   o += w.row_words;
-  w.tags = o;  // one byte per cell: the lane that wrote it last
-  o += (ncell + 3) / 4;
   w.lead = h > kBitOff ? (h - kBitOff + 31) / 32 : 0;
   w.bw = (ncell + h + kBitOff + 31) / 32 + 2;
   w.bm = o + w.lead;
   o += w.lead + w.bw;
-  w.scr = o;
-  o += 32;
-  w.touched = o;  // cells written by the current row (16 bits each)
+  w.cells = o;  // cells accepted by the current row (16 bits each)
   o += kTouchCap / 2;
   w.score = o + 4;  // 4 words of margin below: the maxima scan reads 2 cycles early
-  o += ncell + ncell / S + 12;
+  o += cc + cc / S + 12;
   o = (o + 1) & ~1;
-  w.lst = o;  // one pass of non-zero convolved values: (value, score address) pairs
+  // one pass of convolved values as (value, score address) pairs; before it, while the
+  // row is gathered, the accepted entries' intensities (kTouchCap words)
+  w.lst = o;
   o += 2 * 32 * S;
   w.mx = maxima_cap(ncell);
   if (2 * w.mx <= 2 * 32 * S) {
@@ -153,8 +158,10 @@ __host__ __device__ inline WarpPlan warp_plan(int S, int h, int ncell) {
   return w;
 }
 
-__host__ __device__ inline size_t search_smem_bytes(int nw, int S, int h, int ncell, bool grow = false) {
-  return (size_t)(block_header_words(h) + (grow ? 0 : nw * warp_plan(S, h, ncell).total)) * 4;
+__host__ __device__ inline size_t search_smem_bytes(int nw, int S, int h, int ncell, int c_max,
+                                                    bool grow = false) {
+  return (size_t)(block_header_words(h) +
+                  nw * (kStageWords + (grow ? 0 : warp_plan(S, h, ncell, c_max).total))) * 4;
 }
 
 // Launch bounds of an instance.  The FP32 shared-memory instances for half widths 10
@@ -198,60 +205,76 @@ struct Counters {
   Count<ON> read, acc, off, pairs, bins1, frag;
 };
 
-// The rare case of add_chunk: lanes that hit the same cycle are grouped and summed
+// One fragment row being gathered.  Accepted entries are appended, in CSR order, to a list
+// (cell, intensity) and added to the row 32 at a time, so that the adds run with full
+// warps however few entries of a chunk lie in the RT window (7 of 32 on average on
+// 3000 x 300 data); the list is also what the next row clears.
+struct RowList {
+  float* row;
+  uint32_t* bm;
+  uint16_t* cells;  // entry i at i % kTouchCap
+  float* vals;      // likewise
+  int n;            // entries appended (warp-uniform)
+  int done;         // of them added to the row
+};
+
+// The rare case of add_entries: lanes that hit the same cycle are grouped and summed
 // by their lowest lane in lane order (kept out of line: it is seldom taken).
-static __device__ __noinline__ void add_chunk_grouped(bool inc, int cell, int addr, float v,
-                                                      int lane, float* row, uint32_t* bm,
-                                                      float* scr) {
-  const int key = inc ? cell : (-1 - lane);
+static __device__ __noinline__ void add_grouped(bool act, int cell, int addr, int first, int lane,
+                                                float* row, const float* vals) {
+  const int key = act ? cell : (-1 - lane);
   const unsigned grp = __match_any_sync(kFull, key);
-  scr[lane] = v;
-  __syncwarp();
-  if (inc && lane == __ffs(grp) - 1) {
+  if (act && lane == __ffs(grp) - 1) {
     float acc = row[addr];
     unsigned g = grp;
     while (g) {
       const int l = __ffs(g) - 1;
-      acc = __fadd_rn(acc, scr[l]);
+      acc = __fadd_rn(acc, vals[(first + l) % kTouchCap]);
       g &= g - 1;
     }
     row[addr] = acc;
-    const int bit = cell + kBitOff;
-    atomicOr(bm + (bit >> 5), 1u << (bit & 31));
   }
 }
 
-// Adds one chunk of 32 CSR-consecutive entries to the XIC row in lane order (the
-// reference's `dense_xic[c] += intensity`, src/quadrupole_observation/mod.rs:96-105).
-// Every accepted lane writes its lane number into its cycle's tag; a lane that
-// reads back another number shares the cycle, and only then are the lanes grouped
-// and summed by their lowest lane one rounded add at a time.
-// Accepted cells are also appended to `touched` (the next row clears them).
-template <class Acc>
-__device__ __forceinline__ void add_chunk(bool inc, int cell, int addr, float v, int lane,
-                                          float* row, uint32_t* bm, uint8_t* tags, float* scr,
-                                          Acc& n_acc, uint16_t* touched, int& n_touched) {
-  const unsigned act = __ballot_sync(kFull, inc);
-  if (act == 0) return;
-  n_acc += (unsigned int)__popc(act);
-  if (inc) {
-    const int at = n_touched + __popc(act & ((1u << lane) - 1u));
-    if (at < kTouchCap) touched[at] = (uint16_t)cell;
-  }
-  n_touched += __popc(act);
-  if (inc) tags[cell] = (uint8_t)lane;
+// Adds the next m (1 to 32) listed entries to the XIC row in list order (the reference's
+// `dense_xic[c] += intensity`, src/quadrupole_observation/mod.rs:96-105).  Setting a
+// cell's bit tells whether it was touched before, by an earlier entry or by another lane:
+// if none was, every cell holds 0 and takes its intensity; else the lanes are grouped by
+// cell and summed by their lowest lane one rounded add at a time.
+template <int S>
+__device__ __forceinline__ void add_entries(RowList& r, int m, int off, int lane) {
   __syncwarp();
-  const bool dup = inc && tags[cell] != (uint8_t)lane;
-  const int bit = cell + kBitOff;
-  if (!__any_sync(kFull, dup)) {
-    if (inc) {
-      row[addr] = __fadd_rn(row[addr], v);
-      atomicOr(bm + (bit >> 5), 1u << (bit & 31));
-    }
+  const int i = (r.done + lane) % kTouchCap;
+  const bool act = lane < m;
+  const int cell = r.cells[i];
+  const float v = r.vals[i];
+  const int addr = raddr<S>(cell + off);
+  const uint32_t bit = 1u << (cell & 31);
+  bool again = false;
+  if (act) again = (atomicOr(r.bm + ((cell + kBitOff) >> 5), bit) & bit) != 0u;
+  if (!__any_sync(kFull, again)) {
+    if (act) r.row[addr] = v;
   } else {
-    add_chunk_grouped(inc, cell, addr, v, lane, row, bm, scr);
+    add_grouped(act, cell, addr, r.done, lane, r.row, r.vals);
   }
-  __syncwarp();
+  r.done += m;
+}
+
+// Appends the lanes' entries marked `in`, in lane order.
+template <int S, class Acc>
+__device__ __forceinline__ void append_entries(RowList& r, bool in, int cell, float v, int off,
+                                               int lane, Acc& n_acc) {
+  const unsigned act = __ballot_sync(kFull, in);
+  if (act == 0) return;
+  if (in) {
+    const int at = (r.n + __popc(act & ((1u << lane) - 1u))) % kTouchCap;
+    r.cells[at] = (uint16_t)cell;
+    r.vals[at] = v;
+  }
+  const int k = __popc(act);
+  n_acc += (unsigned int)k;
+  r.n += k;
+  if (r.n - r.done >= 32) add_entries<S>(r, 32, off, lane);
 }
 
 // Is `pos` the first entry of one of the bins (b0, b1)?  (slice_starts[b] == pos)
@@ -269,107 +292,119 @@ static __device__ __noinline__ bool bin_starts_at(const uint32_t* ssw, uint32_t 
   return lo < b1 && __ldg(ssw + lo) == pos;
 }
 
-// fill_xic_slice for one (fragment, window) pair whose bin range [b0, b1) spans
-// the CSR entries [rs, re) of the window.  Two exact strategies:
-//   scan     read every entry of the range, keep start < cycle < stop plus, per
-//            bin, the last entry at cycle == start (where Rust's binary_search
-//            lands, src/quadrupole_observation/mod.rs:91-94);
-//   bsearch  per bin, binary-search the first kept entry and the first entry at or
-//            past stop, then read only the kept entries.
-// Up to 32 * NC CSR entries (cycle, intensity) of a scanned range, one per lane and
-// chunk, -1 / 0 past its end.
-template <int NC>
-struct ScanBatch {
-  int c[NC];
-  float v[NC];
-};
-
-// Entries of one observation: CSR positions are 32-bit offsets from its base.
-struct WinEntries {
-  const uint16_t* cy;
-  const float* in;
-  const uint16_t* in16;  // bfloat16 copy (BF16-storage searches)
-};
-
-__device__ __forceinline__ WinEntries win_entries(const SearchArgs& a, int64_t wbase) {
-  return WinEntries{a.cyc + wbase, a.inten + wbase, a.inten_bf16 + wbase};
+// Entries of one run, addressed by absolute CSR position (64 bits: a run may hold more
+// than 2^32 entries).
+template <bool FAST>
+__device__ __forceinline__ float ld_intensity(const SearchArgs& a, int64_t q) {
+  if (FAST) return __uint_as_float((uint32_t)__ldg(a.inten_bf16 + q) << 16);
+  return __ldg(a.inten + q);
 }
 
-// Intensity of entry q: f32, or (BF16 storage) the bfloat16 copy widened.
-template <bool FAST>
-__device__ __forceinline__ float ld_intensity(const WinEntries& e, uint32_t q) {
-  if (FAST) return __uint_as_float((uint32_t)__ldg(e.in16 + q) << 16);
-  return __ldg(e.in + q);
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
+// Starts copying entries [q0, q0 + m) (m <= kStageEntries) into the staging area: lane k
+// takes 16-byte pieces k, k + 32 of the intensities' pieces followed by the cycles'.  A
+// range of up to about 76 FP32 (120 BF16) entries is one instruction of the warp; through
+// registers, 64 (96) entries took 4 to 6 loads and as many live registers across the
+// stencil.
 template <bool FAST>
-__device__ __forceinline__ void load_batch(const WinEntries& e, uint32_t q0, uint32_t re, int lane,
-                                           ScanBatch<kPrefetchChunks<FAST>>& b) {
-#pragma unroll
-  for (int u = 0; u < kPrefetchChunks<FAST>; ++u) {
-    const uint32_t q = q0 + u * 32 + lane;
-    b.c[u] = q < re ? (int)__ldg(e.cy + q) : -1;
-    b.v[u] = q < re ? ld_intensity<FAST>(e, q) : 0.0f;
+__device__ __forceinline__ void stage_entries(const SearchArgs& a, int64_t q0, int m, uint32_t stage,
+                                              int lane) {
+  constexpr int PI = FAST ? 8 : 4;  // intensities in 16 bytes
+  const char* in = FAST ? reinterpret_cast<const char*>(a.inten_bf16) + (q0 & ~(int64_t)7) * 2
+                        : reinterpret_cast<const char*>(a.inten) + (q0 & ~(int64_t)3) * 4;
+  const char* cy = reinterpret_cast<const char*>(a.cyc) + (q0 & ~(int64_t)7) * 2;
+  const int ni = ((int)(q0 & (PI - 1)) + m + PI - 1) / PI;
+  const int nc = ((int)(q0 & 7) + m + 7) / 8;
+  for (int k = lane; k < ni + nc; k += 32) {
+    if (k < ni)
+      cp_async16(stage + k * 16, in + k * 16);
+    else
+      cp_async16(stage + kStageCycOff + (k - ni) * 16, cy + (k - ni) * 16);
   }
+}
+
+__device__ __forceinline__ void stage_wait() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
 }
 
 __device__ __forceinline__ bool scans(const SearchArgs& a, uint32_t n) {
   return a.gather_mode == 1 || (a.gather_mode == 0 && n <= (uint32_t)a.scan_thresh);
 }
 
-// `pre`: the range's first batch, already loaded (or null).
+// The CSR ranges of a precursor's (fragment, window) pairs, fetched 32 at a time
+// (lane q holds pair pb + q), and the pair whose first entries are staged.
+struct PairCursor {
+  int pb = -64;
+  uint32_t rs = 0, n = 0, b0 = 0, b1 = 0;
+  int wsel = 0;
+  int64_t wbase = 0;
+  int pre_pi = -1;
+};
+
+// The pair in lane q of the cursor.
+struct Pair {
+  int64_t q;   // absolute position of its first entry
+  uint32_t n;  // entries
+};
+__device__ __forceinline__ Pair pair_of(const PairCursor& pc, int q) {
+  return Pair{__shfl_sync(kFull, pc.wbase + pc.rs, q), __shfl_sync(kFull, pc.n, q)};
+}
+
+// fill_xic_slice for the (fragment, window) pair in lane `pq` of the cursor.  Two exact
+// strategies:
+//   scan     read every entry of the range, keep start < cycle < stop plus, per
+//            bin, the last entry at cycle == start (where Rust's binary_search
+//            lands, src/quadrupole_observation/mod.rs:91-94);
+//   bsearch  per bin, binary-search the first kept entry and the first entry at or
+//            past stop, then read only the kept entries.
+// `staged`: the range's first kStageEntries entries are already on their way.
 template <int S, bool FAST, bool STATS>
-__device__ __forceinline__ void gather_pair(const SearchArgs& a, int wsel, int64_t wbase,
-                                            uint32_t b0, uint32_t b1, uint32_t rs, uint32_t re,
-                                            int cs, int ce, int lane, float* row, int off,
-                                            uint32_t* bm, uint8_t* tags, float* scr,
-                                            Counters<STATS>& k,
-                                            const ScanBatch<kPrefetchChunks<FAST>>* pre,
-                                            uint16_t* touched,
-                                            int& n_touched) {
-  if (re <= rs) return;
-  const uint32_t n = re - rs;
-  const WinEntries e = win_entries(a, wbase);
-  if (scans(a, n)) {
-    k.read += (unsigned int)n;
-    constexpr int NC = kPrefetchChunks<FAST>;
-    for (uint32_t q0 = rs; q0 < re; q0 += 32 * NC) {
-      ScanBatch<NC> bt;
-      if (pre != nullptr && q0 == rs)
-        bt = *pre;
-      else
-        load_batch<FAST>(e, q0, re, lane, bt);
-#pragma unroll
-      for (int u = 0; u < NC; ++u) {
-        const uint32_t qb = q0 + u * 32;
-        if (qb >= re) break;
-        const uint32_t q = qb + lane;
-        const int cu = bt.c[u];
-        bool inc = q < re && cu > cs && cu < ce;
-        const bool at_start = q < re && cu == cs;
-        if (__any_sync(kFull, at_start)) {
-          int nxt = __shfl_down_sync(kFull, cu, 1);
-          const int nxt_first = __shfl_sync(kFull, bt.c[u + 1 < NC ? u + 1 : u], 0);
-          if (lane == 31) nxt = (u + 1 < NC) ? nxt_first : -2;
-          if (at_start) {
-            const uint32_t qn = q + 1;
-            bool last = qn >= re;
-            if (!last) last = bin_starts_at(a.ss + a.win[wsel].ss_off, b0, b1, qn);
-            if (!last) {
-              const int cn = nxt == -2 ? (int)__ldg(e.cy + qn) : nxt;
-              last = cn != cs;
+__device__ __forceinline__ void gather_pair(const SearchArgs& a, const PairCursor& pc, int pq,
+                                            Pair pr, bool staged, int cs, int C, int lane,
+                                            uint32_t stage, const unsigned char* stage_p,
+                                            RowList& r, int off, Counters<STATS>& k) {
+  if (scans(a, pr.n)) {
+    k.read += pr.n;
+    for (uint32_t q0 = 0; q0 < pr.n; q0 += kStageEntries) {
+      const int m = (int)min(pr.n - q0, (uint32_t)kStageEntries);
+      const int64_t q = pr.q + q0;
+      if (!(staged && q0 == 0)) {
+        __syncwarp();  // the area's previous entries have been read
+        stage_entries<FAST>(a, q, m, stage, lane);
+      }
+      stage_wait();
+      const uint16_t* sc = reinterpret_cast<const uint16_t*>(stage_p + kStageCycOff) + (q & 7);
+      const float* sf = reinterpret_cast<const float*>(stage_p) + (q & 3);
+      const uint16_t* sh = reinterpret_cast<const uint16_t*>(stage_p) + (q & 7);
+      for (int t = lane; t < ((m + 31) & ~31); t += 32) {
+        const int cell = (int)sc[t] - cs;
+        bool in = t < m && (unsigned)cell < (unsigned)C;
+        const float v = FAST ? __uint_as_float((uint32_t)sh[t] << 16) : sf[t];
+        if (__any_sync(kFull, in && cell == 0)) {
+          const uint32_t rs = __shfl_sync(kFull, pc.rs, pq);
+          const uint32_t b0 = __shfl_sync(kFull, pc.b0, pq), b1 = __shfl_sync(kFull, pc.b1, pq);
+          const int wsel = __shfl_sync(kFull, pc.wsel, pq);
+          if (in && cell == 0) {
+            const uint32_t tn = q0 + (uint32_t)t + 1;  // the next entry of the range
+            if (tn < pr.n && !bin_starts_at(a.ss + a.win[wsel].ss_off, b0, b1, rs + tn)) {
+              const int cn = t + 1 < m ? (int)sc[t + 1] : (int)__ldg(a.cyc + pr.q + tn);
+              in = cn != cs;
             }
-            inc = last;
           }
         }
-        const int cell = cu - cs;
-        add_chunk(inc, cell, inc ? raddr<S>(cell + off) : 0, bt.v[u], lane, row, bm, tags, scr,
-                  k.acc, touched, n_touched);
+        append_entries<S>(r, in, cell, v, off, lane, k.acc);
       }
     }
   } else {
+    const uint32_t b0 = __shfl_sync(kFull, pc.b0, pq), b1 = __shfl_sync(kFull, pc.b1, pq);
+    const int wsel = __shfl_sync(kFull, pc.wsel, pq);
+    const int64_t wbase = __shfl_sync(kFull, pc.wbase, pq);
     const uint32_t* ssw = a.ss + a.win[wsel].ss_off;
-    const uint16_t* cy = e.cy;
+    const uint16_t* cy = a.cyc + wbase;
     for (uint32_t bb = b0; bb < b1; bb += 32) {
       const uint32_t b = bb + lane;
       const bool vb = b < b1;
@@ -377,7 +412,7 @@ __device__ __forceinline__ void gather_pair(const SearchArgs& a, int wsel, int64
       if (vb) {
         const int64_t s0 = __ldg(ssw + b), s1 = __ldg(ssw + b + 1);
         pos = s0 + rust_bsearch_u16(cy + s0, s1 - s0, cs);
-        const int64_t end = pos + lower_bound_u16(cy + pos, s1 - pos, ce);
+        const int64_t end = pos + lower_bound_u16(cy + pos, s1 - pos, cs + C);
         cnt = end - pos;
       }
       k.off += 2u * (unsigned int)__popc(__ballot_sync(kFull, vb));
@@ -404,10 +439,8 @@ __device__ __forceinline__ void gather_pair(const SearchArgs& a, int wsel, int64
         const bool vt = t < total;
         const int64_t q = opos + (t - oex);
         const int c = vt ? (int)__ldg(cy + q) : 0;
-        const float v = vt ? ld_intensity<FAST>(e, (uint32_t)q) : 0.0f;
-        const int cell = c - cs;
-        add_chunk(vt, cell, vt ? raddr<S>(cell + off) : 0, v, lane, row, bm, tags, scr, k.acc,
-                  touched, n_touched);
+        const float v = vt ? ld_intensity<FAST>(a, wbase + q) : 0.0f;
+        append_entries<S>(r, vt, c - cs, v, off, lane, k.acc);
       }
     }
   }
@@ -543,79 +576,73 @@ __device__ __forceinline__ void warp_merge_best_first(float& v, int& i, int lane
   for (int j = 16; j > 0; j >>= 1) cmpx(v, i, j, (lane & j) == 0);
 }
 
-// The CSR ranges of a precursor's (fragment, window) pairs, fetched 32 at a time
-// (lane q holds pair pb + q), and the first batch of the next row's first pair,
-// loaded while the current row is convolved.
+// Moves the cursor to pairs [pi, pi + 32).
+__device__ __forceinline__ void load_pairs(const SearchArgs& a, int64_t p, int pi, int nwin,
+                                           int npairs, int lane, PairCursor& pc) {
+  pc.pb = pi;
+  const int pj = pi + lane;
+  pc.rs = pc.n = 0;
+  pc.b0 = pc.b1 = 0;
+  pc.wsel = 0;
+  pc.wbase = 0;
+  if (pj < npairs) {
+    const int fj = nwin == 1 ? pj : pj / nwin, wj = pj - fj * nwin;
+    const int64_t fo = p * a.kf + fj;
+    pc.b0 = a.blo[fo];
+    pc.b1 = a.bhi[fo];
+    pc.wsel = a.wins[p * a.maxw + wj];
+    if (pc.b1 > pc.b0) {
+      const WinInfo w = a.win[pc.wsel];
+      pc.wbase = w.base;
+      pc.rs = __ldg(a.ss + w.ss_off + pc.b0);
+      pc.n = __ldg(a.ss + w.ss_off + pc.b1) - pc.rs;
+    }
+  }
+}
+
+// Starts staging pair pi's first entries (after the area's last ones have been read).
 template <bool FAST>
-struct PairCursor {
-  int pb = -64;
-  uint32_t rs = 0, re = 0, b0 = 0, b1 = 0;
-  int wsel = 0;
-  int64_t wbase = 0;
-  ScanBatch<kPrefetchChunks<FAST>> pre;
-  int pre_pi = -1;
-};
+__device__ __forceinline__ void stage_pair(const SearchArgs& a, int64_t p, int pi, int nwin,
+                                           int npairs, int lane, PairCursor& pc, uint32_t stage) {
+  pc.pre_pi = -1;
+  if (pi >= npairs) return;
+  if (pi >= pc.pb + 32) load_pairs(a, p, pi, nwin, npairs, lane, pc);
+  const Pair pr = pair_of(pc, pi - pc.pb);
+  if (pr.n > 0 && scans(a, pr.n)) {
+    __syncwarp();
+    stage_entries<FAST>(a, pr.q, (int)min(pr.n, (uint32_t)kStageEntries), stage, lane);
+    pc.pre_pi = pi;
+  }
+}
 
 // Gathers fragment f's XIC row: its (fragment, window) pairs in window order (the
 // reference's DenseXICObservation::new, src/dense_xic_observation/mod.rs:30-64),
-// then prefetches the first batch of the next fragment's first pair.
+// then starts staging the next fragment's first pair, which arrives while this row is
+// convolved.
 template <int S, bool FAST, bool STATS>
 __device__ __forceinline__ void gather_row(const SearchArgs& a, int64_t p, int f, int nwin,
-                                           int npairs, int cs, int ce, int lane,
-                                           PairCursor<FAST>& pc, float* row, int off,
-                                           uint32_t* bm, uint8_t* tags, float* scr,
-                                           Counters<STATS>& k,
-                                           uint16_t* touched, int& n_touched) {
+                                           int npairs, int cs, int C, int lane, PairCursor& pc,
+                                           uint32_t stage, const unsigned char* stage_p, RowList& r,
+                                           int off, Counters<STATS>& k) {
   for (int wi = 0; wi < nwin; ++wi) {
     const int pi = f * nwin + wi;
-    if (pi >= pc.pb + 32) {
-      pc.pb = pi;
-      const int pj = pc.pb + lane;
-      pc.rs = pc.re = 0;
-      pc.b0 = pc.b1 = 0;
-      pc.wsel = 0;
-      pc.wbase = 0;
-      if (pj < npairs) {
-        const int fj = pj / nwin, wj = pj - fj * nwin;
-        const int64_t fo = p * a.kf + fj;
-        pc.b0 = a.blo[fo];
-        pc.b1 = a.bhi[fo];
-        pc.wsel = a.wins[p * a.maxw + wj];
-        if (pc.b1 > pc.b0) {
-          const WinInfo w = a.win[pc.wsel];
-          pc.wbase = w.base;
-          pc.rs = __ldg(a.ss + w.ss_off + pc.b0);
-          pc.re = __ldg(a.ss + w.ss_off + pc.b1);
-        }
+    if (pi >= pc.pb + 32) load_pairs(a, p, pi, nwin, npairs, lane, pc);
+    const int q = pi - pc.pb;
+    const Pair pr = pair_of(pc, q);
+    if (STATS) {
+      const uint32_t b0 = __shfl_sync(kFull, pc.b0, q), b1 = __shfl_sync(kFull, pc.b1, q);
+      if (b1 > b0) {
+        k.off += 2u;
+        k.pairs += 1u;
+        k.bins1 += b1 - b0 + 1;
       }
     }
-    const int q = pi - pc.pb;
-    const uint32_t qrs = __shfl_sync(kFull, pc.rs, q);
-    const uint32_t qre = __shfl_sync(kFull, pc.re, q);
-    const uint32_t qb0 = __shfl_sync(kFull, pc.b0, q);
-    const uint32_t qb1 = __shfl_sync(kFull, pc.b1, q);
-    const int qw = __shfl_sync(kFull, pc.wsel, q);
-    const int64_t qbase = __shfl_sync(kFull, pc.wbase, q);
-    if (qb1 <= qb0) continue;
-    k.off += 2u;
-    k.pairs += 1u;
-    k.bins1 += qb1 - qb0 + 1;
-    gather_pair<S, FAST, STATS>(a, qw, qbase, qb0, qb1, qrs, qre, cs, ce, lane, row, off, bm, tags, scr,
-                         k, pi == pc.pre_pi ? &pc.pre : nullptr, touched, n_touched);
+    if (pr.n == 0) continue;
+    gather_pair<S, FAST, STATS>(a, pc, q, pr, pi == pc.pre_pi, cs, C, lane, stage, stage_p, r, off, k);
   }
+  if (r.n > r.done) add_entries<S>(r, r.n - r.done, off, lane);
+  stage_pair<FAST>(a, p, (f + 1) * nwin, nwin, npairs, lane, pc, stage);
   __syncwarp();
-  const int pn = (f + 1) * nwin;
-  pc.pre_pi = -1;
-  if (pn < npairs && pn < pc.pb + 32) {
-    const int q = pn - pc.pb;
-    const uint32_t nrs = __shfl_sync(kFull, pc.rs, q), nre = __shfl_sync(kFull, pc.re, q);
-    const uint32_t nb0 = __shfl_sync(kFull, pc.b0, q), nb1 = __shfl_sync(kFull, pc.b1, q);
-    const int64_t nbase = __shfl_sync(kFull, pc.wbase, q);
-    if (nb1 > nb0 && nre > nrs && scans(a, nre - nrs)) {
-      load_batch<FAST>(win_entries(a, nbase), nrs, nre, lane, pc.pre);
-      pc.pre_pi = pn;
-    }
-  }
 }
 
 // Strict 5-point local maxima of a precursor's scores (src/peak_group_selection/mod.rs:33-43),
@@ -756,20 +783,23 @@ __global__ void __launch_bounds__(LaunchShape<H, FAST, GROW>::threads, LaunchSha
   extern __shared__ __align__(16) float smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = H > 0 ? H : a.h;
-  const WarpPlan P = warp_plan(S, h, a.ncell);
+  const WarpPlan P = warp_plan(S, h, a.ncell, a.c_max);
   double2* lnt = reinterpret_cast<double2*>(smem_raw);
   float* kw_s = smem_raw + kLnTableSize * 4;
-  float* wb = GROW ? a.grow + ((size_t)blockIdx.x * (blockDim.x >> 5) + warp) * (size_t)P.total
-                   : smem_raw + block_header_words(h) + warp * P.total;
+  const int nw = blockDim.x >> 5;
+  float* areas = smem_raw + block_header_words(h);
+  const unsigned char* stage_p = reinterpret_cast<const unsigned char*>(areas + warp * kStageWords);
+  const uint32_t stage = (uint32_t)__cvta_generic_to_shared(stage_p);
+  float* wb = GROW ? a.grow + ((size_t)blockIdx.x * nw + warp) * (size_t)P.total
+                   : areas + nw * kStageWords + warp * P.total;
   float* row = wb + P.row;
-  uint8_t* tags = reinterpret_cast<uint8_t*>(wb + P.tags);
   uint32_t* bm = reinterpret_cast<uint32_t*>(wb + P.bm);
-  float* scr = wb + P.scr;
   float* score = wb + P.score;
   float* mval = wb + P.mval;
   int* midx = reinterpret_cast<int*>(wb + P.midx);
-  uint16_t* touched = reinterpret_cast<uint16_t*>(wb + P.touched);
-  int n_touched = 0;  // cells the last row wrote (warp-uniform)
+  float2* lst = reinterpret_cast<float2*>(wb + P.lst);
+  // r.n: also the cells the previous row left to clear
+  RowList r{row, bm, reinterpret_cast<uint16_t*>(wb + P.cells), wb + P.lst, 0, 0};
   {
     float4* r4 = reinterpret_cast<float4*>(row);
     for (int i = lane; i < P.row_words / 4; i += 32) r4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -809,27 +839,28 @@ __global__ void __launch_bounds__(LaunchShape<H, FAST, GROW>::threads, LaunchSha
     k.frag += F;
     // fragment weights, lane f holding fragment f's (fetched once per precursor)
     const float wf_lane = lane < F ? __ldg(a.fw + p * a.kf + lane) : 0.0f;
+    PairCursor pc;
+    load_pairs(a, p, 0, nwin, npairs, lane, pc);
+    stage_pair<FAST>(a, p, 0, nwin, npairs, lane, pc, stage);
     for (int i = lane; i <= C + C / S; i += 32) score[i] = 0.0f;  // cycles [0, C) with pads
 
-    PairCursor<FAST> pc;
     for (int f = 0; f < F; ++f) {
       // the previous row's cells (and bitmap words) back to zero
-      if (n_touched > kTouchCap) {
+      if (r.n > kTouchCap) {
         float4* r4 = reinterpret_cast<float4*>(row);
         for (int i = lane; i < P.row_words / 4; i += 32) r4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int i = lane; i < P.bw; i += 32) bm[i] = 0u;
       } else {
-        for (int i = lane; i < n_touched; i += 32) {
-          const int c = touched[i];
+        for (int i = lane; i < r.n; i += 32) {
+          const int c = r.cells[i];
           row[raddr<S>(c + P.off)] = 0.0f;
           bm[(c + kBitOff) >> 5] = 0u;
         }
       }
-      n_touched = 0;
+      r.n = r.done = 0;
       __syncwarp();
       // ---- 1. gather: the fragment's pairs in window order
-      gather_row<S, FAST, STATS>(a, p, f, nwin, npairs, cs, ce, lane, pc, row, P.off, bm, tags,
-                                 scr, k, touched, n_touched);
+      gather_row<S, FAST, STATS>(a, p, f, nwin, npairs, cs, C, lane, pc, stage, stage_p, r, P.off, k);
       float wf = __shfl_sync(kFull, wf_lane, f & 31);
       if (f >= 32) wf = __ldg(a.fw + p * a.kf + f);
       if (!isfinite(wf)) {
@@ -842,17 +873,38 @@ __global__ void __launch_bounds__(LaunchShape<H, FAST, GROW>::threads, LaunchSha
         __syncwarp();
         continue;
       }
-      if (n_touched == 0) continue;  // no entry accepted: every term is +0
-      // ---- 2./3. convolution of this lane's cycles, then the score terms of its
-      // non-zero outputs.  A zero output adds ln(1) * w = +0, which leaves a score as
-      // it is, so only non-zero outputs of the valid range [h, C - h) are listed
-      // (warp-compacted, in lane order) and take a logarithm.
-      float2* lst = reinterpret_cast<float2*>(wb + P.lst);
+      if (r.n == 0) continue;  // no entry accepted: every term is +0
+      // ---- 2./3. convolution of this lane's cycles, then the score terms of the
+      // outputs of the valid range [h, C - h) that a touched cycle reaches.  Every other
+      // output is zero and adds ln(1) * w = +0, which leaves a score as it is, so only
+      // those are listed (warp-compacted, in lane order) and take a logarithm.
       for (int ps = 0; ps < passes; ++ps) {
         const int j0 = ps * 32 * S + lane * S;
-        const bool act = j0 + S > h && j0 < C - h && bits_any(bm, j0 - h + kBitOff, S + 2 * h);
+        uint32_t mk = 0;  // outputs j0 + m to list
+        bool act;
+        if (H > 0) {
+          // bits j0 - H .. j0 + S - 1 + H of the touched cycles, each spread over the
+          // 2H + 1 outputs it reaches
+          const int lo = j0 - H + kBitOff;
+          const uint32_t* bw = bm + (lo >> 5);
+          const uint32_t x0 = bw[0], x1 = bw[1], x2 = bw[2];
+          unsigned long long x = ((unsigned long long)__funnelshift_r(x1, x2, lo) << 32) |
+                                 __funnelshift_r(x0, x1, lo);
+          int reach = 1;
+#pragma unroll
+          for (int g = 0; g < 5; ++g)
+            if (2 * reach <= 2 * H + 1) {
+              x |= x >> reach;
+              reach *= 2;
+            }
+          x |= x >> (2 * H + 1 - reach);
+          const int m0 = max(H - j0, 0), m1 = max(min(C - H - j0, S), 0);
+          mk = (uint32_t)x & ((1u << m1) - 1u) & (0xffffffffu << m0);
+          act = mk != 0u;
+        } else {
+          act = j0 + S > h && j0 < C - h && bits_any(bm, j0 - h + kBitOff, S + 2 * h);
+        }
         if (!__any_sync(kFull, act)) continue;
-        uint32_t mk = 0;
         float cv[S];
         if (H > 0) {
           if (act) {
@@ -899,7 +951,7 @@ __global__ void __launch_bounds__(LaunchShape<H, FAST, GROW>::threads, LaunchSha
             cv[m] = (j >= h && j < C - h) ? conv_at<S, FAST>(row, P.off, kw_s, h, j) : 0.0f;
           }
         }
-        if (act) {
+        if (H == 0 && act) {
           const int m0 = max(h - j0, 0), m1 = min(C - h - j0, S);
 #pragma unroll
           for (int m = 0; m < S; ++m)
