@@ -277,7 +277,7 @@ std::vector<float> gaussian_kernel(float fwhm_rt, float sigma_scale_rt, int64_t 
 extern "C" const char* ads_last_error(void) { return ads::g_last_error.c_str(); }
 
 namespace {
-__global__ void selftest_ln_kernel(uint32_t lo, uint32_t hi, const double2* tab,
+__global__ void selftest_ln_kernel(uint32_t lo, uint32_t hi, const double2* tab, ads::LnCoef k,
                                    unsigned long long* out) {
   unsigned long long bad = 0, slow = 0;
   const uint64_t n = (uint64_t)hi - lo;
@@ -285,7 +285,7 @@ __global__ void selftest_ln_kernel(uint32_t lo, uint32_t hi, const double2* tab,
        i += (uint64_t)gridDim.x * blockDim.x) {
     const float x = __uint_as_float(lo + (uint32_t)i);
     bool s = false;
-    const float a = ads::ln_fast(x, tab, &s);
+    const float a = ads::ln_fast(x, tab, k, &s);
     const float b = ads::ln_rn(x);
     bad += __float_as_uint(a) != __float_as_uint(b);
     slow += s;
@@ -306,7 +306,7 @@ extern "C" int ads_selftest_ln(int device, uint32_t lo_bits, uint32_t hi_bits, i
     DevBuf<unsigned long long> out;
     ADS_TRY(out.alloc(2));
     ADS_CUDA(cudaMemset(out.p, 0, 16));
-    selftest_ln_kernel<<<148 * 16, 256>>>(lo_bits, hi_bits, tab, out.p);
+    selftest_ln_kernel<<<148 * 16, 256>>>(lo_bits, hi_bits, tab, LnCoef(), out.p);
     ADS_LAUNCH_CHECK();
     unsigned long long h[2];
     ADS_CUDA(cudaMemcpy(h, out.p, 16, cudaMemcpyDeviceToHost));

@@ -227,11 +227,20 @@ std::vector<double2> host_ln_table();  // the values device_ln_table uploads
 // halfway pattern (about one input in 2^14); there ln_rn decides.  Checked against
 // ln_rn for every float in (1, inf).  `tab` is the table of device_ln_table
 // (usually staged in shared memory).
-__device__ __forceinline__ float ln_fast(float x, const double2* tab, bool* slow = nullptr) {
+//
+// The coefficients come as an argument: kernels pass them in their parameters, which the
+// double-precision instructions read in place (as literals each took two moves per use,
+// 50 of the search kernel's 1160 instructions per fragment row).
+//
+// ln_table: *y = ln(x) unless it returns true, when ln_rn must decide (x < 1, infinite or
+// NaN, or a result too near a rounding boundary).  x = 1 gives exactly 0.
+struct LnCoef {
+  double ln2 = 0.6931471805599453094172321, c2 = -1.0 / 2.0, c3 = 1.0 / 3.0, c4 = -1.0 / 4.0,
+         c5 = 1.0 / 5.0, one = 1.0;
+};
+
+__device__ __forceinline__ bool ln_table(float x, const double2* tab, const LnCoef& k, float* y) {
   const uint32_t b = __float_as_uint(x);
-  if (b <= 0x3F800000u || b >= 0x7F800000u) {  // x <= 1, negative, inf or NaN
-    return b == 0x3F800000u ? 0.0f : ln_rn_slow(x);
-  }
   const int e = (int)(b >> 23) - 127;
   const uint32_t j = (b >> (23 - kLnTableBits)) & (kLnTableSize - 1);
   const double m = (double)__uint_as_float((b & 0x007FFFFFu) | 0x3F800000u);
@@ -240,17 +249,23 @@ __device__ __forceinline__ float ln_fast(float x, const double2* tab, bool* slow
   // 1 - r/2 + r^2/3 - r^3/4 + r^4/5 as (1 - r/2) + r^2 * ((1/3 - r/4) + r^2/5): three
   // dependent steps after r instead of four; e*ln2 + ln(c_j) forms alongside
   const double r2 = r * r;
-  const double c0 = fma(r, -1.0 / 2.0, 1.0);
-  const double c1 = fma(r, -1.0 / 4.0, 1.0 / 3.0);
-  const double p = fma(r2, fma(r2, 1.0 / 5.0, c1), c0);
-  const double ln2 = 0.6931471805599453094172321;
-  const double y = fma(p, r, fma((double)e, ln2, t.y));
-  const uint32_t low = (uint32_t)__double2loint(y) & 0x1FFFFFFFu;
-  if (low - (0x10000000u - 0x4000u) < 0x8000u) {
-    if (slow) *slow = true;
+  const double c0 = fma(r, k.c2, k.one);
+  const double c1 = fma(r, k.c4, k.c3);
+  const double p = fma(r2, fma(r2, k.c5, c1), c0);
+  const double v = fma(p, r, fma((double)e, k.ln2, t.y));
+  *y = __double2float_rn(v);
+  const uint32_t low = (uint32_t)__double2loint(v) & 0x1FFFFFFFu;
+  return b - 0x3F800000u >= 0x40000000u || low - (0x10000000u - 0x4000u) < 0x8000u;
+}
+
+__device__ __forceinline__ float ln_fast(float x, const double2* tab, const LnCoef& k,
+                                         bool* slow = nullptr) {
+  float y;
+  if (ln_table(x, tab, k, &y)) {
+    if (slow) *slow = x > 1.0f && x < INFINITY;
     return ln_rn_slow(x);
   }
-  return __double2float_rn(y);
+  return y;
 }
 
 // ------------------------------------------------------------- structures

@@ -487,6 +487,7 @@ void set_taps(SearchArgs* sa, const float* kernel, int h, const float* kw_dev) {
   }
   sa->zero2 = 0ull;
   sa->nzero2 = 0x8000000080000000ull;
+  sa->ln = LnCoef();
 }
 
 // ------------------------------------------------------------ compaction
@@ -972,7 +973,7 @@ int enqueue_search(AdsSelection* s, const AdsDia* d, const AdsLib* l, AdsCandida
   ADS_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
 
   SearchArgs sa;
-  std::memset(&sa, 0, sizeof(sa));
+  std::memset(static_cast<void*>(&sa), 0, sizeof(sa));
   sa.n_prec = P;
   sa.nf = s->nf.p;
   sa.cs = s->cs.p;
@@ -1742,7 +1743,7 @@ int select_noalloc(const AdsDia* d, const AdsLib* l, const AdsSelectionParams* p
   ADS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, nw * 32, smem));
   if (occ <= 0) return fail(ADS_ERR_INTERNAL, "search kernel cannot be resident");
   SearchArgs sa;
-  std::memset(&sa, 0, sizeof(sa));
+  std::memset(static_cast<void*>(&sa), 0, sizeof(sa));
   sa.n_prec = P;
   sa.nf = nf;
   sa.cs = cs;

@@ -43,6 +43,7 @@ struct SearchArgs {
   unsigned long long kw2[kMaxHalf + 1];  // the same taps, each twice (packed f32x2 operands)
   unsigned long long zero2;   // +0.0f twice
   unsigned long long nzero2;  // -0.0f twice
+  LnCoef ln;
   int h;
   int k_out;   // candidates kept per precursor
   int c_max;   // largest cycle range of the precursors this launch searches
@@ -135,13 +136,14 @@ __host__ __device__ inline WarpPlan warp_plan(int S, int h, int ncell, int c_max
   o += w.lead + w.bw;
   w.cells = o;  // cells accepted by the current row (16 bits each)
   o += kTouchCap / 2;
-  w.score = o + 4;  // 4 words of margin below: the maxima scan reads 2 cycles early
+  w.score = o + 4;  // 4 words of margin below: the maxima scan reads 2 cycles early, and
+                    // idle lanes of the score terms work on the lowest
   o += cc + cc / S + 12;
   o = (o + 1) & ~1;
-  // one pass of convolved values as (value, score address) pairs; before it, while the
-  // row is gathered, the accepted entries' intensities (kTouchCap words)
+  // one pass of convolved values as (value, score address) pairs, and a warp of idle ones;
+  // before it, while the row is gathered, the accepted entries' intensities (kTouchCap words)
   w.lst = o;
-  o += 2 * 32 * S;
+  o += 2 * 32 * (S + 1);
   w.mx = maxima_cap(ncell);
   if (2 * w.mx <= 2 * 32 * S) {
     // the maxima are collected after the precursor's last row is scored, when the
@@ -205,6 +207,18 @@ struct Counters {
   Count<ON> read, acc, off, pairs, bins1, frag;
 };
 
+// A value that is the same in all lanes, as the result of a warp reduction, which the
+// compiler knows to be uniform: branches and loops on it need no reconvergence code, and
+// the collectives inside them no divergence check (24 of 1160 instructions per fragment
+// row, and as many again for the barriers around them).
+__device__ __forceinline__ int uniform(int x) {
+  return (int)__reduce_max_sync(kFull, (unsigned)x);
+}
+// Lane q's value (x >= 0), uniform as above.
+__device__ __forceinline__ unsigned from_lane(unsigned x, int q, int lane) {
+  return __reduce_max_sync(kFull, lane == q ? x : 0u);
+}
+
 // One fragment row being gathered.  Accepted entries are appended, in CSR order, to a list
 // (cell, intensity) and added to the row 32 at a time, so that the adds run with full
 // warps however few entries of a chunk lie in the RT window (7 of 32 on average on
@@ -227,6 +241,7 @@ static __device__ __noinline__ void add_grouped(bool act, int cell, int addr, in
   if (act && lane == __ffs(grp) - 1) {
     float acc = row[addr];
     unsigned g = grp;
+#pragma unroll 1
     while (g) {
       const int l = __ffs(g) - 1;
       acc = __fadd_rn(acc, vals[(first + l) % kTouchCap]);
@@ -261,19 +276,16 @@ __device__ __forceinline__ void add_entries(RowList& r, int m, int off, int lane
 }
 
 // Appends the lanes' entries marked `in`, in lane order.
-template <int S, class Acc>
+template <int S>
 __device__ __forceinline__ void append_entries(RowList& r, bool in, int cell, float v, int off,
-                                               int lane, Acc& n_acc) {
+                                               int lane) {
   const unsigned act = __ballot_sync(kFull, in);
-  if (act == 0) return;
   if (in) {
     const int at = (r.n + __popc(act & ((1u << lane) - 1u))) % kTouchCap;
     r.cells[at] = (uint16_t)cell;
     r.vals[at] = v;
   }
-  const int k = __popc(act);
-  n_acc += (unsigned int)k;
-  r.n += k;
+  r.n += __popc(act);
   if (r.n - r.done >= 32) add_entries<S>(r, 32, off, lane);
 }
 
@@ -282,6 +294,7 @@ __device__ __forceinline__ void append_entries(RowList& r, bool in, int cell, fl
 static __device__ __noinline__ bool bin_starts_at(const uint32_t* ssw, uint32_t b0, uint32_t b1,
                                                   uint32_t pos) {
   uint32_t lo = b0 + 1, hi = b1;
+#pragma unroll 1
   while (lo < hi) {
     const uint32_t mid = (lo + hi) >> 1;
     if (__ldg(ssw + mid) < pos)
@@ -318,11 +331,13 @@ __device__ __forceinline__ void stage_entries(const SearchArgs& a, int64_t q0, i
   const char* cy = reinterpret_cast<const char*>(a.cyc) + (q0 & ~(int64_t)7) * 2;
   const int ni = ((int)(q0 & (PI - 1)) + m + PI - 1) / PI;
   const int nc = ((int)(q0 & 7) + m + 7) / 8;
-  for (int k = lane; k < ni + nc; k += 32) {
-    if (k < ni)
-      cp_async16(stage + k * 16, in + k * 16);
-    else
-      cp_async16(stage + kStageCycOff + (k - ni) * 16, cy + (k - ni) * 16);
+  // (piece k of the cycles, counted from the intensities' first)
+  const char* cy0 = cy - ni * 16;
+  const uint32_t cyc_stage = stage + kStageCycOff - ni * 16;
+#pragma unroll 1
+  for (int k0 = 0; k0 < ni + nc; k0 += 32) {
+    const int k = k0 + lane;
+    if (k < ni + nc) cp_async16((k < ni ? stage : cyc_stage) + k * 16, (k < ni ? in : cy0) + k * 16);
   }
 }
 
@@ -350,18 +365,85 @@ struct Pair {
   int64_t q;   // absolute position of its first entry
   uint32_t n;  // entries
 };
-__device__ __forceinline__ Pair pair_of(const PairCursor& pc, int q) {
-  return Pair{__shfl_sync(kFull, pc.wbase + pc.rs, q), __shfl_sync(kFull, pc.n, q)};
+__device__ __forceinline__ Pair pair_of(const PairCursor& pc, int q, int lane) {
+  return Pair{__shfl_sync(kFull, pc.wbase + pc.rs, q), from_lane(pc.n, q, lane)};
 }
 
-// fill_xic_slice for the (fragment, window) pair in lane `pq` of the cursor.  Two exact
-// strategies:
-//   scan     read every entry of the range, keep start < cycle < stop plus, per
-//            bin, the last entry at cycle == start (where Rust's binary_search
-//            lands, src/quadrupole_observation/mod.rs:91-94);
-//   bsearch  per bin, binary-search the first kept entry and the first entry at or
-//            past stop, then read only the kept entries.
-// `staged`: the range's first kStageEntries entries are already on their way.
+// An entry at the window's first cycle counts only if it is the last of its bin there
+// (where Rust's binary_search lands, src/quadrupole_observation/mod.rs:91-94): is the
+// next entry, entry `tn` of the pair's n, in another bin or at another cycle?  Out of
+// line: about one range in fifty holds such an entry.
+static __device__ __noinline__ bool last_at_start(const SearchArgs& a, int wsel, uint32_t b0,
+                                                  uint32_t b1, uint32_t rs, int64_t q, uint32_t tn,
+                                                  uint32_t n, int cs) {
+  if (tn >= n || bin_starts_at(a.ss + a.win[wsel].ss_off, b0, b1, rs + tn)) return true;
+  return (int)__ldg(a.cyc + q + tn) != cs;
+}
+
+// The rare strategy of gather_pair, out of line: per bin, binary-search the first kept
+// entry and the first entry at or past stop, then read only the kept entries.
+struct SearchedPair {
+  int n, done;           // of the row list
+  unsigned read, offs;   // entries and offsets read
+};
+template <int S, bool FAST>
+static __device__ __noinline__ SearchedPair gather_searched(const SearchArgs& a, uint32_t b0,
+                                                            uint32_t b1, int wsel, int64_t wbase,
+                                                            int cs, int C, int lane, RowList r,
+                                                            int off) {
+  SearchedPair out{0, 0, 0, 0};
+  const uint32_t* ssw = a.ss + a.win[wsel].ss_off;
+  const uint16_t* cy = a.cyc + wbase;
+#pragma unroll 1
+  for (uint32_t bb = b0; bb < b1; bb += 32) {
+    const uint32_t b = bb + lane;
+    const bool vb = b < b1;
+    int64_t pos = 0, cnt = 0;
+    if (vb) {
+      const int64_t s0 = __ldg(ssw + b), s1 = __ldg(ssw + b + 1);
+      pos = s0 + rust_bsearch_u16(cy + s0, s1 - s0, cs);
+      const int64_t end = pos + lower_bound_u16(cy + pos, s1 - pos, cs + C);
+      cnt = end - pos;
+    }
+    out.offs += 2u * (unsigned int)__popc(__ballot_sync(kFull, vb));
+    int64_t incl = cnt;
+#pragma unroll 1
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t t = __shfl_up_sync(kFull, incl, o);
+      if (lane >= o) incl += t;
+    }
+    const int64_t total = __shfl_sync(kFull, incl, 31);
+    const int64_t excl = incl - cnt;
+    out.read += (unsigned int)total;
+#pragma unroll 1
+    for (int64_t t0 = 0; t0 < total; t0 += 32) {
+      const int64_t t = t0 + lane;
+      int l = 0;
+#pragma unroll 1
+      for (int st = 16; st >= 1; st >>= 1) {
+        const int c = l + st;
+        const int64_t ec = __shfl_sync(kFull, excl, c);
+        if (ec <= t) l = c;
+      }
+      const int64_t opos = __shfl_sync(kFull, pos, l);
+      const int64_t oex = __shfl_sync(kFull, excl, l);
+      const bool vt = t < total;
+      const int64_t q = opos + (t - oex);
+      const int c = vt ? (int)__ldg(cy + q) : 0;
+      const float v = vt ? ld_intensity<FAST>(a, wbase + q) : 0.0f;
+      append_entries<S>(r, vt, c - cs, v, off, lane);
+    }
+  }
+  out.n = r.n;
+  out.done = r.done;
+  return out;
+}
+
+// fill_xic_slice for the (fragment, window) pair in lane `pq` of the cursor: its entries
+// inside the RT window are listed, in CSR order.  Two exact strategies: scan, which reads
+// every entry of the range and keeps start < cycle < stop plus, per bin, the last entry
+// at cycle == start; or, for long ranges, gather_searched.  `staged`: the range's first
+// kStageEntries entries are already on their way.
 template <int S, bool FAST, bool STATS>
 __device__ __forceinline__ void gather_pair(const SearchArgs& a, const PairCursor& pc, int pq,
                                             Pair pr, bool staged, int cs, int C, int lane,
@@ -369,18 +451,22 @@ __device__ __forceinline__ void gather_pair(const SearchArgs& a, const PairCurso
                                             RowList& r, int off, Counters<STATS>& k) {
   if (scans(a, pr.n)) {
     k.read += pr.n;
+#pragma unroll 1
     for (uint32_t q0 = 0; q0 < pr.n; q0 += kStageEntries) {
       const int m = (int)min(pr.n - q0, (uint32_t)kStageEntries);
       const int64_t q = pr.q + q0;
-      if (!(staged && q0 == 0)) {
+      if (!staged) {
         __syncwarp();  // the area's previous entries have been read
         stage_entries<FAST>(a, q, m, stage, lane);
       }
+      staged = false;
       stage_wait();
       const uint16_t* sc = reinterpret_cast<const uint16_t*>(stage_p + kStageCycOff) + (q & 7);
       const float* sf = reinterpret_cast<const float*>(stage_p) + (q & 3);
       const uint16_t* sh = reinterpret_cast<const uint16_t*>(stage_p) + (q & 7);
-      for (int t = lane; t < ((m + 31) & ~31); t += 32) {
+#pragma unroll 1
+      for (int t0 = 0; t0 < m; t0 += 32) {
+        const int t = t0 + lane;
         const int cell = (int)sc[t] - cs;
         bool in = t < m && (unsigned)cell < (unsigned)C;
         const float v = FAST ? __uint_as_float((uint32_t)sh[t] << 16) : sf[t];
@@ -388,61 +474,20 @@ __device__ __forceinline__ void gather_pair(const SearchArgs& a, const PairCurso
           const uint32_t rs = __shfl_sync(kFull, pc.rs, pq);
           const uint32_t b0 = __shfl_sync(kFull, pc.b0, pq), b1 = __shfl_sync(kFull, pc.b1, pq);
           const int wsel = __shfl_sync(kFull, pc.wsel, pq);
-          if (in && cell == 0) {
-            const uint32_t tn = q0 + (uint32_t)t + 1;  // the next entry of the range
-            if (tn < pr.n && !bin_starts_at(a.ss + a.win[wsel].ss_off, b0, b1, rs + tn)) {
-              const int cn = t + 1 < m ? (int)sc[t + 1] : (int)__ldg(a.cyc + pr.q + tn);
-              in = cn != cs;
-            }
-          }
+          if (in && cell == 0)
+            in = last_at_start(a, wsel, b0, b1, rs, pr.q, q0 + (uint32_t)t + 1, pr.n, cs);
         }
-        append_entries<S>(r, in, cell, v, off, lane, k.acc);
+        append_entries<S>(r, in, cell, v, off, lane);
       }
     }
   } else {
-    const uint32_t b0 = __shfl_sync(kFull, pc.b0, pq), b1 = __shfl_sync(kFull, pc.b1, pq);
-    const int wsel = __shfl_sync(kFull, pc.wsel, pq);
-    const int64_t wbase = __shfl_sync(kFull, pc.wbase, pq);
-    const uint32_t* ssw = a.ss + a.win[wsel].ss_off;
-    const uint16_t* cy = a.cyc + wbase;
-    for (uint32_t bb = b0; bb < b1; bb += 32) {
-      const uint32_t b = bb + lane;
-      const bool vb = b < b1;
-      int64_t pos = 0, cnt = 0;
-      if (vb) {
-        const int64_t s0 = __ldg(ssw + b), s1 = __ldg(ssw + b + 1);
-        pos = s0 + rust_bsearch_u16(cy + s0, s1 - s0, cs);
-        const int64_t end = pos + lower_bound_u16(cy + pos, s1 - pos, cs + C);
-        cnt = end - pos;
-      }
-      k.off += 2u * (unsigned int)__popc(__ballot_sync(kFull, vb));
-      int64_t incl = cnt;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int64_t t = __shfl_up_sync(kFull, incl, o);
-        if (lane >= o) incl += t;
-      }
-      const int64_t total = __shfl_sync(kFull, incl, 31);
-      const int64_t excl = incl - cnt;
-      k.read += (unsigned int)total;
-      for (int64_t t0 = 0; t0 < total; t0 += 32) {
-        const int64_t t = t0 + lane;
-        int l = 0;
-#pragma unroll
-        for (int st = 16; st >= 1; st >>= 1) {
-          const int c = l + st;
-          const int64_t ec = __shfl_sync(kFull, excl, c);
-          if (ec <= t) l = c;
-        }
-        const int64_t opos = __shfl_sync(kFull, pos, l);
-        const int64_t oex = __shfl_sync(kFull, excl, l);
-        const bool vt = t < total;
-        const int64_t q = opos + (t - oex);
-        const int c = vt ? (int)__ldg(cy + q) : 0;
-        const float v = vt ? ld_intensity<FAST>(a, wbase + q) : 0.0f;
-        append_entries<S>(r, vt, c - cs, v, off, lane, k.acc);
-      }
-    }
+    const SearchedPair sp = gather_searched<S, FAST>(
+        a, __shfl_sync(kFull, pc.b0, pq), __shfl_sync(kFull, pc.b1, pq),
+        __shfl_sync(kFull, pc.wsel, pq), __shfl_sync(kFull, pc.wbase, pq), cs, C, lane, r, off);
+    r.n = uniform(sp.n);
+    r.done = uniform(sp.done);
+    k.read += sp.read;
+    k.off += sp.offs;
   }
 }
 
@@ -453,6 +498,7 @@ __device__ __forceinline__ bool bits_any(const uint32_t* bm, int lo, int n) {
   const int last = lo + n - 1;
   const int w0 = lo >> 5, w1 = last >> 5;
   uint32_t acc = 0;
+#pragma unroll 1
   for (int w = w0; w <= w1; ++w) {
     uint32_t v = bm[w];
     if (w == w0) v &= 0xffffffffu << (lo & 31);
@@ -505,6 +551,7 @@ template <int S, bool FAST>
 __device__ __forceinline__ float conv_at(const float* row, int off, const float* kw_s, int h,
                                          int j) {
   float s = __fadd_rn(0.0f, __fmul_rn(row[raddr<S>(j + off)], kw_s[h]));
+#pragma unroll 1
   for (int t = 0; t < h; ++t) {
     const float lr = __fadd_rn(row[raddr<S>(j - h + t + off)], row[raddr<S>(j + h - t + off)]);
     s = FAST ? __fmaf_rn(lr, kw_s[t], s) : __fadd_rn(s, __fmul_rn(lr, kw_s[t]));
@@ -527,53 +574,77 @@ __device__ __forceinline__ float ln1p_fast(float c) {
   return fabsf(c) < 0.0625f ? series : __logf(__fadd_rn(c, 1.0f));
 }
 
-// score[j] += ln(c + 1) * w (src/score/scalar.rs:16-22): one rounded operation at a
-// time with the exact ln; FAST (BF16 storage) takes the hardware log2 and a fused
-// multiply-add.
+// s + ln(c + 1) * w (src/score/scalar.rs:16-22): one rounded operation at a time with the
+// exact ln; FAST (BF16 storage) takes the hardware log2 and a fused multiply-add.  Called
+// by whole warps: the slow path of the exact ln is behind one vote.
 template <bool FAST>
-__device__ __forceinline__ float score_term(float s, float c, float w, const double2* lnt) {
+__device__ __forceinline__ float score_term(float s, float c, float w, const double2* lnt,
+                                            const LnCoef& k) {
   if (FAST) return __fmaf_rn(ln1p_fast(c), w, s);
-  return __fadd_rn(s, __fmul_rn(ln_fast(__fadd_rn(c, 1.0f), lnt), w));
+  const float x = __fadd_rn(c, 1.0f);
+  float y;
+  const bool slow = ln_table(x, lnt, k, &y);
+  if (__any_sync(kFull, slow)) y = slow ? ln_rn_slow(x) : y;
+  return __fadd_rn(s, __fmul_rn(y, w));
+}
+
+// Where the list of a pass's outputs, (value, score index) pairs, is appended to: a
+// shared-memory address, or (GROW) a pointer.
+template <bool GROW>
+struct OutEnd;
+template <>
+struct OutEnd<false> {
+  uint32_t to;
+  __device__ OutEnd(float2* at) : to((uint32_t)__cvta_generic_to_shared(at)) {}
+  // Appends (v, at) where bit m of mk is set: test, store, advance, all predicated (a
+  // branch around each store cost three times as much).
+  __device__ __forceinline__ void put(uint32_t mk, int m, float v, int at) {
+    asm volatile(
+        "{\n .reg .pred q;\n .reg .b32 t;\n and.b32 t, %1, %2;\n setp.ne.u32 q, t, 0;\n"
+        " @q st.shared.v2.b32 [%0], {%3, %4};\n @q add.u32 %0, %0, 8;\n}"
+        : "+r"(to)
+        : "r"(mk), "r"(1u << m), "r"(__float_as_uint(v)), "r"(at)
+        : "memory");
+  }
+};
+template <>
+struct OutEnd<true> {
+  float2* to;
+  __device__ OutEnd(float2* at) : to(at) {}
+  __device__ __forceinline__ void put(uint32_t mk, int m, float v, int at) {
+    if ((mk >> m) & 1u) *to++ = make_float2(v, __int_as_float(at));
+  }
+};
+
+// Spreads every set bit of x over the LEN bits at and below it: bit m of the result is set
+// where any of bits m .. m + LEN - 1 is.
+template <int LEN, class U>
+__device__ __forceinline__ U spread_down(U x) {
+  int reach = 1;
+#pragma unroll
+  for (int g = 0; g < 5; ++g)
+    if (2 * reach <= LEN) {
+      x |= x >> reach;
+      reach *= 2;
+    }
+  if (reach < LEN) x |= x >> (LEN - reach);
+  return x;
 }
 
 template <bool FAST>
 __device__ __forceinline__ void score_add(float* score, int addr, float c, float w,
-                                          const double2* lnt) {
+                                          const double2* lnt, const LnCoef& k) {
   if (FAST)
     score[addr] = __fmaf_rn(ln1p_fast(c), w, score[addr]);
   else
-    score[addr] = __fadd_rn(score[addr], __fmul_rn(ln_fast(__fadd_rn(c, 1.0f), lnt), w));
+    score[addr] = __fadd_rn(score[addr], __fmul_rn(ln_fast(__fadd_rn(c, 1.0f), lnt, k), w));
 }
 
-// Candidate order: value descending, then cycle ascending (maxima values are never
-// NaN: every comparison with NaN is false, so NaN is never a strict maximum).
-__device__ __forceinline__ bool better(float av, int ai, float bv, int bi) {
-  return av > bv || (av == bv && ai < bi);
-}
-
-// Compare-exchange between lanes l and l ^ j, the better key going to the lane
-// that `keep_best` marks.
-__device__ __forceinline__ void cmpx(float& v, int& i, int j, bool keep_best) {
-  const float ov = __shfl_xor_sync(kFull, v, j);
-  const int oi = __shfl_xor_sync(kFull, i, j);
-  if (keep_best ? better(ov, oi, v, i) : better(v, i, ov, oi)) {
-    v = ov;
-    i = oi;
-  }
-}
-
-// Bitonic sort of one key per lane, best in lane 0.
-__device__ __forceinline__ void warp_sort_best_first(float& v, int& i, int lane) {
-#pragma unroll 1
-  for (int k = 2; k <= 32; k <<= 1)
-#pragma unroll 1
-    for (int j = k >> 1; j > 0; j >>= 1) cmpx(v, i, j, ((lane & j) == 0) == ((lane & k) == 0));
-}
-
-// Sorts a bitonic sequence across the lanes, best in lane 0.
-__device__ __forceinline__ void warp_merge_best_first(float& v, int& i, int lane) {
-#pragma unroll 1
-  for (int j = 16; j > 0; j >>= 1) cmpx(v, i, j, (lane & j) == 0);
+// An unsigned key ordered like the value (-0 as +0), at least 1; NaN has key 0.
+__device__ __forceinline__ uint32_t order_key(float v) {
+  const uint32_t b = __float_as_uint(__fadd_rn(v, 0.0f));
+  const uint32_t k = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+  return v != v ? 0u : k;
 }
 
 // Moves the cursor to pairs [pi, pi + 32).
@@ -607,7 +678,7 @@ __device__ __forceinline__ void stage_pair(const SearchArgs& a, int64_t p, int p
   pc.pre_pi = -1;
   if (pi >= npairs) return;
   if (pi >= pc.pb + 32) load_pairs(a, p, pi, nwin, npairs, lane, pc);
-  const Pair pr = pair_of(pc, pi - pc.pb);
+  const Pair pr = pair_of(pc, pi - pc.pb, lane);
   if (pr.n > 0 && scans(a, pr.n)) {
     __syncwarp();
     stage_entries<FAST>(a, pr.q, (int)min(pr.n, (uint32_t)kStageEntries), stage, lane);
@@ -616,19 +687,18 @@ __device__ __forceinline__ void stage_pair(const SearchArgs& a, int64_t p, int p
 }
 
 // Gathers fragment f's XIC row: its (fragment, window) pairs in window order (the
-// reference's DenseXICObservation::new, src/dense_xic_observation/mod.rs:30-64),
-// then starts staging the next fragment's first pair, which arrives while this row is
-// convolved.
+// reference's DenseXICObservation::new, src/dense_xic_observation/mod.rs:30-64).
 template <int S, bool FAST, bool STATS>
 __device__ __forceinline__ void gather_row(const SearchArgs& a, int64_t p, int f, int nwin,
                                            int npairs, int cs, int C, int lane, PairCursor& pc,
                                            uint32_t stage, const unsigned char* stage_p, RowList& r,
                                            int off, Counters<STATS>& k) {
+#pragma unroll 1
   for (int wi = 0; wi < nwin; ++wi) {
     const int pi = f * nwin + wi;
     if (pi >= pc.pb + 32) load_pairs(a, p, pi, nwin, npairs, lane, pc);
     const int q = pi - pc.pb;
-    const Pair pr = pair_of(pc, q);
+    const Pair pr = pair_of(pc, q, lane);
     if (STATS) {
       const uint32_t b0 = __shfl_sync(kFull, pc.b0, q), b1 = __shfl_sync(kFull, pc.b1, q);
       if (b1 > b0) {
@@ -638,11 +708,44 @@ __device__ __forceinline__ void gather_row(const SearchArgs& a, int64_t p, int f
       }
     }
     if (pr.n == 0) continue;
-    gather_pair<S, FAST, STATS>(a, pc, q, pr, pi == pc.pre_pi, cs, C, lane, stage, stage_p, r, off, k);
+    gather_pair<S, FAST, STATS>(a, pc, q, pr, pi == pc.pre_pi, cs, C, lane, stage,
+                                stage_p, r, off, k);
   }
-  if (r.n > r.done) add_entries<S>(r, r.n - r.done, off, lane);
-  stage_pair<FAST>(a, p, (f + 1) * nwin, nwin, npairs, lane, pc, stage);
+  if (r.done < r.n) add_entries<S>(r, r.n - r.done, off, lane);
+}
+
+// The last gathered row's cells (and bitmap words) back to zero.
+template <int S>
+__device__ __forceinline__ void clear_row(RowList& r, const WarpPlan& P, int lane) {
+  if (r.n > kTouchCap) {
+    float4* r4 = reinterpret_cast<float4*>(r.row);
+#pragma unroll 1
+    for (int i = lane; i < P.row_words / 4; i += 32) r4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+    for (int i = lane; i < P.bw; i += 32) r.bm[i] = 0u;
+  } else {
+#pragma unroll 1
+    for (int i = lane; i < r.n; i += 32) {
+      const int c = r.cells[i];
+      r.row[raddr<S>(c + P.off)] = 0.0f;
+      r.bm[(c + kBitOff) >> 5] = 0u;
+    }
+  }
+  r.n = r.done = 0;
   __syncwarp();
+}
+
+// A row whose weight is not finite, out of line: ln(conv + 1) * w is NaN even where conv
+// is zero, so every column takes its term, as in the reference.
+template <int S, bool FAST>
+static __device__ __noinline__ void score_every_column(const SearchArgs& a, const float* row, int off,
+                                                       const float* kw_s, int h, int C, float wf,
+                                                       float* score, const double2* lnt, int lane) {
+#pragma unroll 1
+  for (int j = lane; j < C; j += 32) {
+    const float c = (j >= h && j < C - h) ? conv_at<S, FAST>(row, off, kw_s, h, j) : 0.0f;
+    score_add<FAST>(score, xaddr<S>(j), c, wf, lnt, a.ln);
+  }
 }
 
 // Strict 5-point local maxima of a precursor's scores (src/peak_group_selection/mod.rs:33-43),
@@ -657,6 +760,7 @@ __device__ __forceinline__ void pick_top_k(const SearchArgs& a, int64_t p, int c
   const int passes = (C + 32 * S - 1) / (32 * S);
   // lane l's maxima of a pass go after those of lanes < l
   int nmax = 0;
+#pragma unroll 1
   for (int ps = 0; ps < passes; ++ps) {
     const int seg = ps * 32 + lane;
     const float* sb = score + seg * (S + 1);
@@ -681,6 +785,7 @@ __device__ __forceinline__ void pick_top_k(const SearchArgs& a, int64_t p, int c
       if (lane >= o) incl += t;
     }
     int pos = nmax + incl - cnt;
+#pragma unroll 1
     while (mk) {
       const int m = __ffs(mk) - 1;
       if (pos < mx) {
@@ -698,64 +803,37 @@ __device__ __forceinline__ void pick_top_k(const SearchArgs& a, int64_t p, int c
     nmax = mx;
   }
   const int kk = min(a.k_out, nmax);
-  if (a.k_out <= 32) {
-    // the best 32 of the maxima, sorted in the lanes: chunks of 32 are sorted
-    // and merged into the running best 32
-    float bv = -INFINITY;
-    int bi = INT_MAX;
-    for (int q0 = 0; q0 < nmax; q0 += 32) {
-      float v = q0 + lane < nmax ? mval[q0 + lane] : -INFINITY;
-      int i = q0 + lane < nmax ? midx[q0 + lane] : INT_MAX;
-      warp_sort_best_first(v, i, lane);
-      if (q0 == 0) {
-        bv = v;
-        bi = i;
-      } else {
-        const float rv = __shfl_sync(kFull, v, 31 - lane);
-        const int ri = __shfl_sync(kFull, i, 31 - lane);
-        if (better(rv, ri, bv, bi)) {
-          bv = rv;
-          bi = ri;
+  // one selection per candidate: every lane holds the best of its maxima (lane,
+  // lane + 32, ...), two reductions find the best value and its first cycle, and the lane
+  // that held it looks for its next.  Sorting 32 at a time took ten times the instructions
+  // for the usual 3 or 5 candidates.
+  uint32_t key = 0;
+  int at = -1;
+  bool look = true;
+#pragma unroll 1
+  for (int r = 0; r < kk; ++r) {
+    if (look) {
+      key = 0;
+#pragma unroll 1
+      for (int q = lane; q < nmax; q += 32) {
+        const uint32_t x = order_key(mval[q]);
+        if (x > key) {
+          key = x;
+          at = q;
         }
-        warp_merge_best_first(bv, bi, lane);
       }
     }
-    if (lane < kk) {
-      a.cand_score[p * a.k_out + lane] = bv;
-      a.cand_center[p * a.k_out + lane] = cs + bi;
+    const uint32_t top = __reduce_max_sync(kFull, key);
+    // maxima are listed in cycle order, so the first in the list is the first cycle
+    const unsigned pos = __reduce_min_sync(kFull, key == top ? (unsigned)at : 0xffffffffu);
+    look = (unsigned)at == pos && key == top;
+    if (look) {
+      a.cand_score[p * a.k_out + r] = mval[pos];
+      a.cand_center[p * a.k_out + r] = cs + midx[pos];
+      mval[pos] = __int_as_float(0x7fc00000);  // taken: key 0
     }
   }
-  for (int r = 0; a.k_out > 32 && r < kk; ++r) {
-    float bv = 0.0f;
-    int bi = -1, bk = -1;
-    for (int q = lane; q < nmax; q += 32) {
-      const float v = mval[q];
-      const int i = midx[q];
-      if (v != v) continue;  // already taken
-      if (bk < 0 || v > bv || (v == bv && i < bi)) {
-        bv = v;
-        bi = i;
-        bk = q;
-      }
-    }
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) {
-      const float ov = __shfl_xor_sync(kFull, bv, o);
-      const int oi = __shfl_xor_sync(kFull, bi, o);
-      const int ok = __shfl_xor_sync(kFull, bk, o);
-      if (ok >= 0 && (bk < 0 || ov > bv || (ov == bv && oi < bi))) {
-        bv = ov;
-        bi = oi;
-        bk = ok;
-      }
-    }
-    if (lane == 0) {
-      a.cand_score[p * a.k_out + r] = bv;
-      a.cand_center[p * a.k_out + r] = cs + bi;
-      mval[bk] = __int_as_float(0x7fc00000);
-    }
-    __syncwarp();
-  }
+  __syncwarp();
   if (lane == 0) a.cand_n[p] = kk;
 }
 
@@ -779,7 +857,7 @@ __device__ __forceinline__ void flush_counters(const SearchArgs& a, const Counte
 // STATS: the statistics pass's work counters (compiled in only for it).
 template <int H, int S, bool FAST, bool GROW, bool STATS>
 __global__ void __launch_bounds__(LaunchShape<H, FAST, GROW>::threads, LaunchShape<H, FAST, GROW>::blocks)
-    search_kernel(SearchArgs a) {
+    search_kernel(const __grid_constant__ SearchArgs a) {
   extern __shared__ __align__(16) float smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = H > 0 ? H : a.h;
@@ -802,26 +880,30 @@ __global__ void __launch_bounds__(LaunchShape<H, FAST, GROW>::threads, LaunchSha
   RowList r{row, bm, reinterpret_cast<uint16_t*>(wb + P.cells), wb + P.lst, 0, 0};
   {
     float4* r4 = reinterpret_cast<float4*>(row);
+#pragma unroll 1
     for (int i = lane; i < P.row_words / 4; i += 32) r4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
     for (int i = lane - P.lead; i < P.bw; i += 32) bm[i] = 0u;
   }
 
+#pragma unroll 1
   for (int i = threadIdx.x; i < kLnTableSize; i += blockDim.x) lnt[i] = a.ln_tab[i];
+#pragma unroll 1
   for (int i = threadIdx.x; i <= a.h; i += blockDim.x) kw_s[i] = a.kw_dev ? a.kw_dev[i] : a.kw[i];
   __syncthreads();
   Counters<STATS> k;
 
-  const unsigned long long n_work = a.list ? (unsigned long long)*a.list_len
-                                            : (unsigned long long)a.n_prec;
+  const unsigned n_work = a.list ? (unsigned)uniform((int)*a.list_len) : (unsigned)a.n_prec;
+#pragma unroll 1
   for (;;) {
-    unsigned long long pw = 0;
-    if (lane == 0) pw = atomicAdd(a.work, 1ull);
-    pw = __shfl_sync(kFull, pw, 0);
+    unsigned pw = 0;
+    if (lane == 0) pw = (unsigned)min(atomicAdd(a.work, 1ull), 0xffffffffull);
+    pw = __reduce_max_sync(kFull, pw);
     if (pw >= n_work) break;
-    const int64_t p = a.list ? (int64_t)a.list[pw] : (int64_t)pw;
-    const int F = a.nf[p];
-    const int cs = a.cs[p], ce = a.ce[p];
-    const int C = ce - cs;
+    const int64_t p = a.list ? (int64_t)uniform(a.list[pw]) : (int64_t)pw;
+    const int F = uniform(a.nf[p]);
+    const int cs = uniform(a.cs[p]);
+    const int C = uniform(a.ce[p]) - cs;
     if (F == 0 || C <= 0) {
       if (lane == 0) a.cand_n[p] = 0;
       continue;
@@ -833,43 +915,34 @@ __global__ void __launch_bounds__(LaunchShape<H, FAST, GROW>::threads, LaunchSha
       }
       continue;
     }
-    const int nwin = a.nwin[p];
+    const int nwin = uniform(a.nwin[p]);
     const int npairs = F * nwin;
     const int passes = (C + 32 * S - 1) / (32 * S);
     k.frag += F;
     // fragment weights, lane f holding fragment f's (fetched once per precursor)
     const float wf_lane = lane < F ? __ldg(a.fw + p * a.kf + lane) : 0.0f;
     PairCursor pc;
-    load_pairs(a, p, 0, nwin, npairs, lane, pc);
-    stage_pair<FAST>(a, p, 0, nwin, npairs, lane, pc, stage);
-    for (int i = lane; i <= C + C / S; i += 32) score[i] = 0.0f;  // cycles [0, C) with pads
-
-    for (int f = 0; f < F; ++f) {
-      // the previous row's cells (and bitmap words) back to zero
-      if (r.n > kTouchCap) {
-        float4* r4 = reinterpret_cast<float4*>(row);
-        for (int i = lane; i < P.row_words / 4; i += 32) r4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int i = lane; i < P.bw; i += 32) bm[i] = 0u;
-      } else {
-        for (int i = lane; i < r.n; i += 32) {
-          const int c = r.cells[i];
-          row[raddr<S>(c + P.off)] = 0.0f;
-          bm[(c + kBitOff) >> 5] = 0u;
-        }
+    // f = -1: only starts the first row's entries on their way
+#pragma unroll 1
+    for (int f = -1; f < F; ++f) {
+      if (f >= 0) {
+        // ---- 1. gather: the fragment's pairs in window order
+        clear_row<S>(r, P, lane);
+        gather_row<S, FAST, STATS>(a, p, f, nwin, npairs, cs, C, lane, pc, stage, stage_p, r, P.off, k);
+        k.acc += (unsigned int)r.n;
       }
-      r.n = r.done = 0;
+      // the next fragment's first pair arrives while this row is convolved
+      stage_pair<FAST>(a, p, (f + 1) * nwin, nwin, npairs, lane, pc, stage);
+      if (f < 0) {
+#pragma unroll 1
+        for (int i = lane; i <= C + C / S; i += 32) score[i] = 0.0f;  // cycles [0, C) with pads
+        continue;
+      }
       __syncwarp();
-      // ---- 1. gather: the fragment's pairs in window order
-      gather_row<S, FAST, STATS>(a, p, f, nwin, npairs, cs, C, lane, pc, stage, stage_p, r, P.off, k);
       float wf = __shfl_sync(kFull, wf_lane, f & 31);
       if (f >= 32) wf = __ldg(a.fw + p * a.kf + f);
       if (!isfinite(wf)) {
-        // ln(conv + 1) * inf is NaN even where conv is zero: every column takes
-        // its term, as in the reference
-        for (int j = lane; j < C; j += 32) {
-          const float c = (j >= h && j < C - h) ? conv_at<S, FAST>(row, P.off, kw_s, h, j) : 0.0f;
-          score_add<FAST>(score, xaddr<S>(j), c, wf, lnt);
-        }
+        score_every_column<S, FAST>(a, row, P.off, kw_s, h, C, wf, score, lnt, lane);
         __syncwarp();
         continue;
       }
@@ -878,6 +951,7 @@ __global__ void __launch_bounds__(LaunchShape<H, FAST, GROW>::threads, LaunchSha
       // outputs of the valid range [h, C - h) that a touched cycle reaches.  Every other
       // output is zero and adds ln(1) * w = +0, which leaves a score as it is, so only
       // those are listed (warp-compacted, in lane order) and take a logarithm.
+#pragma unroll 1
       for (int ps = 0; ps < passes; ++ps) {
         const int j0 = ps * 32 * S + lane * S;
         uint32_t mk = 0;  // outputs j0 + m to list
@@ -887,19 +961,16 @@ __global__ void __launch_bounds__(LaunchShape<H, FAST, GROW>::threads, LaunchSha
           // 2H + 1 outputs it reaches
           const int lo = j0 - H + kBitOff;
           const uint32_t* bw = bm + (lo >> 5);
-          const uint32_t x0 = bw[0], x1 = bw[1], x2 = bw[2];
-          unsigned long long x = ((unsigned long long)__funnelshift_r(x1, x2, lo) << 32) |
-                                 __funnelshift_r(x0, x1, lo);
-          int reach = 1;
-#pragma unroll
-          for (int g = 0; g < 5; ++g)
-            if (2 * reach <= 2 * H + 1) {
-              x |= x >> reach;
-              reach *= 2;
-            }
-          x |= x >> (2 * H + 1 - reach);
+          uint32_t x;
+          if (S + 2 * H <= 32) {
+            x = spread_down<2 * H + 1>(__funnelshift_r(bw[0], bw[1], lo));
+          } else {
+            const uint32_t x0 = bw[0], x1 = bw[1], x2 = bw[2];
+            x = (uint32_t)spread_down<2 * H + 1>(
+                ((unsigned long long)__funnelshift_r(x1, x2, lo) << 32) | __funnelshift_r(x0, x1, lo));
+          }
           const int m0 = max(H - j0, 0), m1 = max(min(C - H - j0, S), 0);
-          mk = (uint32_t)x & ((1u << m1) - 1u) & (0xffffffffu << m0);
+          mk = x & ((1u << m1) - 1u) & (0xffffffffu << m0);
           act = mk != 0u;
         } else {
           act = j0 + S > h && j0 < C - h && bits_any(bm, j0 - h + kBitOff, S + 2 * h);
@@ -907,51 +978,52 @@ __global__ void __launch_bounds__(LaunchShape<H, FAST, GROW>::threads, LaunchSha
         if (!__any_sync(kFull, act)) continue;
         float cv[S];
         if (H > 0) {
-          if (act) {
-            // cells u in [UB, UE) of this lane's segment as 8-byte pairs (u even);
-            // every output is formed in the reference's order: 0 + x[j]*w[h], then
-            // + (x[j-d] + x[j+d]) * w[h-d] for d = h..1, two outputs (m, m + 1) per
-            // packed instruction.  For odd d the pair sums straddle the register
-            // pairs and are formed by two scalar adds.
-            constexpr int UB = -((H + 1) & ~1);
-            constexpr int UE = (S + H + 1) & ~1;
-            constexpr int NX = UE - UB;
-            const float* rb = row + (ps * 32 + lane + P.off / S) * row_stride(S);
-            float xv[NX];
+          // cells u in [UB, UE) of this lane's segment as 8-byte pairs (u even; a lane
+          // without outputs computes the first segment's); every output is formed in the
+          // reference's order: 0 + x[j]*w[h], then + (x[j-d] + x[j+d]) * w[h-d] for
+          // d = h..1, two outputs (m, m + 1) per packed instruction.  For odd d the pair
+          // sums straddle the register pairs and are formed by two scalar adds.
+          constexpr int UB = -((H + 1) & ~1);
+          constexpr int UE = (S + H + 1) & ~1;
+          constexpr int NX = UE - UB;
+          const float* rb = row + ((act ? ps * 32 + lane : 0) + P.off / S) * row_stride(S);
+          float xv[NX];
 #pragma unroll
-            for (int q = 0; q < NX; q += 2) {
-              const int u = UB + q;
-              const float2 v =
-                  *reinterpret_cast<const float2*>(rb + u + floordiv(u, S) * (row_stride(S) - S));
-              xv[q] = v.x;
-              xv[q + 1] = v.y;
-            }
+          for (int q = 0; q < NX; q += 2) {
+            const int u = UB + q;
+            const float2 v =
+                *reinterpret_cast<const float2*>(rb + u + floordiv(u, S) * (row_stride(S) - S));
+            xv[q] = v.x;
+            xv[q + 1] = v.y;
+          }
+          f32x2 acc[S / 2];
+#pragma unroll
+          for (int m = 0; m < S; m += 2)
+            acc[m / 2] = add2(a.zero2, fma2(pk2(xv[m - UB], xv[m + 1 - UB]), a.kw2[H], a.nzero2));
+#pragma unroll
+          for (int t = 0; t < H; ++t) {
+            const int d = H - t;
 #pragma unroll
             for (int m = 0; m < S; m += 2) {
-              f32x2 acc = add2(a.zero2, fma2(pk2(xv[m - UB], xv[m + 1 - UB]), a.kw2[H], a.nzero2));
-#pragma unroll
-              for (int t = 0; t < H; ++t) {
-                const int d = H - t;
-                f32x2 lr;
-                if (d % 2 == 0)
-                  lr = add2(pk2(xv[m - d - UB], xv[m - d + 1 - UB]),
-                            pk2(xv[m + d - UB], xv[m + d + 1 - UB]));
-                else
-                  lr = pk2(__fadd_rn(xv[m - d - UB], xv[m + d - UB]),
-                           __fadd_rn(xv[m + 1 - d - UB], xv[m + 1 + d - UB]));
-                acc = FAST ? fma2(lr, a.kw2[t], acc) : add2(acc, fma2(lr, a.kw2[t], a.nzero2));
-              }
-              unpk2(acc, cv[m], cv[m + 1]);
+              f32x2 lr;
+              if (d % 2 == 0)
+                lr = add2(pk2(xv[m - d - UB], xv[m - d + 1 - UB]),
+                          pk2(xv[m + d - UB], xv[m + d + 1 - UB]));
+              else
+                lr = pk2(__fadd_rn(xv[m - d - UB], xv[m + d - UB]),
+                         __fadd_rn(xv[m + 1 - d - UB], xv[m + 1 + d - UB]));
+              acc[m / 2] = FAST ? fma2(lr, a.kw2[t], acc[m / 2])
+                                : add2(acc[m / 2], fma2(lr, a.kw2[t], a.nzero2));
             }
           }
+#pragma unroll
+          for (int m = 0; m < S; m += 2) unpk2(acc[m / 2], cv[m], cv[m + 1]);
         } else if (act) {
 #pragma unroll
           for (int m = 0; m < S; ++m) {
             const int j = j0 + m;
             cv[m] = (j >= h && j < C - h) ? conv_at<S, FAST>(row, P.off, kw_s, h, j) : 0.0f;
           }
-        }
-        if (H == 0 && act) {
           const int m0 = max(h - j0, 0), m1 = min(C - h - j0, S);
 #pragma unroll
           for (int m = 0; m < S; ++m)
@@ -964,17 +1036,19 @@ __global__ void __launch_bounds__(LaunchShape<H, FAST, GROW>::threads, LaunchSha
           const int t = __shfl_up_sync(kFull, incl, o);
           if (lane >= o) incl += t;
         }
-        const int total = __shfl_sync(kFull, incl, 31);
-        int pos = incl - cnt;
-        const int sbase = (ps * 32 + lane) * (S + 1);  // score address of cycle j0
+        const int total = (int)__reduce_add_sync(kFull, (unsigned)cnt);
+        const int sbase = (ps * 32 + lane) * (S + 1);  // score index of cycle j0
+        OutEnd<GROW> end(lst + (incl - cnt));
 #pragma unroll
-        for (int m = 0; m < S; ++m)
-          if ((mk >> m) & 1u) lst[pos++] = make_float2(cv[m], __int_as_float(sbase + m));
+        for (int m = 0; m < S; ++m) end.put(mk, m, cv[m], sbase + m);
+        // idle entries up to a whole warp, which work on a word below the scores
+        lst[total + lane] = make_float2(0.0f, __int_as_float(-4));
         __syncwarp();
-        for (int i = lane; i < total; i += 32) {
-          const float2 e = lst[i];
-          const int at = __float_as_int(e.y);
-          score[at] = score_term<FAST>(score[at], e.x, wf, lnt);
+#pragma unroll 1
+        for (int i0 = 0; i0 < total; i0 += 32) {
+          const float2 e = lst[i0 + lane];
+          float* sp = score + __float_as_int(e.y);
+          *sp = score_term<FAST>(*sp, e.x, wf, lnt, a.ln);
         }
         __syncwarp();
       }
