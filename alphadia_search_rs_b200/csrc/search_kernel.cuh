@@ -254,8 +254,10 @@ static __device__ __noinline__ void add_grouped(bool act, int cell, int addr, in
 // Adds the next m (1 to 32) listed entries to the XIC row in list order (the reference's
 // `dense_xic[c] += intensity`, src/quadrupole_observation/mod.rs:96-105).  Setting a
 // cell's bit tells whether it was touched before, by an earlier entry or by another lane:
-// if none was, every cell holds 0 and takes its intensity; else the lanes are grouped by
-// cell and summed by their lowest lane one rounded add at a time.
+// if none was, every cell holds 0 and takes its intensity.  If one lane's was (a third of
+// the rows), that lane adds after the others have stored: to what an earlier entry left, or
+// to another lane's intensity, where 0 + a + b and 0 + b + a round alike.  Else the lanes
+// are grouped by cell and summed by their lowest lane one rounded add at a time.
 template <int S>
 __device__ __forceinline__ void add_entries(RowList& r, int m, int off, int lane) {
   __syncwarp();
@@ -267,8 +269,11 @@ __device__ __forceinline__ void add_entries(RowList& r, int m, int off, int lane
   const uint32_t bit = 1u << (cell & 31);
   bool again = false;
   if (act) again = (atomicOr(r.bm + ((cell + kBitOff) >> 5), bit) & bit) != 0u;
-  if (!__any_sync(kFull, again)) {
-    if (act) r.row[addr] = v;
+  const unsigned later = __ballot_sync(kFull, again);
+  if ((later & (later - 1u)) == 0u) {
+    if (act && !again) r.row[addr] = v;
+    __syncwarp();
+    if (again) r.row[addr] = __fadd_rn(r.row[addr], v);
   } else {
     add_grouped(act, cell, addr, r.done, lane, r.row, r.vals);
   }
@@ -281,12 +286,32 @@ __device__ __forceinline__ void append_entries(RowList& r, bool in, int cell, fl
                                                int lane) {
   const unsigned act = __ballot_sync(kFull, in);
   if (in) {
-    const int at = (r.n + __popc(act & ((1u << lane) - 1u))) % kTouchCap;
+    const int at = (r.n + __popc(act & lanemask_lt())) % kTouchCap;
     r.cells[at] = (uint16_t)cell;
     r.vals[at] = v;
   }
   r.n += __popc(act);
   if (r.n - r.done >= 32) add_entries<S>(r, 32, off, lane);
+}
+
+// The same for two consecutive entries per lane.
+template <int S>
+__device__ __forceinline__ void append_pairs(RowList& r, bool in0, bool in1, int cell0, int cell1,
+                                             float v0, float v1, int off, int lane) {
+  const unsigned act0 = __ballot_sync(kFull, in0), act1 = __ballot_sync(kFull, in1);
+  const int at = r.n + __popc(act0 & lanemask_lt()) + __popc(act1 & lanemask_lt());
+  if (in0) {
+    r.cells[at % kTouchCap] = (uint16_t)cell0;
+    r.vals[at % kTouchCap] = v0;
+  }
+  if (in1) {
+    const int to = (at + (in0 ? 1 : 0)) % kTouchCap;
+    r.cells[to] = (uint16_t)cell1;
+    r.vals[to] = v1;
+  }
+  r.n += __popc(act0) + __popc(act1);
+#pragma unroll 1
+  while (r.n - r.done >= 32) add_entries<S>(r, 32, off, lane);
 }
 
 // Is `pos` the first entry of one of the bins (b0, b1)?  (slice_starts[b] == pos)
@@ -461,23 +486,44 @@ __device__ __forceinline__ void gather_pair(const SearchArgs& a, const PairCurso
       }
       staged = false;
       stage_wait();
-      const uint16_t* sc = reinterpret_cast<const uint16_t*>(stage_p + kStageCycOff) + (q & 7);
-      const float* sf = reinterpret_cast<const float*>(stage_p) + (q & 3);
-      const uint16_t* sh = reinterpret_cast<const uint16_t*>(stage_p) + (q & 7);
+      // two consecutive entries per lane, from the even position at or below the first
+      const int odd = (int)(q & 1);
+      const uint32_t* sc = reinterpret_cast<const uint32_t*>(stage_p + kStageCycOff) + ((q & 7) >> 1);
+      const float2* sf = reinterpret_cast<const float2*>(stage_p) + ((q & 3) >> 1);
+      const uint32_t* sh = reinterpret_cast<const uint32_t*>(stage_p) + ((q & 7) >> 1);
 #pragma unroll 1
-      for (int t0 = 0; t0 < m; t0 += 32) {
-        const int t = t0 + lane;
-        const int cell = (int)sc[t] - cs;
-        bool in = t < m && (unsigned)cell < (unsigned)C;
-        const float v = FAST ? __uint_as_float((uint32_t)sh[t] << 16) : sf[t];
-        if (__any_sync(kFull, in && cell == 0)) {
+      for (int i0 = 0; i0 < m + odd; i0 += 64) {
+        const int t = i0 + 2 * lane - odd;
+        const int i = min((i0 >> 1) + lane, kStageEntries / 2);  // the area's last pair
+        const uint32_t cc = sc[i];
+        float2 v;
+        if (FAST) {
+          const uint32_t b = sh[i];
+          v = make_float2(__uint_as_float(b << 16), __uint_as_float(b & 0xffff0000u));
+        } else {
+          v = sf[i];
+        }
+        const int cell0 = (int)(cc & 0xffffu) - cs, cell1 = (int)(cc >> 16) - cs;
+        bool in0 = (unsigned)t < (unsigned)m && (unsigned)cell0 < (unsigned)C;
+        bool in1 = t + 1 < m && (unsigned)cell1 < (unsigned)C;
+        if (__any_sync(kFull, (in0 && cell0 == 0) || (in1 && cell1 == 0))) {
           const uint32_t rs = __shfl_sync(kFull, pc.rs, pq);
           const uint32_t b0 = __shfl_sync(kFull, pc.b0, pq), b1 = __shfl_sync(kFull, pc.b1, pq);
           const int wsel = __shfl_sync(kFull, pc.wsel, pq);
-          if (in && cell == 0)
-            in = last_at_start(a, wsel, b0, b1, rs, pr.q, q0 + (uint32_t)t + 1, pr.n, cs);
+#pragma unroll 1
+          for (int e = 0; e < 2; ++e) {
+            const bool ask = e == 0 ? in0 && cell0 == 0 : in1 && cell1 == 0;
+            if (ask) {
+              const bool keep = last_at_start(a, wsel, b0, b1, rs, pr.q, q0 + (uint32_t)(t + e) + 1,
+                                              pr.n, cs);
+              if (e == 0)
+                in0 = keep;
+              else
+                in1 = keep;
+            }
+          }
         }
-        append_entries<S>(r, in, cell, v, off, lane);
+        append_pairs<S>(r, in0, in1, cell0, cell1, v.x, v.y, off, lane);
       }
     }
   } else {
