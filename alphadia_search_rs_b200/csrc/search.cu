@@ -353,113 +353,58 @@ __global__ void __launch_bounds__(kPrepThreads, 8) prep_kernel(PrepArgs a) {
 
 #include "search_kernel.cuh"
 
-// Cycles per lane the search kernel is compiled for, and its instances: fully
-// unrolled stencils for the half widths of kernel_size 20, 21-22 and 31-32, any
-// other half width through the generic path.
+// Values of the cycles_per_lane option: 0 for length classes, any other for one class over
+// all RT windows up to kSmemMaxCycles.
 constexpr int kLaneCycles[] = {4, 8, 10, 12, 16};
-constexpr int kGrowLaneCycles = 16;  // cycles per lane of long-window (GROW) launches
 // Global working sets of one long-window launch: at most this many bytes (the grid
 // is trimmed to fit; a warp's set is about 15 bytes per cycle of the longest window).
 constexpr int64_t kGrowBudgetBytes = int64_t(1) << 30;
 constexpr int kDefaultWarpsPerBlock = 4;
 constexpr int kMaxClasses = 10;
+constexpr int kClassBounds[] = {512, 768, 1024, 1408};
 constexpr int kStats = 7;  // statistics-pass counters (ads_selection_last_stats)
 
-// Length classes of one search: class b covers C <= bound[b] with S[b] cycles per
-// lane (bound[last] = the longest window, searched in one or more passes).
+// Length classes of one search: class b covers C <= bound[b] (bound[last] = the longest
+// window).  They differ in the shared memory a warp takes, so in the warps an SM holds.
 struct LenClasses {
   int bound[kMaxClasses];
-  int S[kMaxClasses];
 };
 
-// Relative cost of searching a c-cycle window with S cycles per lane: passes times
-// (S outputs + about 6 outputs' worth of per-pass loads and control per lane).
-int lane_cost(int64_t c, int S) { return (int)((c + 32 * S - 1) / (32 * S)) * (S + 6); }
-
-// The cheapest lane width for a c-cycle window, ties to the larger S.
-int best_lane_cycles(int64_t c) {
-  int S = kLaneCycles[0];
-  int best = -1;
-  for (int cand : kLaneCycles) {
-    const int cost = lane_cost(c, cand);
-    if (best < 0 || cost <= best) {
-      best = cost;
-      S = cand;
-    }
-  }
-  return S;
-}
-
-// Length classes: every bound 32 * S * k (k <= 4 passes) below the longest window, at
-// least 20 % apart, each with its cheapest lane width, then one class for the rest.
-// A fixed cycles_per_lane gives a single class.  Windows longer than kSmemMaxCycles
-// get a class of their own, searched with the warps' working sets in global memory
-// (GROW, kGrowLaneCycles cycles per lane); everything up to kSmemMaxCycles then stays
-// in shared-memory classes.
-int plan_classes(int64_t c_max, int fixed_S, LenClasses* out) {
+int plan_classes(int64_t c_max, bool one_class, LenClasses* out) {
   int n = 0;
   const bool grow = c_max > kSmemMaxCycles;
   const int64_t c_sm = std::min<int64_t>(c_max, kSmemMaxCycles);
-  if (fixed_S == 0) {
-    std::vector<int> bounds;
-    for (int S : kLaneCycles)
-      for (int k = 1; k <= 4; ++k)
-        if ((int64_t)32 * S * k < c_sm) bounds.push_back(32 * S * k);
-    std::sort(bounds.begin(), bounds.end());
-    int last = 0;
-    for (int b : bounds) {
-      if (n == kMaxClasses - 1 - (grow ? 1 : 0)) break;
-      if (last > 0 && (int64_t)b * 5 < (int64_t)last * 6) continue;
-      out->bound[n] = b;
-      out->S[n] = best_lane_cycles(b);
-      last = b;
-      ++n;
-    }
-  }
-  if (grow) {
-    out->bound[n] = kSmemMaxCycles;
-    out->S[n] = fixed_S ? fixed_S : best_lane_cycles(kSmemMaxCycles);
-    ++n;
-    out->bound[n] = (int)c_max;
-    out->S[n] = kGrowLaneCycles;
-    return n + 1;
-  }
-  out->bound[n] = (int)c_max;
-  out->S[n] = fixed_S ? fixed_S : best_lane_cycles(c_max);
-  return n + 1;
+  if (!one_class)
+    for (int b : kClassBounds)
+      if ((int64_t)b * 5 < c_sm * 4) out->bound[n++] = b;
+  if (grow) out->bound[n++] = kSmemMaxCycles;
+  out->bound[n++] = (int)c_max;
+  return n;
 }
 
 template <int H, bool FAST, bool STATS>
-void (*pick_for_h(int S, bool grow))(SearchArgs) {
-  if (grow) return search_kernel<H, kGrowLaneCycles, FAST, true, STATS>;
-  switch (S) {
-    case 4: return search_kernel<H, 4, FAST, false, STATS>;
-    case 8: return search_kernel<H, 8, FAST, false, STATS>;
-    case 10: return search_kernel<H, 10, FAST, false, STATS>;
-    case 12: return search_kernel<H, 12, FAST, false, STATS>;
-    default: return search_kernel<H, 16, FAST, false, STATS>;
-  }
+void (*pick_for_h(bool grow))(SearchArgs) {
+  return grow ? search_kernel<H, FAST, true, STATS> : search_kernel<H, FAST, false, STATS>;
 }
 
 // The statistics pass counts gather work, which the half width does not change: it
 // runs the generic-h instances with the counters compiled in.
 template <bool FAST>
-void (*pick_for_precision(int h, int S, bool grow, bool stats))(SearchArgs) {
-  if (stats) return pick_for_h<0, FAST, true>(S, grow);
+void (*pick_for_precision(int h, bool grow, bool stats))(SearchArgs) {
+  if (stats) return pick_for_h<0, FAST, true>(grow);
   switch (h) {
-    case 10: return pick_for_h<10, FAST, false>(S, grow);
-    case 11: return pick_for_h<11, FAST, false>(S, grow);
-    case 16: return pick_for_h<16, FAST, false>(S, grow);
-    default: return pick_for_h<0, FAST, false>(S, grow);
+    case 10: return pick_for_h<10, FAST, false>(grow);
+    case 11: return pick_for_h<11, FAST, false>(grow);
+    case 16: return pick_for_h<16, FAST, false>(grow);
+    default: return pick_for_h<0, FAST, false>(grow);
   }
 }
 
 // fast: BF16 intensity storage with the fast f32 arithmetic (ADS_PRECISION_BF16);
-// grow: working sets in global memory (long windows; S must be kGrowLaneCycles);
+// grow: working sets in global memory (long windows);
 // stats: the statistics pass's instances (work counters compiled in)
-void (*pick_search_kernel(int h, int S, bool fast, bool grow, bool stats))(SearchArgs) {
-  return fast ? pick_for_precision<true>(h, S, grow, stats)
-              : pick_for_precision<false>(h, S, grow, stats);
+void (*pick_search_kernel(int h, bool fast, bool grow, bool stats))(SearchArgs) {
+  return fast ? pick_for_precision<true>(h, grow, stats) : pick_for_precision<false>(h, grow, stats);
 }
 
 // Largest block (in warps) an instance may launch: its launch bounds (LaunchShape); the
@@ -855,10 +800,8 @@ int enqueue_search(AdsSelection* s, const AdsDia* d, const AdsLib* l, AdsCandida
   const bool bf16 = s->o.precision == ADS_PRECISION_BF16;
   if (!bf16) ADS_TRY(need_f32_intensities(d, "an FP32 search"));
   LenClasses cls;
-  const int n_cls = plan_classes(c_max, S_fixed, &cls);
-  const int S_last = cls.S[n_cls - 1];
-  const int ncell = (int)((c_max + 32 * S_last - 1) / (32 * S_last) * 32 * S_last);
-  const int k_out = (int)std::max<int64_t>(0, std::min<int64_t>(prm.candidate_count, maxima_cap(ncell)));
+  const int n_cls = plan_classes(c_max, S_fixed != 0, &cls);
+  const int k_out = (int)std::max<int64_t>(0, std::min<int64_t>(prm.candidate_count, maxima_cap((int)c_max)));
   const int kf = (int)std::max<int64_t>(1, std::min<int64_t>(prm.top_k_fragments, l->max_frag));
   const int maxw = std::max(1, d->max_overlap);
 
@@ -1024,24 +967,20 @@ int enqueue_search(AdsSelection* s, const AdsDia* d, const AdsLib* l, AdsCandida
     ++launches;
   }
   for (int b = 0; b < n_cls; ++b) {
-    int S = cls.S[b];
     const int cmax_b = cls.bound[b];
     // block shape: warps per block (one precursor per warp at a time); 4 by default,
     // which packs long-window classes into shared memory better than 8
     bool grow = cmax_b > kSmemMaxCycles;
     int nw = s->o.warps_per_block > 0 ? s->o.warps_per_block : kDefaultWarpsPerBlock;
-    if (!grow && search_smem_bytes(1, S, s->h, (cmax_b + 32 * S - 1) / (32 * S) * 32 * S, cmax_b, false) >
-                     (size_t)max_smem)
+    if (!grow && search_smem_bytes(1, s->h, cmax_b, false) > (size_t)max_smem)
       grow = true;  // a very wide kernel: even one warp's plan exceeds shared memory
-    if (grow) S = kGrowLaneCycles;
     nw = std::max(1, std::min(nw, max_warps_per_block(bf16, s->h, grow, s->stats_on)));
-    const int ncell_b = (cmax_b + 32 * S - 1) / (32 * S) * 32 * S;
-    while (nw > 1 && search_smem_bytes(nw, S, s->h, ncell_b, cmax_b, grow) > (size_t)max_smem) --nw;
-    const size_t smem = search_smem_bytes(nw, S, s->h, ncell_b, cmax_b, grow);
+    while (nw > 1 && search_smem_bytes(nw, s->h, cmax_b, grow) > (size_t)max_smem) --nw;
+    const size_t smem = search_smem_bytes(nw, s->h, cmax_b, grow);
     if (smem > (size_t)max_smem)
       return fail(ADS_ERR_INTERNAL, "search kernel plan exceeds shared memory (" +
                                         std::to_string(cmax_b) + " cycles)");
-    void (*kern)(SearchArgs) = pick_search_kernel(s->h, S, bf16, grow, s->stats_on);
+    void (*kern)(SearchArgs) = pick_search_kernel(s->h, bf16, grow, s->stats_on);
     ADS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int occ = 0;
     ADS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, nw * 32, smem));
@@ -1050,12 +989,11 @@ int enqueue_search(AdsSelection* s, const AdsDia* d, const AdsLib* l, AdsCandida
     sa.list = use_lists ? s->class_lists.p + (int64_t)b * P : nullptr;
     sa.list_len = use_lists ? class_len + b : nullptr;
     sa.c_max = cmax_b;
-    sa.ncell = ncell_b;
     sa.work = s->work.p + b;
     int64_t blocks = std::min<int64_t>((int64_t)s->num_sms * bps, (P + nw - 1) / nw);
     sa.grow = nullptr;
     if (grow) {
-      const size_t warp_bytes = (size_t)warp_plan(S, s->h, ncell_b, cmax_b).total * 4;
+      const size_t warp_bytes = (size_t)warp_plan(s->h, cmax_b).total * 4;
       blocks = grow_blocks(blocks, nw, warp_bytes, (size_t)kGrowBudgetBytes);
       ADS_TRY(s->grow.reserve((size_t)blocks * nw * warp_bytes / 4));
       sa.grow = s->grow.p;
@@ -1146,8 +1084,7 @@ int autotune(AdsSelection* s, const AdsDia* d, const AdsLib* l, int32_t repeats,
     for (int nw : {2, 4, 8}) {
       if (nw > max_warps_per_block(s->o.precision == ADS_PRECISION_BF16, s->h, false, false))
         continue;
-      for (int S : {0, 4, 8, 10, 12, 16}) {
-        if (S != 0 && (int64_t)32 * S * 8 < key.c_max) continue;  // more than 8 passes
+      for (int S : {0, 16}) {  // length classes, or one class
         s->o.warps_per_block = nw;
         s->o.cycles_per_lane = S;
         rc = enqueue_search(s, d, l, &scratch, false);  // warm-up (and buffer sizing)
@@ -1623,13 +1560,8 @@ int select_noalloc(const AdsDia* d, const AdsLib* l, const AdsSelectionParams* p
   // long-window launch whose warps' working sets are carved from the scratch
   int max_smem = 0;
   ADS_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, d->device));
-  const int S0 = best_lane_cycles(c_max);
-  const bool grow =
-      c_max > kSmemMaxCycles ||
-      search_smem_bytes(1, S0, h, (int)((c_max + 32 * S0 - 1) / (32 * S0) * 32 * S0), (int)c_max) > (size_t)max_smem;
-  const int S = grow ? kGrowLaneCycles : S0;
-  const int ncell = (int)((c_max + 32 * S - 1) / (32 * S) * 32 * S);
-  const int k_out = (int)std::max<int64_t>(0, std::min<int64_t>(prm.candidate_count, maxima_cap(ncell)));
+  const bool grow = c_max > kSmemMaxCycles || search_smem_bytes(1, h, (int)c_max) > (size_t)max_smem;
+  const int k_out = (int)std::max<int64_t>(0, std::min<int64_t>(prm.candidate_count, maxima_cap((int)c_max)));
   const int kf = (int)std::max<int64_t>(1, std::min<int64_t>(prm.top_k_fragments, l->max_frag));
   const int maxw = std::max(1, d->max_overlap);
   const int64_t rows_needed = P * (int64_t)k_out;
@@ -1666,7 +1598,7 @@ int select_noalloc(const AdsDia* d, const AdsLib* l, const AdsSelectionParams* p
   float* taps = h > kMaxHalf ? sc.take<float>(L) : nullptr;  // wide kernels: taps on the device
   // long windows: at least one block of warps' working sets must fit after the rest
   const int nw0 = kDefaultWarpsPerBlock;
-  const size_t grow_warp_bytes = grow ? (size_t)warp_plan(S, h, ncell, (int)c_max).total * 4 : 0;
+  const size_t grow_warp_bytes = grow ? (size_t)warp_plan(h, (int)c_max).total * 4 : 0;
   float* grow_sets = nullptr;
   size_t grow_bytes = 0;
   if (grow) {  // the rest of the array, which must hold one block's working sets
@@ -1732,12 +1664,12 @@ int select_noalloc(const AdsDia* d, const AdsLib* l, const AdsSelectionParams* p
   ADS_LAUNCH_CHECK();
 
   int nw = nw0;
-  while (nw > 1 && search_smem_bytes(nw, S, h, ncell, (int)c_max, grow) > (size_t)max_smem) --nw;
-  const size_t smem = search_smem_bytes(nw, S, h, ncell, (int)c_max, grow);
+  while (nw > 1 && search_smem_bytes(nw, h, (int)c_max, grow) > (size_t)max_smem) --nw;
+  const size_t smem = search_smem_bytes(nw, h, (int)c_max, grow);
   if (smem > (size_t)max_smem)
     return fail(ADS_ERR_INTERNAL, "search kernel plan exceeds shared memory (" +
                                       std::to_string(c_max) + " cycles)");
-  void (*kern)(SearchArgs) = pick_search_kernel(h, S, false, grow, false);
+  void (*kern)(SearchArgs) = pick_search_kernel(h, false, grow, false);
   ADS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int occ = 0;
   ADS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, nw * 32, smem));
@@ -1766,7 +1698,6 @@ int select_noalloc(const AdsDia* d, const AdsLib* l, const AdsSelectionParams* p
   sa.h = h;
   sa.k_out = k_out;
   sa.c_max = (int)c_max;
-  sa.ncell = ncell;
   sa.gather_mode = 0;
   sa.scan_thresh = kScanThreshFp32;
   sa.work = work;

@@ -9,9 +9,9 @@
 //   1. gathers the fragment's XIC row into its shared-memory row: the CSR
 //      entries of every (fragment, window) pair are read up to 128 at a time and
 //      added to the row in CSR order (the reference's `dense_xic[c] += intensity`);
-//   2. convolves the row: lane l owns S consecutive output cycles per pass of
-//      32*S cycles and holds the S + 2h inputs they need in registers;
-//   3. adds ln(conv + 1) * w_f to its own columns' scores.  Fragments are taken
+//   2. convolves the segments of 4 output cycles that a touched cycle reaches, one per
+//      lane, the 4 + 2h inputs in registers;
+//   3. adds ln(conv + 1) * w_f to the scores of the non-zero outputs.  Fragments are taken
 //      in order, which is the reference's row-major accumulation
 //      (src/score/scalar.rs:16-22).
 // Then 5-point local maxima over the scores and a warp top-K.  All f32
@@ -47,7 +47,6 @@ struct SearchArgs {
   int h;
   int k_out;   // candidates kept per precursor
   int c_max;   // largest cycle range of the precursors this launch searches
-  int ncell;   // cycles a warp's row holds: passes * 32 * S >= c_max
   int gather_mode;
   int scan_thresh;
   float* grow;  // per-warp working sets of a long-window launch (GROW), else null
@@ -68,102 +67,70 @@ constexpr int kStageCycOff = kStageEntries * 4 + 16;                   // bytes
 constexpr int kStageWords = (kStageCycOff + kStageEntries * 2 + 16) / 4;
 // Bin ranges of more entries than this are binary-searched per bin instead of scanned.
 constexpr int kScanThreshFp32 = 256, kScanThreshBf16 = 384;
-constexpr int kBitOff = 32;         // bitmap bit of cycle c is c + kBitOff (room for -h)
+constexpr int kSeg = 4;               // output cycles of one segment
 constexpr int kSmemMaxCycles = 2048;  // longest RT window (cycles) a warp's shared-memory plan
                                       // holds; longer windows run with GROW
-constexpr int kTouchCap = 256;      // accepted cells a row records for clearing; beyond it the
-                                    // row is zeroed whole
+constexpr int kTouchCap = 256;        // accepted cells a row records for clearing; beyond it the
+                                      // row is zeroed whole
+// Listed outputs: up to 31 left over, 4 per lane of one round, a warp of idle ones.
+constexpr int kOutCap = 31 + 32 * kSeg + 32;
 
-__host__ __device__ inline int maxima_cap(int ncell) { return ncell / 4 + 8; }
-
-// Shared-memory address of stored index i (cycle + off) in a score array whose
-// lanes own S consecutive cycles: one pad word after every S cells, so that the 32
-// lanes of a warp, reading at the same offset within their segments, hit 32
-// different banks.
-template <int S>
-__device__ __forceinline__ int xaddr(int i) {
-  return i + i / S;
-}
-
-// The XIC row is read as 8-byte pairs of cells (u, u + 1), u even within a lane's
-// segment, so its segments of S cells (S even) sit at an even stride of
-// row_stride(S) words whose half is odd: the 16 lanes of each half-warp then hit 16
-// different bank pairs.
-__host__ __device__ constexpr int row_stride(int S) {
-  return ((S + 2) / 2) % 2 == 1 ? S + 2 : S + 4;
-}
-
-template <int S>
-__device__ __forceinline__ int raddr(int i) {
-  return i + (i / S) * (row_stride(S) - S);
-}
-
-// Floor division, for offsets known at compile time.
-__host__ __device__ constexpr int floordiv(int a, int b) {
-  return a >= 0 ? a / b : -((-a + b - 1) / b);
-}
+__host__ __device__ inline int maxima_cap(int c_max) { return c_max / 4 + 8; }
 
 // Per-warp shared-memory plan, in 4-byte words.  The block's ln table (double2 x
 // 256 = 1024 words), kernel taps (h + 1 words, at least 32) and the warps' staging
-// areas come first.  `ncell` (passes * 32 * S) sizes the bitmap, which every lane reads;
-// the row and the scores, of which only lanes with an output below c_max touch theirs,
-// are sized by c_max (a 801-cycle class of S = 16 would else hold 1024 cycles).
+// areas come first.
 struct WarpPlan {
-  int row, bm, cells, score, lst, mval, midx, total;
-  int off;        // stored index of cycle c is c + off (off >= h, a multiple of S)
+  int row, bm, cells, segbits, segs, score, lst, mval, midx, total;
+  int off;        // the row holds cycle c at c + off (off >= h, a multiple of kSeg)
   int row_words;  // words of the row, a multiple of 4
-  int lead;       // bitmap words below bm[0]: a window reaching h cycles before cycle 0
-                  // reads them (always zero)
-  int bw;         // bitmap words from bm[0]
+  int bw;         // words of the touched-cycle bitmap
+  int sw;         // words of the segment bitmap
   int mx;         // maxima capacity
 };
 __host__ __device__ inline int block_header_words(int h) {
   return kLnTableSize * 4 + ((h + 1 + 31) / 32) * 32;
 }
 
-__host__ __device__ inline WarpPlan warp_plan(int S, int h, int ncell, int c_max) {
+__host__ __device__ inline WarpPlan warp_plan(int h, int c_max) {
   WarpPlan w;
-  const int cc = (c_max + S - 1) / S * S;
-  w.off = (h + S - 1) / S * S;
-  const int span = cc + h + w.off + S;  // stored indices [0, span) cover every read
-  w.row_words = (span + (span / S + 1) * (row_stride(S) - S) + 3) & ~3;
+  const int cc = (c_max + kSeg - 1) / kSeg * kSeg;
+  w.off = (h + kSeg - 1) / kSeg * kSeg;
+  w.row_words = cc + 2 * w.off + kSeg;
   int o = 0;
   w.row = o;
   o += w.row_words;
-  w.lead = h > kBitOff ? (h - kBitOff + 31) / 32 : 0;
-  w.bw = (ncell + h + kBitOff + 31) / 32 + 2;
-  w.bm = o + w.lead;
-  o += w.lead + w.bw;
+  w.score = o + 4;  // 4 words of margin on both sides: the maxima scan reads them, and idle
+                    // lanes of the score terms work on the lowest
+  o += cc + 8;
+  w.bm = o;  // a bit per touched cycle
+  w.bw = (cc + 31) / 32;
+  o += w.bw;
+  w.segbits = o;  // a bit per segment that a touched cycle reaches
+  w.sw = (cc / kSeg + 31) / 32 + 1;
+  o += w.sw;
+  w.segs = o;  // those segments, listed (16 bits each)
+  o += (cc / kSeg + 1) / 2;
   w.cells = o;  // cells accepted by the current row (16 bits each)
   o += kTouchCap / 2;
-  w.score = o + 4;  // 4 words of margin below: the maxima scan reads 2 cycles early, and
-                    // idle lanes of the score terms work on the lowest
-  o += cc + cc / S + 12;
   o = (o + 1) & ~1;
-  // one pass of convolved values as (value, score address) pairs, and a warp of idle ones;
-  // before it, while the row is gathered, the accepted entries' intensities (kTouchCap words)
+  // non-zero outputs as (value, score index) pairs; before them, while the row is gathered,
+  // the accepted entries' intensities (kTouchCap words); after the last row, the maxima
   w.lst = o;
-  o += 2 * 32 * (S + 1);
-  w.mx = maxima_cap(ncell);
-  if (2 * w.mx <= 2 * 32 * S) {
-    // the maxima are collected after the precursor's last row is scored, when the
-    // output list is free
-    w.mval = w.lst;
-    w.midx = w.lst + w.mx;
-  } else {
-    w.mval = o;
-    o += w.mx;
-    w.midx = o;
-    o += w.mx;
-  }
+  w.mx = maxima_cap(cc);
+  w.mval = o;
+  w.midx = o + w.mx;
+  int lw = 2 * kOutCap;
+  if (lw < kTouchCap) lw = kTouchCap;
+  if (lw < 2 * w.mx) lw = 2 * w.mx;
+  o += lw;
   w.total = (o + 3) & ~3;
   return w;
 }
 
-__host__ __device__ inline size_t search_smem_bytes(int nw, int S, int h, int ncell, int c_max,
-                                                    bool grow = false) {
+__host__ __device__ inline size_t search_smem_bytes(int nw, int h, int c_max, bool grow = false) {
   return (size_t)(block_header_words(h) +
-                  nw * (kStageWords + (grow ? 0 : warp_plan(S, h, ncell, c_max).total))) * 4;
+                  nw * (kStageWords + (grow ? 0 : warp_plan(h, c_max).total))) * 4;
 }
 
 // Launch bounds of an instance.  The FP32 shared-memory instances for half widths 10
@@ -224,8 +191,9 @@ __device__ __forceinline__ unsigned from_lane(unsigned x, int q, int lane) {
 // warps however few entries of a chunk lie in the RT window (7 of 32 on average on
 // 3000 x 300 data); the list is also what the next row clears.
 struct RowList {
-  float* row;
-  uint32_t* bm;
+  float* row;         // cycle 0's cell
+  uint32_t* bm;       // touched cycles
+  uint32_t* segbits;  // segments they reach
   uint16_t* cells;  // entry i at i % kTouchCap
   float* vals;      // likewise
   int n;            // entries appended (warp-uniform)
@@ -234,12 +202,12 @@ struct RowList {
 
 // The rare case of add_entries: lanes that hit the same cycle are grouped and summed
 // by their lowest lane in lane order (kept out of line: it is seldom taken).
-static __device__ __noinline__ void add_grouped(bool act, int cell, int addr, int first, int lane,
+static __device__ __noinline__ void add_grouped(bool act, int cell, int first, int lane,
                                                 float* row, const float* vals) {
   const int key = act ? cell : (-1 - lane);
   const unsigned grp = __match_any_sync(kFull, key);
   if (act && lane == __ffs(grp) - 1) {
-    float acc = row[addr];
+    float acc = row[cell];
     unsigned g = grp;
 #pragma unroll 1
     while (g) {
@@ -247,7 +215,7 @@ static __device__ __noinline__ void add_grouped(bool act, int cell, int addr, in
       acc = __fadd_rn(acc, vals[(first + l) % kTouchCap]);
       g &= g - 1;
     }
-    row[addr] = acc;
+    row[cell] = acc;
   }
 }
 
@@ -258,48 +226,66 @@ static __device__ __noinline__ void add_grouped(bool act, int cell, int addr, in
 // the rows), that lane adds after the others have stored: to what an earlier entry left, or
 // to another lane's intensity, where 0 + a + b and 0 + b + a round alike.  Else the lanes
 // are grouped by cell and summed by their lowest lane one rounded add at a time.
-template <int S>
-__device__ __forceinline__ void add_entries(RowList& r, int m, int off, int lane) {
+template <int H>
+__device__ __forceinline__ void add_entries(RowList& r, int m, int h, int C, int lane) {
   __syncwarp();
   const int i = (r.done + lane) % kTouchCap;
   const bool act = lane < m;
   const int cell = r.cells[i];
   const float v = r.vals[i];
-  const int addr = raddr<S>(cell + off);
   const uint32_t bit = 1u << (cell & 31);
   bool again = false;
-  if (act) again = (atomicOr(r.bm + ((cell + kBitOff) >> 5), bit) & bit) != 0u;
+  if (act) again = (atomicOr(r.bm + (cell >> 5), bit) & bit) != 0u;
+  if (act && !again) {
+    // the segments holding outputs cell - h .. cell + h of the valid range
+    const int s0 = max(cell - h, h) / kSeg, s1 = min(cell + h, C - 1) / kSeg;
+    if (H > 0) {
+      if (s1 >= s0) {  // at most (2H + 4) / 4 + 1 <= 10 segments: two words
+        const unsigned long long mask = ((2ull << (s1 - s0)) - 1ull) << (s0 & 31);
+        atomicOr(r.segbits + (s0 >> 5), (uint32_t)mask);
+        if ((uint32_t)(mask >> 32)) atomicOr(r.segbits + (s0 >> 5) + 1, (uint32_t)(mask >> 32));
+      }
+    } else {
+#pragma unroll 1
+      for (int s = s0; s <= s1; s = (s | 31) + 1) {
+        const uint32_t from = 0xffffffffu << (s & 31);
+        const uint32_t to = (s1 | 31) == (s | 31) ? 0xffffffffu >> (31 - (s1 & 31)) : 0xffffffffu;
+        atomicOr(r.segbits + (s >> 5), from & to);
+      }
+    }
+  }
   const unsigned later = __ballot_sync(kFull, again);
   if ((later & (later - 1u)) == 0u) {
-    if (act && !again) r.row[addr] = v;
+    if (act && !again) r.row[cell] = v;
     __syncwarp();
-    if (again) r.row[addr] = __fadd_rn(r.row[addr], v);
+    if (again) r.row[cell] = __fadd_rn(r.row[cell], v);
   } else {
-    add_grouped(act, cell, addr, r.done, lane, r.row, r.vals);
+    add_grouped(act, cell, r.done, lane, r.row, r.vals);
   }
   r.done += m;
 }
 
 // Appends the lanes' entries marked `in`, in lane order.
-template <int S>
-__device__ __forceinline__ void append_entries(RowList& r, bool in, int cell, float v, int off,
+template <int H>
+__device__ __forceinline__ void append_entries(RowList& r, bool in, int cell, float v, int h, int C,
                                                int lane) {
   const unsigned act = __ballot_sync(kFull, in);
   if (in) {
-    const int at = (r.n + __popc(act & lanemask_lt())) % kTouchCap;
+    const int at = (r.n + __popc(act & ((1u << lane) - 1u))) % kTouchCap;
     r.cells[at] = (uint16_t)cell;
     r.vals[at] = v;
   }
   r.n += __popc(act);
-  if (r.n - r.done >= 32) add_entries<S>(r, 32, off, lane);
+  if (r.n - r.done >= 32) add_entries<H>(r, 32, h, C, lane);
 }
 
 // The same for two consecutive entries per lane.
-template <int S>
+template <int H>
 __device__ __forceinline__ void append_pairs(RowList& r, bool in0, bool in1, int cell0, int cell1,
-                                             float v0, float v1, int off, int lane) {
+                                             float v0, float v1, int h, int C, int lane) {
+  const unsigned lt = (1u << lane) - 1u;
   const unsigned act0 = __ballot_sync(kFull, in0), act1 = __ballot_sync(kFull, in1);
-  const int at = r.n + __popc(act0 & lanemask_lt()) + __popc(act1 & lanemask_lt());
+  const int at = r.n + __popc(act0 & lt) + __popc(act1 & lt);
   if (in0) {
     r.cells[at % kTouchCap] = (uint16_t)cell0;
     r.vals[at % kTouchCap] = v0;
@@ -311,7 +297,7 @@ __device__ __forceinline__ void append_pairs(RowList& r, bool in0, bool in1, int
   }
   r.n += __popc(act0) + __popc(act1);
 #pragma unroll 1
-  while (r.n - r.done >= 32) add_entries<S>(r, 32, off, lane);
+  while (r.n - r.done >= 32) add_entries<H>(r, 32, h, C, lane);
 }
 
 // Is `pos` the first entry of one of the bins (b0, b1)?  (slice_starts[b] == pos)
@@ -411,11 +397,11 @@ struct SearchedPair {
   int n, done;           // of the row list
   unsigned read, offs;   // entries and offsets read
 };
-template <int S, bool FAST>
+template <int H, bool FAST>
 static __device__ __noinline__ SearchedPair gather_searched(const SearchArgs& a, uint32_t b0,
                                                             uint32_t b1, int wsel, int64_t wbase,
                                                             int cs, int C, int lane, RowList r,
-                                                            int off) {
+                                                            int h) {
   SearchedPair out{0, 0, 0, 0};
   const uint32_t* ssw = a.ss + a.win[wsel].ss_off;
   const uint16_t* cy = a.cyc + wbase;
@@ -456,7 +442,7 @@ static __device__ __noinline__ SearchedPair gather_searched(const SearchArgs& a,
       const int64_t q = opos + (t - oex);
       const int c = vt ? (int)__ldg(cy + q) : 0;
       const float v = vt ? ld_intensity<FAST>(a, wbase + q) : 0.0f;
-      append_entries<S>(r, vt, c - cs, v, off, lane);
+      append_entries<H>(r, vt, c - cs, v, h, C, lane);
     }
   }
   out.n = r.n;
@@ -469,11 +455,11 @@ static __device__ __noinline__ SearchedPair gather_searched(const SearchArgs& a,
 // every entry of the range and keeps start < cycle < stop plus, per bin, the last entry
 // at cycle == start; or, for long ranges, gather_searched.  `staged`: the range's first
 // kStageEntries entries are already on their way.
-template <int S, bool FAST, bool STATS>
+template <int H, bool FAST, bool STATS>
 __device__ __forceinline__ void gather_pair(const SearchArgs& a, const PairCursor& pc, int pq,
                                             Pair pr, bool staged, int cs, int C, int lane,
                                             uint32_t stage, const unsigned char* stage_p,
-                                            RowList& r, int off, Counters<STATS>& k) {
+                                            RowList& r, int h, Counters<STATS>& k) {
   if (scans(a, pr.n)) {
     k.read += pr.n;
 #pragma unroll 1
@@ -523,35 +509,18 @@ __device__ __forceinline__ void gather_pair(const SearchArgs& a, const PairCurso
             }
           }
         }
-        append_pairs<S>(r, in0, in1, cell0, cell1, v.x, v.y, off, lane);
+        append_pairs<H>(r, in0, in1, cell0, cell1, v.x, v.y, h, C, lane);
       }
     }
   } else {
-    const SearchedPair sp = gather_searched<S, FAST>(
+    const SearchedPair sp = gather_searched<H, FAST>(
         a, __shfl_sync(kFull, pc.b0, pq), __shfl_sync(kFull, pc.b1, pq),
-        __shfl_sync(kFull, pc.wsel, pq), __shfl_sync(kFull, pc.wbase, pq), cs, C, lane, r, off);
+        __shfl_sync(kFull, pc.wsel, pq), __shfl_sync(kFull, pc.wbase, pq), cs, C, lane, r, h);
     r.n = uniform(sp.n);
     r.done = uniform(sp.done);
     k.read += sp.read;
     k.off += sp.offs;
   }
-}
-
-// Any bit set in bm[lo, lo + n)?  (n >= 1; lo may be negative: the shift and mask
-// below are floor division and remainder on two's-complement ints, and the words
-// below bm[0] that such a range reaches are reserved and zero)
-__device__ __forceinline__ bool bits_any(const uint32_t* bm, int lo, int n) {
-  const int last = lo + n - 1;
-  const int w0 = lo >> 5, w1 = last >> 5;
-  uint32_t acc = 0;
-#pragma unroll 1
-  for (int w = w0; w <= w1; ++w) {
-    uint32_t v = bm[w];
-    if (w == w0) v &= 0xffffffffu << (lo & 31);
-    if (w == w1) v &= 0xffffffffu >> (31 - (last & 31));
-    acc |= v;
-  }
-  return acc != 0u;
 }
 
 // Packed f32x2 arithmetic (sm_100a): one instruction performs two independent f32
@@ -593,13 +562,12 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
 // row in shared memory: x[j]*w[h] first, then (x[j-d] + x[j+d]) * w[h-d] for
 // d = h..1.  Any half width; used off the main path.  FAST (BF16 storage) fuses
 // each multiply-add.
-template <int S, bool FAST>
-__device__ __forceinline__ float conv_at(const float* row, int off, const float* kw_s, int h,
-                                         int j) {
-  float s = __fadd_rn(0.0f, __fmul_rn(row[raddr<S>(j + off)], kw_s[h]));
+template <bool FAST>
+__device__ __forceinline__ float conv_at(const float* row, const float* kw_s, int h, int j) {
+  float s = __fadd_rn(0.0f, __fmul_rn(row[j], kw_s[h]));
 #pragma unroll 1
   for (int t = 0; t < h; ++t) {
-    const float lr = __fadd_rn(row[raddr<S>(j - h + t + off)], row[raddr<S>(j + h - t + off)]);
+    const float lr = __fadd_rn(row[j - h + t], row[j + h - t]);
     s = FAST ? __fmaf_rn(lr, kw_s[t], s) : __fadd_rn(s, __fmul_rn(lr, kw_s[t]));
   }
   return s;
@@ -634,47 +602,19 @@ __device__ __forceinline__ float score_term(float s, float c, float w, const dou
   return __fadd_rn(s, __fmul_rn(y, w));
 }
 
-// Where the list of a pass's outputs, (value, score index) pairs, is appended to: a
-// shared-memory address, or (GROW) a pointer.
+// Stores the pair (v, at) where `on`, predicated (a branch around each store cost three
+// times as much).
 template <bool GROW>
-struct OutEnd;
-template <>
-struct OutEnd<false> {
-  uint32_t to;
-  __device__ OutEnd(float2* at) : to((uint32_t)__cvta_generic_to_shared(at)) {}
-  // Appends (v, at) where bit m of mk is set: test, store, advance, all predicated (a
-  // branch around each store cost three times as much).
-  __device__ __forceinline__ void put(uint32_t mk, int m, float v, int at) {
+__device__ __forceinline__ void put_if(bool on, float2* to, float v, int at) {
+  if (GROW) {
+    if (on) *to = make_float2(v, __int_as_float(at));
+  } else {
     asm volatile(
-        "{\n .reg .pred q;\n .reg .b32 t;\n and.b32 t, %1, %2;\n setp.ne.u32 q, t, 0;\n"
-        " @q st.shared.v2.b32 [%0], {%3, %4};\n @q add.u32 %0, %0, 8;\n}"
-        : "+r"(to)
-        : "r"(mk), "r"(1u << m), "r"(__float_as_uint(v)), "r"(at)
+        "{\n .reg .pred q;\n setp.ne.u32 q, %0, 0;\n @q st.shared.v2.b32 [%1], {%2, %3};\n}" ::"r"(
+            (uint32_t)on),
+        "r"((uint32_t)__cvta_generic_to_shared(to)), "r"(__float_as_uint(v)), "r"(at)
         : "memory");
   }
-};
-template <>
-struct OutEnd<true> {
-  float2* to;
-  __device__ OutEnd(float2* at) : to(at) {}
-  __device__ __forceinline__ void put(uint32_t mk, int m, float v, int at) {
-    if ((mk >> m) & 1u) *to++ = make_float2(v, __int_as_float(at));
-  }
-};
-
-// Spreads every set bit of x over the LEN bits at and below it: bit m of the result is set
-// where any of bits m .. m + LEN - 1 is.
-template <int LEN, class U>
-__device__ __forceinline__ U spread_down(U x) {
-  int reach = 1;
-#pragma unroll
-  for (int g = 0; g < 5; ++g)
-    if (2 * reach <= LEN) {
-      x |= x >> reach;
-      reach *= 2;
-    }
-  if (reach < LEN) x |= x >> (LEN - reach);
-  return x;
 }
 
 template <bool FAST>
@@ -734,11 +674,11 @@ __device__ __forceinline__ void stage_pair(const SearchArgs& a, int64_t p, int p
 
 // Gathers fragment f's XIC row: its (fragment, window) pairs in window order (the
 // reference's DenseXICObservation::new, src/dense_xic_observation/mod.rs:30-64).
-template <int S, bool FAST, bool STATS>
+template <int H, bool FAST, bool STATS>
 __device__ __forceinline__ void gather_row(const SearchArgs& a, int64_t p, int f, int nwin,
                                            int npairs, int cs, int C, int lane, PairCursor& pc,
                                            uint32_t stage, const unsigned char* stage_p, RowList& r,
-                                           int off, Counters<STATS>& k) {
+                                           int h, Counters<STATS>& k) {
 #pragma unroll 1
   for (int wi = 0; wi < nwin; ++wi) {
     const int pi = f * nwin + wi;
@@ -754,17 +694,15 @@ __device__ __forceinline__ void gather_row(const SearchArgs& a, int64_t p, int f
       }
     }
     if (pr.n == 0) continue;
-    gather_pair<S, FAST, STATS>(a, pc, q, pr, pi == pc.pre_pi, cs, C, lane, stage,
-                                stage_p, r, off, k);
+    gather_pair<H, FAST, STATS>(a, pc, q, pr, pi == pc.pre_pi, cs, C, lane, stage, stage_p, r, h, k);
   }
-  if (r.done < r.n) add_entries<S>(r, r.n - r.done, off, lane);
+  if (r.done < r.n) add_entries<H>(r, r.n - r.done, h, C, lane);
 }
 
 // The last gathered row's cells (and bitmap words) back to zero.
-template <int S>
-__device__ __forceinline__ void clear_row(RowList& r, const WarpPlan& P, int lane) {
+__device__ __forceinline__ void clear_row(RowList& r, float* row, const WarpPlan& P, int lane) {
   if (r.n > kTouchCap) {
-    float4* r4 = reinterpret_cast<float4*>(r.row);
+    float4* r4 = reinterpret_cast<float4*>(row);
 #pragma unroll 1
     for (int i = lane; i < P.row_words / 4; i += 32) r4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
@@ -773,75 +711,64 @@ __device__ __forceinline__ void clear_row(RowList& r, const WarpPlan& P, int lan
 #pragma unroll 1
     for (int i = lane; i < r.n; i += 32) {
       const int c = r.cells[i];
-      r.row[raddr<S>(c + P.off)] = 0.0f;
-      r.bm[(c + kBitOff) >> 5] = 0u;
+      r.row[c] = 0.0f;
+      r.bm[c >> 5] = 0u;
     }
   }
+#pragma unroll 1
+  for (int i = lane; i < P.sw; i += 32) r.segbits[i] = 0u;
   r.n = r.done = 0;
   __syncwarp();
 }
 
 // A row whose weight is not finite, out of line: ln(conv + 1) * w is NaN even where conv
 // is zero, so every column takes its term, as in the reference.
-template <int S, bool FAST>
-static __device__ __noinline__ void score_every_column(const SearchArgs& a, const float* row, int off,
+template <bool FAST>
+static __device__ __noinline__ void score_every_column(const SearchArgs& a, const float* row,
                                                        const float* kw_s, int h, int C, float wf,
                                                        float* score, const double2* lnt, int lane) {
 #pragma unroll 1
   for (int j = lane; j < C; j += 32) {
-    const float c = (j >= h && j < C - h) ? conv_at<S, FAST>(row, off, kw_s, h, j) : 0.0f;
-    score_add<FAST>(score, xaddr<S>(j), c, wf, lnt, a.ln);
+    const float c = (j >= h && j < C - h) ? conv_at<FAST>(row, kw_s, h, j) : 0.0f;
+    score_add<FAST>(score, j, c, wf, lnt, a.ln);
   }
 }
 
 // Strict 5-point local maxima of a precursor's scores (src/peak_group_selection/mod.rs:33-43),
 // collected in cycle order, and the top K of them by (value descending, cycle
 // ascending), the reference's stable sort (src/peak_group_selection/mod.rs:45-61),
-// written to the candidate slots.  `score` holds cycle j at xaddr<S>(j), with two
-// readable words below cycle 0 and S + 2 cycles past C.
-template <int S>
+// written to the candidate slots.  `score` is 16-byte aligned, with four readable words
+// below cycle 0 and past the last multiple of 4.
 __device__ __forceinline__ void pick_top_k(const SearchArgs& a, int64_t p, int cs, int C,
                                            const float* score, float* mval, int* midx, int mx,
                                            int lane) {
-  const int passes = (C + 32 * S - 1) / (32 * S);
-  // lane l's maxima of a pass go after those of lanes < l
+  const unsigned lt = (1u << lane) - 1u;
   int nmax = 0;
+  // 4 consecutive cycles per lane; two maxima are at least 4 cycles apart, so a lane finds
+  // at most one
 #pragma unroll 1
-  for (int ps = 0; ps < passes; ++ps) {
-    const int seg = ps * 32 + lane;
-    const float* sb = score + seg * (S + 1);
-    uint32_t mk = 0;
-    if (seg * S < C - 2 && seg * S + S > 2) {
-      float v[S + 4];
+  for (int c0 = 0; c0 < C; c0 += 128) {
+    const int j0 = c0 + 4 * lane;
+    int found = -1;
+    if (j0 < C) {
+      const float4* s4 = reinterpret_cast<const float4*>(score + j0);
+      const float4 l = s4[-1], m = s4[0], h = s4[1];
+      const float v[8] = {l.z, l.w, m.x, m.y, m.z, m.w, h.x, h.y};
 #pragma unroll
-      for (int t = 0; t < S + 4; ++t) v[t] = sb[(t - 2) + floordiv(t - 2, S)];
-#pragma unroll
-      for (int m = 0; m < S; ++m) {
-        const int i = seg * S + m;
-        const bool is = i >= 2 && i < C - 2 && v[m] < v[m + 1] && v[m + 1] < v[m + 2] &&
-                        v[m + 2] > v[m + 3] && v[m + 3] > v[m + 4];
-        mk |= (uint32_t)is << m;
+      for (int t = 0; t < 4; ++t) {
+        const int i = j0 + t;
+        if (i >= 2 && i < C - 2 && v[t] < v[t + 1] && v[t + 1] < v[t + 2] && v[t + 2] > v[t + 3] &&
+            v[t + 3] > v[t + 4])
+          found = i;
       }
     }
-    const int cnt = __popc(mk);
-    int incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(kFull, incl, o);
-      if (lane >= o) incl += t;
+    const unsigned b = __ballot_sync(kFull, found >= 0);
+    const int pos = nmax + __popc(b & lt);
+    if (found >= 0 && pos < mx) {
+      mval[pos] = score[found];
+      midx[pos] = found;
     }
-    int pos = nmax + incl - cnt;
-#pragma unroll 1
-    while (mk) {
-      const int m = __ffs(mk) - 1;
-      if (pos < mx) {
-        mval[pos] = sb[m];
-        midx[pos] = seg * S + m;
-      }
-      ++pos;
-      mk &= mk - 1;
-    }
-    nmax += __shfl_sync(kFull, incl, 31);
+    nmax += __popc(b);
   }
   __syncwarp();
   if (nmax > mx) {  // cannot happen: maxima are at least 4 cycles apart
@@ -897,17 +824,17 @@ __device__ __forceinline__ void flush_counters(const SearchArgs& a, const Counte
   }
 }
 
-// GROW: the warp's working set (row, tags, bitmap, scores, lists, maxima) lives in
+// GROW: the warp's working set (row, bitmaps, scores, lists, maxima) lives in
 // a global buffer of P.total words per warp (`a.grow`) instead of shared memory, for
 // RT windows longer than kSmemMaxCycles; the code and every operation are the same.
 // STATS: the statistics pass's work counters (compiled in only for it).
-template <int H, int S, bool FAST, bool GROW, bool STATS>
+template <int H, bool FAST, bool GROW, bool STATS>
 __global__ void __launch_bounds__(LaunchShape<H, FAST, GROW>::threads, LaunchShape<H, FAST, GROW>::blocks)
     search_kernel(const __grid_constant__ SearchArgs a) {
   extern __shared__ __align__(16) float smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = H > 0 ? H : a.h;
-  const WarpPlan P = warp_plan(S, h, a.ncell, a.c_max);
+  const WarpPlan P = warp_plan(h, a.c_max);
   double2* lnt = reinterpret_cast<double2*>(smem_raw);
   float* kw_s = smem_raw + kLnTableSize * 4;
   const int nw = blockDim.x >> 5;
@@ -923,13 +850,15 @@ __global__ void __launch_bounds__(LaunchShape<H, FAST, GROW>::threads, LaunchSha
   int* midx = reinterpret_cast<int*>(wb + P.midx);
   float2* lst = reinterpret_cast<float2*>(wb + P.lst);
   // r.n: also the cells the previous row left to clear
-  RowList r{row, bm, reinterpret_cast<uint16_t*>(wb + P.cells), wb + P.lst, 0, 0};
+  uint32_t* segbits = reinterpret_cast<uint32_t*>(wb + P.segbits);
+  uint16_t* segs = reinterpret_cast<uint16_t*>(wb + P.segs);
+  RowList r{row + P.off, bm, segbits, reinterpret_cast<uint16_t*>(wb + P.cells), wb + P.lst, 0, 0};
   {
     float4* r4 = reinterpret_cast<float4*>(row);
 #pragma unroll 1
     for (int i = lane; i < P.row_words / 4; i += 32) r4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
-    for (int i = lane - P.lead; i < P.bw; i += 32) bm[i] = 0u;
+    for (int i = lane; i < P.bw; i += 32) bm[i] = 0u;
   }
 
 #pragma unroll 1
@@ -938,6 +867,7 @@ __global__ void __launch_bounds__(LaunchShape<H, FAST, GROW>::threads, LaunchSha
   for (int i = threadIdx.x; i <= a.h; i += blockDim.x) kw_s[i] = a.kw_dev ? a.kw_dev[i] : a.kw[i];
   __syncthreads();
   Counters<STATS> k;
+  const unsigned lt = (1u << lane) - 1u;
 
   const unsigned n_work = a.list ? (unsigned)uniform((int)*a.list_len) : (unsigned)a.n_prec;
 #pragma unroll 1
@@ -963,7 +893,6 @@ __global__ void __launch_bounds__(LaunchShape<H, FAST, GROW>::threads, LaunchSha
     }
     const int nwin = uniform(a.nwin[p]);
     const int npairs = F * nwin;
-    const int passes = (C + 32 * S - 1) / (32 * S);
     k.frag += F;
     // fragment weights, lane f holding fragment f's (fetched once per precursor)
     const float wf_lane = lane < F ? __ldg(a.fw + p * a.kf + lane) : 0.0f;
@@ -973,136 +902,121 @@ __global__ void __launch_bounds__(LaunchShape<H, FAST, GROW>::threads, LaunchSha
     for (int f = -1; f < F; ++f) {
       if (f >= 0) {
         // ---- 1. gather: the fragment's pairs in window order
-        clear_row<S>(r, P, lane);
-        gather_row<S, FAST, STATS>(a, p, f, nwin, npairs, cs, C, lane, pc, stage, stage_p, r, P.off, k);
+        clear_row(r, row, P, lane);
+        gather_row<H, FAST, STATS>(a, p, f, nwin, npairs, cs, C, lane, pc, stage, stage_p, r, h, k);
         k.acc += (unsigned int)r.n;
       }
       // the next fragment's first pair arrives while this row is convolved
       stage_pair<FAST>(a, p, (f + 1) * nwin, nwin, npairs, lane, pc, stage);
       if (f < 0) {
 #pragma unroll 1
-        for (int i = lane; i <= C + C / S; i += 32) score[i] = 0.0f;  // cycles [0, C) with pads
+        for (int i = lane; i < C; i += 32) score[i] = 0.0f;
         continue;
       }
       __syncwarp();
       float wf = __shfl_sync(kFull, wf_lane, f & 31);
       if (f >= 32) wf = __ldg(a.fw + p * a.kf + f);
       if (!isfinite(wf)) {
-        score_every_column<S, FAST>(a, row, P.off, kw_s, h, C, wf, score, lnt, lane);
+        score_every_column<FAST>(a, r.row, kw_s, h, C, wf, score, lnt, lane);
         __syncwarp();
         continue;
       }
       if (r.n == 0) continue;  // no entry accepted: every term is +0
-      // ---- 2./3. convolution of this lane's cycles, then the score terms of the
-      // outputs of the valid range [h, C - h) that a touched cycle reaches.  Every other
-      // output is zero and adds ln(1) * w = +0, which leaves a score as it is, so only
-      // those are listed (warp-compacted, in lane order) and take a logarithm.
+      // ---- 2./3. convolution of the segments that a touched cycle reaches (every other
+      // output is zero), one per lane, then the score terms of the non-zero outputs of the
+      // valid range [h, C - h).  A zero output adds ln(1) * w = +0, which leaves a score
+      // as it is, so only the others are listed and take a logarithm, 32 at a time.  Their
+      // order within the row is free: each has its own cycle.
+      const int n_seg = (C - h + kSeg - 1) / kSeg;
+      int nact = 0;
 #pragma unroll 1
-      for (int ps = 0; ps < passes; ++ps) {
-        const int j0 = ps * 32 * S + lane * S;
-        uint32_t mk = 0;  // outputs j0 + m to list
-        bool act;
+      for (int w0 = 0; w0 < n_seg; w0 += 32) {
+        uint32_t x = segbits[w0 / 32];
+        if (w0 + 32 > n_seg) x &= 0xffffffffu >> (32 - (n_seg - w0));
+        if ((x >> lane) & 1u) segs[nact + __popc(x & lt)] = (uint16_t)(w0 + lane);
+        nact += __popc(x);
+      }
+      nact = uniform(nact);
+      __syncwarp();
+      int listed = 0;
+#pragma unroll 1
+      for (int a0 = 0; a0 < nact; a0 += 32) {
+        const bool on = a0 + lane < nact;
+        const int j0 = on ? (int)segs[a0 + lane] * kSeg : 0;  // (idle lanes: segment 0)
+        const int rel = on ? j0 - h : -(1 << 20);             // of output 0 to the valid range
+        float cv[kSeg];
         if (H > 0) {
-          // bits j0 - H .. j0 + S - 1 + H of the touched cycles, each spread over the
-          // 2H + 1 outputs it reaches
-          const int lo = j0 - H + kBitOff;
-          const uint32_t* bw = bm + (lo >> 5);
-          uint32_t x;
-          if (S + 2 * H <= 32) {
-            x = spread_down<2 * H + 1>(__funnelshift_r(bw[0], bw[1], lo));
-          } else {
-            const uint32_t x0 = bw[0], x1 = bw[1], x2 = bw[2];
-            x = (uint32_t)spread_down<2 * H + 1>(
-                ((unsigned long long)__funnelshift_r(x1, x2, lo) << 32) | __funnelshift_r(x0, x1, lo));
-          }
-          const int m0 = max(H - j0, 0), m1 = max(min(C - H - j0, S), 0);
-          mk = x & ((1u << m1) - 1u) & (0xffffffffu << m0);
-          act = mk != 0u;
-        } else {
-          act = j0 + S > h && j0 < C - h && bits_any(bm, j0 - h + kBitOff, S + 2 * h);
-        }
-        if (!__any_sync(kFull, act)) continue;
-        float cv[S];
-        if (H > 0) {
-          // cells u in [UB, UE) of this lane's segment as 8-byte pairs (u even; a lane
-          // without outputs computes the first segment's); every output is formed in the
-          // reference's order: 0 + x[j]*w[h], then + (x[j-d] + x[j+d]) * w[h-d] for
-          // d = h..1, two outputs (m, m + 1) per packed instruction.  For odd d the pair
-          // sums straddle the register pairs and are formed by two scalar adds.
-          constexpr int UB = -((H + 1) & ~1);
-          constexpr int UE = (S + H + 1) & ~1;
-          constexpr int NX = UE - UB;
-          const float* rb = row + ((act ? ps * 32 + lane : 0) + P.off / S) * row_stride(S);
+          // cells j0 - OFF .. j0 + 3 + OFF; every output is formed in the reference's
+          // order: 0 + x[j]*w[h], then + (x[j-d] + x[j+d]) * w[h-d] for d = h..1, two
+          // outputs (m, m + 1) per packed instruction.  For odd d the pair sums straddle
+          // the register pairs and are formed by two scalar adds.
+          constexpr int OFF = (H + kSeg - 1) / kSeg * kSeg;
+          constexpr int NX = kSeg + 2 * OFF;
+          const float4* rb = reinterpret_cast<const float4*>(row + j0);
           float xv[NX];
 #pragma unroll
-          for (int q = 0; q < NX; q += 2) {
-            const int u = UB + q;
-            const float2 v =
-                *reinterpret_cast<const float2*>(rb + u + floordiv(u, S) * (row_stride(S) - S));
+          for (int q = 0; q < NX; q += 4) {
+            const float4 v = rb[q / 4];
             xv[q] = v.x;
             xv[q + 1] = v.y;
+            xv[q + 2] = v.z;
+            xv[q + 3] = v.w;
           }
-          f32x2 acc[S / 2];
+          f32x2 acc[kSeg / 2];
 #pragma unroll
-          for (int m = 0; m < S; m += 2)
-            acc[m / 2] = add2(a.zero2, fma2(pk2(xv[m - UB], xv[m + 1 - UB]), a.kw2[H], a.nzero2));
+          for (int m = 0; m < kSeg; m += 2)
+            acc[m / 2] = add2(a.zero2, fma2(pk2(xv[m + OFF], xv[m + 1 + OFF]), a.kw2[H], a.nzero2));
 #pragma unroll
           for (int t = 0; t < H; ++t) {
             const int d = H - t;
 #pragma unroll
-            for (int m = 0; m < S; m += 2) {
+            for (int m = 0; m < kSeg; m += 2) {
+              const int l = m - d + OFF, u = m + d + OFF;
               f32x2 lr;
               if (d % 2 == 0)
-                lr = add2(pk2(xv[m - d - UB], xv[m - d + 1 - UB]),
-                          pk2(xv[m + d - UB], xv[m + d + 1 - UB]));
+                lr = add2(pk2(xv[l], xv[l + 1]), pk2(xv[u], xv[u + 1]));
               else
-                lr = pk2(__fadd_rn(xv[m - d - UB], xv[m + d - UB]),
-                         __fadd_rn(xv[m + 1 - d - UB], xv[m + 1 + d - UB]));
+                lr = pk2(__fadd_rn(xv[l], xv[u]), __fadd_rn(xv[l + 1], xv[u + 1]));
               acc[m / 2] = FAST ? fma2(lr, a.kw2[t], acc[m / 2])
                                 : add2(acc[m / 2], fma2(lr, a.kw2[t], a.nzero2));
             }
           }
 #pragma unroll
-          for (int m = 0; m < S; m += 2) unpk2(acc[m / 2], cv[m], cv[m + 1]);
-        } else if (act) {
+          for (int m = 0; m < kSeg; m += 2) unpk2(acc[m / 2], cv[m], cv[m + 1]);
+        } else {
 #pragma unroll
-          for (int m = 0; m < S; ++m) {
-            const int j = j0 + m;
-            cv[m] = (j >= h && j < C - h) ? conv_at<S, FAST>(row, P.off, kw_s, h, j) : 0.0f;
+          for (int m = 0; m < kSeg; ++m) {
+            cv[m] = 0.0f;
+            if ((unsigned)(rel + m) < (unsigned)(C - 2 * h)) cv[m] = conv_at<FAST>(r.row, kw_s, h, j0 + m);
           }
-          const int m0 = max(h - j0, 0), m1 = min(C - h - j0, S);
-#pragma unroll
-          for (int m = 0; m < S; ++m)
-            mk |= (uint32_t)(m >= m0 && m < m1 && cv[m] != 0.0f) << m;
         }
-        const int cnt = __popc(mk);
-        int incl = cnt;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int t = __shfl_up_sync(kFull, incl, o);
-          if (lane >= o) incl += t;
+        for (int m = 0; m < kSeg; ++m) {
+          const bool ok = (unsigned)(rel + m) < (unsigned)(C - 2 * h) && cv[m] != 0.0f;
+          const unsigned b = __ballot_sync(kFull, ok);
+          put_if<GROW>(ok, lst + listed + __popc(b & lt), cv[m], j0 + m);
+          listed += __popc(b);
         }
-        const int total = (int)__reduce_add_sync(kFull, (unsigned)cnt);
-        const int sbase = (ps * 32 + lane) * (S + 1);  // score index of cycle j0
-        OutEnd<GROW> end(lst + (incl - cnt));
-#pragma unroll
-        for (int m = 0; m < S; ++m) end.put(mk, m, cv[m], sbase + m);
-        // idle entries up to a whole warp, which work on a word below the scores
-        lst[total + lane] = make_float2(0.0f, __int_as_float(-4));
+        if (a0 + 32 >= nact) {
+          // the row's last round: idle entries up to a whole warp, which work on a word
+          // below the scores
+          lst[listed + lane] = make_float2(0.0f, __int_as_float(-4));
+          listed = (listed + 31) & ~31;
+        }
         __syncwarp();
 #pragma unroll 1
-        for (int i0 = 0; i0 < total; i0 += 32) {
-          const float2 e = lst[i0 + lane];
+        while (listed >= 32) {
+          listed -= 32;
+          const float2 e = lst[listed + lane];
           float* sp = score + __float_as_int(e.y);
           *sp = score_term<FAST>(*sp, e.x, wf, lnt, a.ln);
         }
         __syncwarp();
       }
-      __syncwarp();
     }
     __syncwarp();
 
-    pick_top_k<S>(a, p, cs, C, score, mval, midx, P.mx, lane);
+    pick_top_k(a, p, cs, C, score, mval, midx, P.mx, lane);
   }
   flush_counters<STATS>(a, k, lane);
 }
