@@ -407,10 +407,9 @@ void (*pick_search_kernel(int h, bool fast, bool grow, bool stats))(SearchArgs) 
   return fast ? pick_for_precision<true>(h, grow, stats) : pick_for_precision<false>(h, grow, stats);
 }
 
-// Largest block (in warps) an instance may launch: its launch bounds (LaunchShape); the
-// statistics pass runs the generic-h instances (256 threads).
-int max_warps_per_block(bool fast, int h, bool grow, bool stats) {
-  return (stats ? 256 : launch_threads(h, fast, grow)) / 32;
+// Largest block (in warps) an instance may launch: its launch bounds (LaunchShape).
+int max_warps_per_block(bool grow) {
+  return (grow ? LaunchShape<true>::threads : LaunchShape<false>::threads) / 32;
 }
 
 // Long-window launches: blocks whose working sets fit kGrowBudgetBytes (at least one).
@@ -974,7 +973,7 @@ int enqueue_search(AdsSelection* s, const AdsDia* d, const AdsLib* l, AdsCandida
     int nw = s->o.warps_per_block > 0 ? s->o.warps_per_block : kDefaultWarpsPerBlock;
     if (!grow && search_smem_bytes(1, s->h, cmax_b, false) > (size_t)max_smem)
       grow = true;  // a very wide kernel: even one warp's plan exceeds shared memory
-    nw = std::max(1, std::min(nw, max_warps_per_block(bf16, s->h, grow, s->stats_on)));
+    nw = std::max(1, std::min(nw, max_warps_per_block(grow)));
     while (nw > 1 && search_smem_bytes(nw, s->h, cmax_b, grow) > (size_t)max_smem) --nw;
     const size_t smem = search_smem_bytes(nw, s->h, cmax_b, grow);
     if (smem > (size_t)max_smem)
@@ -1082,8 +1081,7 @@ int autotune(AdsSelection* s, const AdsDia* d, const AdsLib* l, int32_t repeats,
     scratch.device = s->device;
     int rc = ADS_OK;
     for (int nw : {2, 4, 8}) {
-      if (nw > max_warps_per_block(s->o.precision == ADS_PRECISION_BF16, s->h, false, false))
-        continue;
+      if (nw > max_warps_per_block(false)) continue;
       for (int S : {0, 16}) {  // length classes, or one class
         s->o.warps_per_block = nw;
         s->o.cycles_per_lane = S;

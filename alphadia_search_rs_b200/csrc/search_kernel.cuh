@@ -133,22 +133,16 @@ __host__ __device__ inline size_t search_smem_bytes(int nw, int h, int c_max, bo
                   nw * (kStageWords + (grow ? 0 : warp_plan(h, c_max).total))) * 4;
 }
 
-// Launch bounds of an instance.  The FP32 shared-memory instances for half widths 10
-// and 11 (kernel sizes 20-22) at 128 threads and 5 blocks per SM: up to 102 registers,
-// 20 warps (on 3000 x 300 data with 301-cycle windows 9 % faster than 256 x 2, without
-// spills worth noting).  Everything else at 256 x 2 (128 registers): the BF16 instances
-// (the 20-warp shape was 1.5 % slower on the uneven workload), half width 16 (spilled
-// up to 256 bytes and ran 13 % slower at kernel size 31), the generic half width and the
-// global-memory (long-window) instances.
-template <int H, bool FAST, bool GROW>
+// Launch bounds of an instance: shared-memory instances at 128 threads and 5 blocks per SM
+// (up to 102 registers, 20 warps), the global-memory (long-window) ones at 256 x 2.  With
+// 6 to 8 blocks (80 to 64 registers) up to 164 bytes of spills meet the little L1 that the
+// warps' shared memory leaves: 200,000 uneven precursors FP32 4.04 ms -> 4.39 to 5.22 ms;
+// at 256 x 2 500,000 uneven BF16 took 9.38 ms against 8.26 ms.
+template <bool GROW>
 struct LaunchShape {
-  static constexpr bool narrow = !FAST && !GROW && (H == 10 || H == 11);
-  static constexpr int threads = narrow ? 128 : 256;
-  static constexpr int blocks = narrow ? 5 : 2;
+  static constexpr int threads = GROW ? 256 : 128;
+  static constexpr int blocks = GROW ? 2 : 5;
 };
-__host__ __device__ constexpr int launch_threads(int h, bool fast, bool grow) {
-  return (!fast && !grow && (h == 10 || h == 11)) ? 128 : 256;
-}
 
 // Per-warp work counters of the statistics pass (ON); 32 bits suffice for one warp's
 // share of a launch.  In the searching instances (ON = false) they hold nothing and
@@ -365,29 +359,41 @@ __device__ __forceinline__ bool scans(const SearchArgs& a, uint32_t n) {
 // (lane q holds pair pb + q), and the pair whose first entries are staged.
 struct PairCursor {
   int pb = -64;
-  uint32_t rs = 0, n = 0, b0 = 0, b1 = 0;
-  int wsel = 0;
-  int64_t wbase = 0;
+  int64_t q = 0;   // absolute position of the pair's first entry
+  uint32_t n = 0;  // entries
   int pre_pi = -1;
 };
 
 // The pair in lane q of the cursor.
 struct Pair {
-  int64_t q;   // absolute position of its first entry
-  uint32_t n;  // entries
+  int64_t q;
+  uint32_t n;
 };
 __device__ __forceinline__ Pair pair_of(const PairCursor& pc, int q, int lane) {
-  return Pair{__shfl_sync(kFull, pc.wbase + pc.rs, q), from_lane(pc.n, q, lane)};
+  return Pair{__shfl_sync(kFull, pc.q, q), from_lane(pc.n, q, lane)};
+}
+
+// Bins and window of pair pi of precursor p, read again where they are rarely needed (kept
+// in registers they cost the hot loop five).
+struct PairBins {
+  uint32_t b0, b1;
+  WinInfo w;
+};
+__device__ __forceinline__ PairBins pair_bins(const SearchArgs& a, int64_t p, int pi, int nwin) {
+  const int f = pi / nwin;
+  const int64_t fo = p * a.kf + f;
+  return PairBins{a.blo[fo], a.bhi[fo], a.win[a.wins[p * a.maxw + (pi - f * nwin)]]};
 }
 
 // An entry at the window's first cycle counts only if it is the last of its bin there
 // (where Rust's binary_search lands, src/quadrupole_observation/mod.rs:91-94): is the
 // next entry, entry `tn` of the pair's n, in another bin or at another cycle?  Out of
 // line: about one range in fifty holds such an entry.
-static __device__ __noinline__ bool last_at_start(const SearchArgs& a, int wsel, uint32_t b0,
-                                                  uint32_t b1, uint32_t rs, int64_t q, uint32_t tn,
-                                                  uint32_t n, int cs) {
-  if (tn >= n || bin_starts_at(a.ss + a.win[wsel].ss_off, b0, b1, rs + tn)) return true;
+static __device__ __noinline__ bool last_at_start(const SearchArgs& a, int64_t p, int pi, int nwin,
+                                                  int64_t q, uint32_t tn, uint32_t n, int cs) {
+  if (tn >= n) return true;
+  const PairBins pb = pair_bins(a, p, pi, nwin);
+  if (bin_starts_at(a.ss + pb.w.ss_off, pb.b0, pb.b1, (uint32_t)(q + tn - pb.w.base))) return true;
   return (int)__ldg(a.cyc + q + tn) != cs;
 }
 
@@ -398,12 +404,14 @@ struct SearchedPair {
   unsigned read, offs;   // entries and offsets read
 };
 template <int H, bool FAST>
-static __device__ __noinline__ SearchedPair gather_searched(const SearchArgs& a, uint32_t b0,
-                                                            uint32_t b1, int wsel, int64_t wbase,
-                                                            int cs, int C, int lane, RowList r,
-                                                            int h) {
+static __device__ __noinline__ SearchedPair gather_searched(const SearchArgs& a, int64_t p, int pi,
+                                                            int nwin, int cs, int C, int lane,
+                                                            RowList r, int h) {
   SearchedPair out{0, 0, 0, 0};
-  const uint32_t* ssw = a.ss + a.win[wsel].ss_off;
+  const PairBins pb = pair_bins(a, p, pi, nwin);
+  const uint32_t b0 = pb.b0, b1 = pb.b1;
+  const int64_t wbase = pb.w.base;
+  const uint32_t* ssw = a.ss + pb.w.ss_off;
   const uint16_t* cy = a.cyc + wbase;
 #pragma unroll 1
   for (uint32_t bb = b0; bb < b1; bb += 32) {
@@ -450,13 +458,13 @@ static __device__ __noinline__ SearchedPair gather_searched(const SearchArgs& a,
   return out;
 }
 
-// fill_xic_slice for the (fragment, window) pair in lane `pq` of the cursor: its entries
+// fill_xic_slice for the (fragment, window) pair pi of precursor p: its entries
 // inside the RT window are listed, in CSR order.  Two exact strategies: scan, which reads
 // every entry of the range and keeps start < cycle < stop plus, per bin, the last entry
 // at cycle == start; or, for long ranges, gather_searched.  `staged`: the range's first
 // kStageEntries entries are already on their way.
 template <int H, bool FAST, bool STATS>
-__device__ __forceinline__ void gather_pair(const SearchArgs& a, const PairCursor& pc, int pq,
+__device__ __forceinline__ void gather_pair(const SearchArgs& a, int64_t p, int pi, int nwin,
                                             Pair pr, bool staged, int cs, int C, int lane,
                                             uint32_t stage, const unsigned char* stage_p,
                                             RowList& r, int h, Counters<STATS>& k) {
@@ -493,14 +501,11 @@ __device__ __forceinline__ void gather_pair(const SearchArgs& a, const PairCurso
         bool in0 = (unsigned)t < (unsigned)m && (unsigned)cell0 < (unsigned)C;
         bool in1 = t + 1 < m && (unsigned)cell1 < (unsigned)C;
         if (__any_sync(kFull, (in0 && cell0 == 0) || (in1 && cell1 == 0))) {
-          const uint32_t rs = __shfl_sync(kFull, pc.rs, pq);
-          const uint32_t b0 = __shfl_sync(kFull, pc.b0, pq), b1 = __shfl_sync(kFull, pc.b1, pq);
-          const int wsel = __shfl_sync(kFull, pc.wsel, pq);
 #pragma unroll 1
           for (int e = 0; e < 2; ++e) {
             const bool ask = e == 0 ? in0 && cell0 == 0 : in1 && cell1 == 0;
             if (ask) {
-              const bool keep = last_at_start(a, wsel, b0, b1, rs, pr.q, q0 + (uint32_t)(t + e) + 1,
+              const bool keep = last_at_start(a, p, pi, nwin, pr.q, q0 + (uint32_t)(t + e) + 1,
                                               pr.n, cs);
               if (e == 0)
                 in0 = keep;
@@ -513,9 +518,7 @@ __device__ __forceinline__ void gather_pair(const SearchArgs& a, const PairCurso
       }
     }
   } else {
-    const SearchedPair sp = gather_searched<H, FAST>(
-        a, __shfl_sync(kFull, pc.b0, pq), __shfl_sync(kFull, pc.b1, pq),
-        __shfl_sync(kFull, pc.wsel, pq), __shfl_sync(kFull, pc.wbase, pq), cs, C, lane, r, h);
+    const SearchedPair sp = gather_searched<H, FAST>(a, p, pi, nwin, cs, C, lane, r, h);
     r.n = uniform(sp.n);
     r.done = uniform(sp.done);
     k.read += sp.read;
@@ -638,21 +641,18 @@ __device__ __forceinline__ void load_pairs(const SearchArgs& a, int64_t p, int p
                                            int npairs, int lane, PairCursor& pc) {
   pc.pb = pi;
   const int pj = pi + lane;
-  pc.rs = pc.n = 0;
-  pc.b0 = pc.b1 = 0;
-  pc.wsel = 0;
-  pc.wbase = 0;
+  pc.q = 0;
+  pc.n = 0;
   if (pj < npairs) {
     const int fj = nwin == 1 ? pj : pj / nwin, wj = pj - fj * nwin;
     const int64_t fo = p * a.kf + fj;
-    pc.b0 = a.blo[fo];
-    pc.b1 = a.bhi[fo];
-    pc.wsel = a.wins[p * a.maxw + wj];
-    if (pc.b1 > pc.b0) {
-      const WinInfo w = a.win[pc.wsel];
-      pc.wbase = w.base;
-      pc.rs = __ldg(a.ss + w.ss_off + pc.b0);
-      pc.n = __ldg(a.ss + w.ss_off + pc.b1) - pc.rs;
+    const uint32_t b0 = a.blo[fo], b1 = a.bhi[fo];
+    const int wsel = a.wins[p * a.maxw + wj];
+    if (b1 > b0) {
+      const WinInfo w = a.win[wsel];
+      const uint32_t rs = __ldg(a.ss + w.ss_off + b0);
+      pc.q = w.base + rs;
+      pc.n = __ldg(a.ss + w.ss_off + b1) - rs;
     }
   }
 }
@@ -686,15 +686,15 @@ __device__ __forceinline__ void gather_row(const SearchArgs& a, int64_t p, int f
     const int q = pi - pc.pb;
     const Pair pr = pair_of(pc, q, lane);
     if (STATS) {
-      const uint32_t b0 = __shfl_sync(kFull, pc.b0, q), b1 = __shfl_sync(kFull, pc.b1, q);
-      if (b1 > b0) {
+      const PairBins pb = pair_bins(a, p, pi, nwin);
+      if (pb.b1 > pb.b0) {
         k.off += 2u;
         k.pairs += 1u;
-        k.bins1 += b1 - b0 + 1;
+        k.bins1 += pb.b1 - pb.b0 + 1;
       }
     }
     if (pr.n == 0) continue;
-    gather_pair<H, FAST, STATS>(a, pc, q, pr, pi == pc.pre_pi, cs, C, lane, stage, stage_p, r, h, k);
+    gather_pair<H, FAST, STATS>(a, p, pi, nwin, pr, pi == pc.pre_pi, cs, C, lane, stage, stage_p, r, h, k);
   }
   if (r.done < r.n) add_entries<H>(r, r.n - r.done, h, C, lane);
 }
@@ -829,7 +829,7 @@ __device__ __forceinline__ void flush_counters(const SearchArgs& a, const Counte
 // RT windows longer than kSmemMaxCycles; the code and every operation are the same.
 // STATS: the statistics pass's work counters (compiled in only for it).
 template <int H, bool FAST, bool GROW, bool STATS>
-__global__ void __launch_bounds__(LaunchShape<H, FAST, GROW>::threads, LaunchShape<H, FAST, GROW>::blocks)
+__global__ void __launch_bounds__(LaunchShape<GROW>::threads, LaunchShape<GROW>::blocks)
     search_kernel(const __grid_constant__ SearchArgs a) {
   extern __shared__ __align__(16) float smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
