@@ -936,8 +936,9 @@ int enqueue_search(AdsSelection* s, const AdsDia* d, const AdsLib* l, AdsCandida
   set_taps(&sa, s->kernel.data(), s->h, s->taps.p);
   sa.h = s->h;
   sa.k_out = k_out;
-  sa.gather_mode = s->o.gather_mode;
-  sa.scan_thresh = bf16 ? kScanThreshBf16 : kScanThreshFp32;
+  sa.scan_thresh = s->o.gather_mode == 1   ? 0xffffffffu
+                   : s->o.gather_mode == 2 ? 0u
+                                           : (bf16 ? kScanThreshBf16 : kScanThreshFp32);
   sa.err = c->err_p;
   sa.cand_n = s->cand_n.p;
   sa.cand_score = s->cand_score.p;
@@ -1696,7 +1697,6 @@ int select_noalloc(const AdsDia* d, const AdsLib* l, const AdsSelectionParams* p
   sa.h = h;
   sa.k_out = k_out;
   sa.c_max = (int)c_max;
-  sa.gather_mode = 0;
   sa.scan_thresh = kScanThreshFp32;
   sa.work = work;
   sa.err = flags;

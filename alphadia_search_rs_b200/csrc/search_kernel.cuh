@@ -47,8 +47,7 @@ struct SearchArgs {
   int h;
   int k_out;   // candidates kept per precursor
   int c_max;   // largest cycle range of the precursors this launch searches
-  int gather_mode;
-  int scan_thresh;
+  uint32_t scan_thresh;  // longest range that is scanned
   float* grow;  // per-warp working sets of a long-window launch (GROW), else null
   unsigned long long* work;
   int* err;
@@ -232,7 +231,7 @@ __device__ __forceinline__ void add_entries(RowList& r, int m, int h, int C, int
   if (act) again = (atomicOr(r.bm + (cell >> 5), bit) & bit) != 0u;
   if (act && !again) {
     // the segments holding outputs cell - h .. cell + h of the valid range
-    const int s0 = max(cell - h, h) / kSeg, s1 = min(cell + h, C - 1) / kSeg;
+    const int s0 = max(cell - h, h) / kSeg, s1 = min(cell + h, C - 1 - h) / kSeg;
     if (H > 0) {
       if (s1 >= s0) {  // at most (2H + 4) / 4 + 1 <= 10 segments: two words
         const unsigned long long mask = ((2ull << (s1 - s0)) - 1ull) << (s0 & 31);
@@ -351,17 +350,17 @@ __device__ __forceinline__ void stage_wait() {
   __syncwarp();
 }
 
+// Is a range of n entries scanned (else binary-searched, or empty)?
 __device__ __forceinline__ bool scans(const SearchArgs& a, uint32_t n) {
-  return a.gather_mode == 1 || (a.gather_mode == 0 && n <= (uint32_t)a.scan_thresh);
+  return n - 1u < a.scan_thresh;
 }
 
 // The CSR ranges of a precursor's (fragment, window) pairs, fetched 32 at a time
-// (lane q holds pair pb + q), and the pair whose first entries are staged.
+// (lane q holds pair pb + q).
 struct PairCursor {
-  int pb = -64;
+  int pb = 0;
   int64_t q = 0;   // absolute position of the pair's first entry
   uint32_t n = 0;  // entries
-  int pre_pi = -1;
 };
 
 // The pair in lane q of the cursor.
@@ -461,24 +460,23 @@ static __device__ __noinline__ SearchedPair gather_searched(const SearchArgs& a,
 // fill_xic_slice for the (fragment, window) pair pi of precursor p: its entries
 // inside the RT window are listed, in CSR order.  Two exact strategies: scan, which reads
 // every entry of the range and keeps start < cycle < stop plus, per bin, the last entry
-// at cycle == start; or, for long ranges, gather_searched.  `staged`: the range's first
-// kStageEntries entries are already on their way.
+// at cycle == start (`staged`: the range's first kStageEntries entries are already on
+// their way); or, for long ranges, gather_searched.
 template <int H, bool FAST, bool STATS>
 __device__ __forceinline__ void gather_pair(const SearchArgs& a, int64_t p, int pi, int nwin,
                                             Pair pr, bool staged, int cs, int C, int lane,
                                             uint32_t stage, const unsigned char* stage_p,
                                             RowList& r, int h, Counters<STATS>& k) {
-  if (scans(a, pr.n)) {
+  if (staged) {
     k.read += pr.n;
 #pragma unroll 1
     for (uint32_t q0 = 0; q0 < pr.n; q0 += kStageEntries) {
       const int m = (int)min(pr.n - q0, (uint32_t)kStageEntries);
       const int64_t q = pr.q + q0;
-      if (!staged) {
+      if (q0 > 0) {
         __syncwarp();  // the area's previous entries have been read
         stage_entries<FAST>(a, q, m, stage, lane);
       }
-      staged = false;
       stage_wait();
       // two consecutive entries per lane, from the even position at or below the first
       const int odd = (int)(q & 1);
@@ -657,46 +655,15 @@ __device__ __forceinline__ void load_pairs(const SearchArgs& a, int64_t p, int p
   }
 }
 
-// Starts staging pair pi's first entries (after the area's last ones have been read).
+// Starts staging a pair's first entries (after the area's last ones have been read).
 template <bool FAST>
-__device__ __forceinline__ void stage_pair(const SearchArgs& a, int64_t p, int pi, int nwin,
-                                           int npairs, int lane, PairCursor& pc, uint32_t stage) {
-  pc.pre_pi = -1;
-  if (pi >= npairs) return;
-  if (pi >= pc.pb + 32) load_pairs(a, p, pi, nwin, npairs, lane, pc);
-  const Pair pr = pair_of(pc, pi - pc.pb, lane);
-  if (pr.n > 0 && scans(a, pr.n)) {
+__device__ __forceinline__ bool stage_pair(const SearchArgs& a, Pair pr, int lane, uint32_t stage) {
+  const bool scan = scans(a, pr.n);
+  if (scan) {
     __syncwarp();
     stage_entries<FAST>(a, pr.q, (int)min(pr.n, (uint32_t)kStageEntries), stage, lane);
-    pc.pre_pi = pi;
   }
-}
-
-// Gathers fragment f's XIC row: its (fragment, window) pairs in window order (the
-// reference's DenseXICObservation::new, src/dense_xic_observation/mod.rs:30-64).
-template <int H, bool FAST, bool STATS>
-__device__ __forceinline__ void gather_row(const SearchArgs& a, int64_t p, int f, int nwin,
-                                           int npairs, int cs, int C, int lane, PairCursor& pc,
-                                           uint32_t stage, const unsigned char* stage_p, RowList& r,
-                                           int h, Counters<STATS>& k) {
-#pragma unroll 1
-  for (int wi = 0; wi < nwin; ++wi) {
-    const int pi = f * nwin + wi;
-    if (pi >= pc.pb + 32) load_pairs(a, p, pi, nwin, npairs, lane, pc);
-    const int q = pi - pc.pb;
-    const Pair pr = pair_of(pc, q, lane);
-    if (STATS) {
-      const PairBins pb = pair_bins(a, p, pi, nwin);
-      if (pb.b1 > pb.b0) {
-        k.off += 2u;
-        k.pairs += 1u;
-        k.bins1 += pb.b1 - pb.b0 + 1;
-      }
-    }
-    if (pr.n == 0) continue;
-    gather_pair<H, FAST, STATS>(a, p, pi, nwin, pr, pi == pc.pre_pi, cs, C, lane, stage, stage_p, r, h, k);
-  }
-  if (r.done < r.n) add_entries<H>(r, r.n - r.done, h, C, lane);
+  return scan;
 }
 
 // The last gathered row's cells (and bitmap words) back to zero.
@@ -859,6 +826,8 @@ __global__ void __launch_bounds__(LaunchShape<GROW>::threads, LaunchShape<GROW>:
     for (int i = lane; i < P.row_words / 4; i += 32) r4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
     for (int i = lane; i < P.bw; i += 32) bm[i] = 0u;
+#pragma unroll 1
+    for (int i = lane; i < P.sw; i += 32) segbits[i] = 0u;
   }
 
 #pragma unroll 1
@@ -897,28 +866,45 @@ __global__ void __launch_bounds__(LaunchShape<GROW>::threads, LaunchShape<GROW>:
     // fragment weights, lane f holding fragment f's (fetched once per precursor)
     const float wf_lane = lane < F ? __ldg(a.fw + p * a.kf + lane) : 0.0f;
     PairCursor pc;
-    // f = -1: only starts the first row's entries on their way
+    load_pairs(a, p, 0, nwin, npairs, lane, pc);
+    Pair next = pair_of(pc, 0, lane);
+    bool staged = stage_pair<FAST>(a, next, lane, stage);
 #pragma unroll 1
-    for (int f = -1; f < F; ++f) {
-      if (f >= 0) {
-        // ---- 1. gather: the fragment's pairs in window order
-        clear_row(r, row, P, lane);
-        gather_row<H, FAST, STATS>(a, p, f, nwin, npairs, cs, C, lane, pc, stage, stage_p, r, h, k);
-        k.acc += (unsigned int)r.n;
-      }
-      // the next fragment's first pair arrives while this row is convolved
-      stage_pair<FAST>(a, p, (f + 1) * nwin, nwin, npairs, lane, pc, stage);
-      if (f < 0) {
+    for (int i = lane; i < C; i += 32) score[i] = 0.0f;
+    int f = -1, wi = 0;
+    // pairs in fragment, then window order (the reference's DenseXICObservation::new,
+    // src/dense_xic_observation/mod.rs:30-64)
 #pragma unroll 1
-        for (int i = lane; i < C; i += 32) score[i] = 0.0f;
-        continue;
+    for (int pi = 0; pi < npairs; ++pi) {
+      // ---- 1. gather
+      if (STATS) {
+        const PairBins pb = pair_bins(a, p, pi, nwin);
+        if (pb.b1 > pb.b0) {
+          k.off += 2u;
+          k.pairs += 1u;
+          k.bins1 += pb.b1 - pb.b0 + 1;
+        }
       }
+      if (next.n > 0)
+        gather_pair<H, FAST, STATS>(a, p, pi, nwin, next, staged, cs, C, lane, stage, stage_p, r, h, k);
+      if (pi + 1 < npairs) {
+        // the next pair's entries arrive while this row is convolved
+        if (pi + 1 >= pc.pb + 32) load_pairs(a, p, pi + 1, nwin, npairs, lane, pc);
+        next = pair_of(pc, pi + 1 - pc.pb, lane);
+        staged = stage_pair<FAST>(a, next, lane, stage);
+      }
+      if (++wi < nwin) continue;  // more windows hold this fragment
+      wi = 0;
+      ++f;
+      k.acc += (unsigned int)r.n;
+      if (r.done < r.n) add_entries<H>(r, r.n - r.done, h, C, lane);
       __syncwarp();
       float wf = __shfl_sync(kFull, wf_lane, f & 31);
       if (f >= 32) wf = __ldg(a.fw + p * a.kf + f);
       if (!isfinite(wf)) {
         score_every_column<FAST>(a, r.row, kw_s, h, C, wf, score, lnt, lane);
         __syncwarp();
+        clear_row(r, row, P, lane);
         continue;
       }
       if (r.n == 0) continue;  // no entry accepted: every term is +0
@@ -931,8 +917,7 @@ __global__ void __launch_bounds__(LaunchShape<GROW>::threads, LaunchShape<GROW>:
       int nact = 0;
 #pragma unroll 1
       for (int w0 = 0; w0 < n_seg; w0 += 32) {
-        uint32_t x = segbits[w0 / 32];
-        if (w0 + 32 > n_seg) x &= 0xffffffffu >> (32 - (n_seg - w0));
+        const uint32_t x = segbits[w0 / 32];
         if ((x >> lane) & 1u) segs[nact + __popc(x & lt)] = (uint16_t)(w0 + lane);
         nact += __popc(x);
       }
@@ -1013,6 +998,7 @@ __global__ void __launch_bounds__(LaunchShape<GROW>::threads, LaunchShape<GROW>:
         }
         __syncwarp();
       }
+      clear_row(r, row, P, lane);
     }
     __syncwarp();
 
