@@ -275,6 +275,33 @@ struct WinInfo {
   int64_t ss_off;    // element offset of its slice_starts, -1 if it holds no peaks
 };
 
+// The non-empty windows that hold an m/z, by lookup: the m distinct window limits v
+// (ascending) cut the axis into 2m + 1 classes, the limits themselves (2i + 1) and what lies
+// below (2i) or above them (2m); class k's windows are list[off[k]] .. list[off[k + 1] - 1],
+// in window order.
+struct WinIndex {
+  const float* v = nullptr;
+  const int* off = nullptr;
+  const int* list = nullptr;
+  int m = 0;
+};
+
+__device__ __forceinline__ void find_windows(const WinIndex& w, float x, int* off, int* len) {
+  *off = *len = 0;
+  if (!(x == x)) return;  // NaN lies in no window
+  int lo = 0, hi = w.m;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (__ldg(w.v + mid) < x)
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  const int k = lo < w.m && __ldg(w.v + lo) == x ? 2 * lo + 1 : 2 * lo;
+  *off = __ldg(w.off + k);
+  *len = __ldg(w.off + k + 1) - *off;
+}
+
 }  // namespace ads
 
 // Elements a run's entry arrays are allocated past their last entry: the search copies
@@ -297,6 +324,14 @@ struct AdsDia {
   bool bf16_only = false;              // f32 intensities released (ads_dia_keep_bf16_only)
   int64_t n_entries = 0;
   int max_overlap = 0;                 // max number of non-empty windows covering one m/z
+  ads::DevBuf<int> win_index_dev;      // WinIndex: v, off, list
+  int win_index_m = 0;
+  bool win_index_ok = false;           // false: too many overlaps to list (windows are scanned)
+  ads::WinIndex win_index() const {
+    const int* p = win_index_dev.p;
+    return ads::WinIndex{reinterpret_cast<const float*>(p), p + win_index_m, p + 3 * win_index_m + 2,
+                         win_index_m};
+  }
   std::vector<float> rt;               // MS1 retention times (RT index)
   float delta_t = 1.0f;
   ads::DevBuf<float> rt_dev;

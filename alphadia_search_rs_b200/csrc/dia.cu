@@ -194,6 +194,46 @@ int build_entries(AdsDia* d, const AdsRawArrays* raw, const std::vector<int32_t>
   return ADS_OK;
 }
 
+// The run's WinIndex on the device.  Left out (windows are then scanned) where its lists
+// would exceed kWinIndexMax entries: thousands of windows all over one another.
+constexpr size_t kWinIndexMax = size_t(1) << 22;
+
+int build_win_index(AdsDia* d) {
+  std::vector<float> v;
+  std::vector<int> open;
+  for (int64_t w = 0; w < d->n_obs; ++w) {
+    const WinInfo& wi = d->win[w];
+    if (wi.ss_off < 0 || !(wi.lo <= wi.hi)) continue;  // holds no peaks, or no m/z
+    v.push_back(wi.lo);
+    v.push_back(wi.hi);
+    open.push_back((int)w);
+  }
+  std::sort(v.begin(), v.end());
+  v.erase(std::unique(v.begin(), v.end()), v.end());
+  const int m = (int)v.size();
+  auto at = [&](float x) { return (int)(std::lower_bound(v.begin(), v.end(), x) - v.begin()); };
+  // windows hold the classes from their lower limit's to their upper limit's
+  std::vector<int> off(2 * (size_t)m + 2, 0);
+  size_t total = 0;
+  for (int w : open) total += 2 * (size_t)(at(d->win[w].hi) - at(d->win[w].lo)) + 1;
+  if (total > kWinIndexMax) return ADS_OK;
+  for (int w : open)
+    for (int k = 2 * at(d->win[w].lo) + 1; k <= 2 * at(d->win[w].hi) + 1; ++k) ++off[k + 1];
+  for (size_t k = 1; k < off.size(); ++k) off[k] += off[k - 1];
+  std::vector<int> cur(off.begin(), off.end() - 1), list(total);
+  for (int w : open)  // ascending, so every class's list is in window order
+    for (int k = 2 * at(d->win[w].lo) + 1; k <= 2 * at(d->win[w].hi) + 1; ++k) list[cur[k]++] = w;
+  std::vector<int> host(3 * (size_t)m + 2 + total);
+  if (m) std::memcpy(host.data(), v.data(), (size_t)m * 4);
+  std::copy(off.begin(), off.end(), host.begin() + m);
+  std::copy(list.begin(), list.end(), host.begin() + 3 * (size_t)m + 2);
+  ADS_TRY(d->win_index_dev.alloc(host.size()));
+  ADS_CUDA(cudaMemcpy(d->win_index_dev.p, host.data(), host.size() * 4, cudaMemcpyHostToDevice));
+  d->win_index_m = m;
+  d->win_index_ok = true;
+  return ADS_OK;
+}
+
 int dia_create(const AdsRawArrays* raw, int device, AdsDia** out) {
   if (!raw || !out) return fail(ADS_ERR_INVALID_ARGUMENT, "null argument");
   *out = nullptr;
@@ -348,6 +388,7 @@ int dia_create(const AdsRawArrays* raw, int device, AdsDia** out) {
   ADS_TRY(d->win_dev.alloc(std::max<int64_t>(n_obs, 1)));
   if (n_obs)
     ADS_CUDA(cudaMemcpy(d->win_dev.p, d->win.data(), n_obs * sizeof(WinInfo), cudaMemcpyHostToDevice));
+  ADS_TRY(build_win_index(d));
   ADS_TRY(d->rt_dev.alloc(std::max<int64_t>(n_rt, 1)));
   if (n_rt) ADS_CUDA(cudaMemcpy(d->rt_dev.p, d->rt.data(), n_rt * 4, cudaMemcpyHostToDevice));
   // copies from pageable memory may return before their DMA ends; searches read these

@@ -102,6 +102,7 @@ struct ScoreArgs {
   float idf_total;
   const WinInfo* win;
   int n_obs;
+  WinIndex wi;  // (with kBlock kernels) windows by precursor m/z
   const uint32_t* ss;
   const uint16_t* cyc;
   const float* inten;
@@ -131,6 +132,7 @@ int64_t scratch_words(int Fm, int Fraw, int Cm) {
 
 // One thread's view of the interleaved scratch.
 struct Scr {
+  typedef int64_t I;
   uint32_t* base;
   int64_t T, t;
   __device__ float f(int64_t e) const { return __uint_as_float(base[e * T + t]); }
@@ -157,18 +159,20 @@ __device__ __forceinline__ int64_t bsearch_u16_rust(const uint16_t* a, int64_t n
 }
 
 // Iterator::sum on f32 (Rust 1.88): a left fold from -0.0.
-__device__ float rust_sum(const Scr& s, int64_t e0, int64_t n) {
+template <class M>
+__device__ float rust_sum(const M& s, typename M::I e0, typename M::I n) {
   float acc = -0.0f;
-  for (int64_t i = 0; i < n; ++i) acc = __fadd_rn(acc, s.f(e0 + i));
+  for (typename M::I i = 0; i < n; ++i) acc = __fadd_rn(acc, s.f(e0 + i));
   return acc;
 }
 
 // ndarray 0.16 numeric_util::unrolled_fold with A::add (ArrayBase::sum of a
 // contiguous row, as sum_axis(Axis(1)) uses it).
-__device__ float ndarray_sum(const Scr& s, int64_t e0, int64_t n) {
+template <class M>
+__device__ float ndarray_sum(const M& s, typename M::I e0, typename M::I n) {
   float acc = 0.0f;
   float p[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  int64_t i = 0;
+  typename M::I i = 0;
   for (; n - i >= 8; i += 8)
 #pragma unroll
     for (int k = 0; k < 8; ++k) p[k] = __fadd_rn(p[k], s.f(e0 + i + k));
@@ -176,18 +180,19 @@ __device__ float ndarray_sum(const Scr& s, int64_t e0, int64_t n) {
   acc = __fadd_rn(acc, __fadd_rn(p[1], p[5]));
   acc = __fadd_rn(acc, __fadd_rn(p[2], p[6]));
   acc = __fadd_rn(acc, __fadd_rn(p[3], p[7]));
-  for (int64_t k = 0; i + k < n && k < 7; ++k) acc = __fadd_rn(acc, s.f(e0 + i + k));
+  for (typename M::I k = 0; i + k < n && k < 7; ++k) acc = __fadd_rn(acc, s.f(e0 + i + k));
   return acc;
 }
 
 // src/peak_group_scoring/utils.rs:126-172 over scratch vectors
-__device__ float correlation_safe(const Scr& s, int64_t ex, int64_t ey, int64_t n) {
+template <class M>
+__device__ float correlation_safe(const M& s, typename M::I ex, typename M::I ey, typename M::I n) {
   if (n == 0) return 0.0f;
   const float xs = rust_sum(s, ex, n), ys = rust_sum(s, ey, n);
   if (xs == 0.0f || ys == 0.0f) return 0.0f;
   const float xm = __fdiv_rn(xs, (float)n), ym = __fdiv_rn(ys, (float)n);
   float xv = 0.0f, yv = 0.0f, cv = 0.0f;
-  for (int64_t i = 0; i < n; ++i) {
+  for (typename M::I i = 0; i < n; ++i) {
     const float dx = __fsub_rn(s.f(ex + i), xm), dy = __fsub_rn(s.f(ey + i), ym);
     xv = __fadd_rn(xv, __fmul_rn(dx, dx));
     yv = __fadd_rn(yv, __fmul_rn(dy, dy));
@@ -205,26 +210,28 @@ struct XStats {
   float xs, xm, xv;
 };
 
-__device__ XStats x_stats(const Scr& s, int64_t ex, int64_t n) {
+template <class M>
+__device__ XStats x_stats(const M& s, typename M::I ex, typename M::I n) {
   XStats r{0.0f, 0.0f, 0.0f};
   if (n == 0) return r;
   r.xs = rust_sum(s, ex, n);
   r.xm = __fdiv_rn(r.xs, (float)n);
-  for (int64_t i = 0; i < n; ++i) {
+  for (typename M::I i = 0; i < n; ++i) {
     const float dx = __fsub_rn(s.f(ex + i), r.xm);
     r.xv = __fadd_rn(r.xv, __fmul_rn(dx, dx));
   }
   return r;
 }
 
-__device__ float correlation_fixed_x(const Scr& s, const XStats& X, int64_t ex, int64_t ey,
-                                     int64_t n) {
+template <class M>
+__device__ float correlation_fixed_x(const M& s, const XStats& X, typename M::I ex, typename M::I ey,
+                                     typename M::I n) {
   if (n == 0) return 0.0f;
   const float ys = rust_sum(s, ey, n);
   if (X.xs == 0.0f || ys == 0.0f) return 0.0f;
   const float ym = __fdiv_rn(ys, (float)n);
   float yv = 0.0f, cv = 0.0f;
-  for (int64_t i = 0; i < n; ++i) {
+  for (typename M::I i = 0; i < n; ++i) {
     const float dx = __fsub_rn(s.f(ex + i), X.xm), dy = __fsub_rn(s.f(ey + i), ym);
     yv = __fadd_rn(yv, __fmul_rn(dy, dy));
     cv = __fadd_rn(cv, __fmul_rn(dx, dy));
@@ -236,10 +243,11 @@ __device__ float correlation_fixed_x(const Scr& s, const XStats& X, int64_t ex, 
 }
 
 // Stable ascending insertion sort of n floats at e0 (slice::sort_by(partial_cmp)).
-__device__ void sort_floats(const Scr& s, int64_t e0, int64_t n) {
-  for (int64_t i = 1; i < n; ++i) {
+template <class M>
+__device__ void sort_floats(const M& s, typename M::I e0, typename M::I n) {
+  for (typename M::I i = 1; i < n; ++i) {
     const float v = s.f(e0 + i);
-    int64_t j = i;
+    typename M::I j = i;
     while (j > 0 && v < s.f(e0 + j - 1)) {
       s.sf(e0 + j, s.f(e0 + j - 1));
       --j;
@@ -249,21 +257,23 @@ __device__ void sort_floats(const Scr& s, int64_t e0, int64_t n) {
 }
 
 // src/utils/mod.rs:120-143 (v copied into the sort buffer first)
-__device__ float median_of(const Scr& s, int64_t ev, int64_t n, int64_t etmp) {
+template <class M>
+__device__ float median_of(const M& s, typename M::I ev, typename M::I n, typename M::I etmp) {
   if (n == 0) return 0.0f;
-  for (int64_t i = 0; i < n; ++i) s.sf(etmp + i, s.f(ev + i));
+  for (typename M::I i = 0; i < n; ++i) s.sf(etmp + i, s.f(ev + i));
   sort_floats(s, etmp, n);
-  const int64_t mid = n / 2;
+  const typename M::I mid = n / 2;
   return n % 2 == 0 ? __fdiv_rn(__fadd_rn(s.f(etmp + mid - 1), s.f(etmp + mid)), 2.0f)
                     : s.f(etmp + mid);
 }
 
 // src/utils/mod.rs:146-173
-__device__ float std_of(const Scr& s, int64_t ev, int64_t n) {
+template <class M>
+__device__ float std_of(const M& s, typename M::I ev, typename M::I n) {
   if (n < 2) return 0.0f;
   const float mean = __fdiv_rn(rust_sum(s, ev, n), (float)n);
   float acc = -0.0f;
-  for (int64_t i = 0; i < n; ++i) {
+  for (typename M::I i = 0; i < n; ++i) {
     const float d = __fsub_rn(s.f(ev + i), mean);
     acc = __fadd_rn(acc, __fmul_rn(d, d));
   }
@@ -275,12 +285,13 @@ __device__ float std_of(const Scr& s, int64_t ev, int64_t n) {
 // unordered pairs go to the lower index) plus the later elements above it.  The two
 // halves are separate loops: nvcc 12.9 at -O3 dropped the tie term of the one-loop
 // form `(w > v) || (!(w < v) && !(w > v) && j < i)` (every tie ranked 0).
-__device__ void ranked_mask(const Scr& s, int64_t ev, int64_t n, int r1, int r2, int64_t em) {
-  for (int64_t i = 0; i < n; ++i) {
+template <class M>
+__device__ void ranked_mask(const M& s, typename M::I ev, typename M::I n, int r1, int r2, typename M::I em) {
+  for (typename M::I i = 0; i < n; ++i) {
     const float v = s.f(ev + i);
-    int64_t rank = 0;
-    for (int64_t j = 0; j < i; ++j) rank += !(s.f(ev + j) < v);
-    for (int64_t j = i + 1; j < n; ++j) rank += s.f(ev + j) > v;
+    typename M::I rank = 0;
+    for (typename M::I j = 0; j < i; ++j) rank += !(s.f(ev + j) < v);
+    for (typename M::I j = i + 1; j < n; ++j) rank += s.f(ev + j) > v;
     s.su(em + i, (rank >= r1 && rank < r2) ? 1u : 0u);
   }
 }
@@ -295,43 +306,51 @@ __device__ float gamma_ln(float x) {
   return __fadd_rn(__fsub_rn(__fmul_rn(__fsub_rn(x, 0.5f), ln_rn(x)), x), __fmul_rn(0.5f, ln_2pi));
 }
 
-// src/peak_group_scoring/utils.rs:193-279 (ew < 0: weights 1.0)
-__device__ float hyperscore(const Scr& s, int64_t etype, int64_t eint, int64_t emask, int64_t ew,
-                            int64_t n) {
+// src/peak_group_scoring/utils.rs:193-279: the sums over b and y fragments
+struct HyperSums {
   uint32_t nb = 0, ny = 0;
   float sb = 0.0f, sy = 0.0f;
-  for (int64_t i = 0; i < n; ++i) {
-    const float v = s.f(eint + i);
-    if (!s.u(emask + i) || v == 0.0f) continue;
-    const float wi = __fmul_rn(v, ew >= 0 ? s.f(ew + i) : 1.0f);
-    const uint32_t t = s.u(etype + i);
-    if (t == 98) {
+  __device__ void add(uint32_t type, float wi) {
+    if (type == 98) {
       ++nb;
       sb = __fadd_rn(sb, wi);
-    } else if (t == 121) {
+    } else if (type == 121) {
       ++ny;
       sy = __fadd_rn(sy, wi);
     }
   }
-  if (nb == 0 && ny == 0) return 0.0f;
-  const float fb = nb > 0 ? gamma_ln(__fadd_rn((float)nb, 1.0f)) : 0.0f;
-  const float fy = ny > 0 ? gamma_ln(__fadd_rn((float)ny, 1.0f)) : 0.0f;
-  const float lb = sb > 0.0f ? ln_rn(sb) : 0.0f;
-  const float ly = sy > 0.0f ? ln_rn(sy) : 0.0f;
-  const float h = __fadd_rn(__fadd_rn(__fadd_rn(fb, fy), lb), ly);
-  return isfinite(h) ? h : 0.0f;
+  __device__ float value() const {
+    if (nb == 0 && ny == 0) return 0.0f;
+    const float fb = nb > 0 ? gamma_ln(__fadd_rn((float)nb, 1.0f)) : 0.0f;
+    const float fy = ny > 0 ? gamma_ln(__fadd_rn((float)ny, 1.0f)) : 0.0f;
+    const float lb = sb > 0.0f ? ln_rn(sb) : 0.0f;
+    const float ly = sy > 0.0f ? ln_rn(sy) : 0.0f;
+    const float h = __fadd_rn(__fadd_rn(__fadd_rn(fb, fy), lb), ly);
+    return isfinite(h) ? h : 0.0f;
+  }
+};
+
+// (ew < 0: weights 1.0)
+template <class M>
+__device__ float hyperscore(const M& s, typename M::I etype, typename M::I eint, typename M::I emask,
+                            typename M::I ew, typename M::I n) {
+  HyperSums h;
+  for (typename M::I i = 0; i < n; ++i) {
+    const float v = s.f(eint + i);
+    if (!s.u(emask + i) || v == 0.0f) continue;
+    h.add(s.u(etype + i), __fmul_rn(v, ew >= 0 ? s.f(ew + i) : 1.0f));
+  }
+  return h.value();
 }
 
-// src/peak_group_scoring/utils.rs:314-372 for one series (numbers sorted in etmp)
-__device__ uint32_t longest_series(const Scr& s, int64_t etype, int64_t enum_, int64_t emask,
-                                   int64_t n, uint32_t type, int64_t etmp) {
-  int64_t m = 0;
-  for (int64_t i = 0; i < n; ++i)
-    if (s.u(emask + i) && s.u(etype + i) == type) s.su(etmp + m++, s.u(enum_ + i));
+// src/peak_group_scoring/utils.rs:314-372: the longest run of the m numbers at etmp, which
+// are sorted there
+template <class M>
+__device__ uint32_t longest_run(const M& s, typename M::I etmp, typename M::I m) {
   if (m == 0) return 0;
-  for (int64_t i = 1; i < m; ++i) {  // sort_unstable: any order of equal numbers
+  for (typename M::I i = 1; i < m; ++i) {  // sort_unstable: any order of equal numbers
     const uint32_t v = s.u(etmp + i);
-    int64_t j = i;
+    typename M::I j = i;
     while (j > 0 && v < s.u(etmp + j - 1)) {
       s.su(etmp + j, s.u(etmp + j - 1));
       --j;
@@ -339,7 +358,7 @@ __device__ uint32_t longest_series(const Scr& s, int64_t etype, int64_t enum_, i
     s.su(etmp + j, v);
   }
   uint32_t mx = 1, cur = 1;  // u8 arithmetic of the reference: wraps
-  for (int64_t i = 1; i < m; ++i) {
+  for (typename M::I i = 1; i < m; ++i) {
     if (s.u(etmp + i) == ((s.u(etmp + i - 1) + 1u) & 0xFFu)) {
       cur = (cur + 1u) & 0xFFu;
       mx = max(mx, cur);
@@ -348,6 +367,17 @@ __device__ uint32_t longest_series(const Scr& s, int64_t etype, int64_t enum_, i
     }
   }
   return mx;
+}
+
+// One series.
+template <class M>
+__device__ uint32_t longest_series(const M& s, typename M::I etype, typename M::I enum_,
+                                   typename M::I emask, typename M::I n, uint32_t type,
+                                   typename M::I etmp) {
+  typename M::I m = 0;
+  for (typename M::I i = 0; i < n; ++i)
+    if (s.u(emask + i) && s.u(etype + i) == type) s.su(etmp + m++, s.u(enum_ + i));
+  return longest_run(s, etmp, m);
 }
 
 // Sort key of each candidate for the work order: its precursor's library fragment count
@@ -886,6 +916,8 @@ __global__ void __launch_bounds__(kScoreBlock) quant_kernel(QuantArgs qa) {
   }
 }
 
+#include "score_block.cuh"
+
 // SpecLibFlatQuantified::from_precursor_quantified_vec (src/speclib_flat_quantified/mod.rs:
 // 212-333), step 1: the kept candidates' precursor rows (candidate order, not yet sorted)
 // and their fragments, flat in candidate order.
@@ -1017,6 +1049,26 @@ int quant_assemble(AdsQuant* r, const uint64_t* d_off, const int* d_pos, cudaStr
   return ADS_OK;
 }
 
+// The candidates a block of score_block_kernel takes, or 0 where the per-candidate kernels
+// run: candidates of so many fragments or cycles that fewer than 4 fit a block's shared
+// memory (whole-run cycle ranges), or a run without a window index.
+int block_group(const AdsDia* d, const BlockPlan& b, int64_t C) {
+  if (!d->win_index_ok || C > 4096) return 0;
+  int group = kGroup;
+  while (group > 4 && block_smem_bytes(b, group) > kBlockSmem) group /= 2;
+  return block_smem_bytes(b, group) <= kBlockSmem ? group : 0;
+}
+
+template <bool QUANT>
+int launch_block(const QuantArgs& qa, const BlockPlan& b, int group, cudaStream_t st) {
+  const size_t smem = block_smem_bytes(b, group);
+  ADS_CUDA(cudaFuncSetAttribute(score_block_kernel<QUANT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)smem));
+  score_block_kernel<QUANT><<<(int)((qa.s.n + group - 1) / group), kBlockThreads, smem, st>>>(qa, b, group);
+  ADS_LAUNCH_CHECK();
+  return ADS_OK;
+}
+
 // The library's IDF histogram, built once per library on the device.
 int ensure_idf(AdsLib* l, const GridView& g, cudaStream_t st) {
   std::lock_guard<std::mutex> lk(l->mu);
@@ -1072,15 +1124,21 @@ int score_device(const AdsScoringParams* p, const AdsDia* d, AdsLib* l, int64_t 
     const int Fm = (int)std::max<int64_t>(1, std::min<int64_t>(p->top_k_fragments, l->max_frag));
     const int Fraw = (int)std::max<int64_t>(1, l->max_frag);
     const int Cm = (int)std::max<int64_t>(1, c_max);
-    const int64_t words = scratch_words(Fm, Fraw, Cm);
-    int n_sm = 0;
-    ADS_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, d->device));
-    int64_t T = std::min<int64_t>(n, (int64_t)n_sm * 16 * kScoreBlock);
-    T = std::max<int64_t>(1, std::min<int64_t>(T, ((int64_t)1 << 28) / words));  // <= 1 GiB
+    const BlockPlan plan = block_plan(Fm, Fraw, Cm);
+    const int group = block_group(d, plan, c_max);
+    int64_t T = 0;
     DevBuf<uint32_t> scratch;
-    ADS_TRY(scratch.alloc((size_t)(T * words)));
-    ScoreArgs a;
-    std::memset(&a, 0, sizeof(a));
+    if (group == 0) {
+      const int64_t words = scratch_words(Fm, Fraw, Cm);
+      int n_sm = 0;
+      ADS_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, d->device));
+      T = std::min<int64_t>(n, (int64_t)n_sm * 16 * kScoreBlock);
+      T = std::max<int64_t>(1, std::min<int64_t>(T, ((int64_t)1 << 28) / words));  // <= 1 GiB
+      ADS_TRY(scratch.alloc((size_t)(T * words)));
+    }
+    QuantArgs qa;
+    std::memset(&qa, 0, sizeof(qa));
+    ScoreArgs& a = qa.s;
     a.n = n;
     a.c_pidx = pidx;
     a.c_rank = rank;
@@ -1104,6 +1162,7 @@ int score_device(const AdsScoringParams* p, const AdsDia* d, AdsLib* l, int64_t 
     a.idf_total = l->idf_total >= 0.0f ? l->idf_total : (float)l->n_frag;
     a.win = d->win_dev.p;
     a.n_obs = (int)d->n_obs;
+    a.wi = d->win_index();
     a.ss = d->slice_starts.p;
     a.cyc = d->cycles.p;
     a.inten = d->intens.p;
@@ -1127,7 +1186,9 @@ int score_device(const AdsScoringParams* p, const AdsDia* d, AdsLib* l, int64_t 
     ADS_CUDA(cudaEventCreate(&ev.a));
     ADS_CUDA(cudaEventCreate(&ev.b));
     ADS_CUDA(cudaEventRecord(ev.a, st));
-    if (a.order)
+    if (group > 0)
+      ADS_TRY(launch_block<false>(qa, plan, group, st));
+    else if (a.order)
       score_kernel<true><<<(int)((T + kScoreBlock - 1) / kScoreBlock), kScoreBlock, 0, st>>>(a);
     else
       score_kernel<false><<<(int)((T + kScoreBlock - 1) / kScoreBlock), kScoreBlock, 0, st>>>(a);
@@ -1215,13 +1276,18 @@ int quant_device(const AdsQuantParams* p, const AdsDia* d, AdsLib* l, int64_t n,
   if (n > 0) {
     ADS_CUDA(cudaMemcpyAsync(r->pidx_p, pidx, (size_t)n * 8, cudaMemcpyDeviceToDevice, st));
     ADS_CUDA(cudaMemcpyAsync(r->rank_p, rank, (size_t)n * 8, cudaMemcpyDeviceToDevice, st));
-    const int64_t words = scratch_words(Fm, Fraw, Cm);
-    int n_sm = 0;
-    ADS_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, d->device));
-    int64_t T = std::min<int64_t>(n, (int64_t)n_sm * 16 * kScoreBlock);
-    T = std::max<int64_t>(1, std::min<int64_t>(T, ((int64_t)1 << 28) / words));  // <= 1 GiB
+    const BlockPlan plan = block_plan(Fm, Fraw, Cm);
+    const int group = block_group(d, plan, c_max);
+    int64_t T = 0;
     DevBuf<uint32_t> scratch;
-    ADS_TRY(scratch.alloc((size_t)(T * words)));
+    if (group == 0) {
+      const int64_t words = scratch_words(Fm, Fraw, Cm);
+      int n_sm = 0;
+      ADS_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, d->device));
+      T = std::min<int64_t>(n, (int64_t)n_sm * 16 * kScoreBlock);
+      T = std::max<int64_t>(1, std::min<int64_t>(T, ((int64_t)1 << 28) / words));  // <= 1 GiB
+      ADS_TRY(scratch.alloc((size_t)(T * words)));
+    }
     QuantArgs qa;
     std::memset(&qa, 0, sizeof(qa));
     ScoreArgs& a = qa.s;
@@ -1243,6 +1309,7 @@ int quant_device(const AdsQuantParams* p, const AdsDia* d, AdsLib* l, int64_t n,
     a.l_ftype = l->ftype_p;
     a.win = d->win_dev.p;
     a.n_obs = (int)d->n_obs;
+    a.wi = d->win_index();
     a.ss = d->slice_starts.p;
     a.cyc = d->cycles.p;
     a.inten = d->intens.p;
@@ -1278,7 +1345,9 @@ int quant_device(const AdsQuantParams* p, const AdsDia* d, AdsLib* l, int64_t n,
     ADS_CUDA(cudaEventCreate(&ev.a));
     ADS_CUDA(cudaEventCreate(&ev.b));
     ADS_CUDA(cudaEventRecord(ev.a, st));
-    if (qa.s.order)
+    if (group > 0)
+      ADS_TRY(launch_block<true>(qa, plan, group, st));
+    else if (qa.s.order)
       quant_kernel<true><<<(int)((T + kScoreBlock - 1) / kScoreBlock), kScoreBlock, 0, st>>>(qa);
     else
       quant_kernel<false><<<(int)((T + kScoreBlock - 1) / kScoreBlock), kScoreBlock, 0, st>>>(qa);

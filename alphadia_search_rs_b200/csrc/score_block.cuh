@@ -1,0 +1,579 @@
+// The block kernel of scoring and quantification: a block of 4 warps takes kGroup
+// candidates through the steps of score_kernel / quant_kernel with one thread per
+// (candidate, fragment), per (candidate, cycle) or per candidate, whatever the step is
+// made of, and everything in shared memory.  Included by score.cu inside namespace
+// ads::{anonymous}; every f32 operation is that of the per-candidate kernels, in their
+// order, through the same helpers.
+//
+// What bounds it: instruction issue.  A thread per candidate (score_kernel) ran 8 of 32
+// lanes per instruction on matrices in a global scratch, and walked every bin of every
+// fragment with a binary search.  Here a row's whole range of entries is read 8 cycle
+// indices at a time, and only an entry inside the window looks up its bin.
+constexpr int kGroup = 32;       // candidates of a block (at most: one lane each)
+constexpr int kBlockWarps = 4;
+constexpr int kBlockThreads = 32 * kBlockWarps;
+// A candidate's shared memory grows with fragments x cycles; beyond this many bytes a block
+// the group is halved, and below 4 candidates the per-candidate kernels run instead.
+constexpr size_t kBlockSmem = 74 * 1024;
+
+// Vectors of one candidate, in words.
+struct BlockPlan {
+  int Fm, Cm;      // most kept fragments, most cycles
+  int Fraw;        // most library fragments
+  int cs;          // row stride of the profiles (odd: rows of consecutive lanes hit different banks)
+  int fmz, fint, idf, tn, obs, corr, err, flag;  // per fragment
+  int med, medf;   // per cycle
+  int prof;        // profiles, before them the raw fragments, after them sort space
+  int words;       // of one candidate (odd)
+  int scratch;     // words of one thread's column or row buffer
+};
+
+__host__ __device__ inline BlockPlan block_plan(int Fm, int Fraw, int Cm) {
+  BlockPlan b;
+  b.Fm = Fm;
+  b.Cm = Cm;
+  b.Fraw = Fraw;
+  b.cs = Cm | 1;
+  int o = 0;
+  b.fmz = o;
+  o += Fm;
+  b.fint = o;
+  o += Fm;
+  b.idf = o;
+  o += Fm;
+  b.tn = o;
+  o += Fm;
+  b.obs = o;
+  o += Fm;
+  b.corr = o;
+  o += Fm;
+  b.err = o;
+  o += Fm;
+  b.flag = o;
+  o += Fm;
+  b.med = o;
+  o += Cm;
+  b.medf = o;
+  o += Cm;
+  b.prof = o;
+  int pw = Fm * b.cs;
+  if (pw < 3 * Fraw) pw = 3 * Fraw;
+  if (pw < 2 * Fm) pw = 2 * Fm;
+  o += pw;
+  b.words = o | 1;
+  b.scratch = Fm > Cm ? Fm : Cm;
+  return b;
+}
+
+// What a block knows of a candidate.
+struct BlockCand {
+  int64_t q;       // its index
+  int64_t fs;      // first library fragment
+  int64_t prec;    // row of its precursor
+  int nraw, F, cs, C;
+  int woff, wlen;  // windows that hold its precursor m/z
+  int nz;          // kept fragments whose profile is not all zero
+  float pmz;
+};
+
+inline size_t block_smem_bytes(const BlockPlan& b, int group) {
+  return (size_t)group * sizeof(BlockCand) + 4 * ((size_t)group * b.words + (size_t)kBlockThreads * b.scratch);
+}
+
+// Words of one candidate, for the shared helpers.
+struct SmVec {
+  typedef int I;
+  uint32_t* base;
+  __device__ float f(int e) const { return __uint_as_float(base[e]); }
+  __device__ void sf(int e, float v) const { base[e] = __float_as_uint(v); }
+  __device__ uint32_t u(int e) const { return base[e]; }
+  __device__ void su(int e, uint32_t v) const { base[e] = v; }
+};
+// One thread's buffer, interleaved across the block's threads.
+struct ThreadVec {
+  typedef int I;
+  uint32_t* base;  // of the thread
+  __device__ float f(int e) const { return __uint_as_float(base[e * kBlockThreads]); }
+  __device__ void sf(int e, float v) const { base[e * kBlockThreads] = __float_as_uint(v); }
+  __device__ uint32_t u(int e) const { return base[e * kBlockThreads]; }
+  __device__ void su(int e, uint32_t v) const { base[e * kBlockThreads] = v; }
+};
+
+// Bin of the window's entry at relative position q, searched in [b, b1).
+__device__ __forceinline__ uint32_t bin_of(const uint32_t* ssw, uint32_t b, uint32_t b1, uint32_t q) {
+  uint32_t lo = b, hi = b1;  // the last bin whose first entry is at or before q
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (__ldg(ssw + mid) <= q)
+      lo = mid;
+    else
+      hi = mid;
+  }
+  return lo;
+}
+
+// One fragment's row of gather_xic_mz: dense XIC (x) and intensity-weighted m/z (z) over
+// cycles [cs, cs + C).
+template <class X, class Z>
+__device__ __forceinline__ void gather_one(const ScoreArgs& a, const X& x, int x0, const Z& z,
+                                           float mz, int cs, int C, int woff, int wlen) {
+  for (int j = 0; j < C; ++j) {
+    x.sf(x0 + j, 0.0f);
+    z.sf(j, 0.0f);
+  }
+  if (C <= 0) return;
+  const float delta = __fmul_rn(__fmul_rn(mz, a.tol), 1e-6f);
+  const uint32_t b0 = grid_lower_bound(a.g, __fsub_rn(mz, delta));
+  const uint32_t b1 = max(b0, grid_upper_bound(a.g, __fadd_rn(mz, delta)));
+  if (b1 <= b0) return;
+  for (int w = 0; w < wlen; ++w) {
+    const WinInfo wi = a.win[__ldg(a.wi.list + woff + w)];
+    const uint32_t* ssw = a.ss + wi.ss_off;
+    const uint32_t r0 = __ldg(ssw + b0), r1 = __ldg(ssw + b1);
+    uint32_t b = b0;
+    // 8 cycle indices at a time from the 16-byte boundary at or below the first entry
+    // (the arrays are allocated kEntrySlack entries past the last one)
+    const int64_t q0 = wi.base + r0, q1 = wi.base + r1;
+#pragma unroll 4
+    for (int64_t c8 = q0 >> 3; c8 < (q1 + 7) >> 3; ++c8) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(a.cyc) + c8);
+      const uint32_t word[4] = {v.x, v.y, v.z, v.w};
+      uint32_t in = 0;
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        in |= (uint32_t)((unsigned)((int)(word[h] & 0xffffu) - cs) < (unsigned)C) << (2 * h);
+        in |= (uint32_t)((unsigned)((int)(word[h] >> 16) - cs) < (unsigned)C) << (2 * h + 1);
+      }
+      const int64_t at = c8 << 3;
+      if (at < q0) in &= 0xffu << (int)(q0 - at);
+      if (at + 8 > q1) in &= 0xffu >> (int)(at + 8 - q1);
+      while (in) {
+        const int h = __ffs(in) - 1;
+        in &= in - 1;
+        const int64_t q = at + h;
+        const uint32_t r = (uint32_t)(q - wi.base);
+        const int c = (int)__ldg(a.cyc + q);
+        b = bin_of(ssw, b, b1, r);
+        // Rust's binary_search lands on the last of a bin's entries at the first cycle
+        if (c == cs && r + 1 < __ldg(ssw + b + 1) && (int)__ldg(a.cyc + q + 1) == cs) continue;
+        const float actual = __ldg(a.g.grid + b);
+        const float y = __ldg(a.inten + q);
+        const float xs = __fadd_rn(x.f(x0 + c - cs), y);
+        x.sf(x0 + c - cs, xs);
+        if (y > 0.0f) {
+          const float prev = __fsub_rn(xs, y);
+          if (prev == 0.0f)
+            z.sf(c - cs, actual);
+          else
+            z.sf(c - cs, __fdiv_rn(__fadd_rn(__fmul_rn(z.f(c - cs), prev), __fmul_rn(actual, y)), xs));
+        }
+      }
+    }
+  }
+}
+
+// hyperscore over the fragments seen (observed intensity above 0); `inverse`: weighted by
+// 1 / (|mass error| + 0.1).
+__device__ __forceinline__ float hyperscore_of(const SmVec& s, const BlockPlan& B, int v0, bool inverse,
+                                               int n) {
+  HyperSums h;
+  for (int i = 0; i < n; ++i) {
+    const float v = s.f(v0 + i);
+    if (!(s.f(B.obs + i) > 0.0f) || v == 0.0f) continue;
+    const float w = inverse ? __fdiv_rn(1.0f, __fadd_rn(fabsf(s.f(B.err + i)), 0.1f)) : 1.0f;
+    h.add(s.u(B.tn + i) & 0xffu, __fmul_rn(v, w));
+  }
+  return h.value();
+}
+
+// longest_series over the fragments seen, numbers sorted at etmp.
+__device__ __forceinline__ uint32_t longest_series_of(const SmVec& s, const BlockPlan& B, int n,
+                                                      uint32_t type, int etmp) {
+  int m = 0;
+  for (int i = 0; i < n; ++i) {
+    const uint32_t tn = s.u(B.tn + i);
+    if (s.f(B.obs + i) > 0.0f && (tn & 0xffu) == type) s.su(etmp + m++, tn >> 8);
+  }
+  return longest_run(s, etmp, m);
+}
+
+// Flags of a kept fragment.
+constexpr uint32_t kFlagNz = 1u;    // profile not all zero
+constexpr uint32_t kFlagTop = 2u;   // among the six highest IDF values
+constexpr int kFlagBand = 2;        // from this bit: intensity rank / 6 (4: rank 24 and on)
+
+template <bool QUANT>
+__global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid_constant__ QuantArgs qa,
+                                                                    const __grid_constant__ BlockPlan B,
+                                                                    int group) {
+  const ScoreArgs& a = qa.s;
+  extern __shared__ __align__(16) unsigned char block_smem[];
+  BlockCand* cand = reinterpret_cast<BlockCand*>(block_smem);
+  uint32_t* vec = reinterpret_cast<uint32_t*>(cand + group);
+  uint32_t* thr = vec + (size_t)group * B.words;
+  __shared__ int sh_max[3];  // of the group: raw fragments, kept fragments, cycles
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const ThreadVec own{thr + tid};
+  const int64_t first = (int64_t)blockIdx.x * group;
+
+  // ---- the candidates and their precursors
+  if (tid < 3) sh_max[tid] = 0;
+  __syncthreads();
+  if (tid < group) {
+    BlockCand k;
+    k.q = -1;
+    k.fs = k.prec = 0;
+    k.nraw = k.F = k.cs = k.C = k.woff = k.wlen = k.nz = 0;
+    k.pmz = 0.0f;
+    if (first + tid < a.n) {
+      const int64_t q = a.order ? (int64_t)a.order[first + tid] : first + tid;
+      const uint64_t pidx = a.c_pidx[q], cs64 = a.c_start[q], ce64 = a.c_stop[q], center = a.c_center[q];
+      bool take = true;
+      if (QUANT) {
+        qa.o_nq[q] = 0;
+        if (ce64 <= cs64 || center < cs64 || center >= ce64) {
+          take = false;  // dropped, as in the reference
+        } else if (ce64 > (uint64_t)a.n_rt || ce64 - cs64 > (uint64_t)B.Cm) {
+          atomicOr(a.err, 1);
+          take = false;
+        }
+      } else {
+        a.o_found[q] = 0;
+        if (cs64 > ce64 || ce64 > (uint64_t)a.n_rt || center >= (uint64_t)a.n_rt ||
+            ce64 - cs64 > (uint64_t)B.Cm) {
+          atomicOr(a.err, 1);
+          take = false;
+        }
+      }
+      if (take && a.P > 0) {
+        // SpecLibFlat::get_precursor_by_idx_filtered: binary search of the sorted idx
+        int64_t size = a.P, base = 0;
+        while (size > 1) {
+          const int64_t half = size / 2, mid = base + half;
+          base = a.l_pidx[mid] > pidx ? base : mid;
+          size -= half;
+        }
+        if (a.l_pidx[base] == pidx) {  // else skipped, as in the reference
+          const int64_t fs = (int64_t)a.l_fs[base], nraw = (int64_t)a.l_fe[base] - fs;
+          if (nraw > B.Fraw) {
+            atomicOr(a.err, 2);
+          } else {
+            k.q = q;
+            k.fs = fs;
+            k.prec = base;
+            k.nraw = (int)nraw;
+            k.cs = (int)cs64;
+            k.C = (int)(ce64 - cs64);
+            k.pmz = a.l_pmz[base];
+            find_windows(a.wi, k.pmz, &k.woff, &k.wlen);
+            atomicMax(sh_max + 0, k.nraw);
+            atomicMax(sh_max + 2, k.C);
+          }
+        }
+      }
+    }
+    cand[tid] = k;
+  }
+  __syncthreads();
+
+  // ---- filter_sort_fragments (select_fragments): raw m/z, intensity and keep mark ...
+  const int RAWM = B.prof, RAWI = B.prof + B.Fraw, KEEP = B.prof + 2 * B.Fraw;
+  const int nraw_max = sh_max[0];
+  for (int t = tid; t < group * nraw_max; t += kBlockThreads) {
+    const int c = t / nraw_max, r = t - c * nraw_max;
+    const BlockCand& k = cand[c];
+    if (r >= k.nraw) continue;
+    const SmVec s{vec + c * B.words};
+    const float I = a.l_fint[k.fs + r];
+    s.sf(RAWM + r, a.l_fmz[k.fs + r]);
+    s.sf(RAWI + r, I);
+    s.su(KEEP + r, I > 0.0f && !(a.l_ftype[k.fs + r] == 121 && a.l_fnum[k.fs + r] == 1) ? 1u : 0u);
+  }
+  __syncthreads();
+  // ... the kept ones counted, and where they are too many the top_k by intensity marked
+  // (ties to the lower position)
+  if (tid < group) {
+    const SmVec s{vec + tid * B.words};
+    int nk = 0;
+    for (int r = 0; r < cand[tid].nraw; ++r) nk += (int)s.u(KEEP + r);
+    cand[tid].F = nk;
+  }
+  __syncthreads();
+  const int top_k = (int)min(a.top_k, (int64_t)INT_MAX);
+  for (int t = tid; t < group * nraw_max; t += kBlockThreads) {
+    const int c = t / nraw_max, r = t - c * nraw_max;
+    const BlockCand& k = cand[c];
+    if (r >= k.nraw || k.F <= top_k) continue;
+    const SmVec s{vec + c * B.words};
+    if (!s.u(KEEP + r)) continue;
+    const float I = s.f(RAWI + r);
+    int rank = 0;
+    for (int j = 0; j < r; ++j)
+      if (s.u(KEEP + j)) rank += !(s.f(RAWI + j) < I);
+    for (int j = r + 1; j < k.nraw; ++j)
+      if (s.u(KEEP + j)) rank += s.f(RAWI + j) > I;
+    if (rank < top_k) s.su(KEEP + r, 2u);  // (only told from 1 after the barrier)
+  }
+  __syncthreads();
+  // ... and put in m/z order (ties keep library order)
+  for (int t = tid; t < group * nraw_max; t += kBlockThreads) {
+    const int c = t / nraw_max, r = t - c * nraw_max;
+    const BlockCand& k = cand[c];
+    if (r >= k.nraw) continue;
+    const SmVec s{vec + c * B.words};
+    const uint32_t need = k.F > top_k ? 2u : 1u;
+    if (s.u(KEEP + r) < need) continue;
+    const float m = s.f(RAWM + r);
+    int pos = 0;
+    for (int j = 0; j < r; ++j)
+      if (s.u(KEEP + j) >= need) pos += !(s.f(RAWM + j) > m);
+    for (int j = r + 1; j < k.nraw; ++j)
+      if (s.u(KEEP + j) >= need) pos += s.f(RAWM + j) < m;
+    s.sf(B.fmz + pos, m);
+    s.sf(B.fint + pos, s.f(RAWI + r));
+    if (QUANT) {
+      s.su(B.tn + pos, (uint32_t)r);
+    } else {
+      s.su(B.tn + pos, (uint32_t)a.l_ftype[k.fs + r] | (uint32_t)a.l_fnum[k.fs + r] << 8);
+      float idf = 1.0f;
+      if (a.idf_total != 0.0f) {
+        const uint32_t cnt = a.idf_counts[grid_find_closest(a.g, a.l_fmzl[k.fs + r])];
+        idf = ln_rn(__fdiv_rn(a.idf_total, (float)max(cnt, 1u)));
+      }
+      s.sf(B.idf + pos, idf);
+    }
+  }
+  __syncthreads();
+  if (tid < group) {
+    cand[tid].F = min(cand[tid].F, top_k);
+    atomicMax(sh_max + 1, cand[tid].F);
+  }
+  __syncthreads();
+
+  // ---- per fragment: XIC row, observed m/z and intensity, normalised profile
+  const int F_max = sh_max[1], C_max = sh_max[2];
+  for (int t = tid; t < group * F_max; t += kBlockThreads) {
+    const int c = t / F_max, f = t - c * F_max;
+    const BlockCand& k = cand[c];
+    if (f >= k.F) continue;
+    const SmVec s{vec + c * B.words};
+    const int X = B.prof + f * B.cs, C = k.C;
+    const float lib = s.f(B.fmz + f);
+    gather_one(a, s, X, own, lib, k.cs, C, k.woff, k.wlen);
+    s.sf(B.obs + f, ndarray_sum(s, X, C));
+    float ws = 0.0f, wsum = 0.0f;
+    for (int j = 0; j < C; ++j) {
+      const float w = s.f(X + j);
+      if (w > 0.0f) {
+        ws = __fadd_rn(ws, __fmul_rn(own.f(j), w));
+        wsum = __fadd_rn(wsum, w);
+      }
+    }
+    const float o = wsum > 0.0f ? __fdiv_rn(ws, wsum) : 0.0f;
+    s.sf(B.err + f, o > 0.0f ? __fmul_rn(__fdiv_rn(__fsub_rn(o, lib), lib), 1e6f) : 0.0f);
+    if (QUANT) s.sf(B.idf + f, o);
+    // normalize_profiles(xic, 1) (normalize_rows), in place
+    const int cc = C / 2;
+    const int c0 = cc > 1 ? cc - 1 : 0, c1 = cc + 2 < C ? cc + 2 : C;
+    float sum = 0.0f;
+    int count = 0;
+    for (int j = c0; j < c1; ++j) {
+      sum = __fadd_rn(sum, s.f(X + j));
+      ++count;
+    }
+    const float mean = count > 0 ? __fdiv_rn(sum, (float)count) : 0.0f;
+    uint32_t nz = 0;
+    for (int j = 0; j < C; ++j) {
+      const float v = mean > 0.0f ? __fdiv_rn(s.f(X + j), mean) : 0.0f;
+      s.sf(X + j, v);
+      nz |= v != 0.0f;
+    }
+    s.su(B.flag + f, nz);
+    if (nz) atomicAdd(&cand[c].nz, 1);
+  }
+  __syncthreads();
+
+  // ---- per cycle: median of all profiles and of those not all zero (zero when none)
+  for (int t = tid; t < group * C_max; t += kBlockThreads) {
+    const int c = t / C_max, j = t - c * C_max;
+    const BlockCand& k = cand[c];
+    if (j >= k.C) continue;
+    const SmVec s{vec + c * B.words};
+    const bool all_nz = k.nz == k.F;  // the two are then the median of the same values
+#pragma unroll 1
+    for (int pass = QUANT || all_nz ? 1 : 0; pass < 2; ++pass) {
+      int R = 0;
+      for (int f = 0; f < k.F; ++f)
+        if (pass == 0 || (s.u(B.flag + f) & kFlagNz)) own.sf(R++, s.f(B.prof + f * B.cs + j));
+      float med = 0.0f;
+      if (R > 0) {
+        sort_floats(own, 0, R);
+        med = R % 2 == 0 ? __fdiv_rn(__fadd_rn(own.f(R / 2 - 1), own.f(R / 2)), 2.0f) : own.f(R / 2);
+      }
+      if (pass == 0 || all_nz) s.sf(B.med + j, med);
+      if (pass == 1) s.sf(B.medf + j, med);
+    }
+  }
+  __syncthreads();
+
+  // ---- per fragment: correlation with the median of the non-zero profiles; ranks
+  for (int t = tid; t < group * F_max; t += kBlockThreads) {
+    const int c = t / F_max, f = t - c * F_max;
+    const BlockCand& k = cand[c];
+    if (f >= k.F) continue;
+    const SmVec s{vec + c * B.words};
+    if (QUANT && !(s.f(B.obs + f) > 0.0f)) continue;  // filter_fragments_by_intensity(0.0)
+    const XStats xmed = x_stats(s, B.medf, k.C);
+    const float corr = correlation_fixed_x(s, xmed, B.medf, B.prof + f * B.cs, k.C);
+    if (QUANT) {
+      int slot = 0;
+      for (int j = 0; j < f; ++j) slot += s.f(B.obs + j) > 0.0f;
+      const int64_t o = k.q * a.Fm + slot;
+      qa.o_frow[o] = (uint64_t)k.fs + s.u(B.tn + f);
+      qa.o_int[o] = s.f(B.obs + f);
+      qa.o_mzo[o] = s.f(B.idf + f);
+      qa.o_err[o] = s.f(B.err + f);
+      qa.o_corr[o] = corr;
+    } else {
+      s.sf(B.corr + f, corr);
+      // create_ranked_mask: earlier not below plus later above (ties to the lower index)
+      const float v = s.f(B.fint + f), w = s.f(B.idf + f);
+      int rank = 0, top = 0;
+      for (int j = 0; j < f; ++j) {
+        rank += !(s.f(B.fint + j) < v);
+        top += !(s.f(B.idf + j) < w);
+      }
+      for (int j = f + 1; j < k.F; ++j) {
+        rank += s.f(B.fint + j) > v;
+        top += s.f(B.idf + j) > w;
+      }
+      s.su(B.flag + f, s.u(B.flag + f) | (top < 6 ? kFlagTop : 0u) |
+                           (uint32_t)(rank < 24 ? rank / 6 : 4) << kFlagBand);
+    }
+  }
+  __syncthreads();
+
+  if (QUANT) {
+    if (tid < group && cand[tid].q >= 0) {
+      const BlockCand& k = cand[tid];
+      const SmVec s{vec + tid * B.words};
+      int nq = 0;
+      for (int f = 0; f < k.F; ++f) nq += s.f(B.obs + f) > 0.0f;
+      qa.o_nq[k.q] = nq;
+      qa.o_prow[k.q] = qa.l_prow[k.prec];
+      qa.o_rt[k.q] = a.rt[a.c_center[k.q]];
+    }
+    return;
+  }
+
+  // ---- per candidate: a lane each, the features divided among the warps
+  if (lane >= group || cand[lane].q < 0) return;
+  const BlockCand& k = cand[lane];
+  const SmVec s{vec + lane * B.words};
+  const int F = k.F, C = k.C;
+  const int64_t n = a.n, q = k.q;
+  float* o = a.o_feat;
+  const int TMP = B.prof + (warp >> 1) * F;  // (warps 0 and 2; the profiles are no longer needed)
+  if (warp == 0) {
+    const float mean_corr = F > 0 ? __fdiv_rn(rust_sum(s, B.corr, F), (float)F) : 0.0f;
+    o[0 * n + q] = a.c_score[q];
+    o[1 * n + q] = mean_corr;
+    o[2 * n + q] = median_of(s, B.corr, F, TMP);
+    o[3 * n + q] = std_of(s, B.corr, F);
+    o[4 * n + q] = correlation_safe(s, B.obs, B.fint, F);
+    o[5 * n + q] = (float)F;
+    o[6 * n + q] = (float)C;
+    // count_values_above (src/utils/mod.rs:223-237), all in one pass
+    int c95 = 0, c90 = 0, c80 = 0, c50 = 0, c0 = 0, t0 = 0, t50 = 0;
+    int b0[4] = {0, 0, 0, 0}, b50[4] = {0, 0, 0, 0};
+    for (int f = 0; f < F; ++f) {
+      const float c = s.f(B.corr + f);
+      const uint32_t flag = s.u(B.flag + f), band = flag >> kFlagBand;
+      const bool top = (flag & kFlagTop) != 0u;
+      c95 += c > 0.95f;
+      c90 += c > 0.90f;
+      c80 += c > 0.80f;
+      c50 += c > 0.50f;
+      c0 += c > 0.0f;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        b0[r] += band == (uint32_t)r && c > 0.0f;
+        b50[r] += band == (uint32_t)r && c > 0.50f;
+      }
+      t0 += top && c > 0.0f;
+      t50 += top && c > 0.50f;
+    }
+    o[7 * n + q] = (float)c95;
+    o[8 * n + q] = (float)c90;
+    o[9 * n + q] = (float)c80;
+    o[10 * n + q] = (float)c50;
+    o[11 * n + q] = (float)c0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      o[(12 + r) * n + q] = (float)b0[r];
+      o[(16 + r) * n + q] = (float)b50[r];
+    }
+    o[39 * n + q] = (float)t0;
+    o[40 * n + q] = (float)t50;
+  } else if (warp == 1) {
+    o[20 * n + q] = hyperscore_of(s, B, B.obs, false, F);
+    o[21 * n + q] = hyperscore_of(s, B, B.fint, false, F);
+    o[22 * n + q] = hyperscore_of(s, B, B.obs, true, F);
+    o[32 * n + q] = hyperscore_of(s, B, B.idf, false, F);
+  } else if (warp == 2) {
+    o[25 * n + q] = (float)longest_series_of(s, B, F, 98, TMP);
+    o[26 * n + q] = (float)longest_series_of(s, B, F, 121, TMP);
+    float ib = 0.0f, iy = 0.0f, wmae_s = 0.0f, wmae_w = 0.0f;
+    for (int f = 0; f < F; ++f) {
+      const float v = s.f(B.obs + f);
+      if (v > 0.0f) {
+        const uint32_t type = s.u(B.tn + f) & 0xffu;
+        if (type == 98) ib = __fadd_rn(ib, v);
+        if (type == 121) iy = __fadd_rn(iy, v);
+      }
+      const float w = s.f(B.fint + f), e = s.f(B.err + f);
+      if (w > 0.0f && e != 0.0f) {
+        wmae_s = __fadd_rn(wmae_s, __fmul_rn(fabsf(e), w));
+        wmae_w = __fadd_rn(wmae_w, w);
+      }
+    }
+    o[28 * n + q] = wmae_w > 0.0f ? __fdiv_rn(wmae_s, wmae_w) : 0.0f;
+    o[29 * n + q] = log10_rn(__fadd_rn(ib, 1e-8f));
+    o[30 * n + q] = log10_rn(__fadd_rn(iy, 1e-8f));
+  } else {
+    const float med_sum = rust_sum(s, B.med, C), med_sum_f = rust_sum(s, B.medf, C);
+    // calculate_fwhm_rt of the filtered median profile
+    float fwhm = 0.0f;
+    if (C > 0) {
+      const int half = C / 2;
+      const float cen = s.f(B.medf + half);
+      for (int j = 0; j < half; ++j) {
+        const float mean = __fdiv_rn(__fadd_rn(s.f(B.medf + half - j), s.f(B.medf + half + j)), 2.0f);
+        if (mean <= __fdiv_rn(cen, 2.0f)) {
+          fwhm = __fsub_rn(a.rt[k.cs + half + j], a.rt[k.cs + half - j]);
+          break;
+        }
+      }
+    }
+    float idf_xic = -0.0f, idf_int = -0.0f;
+    for (int f = 0; f < F; ++f) {
+      idf_xic = __fadd_rn(idf_xic, __fmul_rn(s.f(B.idf + f), s.f(B.corr + f)));
+      idf_int = __fadd_rn(idf_int, __fmul_rn(s.f(B.idf + f), s.f(B.obs + f)));
+    }
+    if (F == 0) idf_xic = idf_int = 0.0f;
+    const float rt_obs = a.rt[a.c_center[q]];
+    o[23 * n + q] = rt_obs;
+    o[24 * n + q] = __fsub_rn(rt_obs, a.l_prt[k.prec]);
+    o[27 * n + q] = (float)a.l_naa[k.prec];
+    o[31 * n + q] = fwhm;
+    o[33 * n + q] = idf_xic;
+    o[34 * n + q] = log10_rn(__fadd_rn(idf_int, 1e-8f));
+    o[35 * n + q] = med_sum;
+    o[36 * n + q] = med_sum_f;
+    o[37 * n + q] = (float)F;
+    o[38 * n + q] = (float)k.nz;
+    a.o_pidx[q] = a.c_pidx[q];
+    a.o_rank[q] = a.c_rank[q];
+    a.o_found[q] = 1;
+  }
+}

@@ -153,21 +153,21 @@ struct PrepArgs {
   uint32_t* blo;
   uint32_t* bhi;
   int* err;
-  int win_in_smem;  // stage the isolation windows / the RT index in shared memory
-  int rt_in_smem;
+  WinIndex wi;      // windows by m/z
+  int indexed;      // (0: the run has no index, windows are scanned)
+  int rt_in_smem;   // stage the RT index in shared memory
 };
 
-// Shared memory of a prep block: the isolation windows, then the MS1 retention times,
-// each when it fits the 48 KB a block gets without opting in.
+// Shared memory of a prep block: the MS1 retention times, when they fit the 48 KB a block
+// gets without opting in.
 constexpr size_t kPrepSmemBytes = 48 * 1024;
 
-__host__ __device__ inline size_t prep_win_bytes(int n_obs) { return ((size_t)n_obs * sizeof(WinInfo) + 15) / 16 * 16; }
-
-size_t plan_prep_smem(PrepArgs* a) {
-  const size_t wb = prep_win_bytes(a->n_obs), rb = (size_t)a->n_rt * sizeof(float);
-  a->win_in_smem = wb <= kPrepSmemBytes;
-  a->rt_in_smem = (a->win_in_smem ? wb : 0) + rb <= kPrepSmemBytes;
-  return (a->win_in_smem ? wb : 0) + (a->rt_in_smem ? rb : 0);
+size_t plan_prep(PrepArgs* a, const AdsDia* d) {
+  a->wi = d->win_index();
+  a->indexed = d->win_index_ok;
+  const size_t rb = (size_t)a->n_rt * sizeof(float);
+  a->rt_in_smem = rb <= kPrepSmemBytes;
+  return a->rt_in_smem ? rb : 0;
 }
 
 // Fragment m/z ordering key: NaN sorts after every number (ties by library
@@ -290,21 +290,11 @@ __global__ void cells_kernel(int64_t n, const int* nf, const int* cs, const int*
 __global__ void __launch_bounds__(kPrepThreads, 8) prep_kernel(PrepArgs a) {
   extern __shared__ __align__(16) unsigned char prep_smem[];
   const int lane = threadIdx.x & 31;
-  const WinInfo* win = a.win;
   const float* rt = a.rt;
-  {
-    size_t o = 0;
-    if (a.win_in_smem) {
-      WinInfo* ws = reinterpret_cast<WinInfo*>(prep_smem);
-      for (int i = threadIdx.x; i < a.n_obs; i += blockDim.x) ws[i] = a.win[i];
-      win = ws;
-      o = prep_win_bytes(a.n_obs);
-    }
-    if (a.rt_in_smem) {
-      float* rs = reinterpret_cast<float*>(prep_smem + o);
-      for (int i = threadIdx.x; i < a.n_rt; i += blockDim.x) rs[i] = __ldg(a.rt + i);
-      rt = rs;
-    }
+  if (a.rt_in_smem) {
+    float* rs = reinterpret_cast<float*>(prep_smem);
+    for (int i = threadIdx.x; i < a.n_rt; i += blockDim.x) rs[i] = __ldg(a.rt + i);
+    rt = rs;
     __syncthreads();
   }
   const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -317,19 +307,25 @@ __global__ void __launch_bounds__(kPrepThreads, 8) prep_kernel(PrepArgs a) {
     int nw = 0;
     if (!skip) {
       const float pmz = __ldg(a.pmz + p);
-      for (int base = 0; base < a.n_obs; base += 32) {
-        const int w = base + lane;
-        bool hit = false;
-        if (w < a.n_obs) {
-          const WinInfo wi = win[w];
-          hit = wi.ss_off >= 0 && wi.lo <= pmz && wi.hi >= pmz;
+      if (a.indexed) {
+        int off;
+        find_windows(a.wi, pmz, &off, &nw);
+        for (int w = lane; w < min(nw, a.maxw); w += 32) a.wins[p * a.maxw + w] = __ldg(a.wi.list + off + w);
+      } else {
+        for (int base = 0; base < a.n_obs; base += 32) {
+          const int w = base + lane;
+          bool hit = false;
+          if (w < a.n_obs) {
+            const WinInfo wi = a.win[w];
+            hit = wi.ss_off >= 0 && wi.lo <= pmz && wi.hi >= pmz;
+          }
+          const unsigned m = __ballot_sync(kFull, hit);
+          if (hit) {
+            const int pos = nw + __popc(m & lanemask_lt());
+            if (pos < a.maxw) a.wins[p * a.maxw + pos] = w;
+          }
+          nw += __popc(m);
         }
-        const unsigned m = __ballot_sync(kFull, hit);
-        if (hit) {
-          const int pos = nw + __popc(m & lanemask_lt());
-          if (pos < a.maxw) a.wins[p * a.maxw + pos] = w;
-        }
-        nw += __popc(m);
       }
       if (nw > a.maxw) {
         if (lane == 0) atomicOr(a.err, 1);
@@ -896,7 +892,7 @@ int enqueue_search(AdsSelection* s, const AdsDia* d, const AdsLib* l, AdsCandida
     ADS_CUDA(cudaEventRecord(s->stage_ev[0], st));
   }
   {
-    const size_t prep_smem = plan_prep_smem(&pa);
+    const size_t prep_smem = plan_prep(&pa, d);
     prep_kernel<<<(int)prep_blocks, kPrepThreads, prep_smem, st>>>(pa);
     ADS_LAUNCH_CHECK();
     ++launches;
@@ -1134,7 +1130,8 @@ std::vector<const void*> graph_key(const AdsSelection* s, const AdsDia* d, const
           s->work.p, s->class_lists.p, s->class_hist.p, s->block_sums.p,
           s->stats_on ? s->stats.p : nullptr,
           d->intens_bf16.p, s->grow.p, s->taps.p,
-          d->slice_starts.p, d->cycles.p, d->intens.p, d->win_dev.p, d->rt_dev.p, v(d->n_obs),
+          d->slice_starts.p, d->cycles.p, d->intens.p, d->win_dev.p, d->rt_dev.p, d->win_index_dev.p,
+          v(d->win_index_m), v(d->win_index_ok), v(d->n_obs),
           v((int64_t)d->rt.size()), v(d->max_overlap),
           l->arena.p, v(l->n_prec), v(l->n_frag), v(l->max_frag), v(l->min_frag), v(l->has_tol),
           v(tol_bits)};
@@ -1658,7 +1655,7 @@ int select_noalloc(const AdsDia* d, const AdsLib* l, const AdsSelectionParams* p
   pa.blo = blo;
   pa.bhi = bhi;
   pa.err = flags;
-  const size_t prep_smem = plan_prep_smem(&pa);
+  const size_t prep_smem = plan_prep(&pa, d);
   prep_kernel<<<(int)prep_blocks, kPrepThreads, prep_smem, st>>>(pa);
   ADS_LAUNCH_CHECK();
 
