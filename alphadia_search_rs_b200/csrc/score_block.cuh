@@ -14,7 +14,7 @@ constexpr int kBlockWarps = 4;
 constexpr int kBlockThreads = 32 * kBlockWarps;
 // A candidate's shared memory grows with fragments x cycles; beyond this many bytes a block
 // the group is halved, and below 4 candidates the per-candidate kernels run instead.
-constexpr size_t kBlockSmem = 74 * 1024;
+constexpr size_t kBlockSmem = 46 * 1024;
 
 // Vectors of one candidate, in words.
 struct BlockPlan {
@@ -129,44 +129,68 @@ __device__ __forceinline__ void gather_one(const ScoreArgs& a, const X& x, int x
   for (int w = 0; w < wlen; ++w) {
     const WinInfo wi = a.win[__ldg(a.wi.list + woff + w)];
     const uint32_t* ssw = a.ss + wi.ss_off;
-    const uint32_t r0 = __ldg(ssw + b0), r1 = __ldg(ssw + b1);
-    uint32_t b = b0;
+    const uint32_t r0 = __ldg(ssw + b0), n = __ldg(ssw + b1) - r0;
     // 8 cycle indices at a time from the 16-byte boundary at or below the first entry
-    // (the arrays are allocated kEntrySlack entries past the last one)
-    const int64_t q0 = wi.base + r0, q1 = wi.base + r1;
-#pragma unroll 4
-    for (int64_t c8 = q0 >> 3; c8 < (q1 + 7) >> 3; ++c8) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(a.cyc) + c8);
-      const uint32_t word[4] = {v.x, v.y, v.z, v.w};
+    // (the arrays are allocated kEntrySlack entries past the last one): position i of the
+    // range is entry skip + i counted from there
+    const int64_t q0 = wi.base + r0;
+    const uint32_t skip = (uint32_t)(q0 & 7);
+    const uint4* c8 = reinterpret_cast<const uint4*>(a.cyc + (q0 - skip));
+    const uint16_t* cy = a.cyc + q0;
+    const float* iy = a.inten + q0;
+    uint32_t b = b0;
+    for (uint32_t j = 0; j < skip + n; j += 8) {
+      const uint4 v = __ldg(c8 + (j >> 3));
       uint32_t in = 0;
 #pragma unroll
       for (int h = 0; h < 4; ++h) {
-        in |= (uint32_t)((unsigned)((int)(word[h] & 0xffffu) - cs) < (unsigned)C) << (2 * h);
-        in |= (uint32_t)((unsigned)((int)(word[h] >> 16) - cs) < (unsigned)C) << (2 * h + 1);
+        const uint32_t word = h == 0 ? v.x : h == 1 ? v.y : h == 2 ? v.z : v.w;
+        in |= (uint32_t)((unsigned)((int)(word & 0xffffu) - cs) < (unsigned)C) << (2 * h);
+        in |= (uint32_t)((unsigned)((int)(word >> 16) - cs) < (unsigned)C) << (2 * h + 1);
       }
-      const int64_t at = c8 << 3;
-      if (at < q0) in &= 0xffu << (int)(q0 - at);
-      if (at + 8 > q1) in &= 0xffu >> (int)(at + 8 - q1);
+      if (j < skip) in &= 0xffu << skip;
+      if (j + 8 > skip + n) in &= 0xffu >> (j + 8 - skip - n);
       while (in) {
-        const int h = __ffs(in) - 1;
-        in &= in - 1;
-        const int64_t q = at + h;
-        const uint32_t r = (uint32_t)(q - wi.base);
-        const int c = (int)__ldg(a.cyc + q);
-        b = bin_of(ssw, b, b1, r);
-        // Rust's binary_search lands on the last of a bin's entries at the first cycle
-        if (c == cs && r + 1 < __ldg(ssw + b + 1) && (int)__ldg(a.cyc + q + 1) == cs) continue;
-        const float actual = __ldg(a.g.grid + b);
-        const float y = __ldg(a.inten + q);
-        const float xs = __fadd_rn(x.f(x0 + c - cs), y);
-        x.sf(x0 + c - cs, xs);
-        if (y > 0.0f) {
-          const float prev = __fsub_rn(xs, y);
-          if (prev == 0.0f)
-            z.sf(c - cs, actual);
-          else
-            z.sf(c - cs, __fdiv_rn(__fadd_rn(__fmul_rn(z.f(c - cs), prev), __fmul_rn(actual, y)), xs));
+        // up to kBatch entries, whose loads do not wait for one another
+        constexpr int kBatch = 4;
+        uint32_t at[kBatch], bin[kBatch];
+        float y[kBatch];
+        int k = 0;
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+          at[u] = 0xffffffffu;
+          if (in) {
+            at[u] = j + (uint32_t)__ffs(in) - 1u - skip;
+            in &= in - 1;
+            ++k;
+          }
         }
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u)
+          if (u < k) {
+            y[u] = __ldg(iy + at[u]);
+            bin[u] = bin_of(ssw, b, b1, r0 + at[u]);
+          }
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u)
+          if (u < k) {
+            const int c = (int)__ldg(cy + at[u]) - cs;
+            const float actual = __ldg(a.g.grid + bin[u]);
+            b = bin[u];
+            // Rust's binary_search lands on the last of a bin's entries at the first cycle
+            if (c == 0 && at[u] + 1 < n && r0 + at[u] + 1 < __ldg(ssw + b + 1) &&
+                (int)__ldg(cy + at[u] + 1) == cs)
+              continue;
+            const float xs = __fadd_rn(x.f(x0 + c), y[u]);
+            x.sf(x0 + c, xs);
+            if (y[u] > 0.0f) {
+              const float prev = __fsub_rn(xs, y[u]);
+              if (prev == 0.0f)
+                z.sf(c, actual);
+              else
+                z.sf(c, __fdiv_rn(__fadd_rn(__fmul_rn(z.f(c), prev), __fmul_rn(actual, y[u])), xs));
+            }
+          }
       }
     }
   }
