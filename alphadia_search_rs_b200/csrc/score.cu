@@ -87,6 +87,7 @@ const char* const kFeatureNames[kFeatures] = {
     "idf_intensity_dot_product", "median_profile_sum", "median_profile_sum_filtered",
     "num_profiles", "num_profiles_filtered", "num_over_0_top6_idf", "num_over_50_top6_idf"};
 
+struct BlockCand;
 struct ScoreArgs {
   int64_t n;
   const uint64_t *c_pidx, *c_rank, *c_center, *c_start, *c_stop;
@@ -112,11 +113,14 @@ struct ScoreArgs {
   float tol;
   int64_t top_k;
   int Fm, Fraw, Cm;  // scratch bounds: kept fragments, raw fragments, cycles
+  const double2* ln_tab;  // (block kernel) table of ln_fast
   uint32_t* scratch;
   int64_t T;  // threads, the scratch's element stride
   uint64_t* o_pidx;
   uint64_t* o_rank;
   float* o_feat;
+  uint32_t* heads;          // (block kernel) the candidates' vectors for feature_kernel, by work order
+  BlockCand* cands;  // and what the block knows of each
   uint8_t* o_found;
   int* err;
   // nullable: the order in which the threads take the candidates (by their precursor's
@@ -162,6 +166,7 @@ __device__ __forceinline__ int64_t bsearch_u16_rust(const uint16_t* a, int64_t n
 template <class M>
 __device__ float rust_sum(const M& s, typename M::I e0, typename M::I n) {
   float acc = -0.0f;
+#pragma unroll 1
   for (typename M::I i = 0; i < n; ++i) acc = __fadd_rn(acc, s.f(e0 + i));
   return acc;
 }
@@ -173,6 +178,7 @@ __device__ float ndarray_sum(const M& s, typename M::I e0, typename M::I n) {
   float acc = 0.0f;
   float p[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   typename M::I i = 0;
+#pragma unroll 1
   for (; n - i >= 8; i += 8)
 #pragma unroll
     for (int k = 0; k < 8; ++k) p[k] = __fadd_rn(p[k], s.f(e0 + i + k));
@@ -180,6 +186,7 @@ __device__ float ndarray_sum(const M& s, typename M::I e0, typename M::I n) {
   acc = __fadd_rn(acc, __fadd_rn(p[1], p[5]));
   acc = __fadd_rn(acc, __fadd_rn(p[2], p[6]));
   acc = __fadd_rn(acc, __fadd_rn(p[3], p[7]));
+#pragma unroll 1
   for (typename M::I k = 0; i + k < n && k < 7; ++k) acc = __fadd_rn(acc, s.f(e0 + i + k));
   return acc;
 }
@@ -192,6 +199,7 @@ __device__ float correlation_safe(const M& s, typename M::I ex, typename M::I ey
   if (xs == 0.0f || ys == 0.0f) return 0.0f;
   const float xm = __fdiv_rn(xs, (float)n), ym = __fdiv_rn(ys, (float)n);
   float xv = 0.0f, yv = 0.0f, cv = 0.0f;
+#pragma unroll 1
   for (typename M::I i = 0; i < n; ++i) {
     const float dx = __fsub_rn(s.f(ex + i), xm), dy = __fsub_rn(s.f(ey + i), ym);
     xv = __fadd_rn(xv, __fmul_rn(dx, dx));
@@ -216,6 +224,7 @@ __device__ XStats x_stats(const M& s, typename M::I ex, typename M::I n) {
   if (n == 0) return r;
   r.xs = rust_sum(s, ex, n);
   r.xm = __fdiv_rn(r.xs, (float)n);
+#pragma unroll 1
   for (typename M::I i = 0; i < n; ++i) {
     const float dx = __fsub_rn(s.f(ex + i), r.xm);
     r.xv = __fadd_rn(r.xv, __fmul_rn(dx, dx));
@@ -231,6 +240,7 @@ __device__ float correlation_fixed_x(const M& s, const XStats& X, typename M::I 
   if (X.xs == 0.0f || ys == 0.0f) return 0.0f;
   const float ym = __fdiv_rn(ys, (float)n);
   float yv = 0.0f, cv = 0.0f;
+#pragma unroll 1
   for (typename M::I i = 0; i < n; ++i) {
     const float dx = __fsub_rn(s.f(ex + i), X.xm), dy = __fsub_rn(s.f(ey + i), ym);
     yv = __fadd_rn(yv, __fmul_rn(dy, dy));
@@ -245,6 +255,7 @@ __device__ float correlation_fixed_x(const M& s, const XStats& X, typename M::I 
 // Stable ascending insertion sort of n floats at e0 (slice::sort_by(partial_cmp)).
 template <class M>
 __device__ void sort_floats(const M& s, typename M::I e0, typename M::I n) {
+#pragma unroll 1
   for (typename M::I i = 1; i < n; ++i) {
     const float v = s.f(e0 + i);
     typename M::I j = i;
@@ -260,6 +271,7 @@ __device__ void sort_floats(const M& s, typename M::I e0, typename M::I n) {
 template <class M>
 __device__ float median_of(const M& s, typename M::I ev, typename M::I n, typename M::I etmp) {
   if (n == 0) return 0.0f;
+#pragma unroll 1
   for (typename M::I i = 0; i < n; ++i) s.sf(etmp + i, s.f(ev + i));
   sort_floats(s, etmp, n);
   const typename M::I mid = n / 2;
@@ -273,6 +285,7 @@ __device__ float std_of(const M& s, typename M::I ev, typename M::I n) {
   if (n < 2) return 0.0f;
   const float mean = __fdiv_rn(rust_sum(s, ev, n), (float)n);
   float acc = -0.0f;
+#pragma unroll 1
   for (typename M::I i = 0; i < n; ++i) {
     const float d = __fsub_rn(s.f(ev + i), mean);
     acc = __fadd_rn(acc, __fmul_rn(d, d));
@@ -287,23 +300,34 @@ __device__ float std_of(const M& s, typename M::I ev, typename M::I n) {
 // form `(w > v) || (!(w < v) && !(w > v) && j < i)` (every tie ranked 0).
 template <class M>
 __device__ void ranked_mask(const M& s, typename M::I ev, typename M::I n, int r1, int r2, typename M::I em) {
+#pragma unroll 1
   for (typename M::I i = 0; i < n; ++i) {
     const float v = s.f(ev + i);
     typename M::I rank = 0;
+#pragma unroll 1
     for (typename M::I j = 0; j < i; ++j) rank += !(s.f(ev + j) < v);
+#pragma unroll 1
     for (typename M::I j = i + 1; j < n; ++j) rank += s.f(ev + j) > v;
     s.su(em + i, (rank >= r1 && rank < r2) ? 1u : 0u);
   }
 }
 
 
+// The natural logarithm of the helpers below: ln_rn, or (a table given) ln_fast, the same
+// value in a quarter of the instructions.
+struct Ln {
+  const double2* tab;
+  LnCoef k;
+  __device__ float operator()(float x) const { return tab ? ln_fast(x, tab, k) : ln_rn(x); }
+};
+
 // src/peak_group_scoring/utils.rs:293-312
-__device__ float gamma_ln(float x) {
+__device__ float gamma_ln(float x, const Ln& ln) {
   if (x <= 0.0f) return 0.0f;
   if (fabsf(__fsub_rn(x, 1.0f)) < 1e-6f) return 0.0f;
   if (fabsf(__fsub_rn(x, 2.0f)) < 1e-6f) return 0.0f;
   const float ln_2pi = 1.837877f;
-  return __fadd_rn(__fsub_rn(__fmul_rn(__fsub_rn(x, 0.5f), ln_rn(x)), x), __fmul_rn(0.5f, ln_2pi));
+  return __fadd_rn(__fsub_rn(__fmul_rn(__fsub_rn(x, 0.5f), ln(x)), x), __fmul_rn(0.5f, ln_2pi));
 }
 
 // src/peak_group_scoring/utils.rs:193-279: the sums over b and y fragments
@@ -319,12 +343,12 @@ struct HyperSums {
       sy = __fadd_rn(sy, wi);
     }
   }
-  __device__ float value() const {
+  __device__ float value(const Ln& ln) const {
     if (nb == 0 && ny == 0) return 0.0f;
-    const float fb = nb > 0 ? gamma_ln(__fadd_rn((float)nb, 1.0f)) : 0.0f;
-    const float fy = ny > 0 ? gamma_ln(__fadd_rn((float)ny, 1.0f)) : 0.0f;
-    const float lb = sb > 0.0f ? ln_rn(sb) : 0.0f;
-    const float ly = sy > 0.0f ? ln_rn(sy) : 0.0f;
+    const float fb = nb > 0 ? gamma_ln(__fadd_rn((float)nb, 1.0f), ln) : 0.0f;
+    const float fy = ny > 0 ? gamma_ln(__fadd_rn((float)ny, 1.0f), ln) : 0.0f;
+    const float lb = sb > 0.0f ? ln(sb) : 0.0f;
+    const float ly = sy > 0.0f ? ln(sy) : 0.0f;
     const float h = __fadd_rn(__fadd_rn(__fadd_rn(fb, fy), lb), ly);
     return isfinite(h) ? h : 0.0f;
   }
@@ -335,12 +359,13 @@ template <class M>
 __device__ float hyperscore(const M& s, typename M::I etype, typename M::I eint, typename M::I emask,
                             typename M::I ew, typename M::I n) {
   HyperSums h;
+#pragma unroll 1
   for (typename M::I i = 0; i < n; ++i) {
     const float v = s.f(eint + i);
     if (!s.u(emask + i) || v == 0.0f) continue;
     h.add(s.u(etype + i), __fmul_rn(v, ew >= 0 ? s.f(ew + i) : 1.0f));
   }
-  return h.value();
+  return h.value(Ln{nullptr, LnCoef()});
 }
 
 // src/peak_group_scoring/utils.rs:314-372: the longest run of the m numbers at etmp, which
@@ -348,6 +373,7 @@ __device__ float hyperscore(const M& s, typename M::I etype, typename M::I eint,
 template <class M>
 __device__ uint32_t longest_run(const M& s, typename M::I etmp, typename M::I m) {
   if (m == 0) return 0;
+#pragma unroll 1
   for (typename M::I i = 1; i < m; ++i) {  // sort_unstable: any order of equal numbers
     const uint32_t v = s.u(etmp + i);
     typename M::I j = i;
@@ -358,6 +384,7 @@ __device__ uint32_t longest_run(const M& s, typename M::I etmp, typename M::I m)
     s.su(etmp + j, v);
   }
   uint32_t mx = 1, cur = 1;  // u8 arithmetic of the reference: wraps
+#pragma unroll 1
   for (typename M::I i = 1; i < m; ++i) {
     if (s.u(etmp + i) == ((s.u(etmp + i - 1) + 1u) & 0xFFu)) {
       cur = (cur + 1u) & 0xFFu;
@@ -375,6 +402,7 @@ __device__ uint32_t longest_series(const M& s, typename M::I etype, typename M::
                                    typename M::I emask, typename M::I n, uint32_t type,
                                    typename M::I etmp) {
   typename M::I m = 0;
+#pragma unroll 1
   for (typename M::I i = 0; i < n; ++i)
     if (s.u(emask + i) && s.u(etype + i) == type) s.su(etmp + m++, s.u(enum_ + i));
   return longest_run(s, etmp, m);
@@ -1050,13 +1078,13 @@ int quant_assemble(AdsQuant* r, const uint64_t* d_off, const int* d_pos, cudaStr
 }
 
 // The candidates a block of score_block_kernel takes, or 0 where the per-candidate kernels
-// run: candidates of so many fragments or cycles that fewer than 4 fit a block's shared
+// run: candidates of so many fragments or cycles that fewer than 2 fit a block's shared
 // memory (whole-run cycle ranges), or a run without a window index.
 int block_group(const AdsDia* d, const BlockPlan& b, int64_t C) {
   if (!d->win_index_ok || C > 4096) return 0;
   int group = kGroup;
-  while (group > 4 && block_smem_bytes(b, group) > kBlockSmem) group /= 2;
-  return block_smem_bytes(b, group) <= kBlockSmem ? group : 0;
+  while (group > 2 && block_smem_bytes(b, group) > kBlockSmem) group /= 2;
+  return block_smem_bytes(b, group) <= kBlockSmem && feature_smem_bytes(b) <= kFeatureSmem ? group : 0;
 }
 
 template <bool QUANT>
@@ -1163,6 +1191,7 @@ int score_device(const AdsScoringParams* p, const AdsDia* d, AdsLib* l, int64_t 
     a.win = d->win_dev.p;
     a.n_obs = (int)d->n_obs;
     a.wi = d->win_index();
+    ADS_TRY(device_ln_table(d->device, &a.ln_tab));
     a.ss = d->slice_starts.p;
     a.cyc = d->cycles.p;
     a.inten = d->intens.p;
@@ -1185,10 +1214,22 @@ int score_device(const AdsScoringParams* p, const AdsDia* d, AdsLib* l, int64_t 
     a.err = err.p;
     ADS_CUDA(cudaEventCreate(&ev.a));
     ADS_CUDA(cudaEventCreate(&ev.b));
+    DevBuf<uint32_t> heads;
+    DevBuf<BlockCand> cands;
+    if (group > 0) {
+      ADS_TRY(heads.alloc((size_t)n * plan.head));
+      ADS_TRY(cands.alloc((size_t)n));
+      a.heads = heads.p;
+      a.cands = cands.p;
+    }
     ADS_CUDA(cudaEventRecord(ev.a, st));
-    if (group > 0)
+    if (group > 0) {
       ADS_TRY(launch_block<false>(qa, plan, group, st));
-    else if (a.order)
+      const size_t fs = feature_smem_bytes(plan);
+      ADS_CUDA(cudaFuncSetAttribute(feature_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fs));
+      feature_kernel<<<(int)((n + kFeatureGroup - 1) / kFeatureGroup), 128, fs, st>>>(qa, plan);
+      ADS_LAUNCH_CHECK();
+    } else if (a.order)
       score_kernel<true><<<(int)((T + kScoreBlock - 1) / kScoreBlock), kScoreBlock, 0, st>>>(a);
     else
       score_kernel<false><<<(int)((T + kScoreBlock - 1) / kScoreBlock), kScoreBlock, 0, st>>>(a);
@@ -1310,6 +1351,7 @@ int quant_device(const AdsQuantParams* p, const AdsDia* d, AdsLib* l, int64_t n,
     a.win = d->win_dev.p;
     a.n_obs = (int)d->n_obs;
     a.wi = d->win_index();
+    ADS_TRY(device_ln_table(d->device, &a.ln_tab));
     a.ss = d->slice_starts.p;
     a.cyc = d->cycles.p;
     a.inten = d->intens.p;

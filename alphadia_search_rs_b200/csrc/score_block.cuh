@@ -9,20 +9,21 @@
 // lanes per instruction on matrices in a global scratch, and walked every bin of every
 // fragment with a binary search.  Here a row's whole range of entries is read 8 cycle
 // indices at a time, and only an entry inside the window looks up its bin.
-constexpr int kGroup = 32;       // candidates of a block (at most: one lane each)
-constexpr int kBlockWarps = 4;
+constexpr int kGroup = 4;        // candidates of a block (at most)
+constexpr int kBlockWarps = 2;
 constexpr int kBlockThreads = 32 * kBlockWarps;
 // A candidate's shared memory grows with fragments x cycles; beyond this many bytes a block
-// the group is halved, and below 4 candidates the per-candidate kernels run instead.
-constexpr size_t kBlockSmem = 46 * 1024;
+// the group is halved, and where not even 2 candidates fit the per-candidate kernels run.
+constexpr size_t kBlockSmem = 64 * 1024;
 
 // Vectors of one candidate, in words.
 struct BlockPlan {
   int Fm, Cm;      // most kept fragments, most cycles
   int Fraw;        // most library fragments
   int cs;          // row stride of the profiles (odd: rows of consecutive lanes hit different banks)
-  int fmz, fint, idf, tn, obs, corr, err, flag;  // per fragment
+  int fmz, fint, idf, tn, obs, corr;  // per fragment (mass error takes the m/z's place)
   int med, medf;   // per cycle
+  int head;        // words of the vectors, all but the profiles
   int prof;        // profiles, before them the raw fragments, after them sort space
   int words;       // of one candidate (odd)
   int scratch;     // words of one thread's column or row buffer
@@ -47,14 +48,11 @@ __host__ __device__ inline BlockPlan block_plan(int Fm, int Fraw, int Cm) {
   o += Fm;
   b.corr = o;
   o += Fm;
-  b.err = o;
-  o += Fm;
-  b.flag = o;
-  o += Fm;
   b.med = o;
   o += Cm;
   b.medf = o;
   o += Cm;
+  b.head = o;
   b.prof = o;
   int pw = Fm * b.cs;
   if (pw < 3 * Fraw) pw = 3 * Fraw;
@@ -112,11 +110,15 @@ __device__ __forceinline__ uint32_t bin_of(const uint32_t* ssw, uint32_t b, uint
   return lo;
 }
 
+// Bit 15 or 31 set where some 16-bit half of z is zero (perhaps also above a zero half).
+__device__ __forceinline__ uint32_t zero_half(uint32_t z) { return (z - 0x00010001u) & ~z; }
+
 // One fragment's row of gather_xic_mz: dense XIC (x) and intensity-weighted m/z (z) over
 // cycles [cs, cs + C).
 template <class X, class Z>
 __device__ __forceinline__ void gather_one(const ScoreArgs& a, const X& x, int x0, const Z& z,
                                            float mz, int cs, int C, int woff, int wlen) {
+#pragma unroll 1
   for (int j = 0; j < C; ++j) {
     x.sf(x0 + j, 0.0f);
     z.sf(j, 0.0f);
@@ -126,6 +128,7 @@ __device__ __forceinline__ void gather_one(const ScoreArgs& a, const X& x, int x
   const uint32_t b0 = grid_lower_bound(a.g, __fsub_rn(mz, delta));
   const uint32_t b1 = max(b0, grid_upper_bound(a.g, __fadd_rn(mz, delta)));
   if (b1 <= b0) return;
+  const uint32_t first2 = (uint32_t)cs * 0x10001u, last2 = (uint32_t)(cs + C - 1) * 0x10001u;
   for (int w = 0; w < wlen; ++w) {
     const WinInfo wi = a.win[__ldg(a.wi.list + woff + w)];
     const uint32_t* ssw = a.ss + wi.ss_off;
@@ -141,6 +144,13 @@ __device__ __forceinline__ void gather_one(const ScoreArgs& a, const X& x, int x
     uint32_t b = b0;
     for (uint32_t j = 0; j < skip + n; j += 8) {
       const uint4 v = __ldg(c8 + (j >> 3));
+      // most groups of 8 hold none: a half of a word is in the window where clamping it
+      // there changes nothing
+      const uint32_t z0 = v.x ^ __vmaxu2(__vminu2(v.x, last2), first2);
+      const uint32_t z1 = v.y ^ __vmaxu2(__vminu2(v.y, last2), first2);
+      const uint32_t z2 = v.z ^ __vmaxu2(__vminu2(v.z, last2), first2);
+      const uint32_t z3 = v.w ^ __vmaxu2(__vminu2(v.w, last2), first2);
+      if (!((zero_half(z0) | zero_half(z1) | zero_half(z2) | zero_half(z3)) & 0x80008000u)) continue;
       uint32_t in = 0;
 #pragma unroll
       for (int h = 0; h < 4; ++h) {
@@ -151,8 +161,8 @@ __device__ __forceinline__ void gather_one(const ScoreArgs& a, const X& x, int x
       if (j < skip) in &= 0xffu << skip;
       if (j + 8 > skip + n) in &= 0xffu >> (j + 8 - skip - n);
       while (in) {
-        // up to kBatch entries, whose loads do not wait for one another
-        constexpr int kBatch = 4;
+        // kBatch entries at once, whose loads do not wait for one another (4: 4 % slower)
+        constexpr int kBatch = 2;
         uint32_t at[kBatch], bin[kBatch];
         float y[kBatch];
         int k = 0;
@@ -198,33 +208,36 @@ __device__ __forceinline__ void gather_one(const ScoreArgs& a, const X& x, int x
 
 // hyperscore over the fragments seen (observed intensity above 0); `inverse`: weighted by
 // 1 / (|mass error| + 0.1).
-__device__ __forceinline__ float hyperscore_of(const SmVec& s, const BlockPlan& B, int v0, bool inverse,
-                                               int n) {
+__device__ float hyperscore_of(const SmVec& s, const BlockPlan& B, int v0, bool inverse, int n,
+                               const Ln& ln) {
   HyperSums h;
+#pragma unroll 1
   for (int i = 0; i < n; ++i) {
     const float v = s.f(v0 + i);
     if (!(s.f(B.obs + i) > 0.0f) || v == 0.0f) continue;
-    const float w = inverse ? __fdiv_rn(1.0f, __fadd_rn(fabsf(s.f(B.err + i)), 0.1f)) : 1.0f;
+    const float w = inverse ? __fdiv_rn(1.0f, __fadd_rn(fabsf(s.f(B.fmz + i)), 0.1f)) : 1.0f;
     h.add(s.u(B.tn + i) & 0xffu, __fmul_rn(v, w));
   }
-  return h.value();
+  return h.value(ln);
 }
 
 // longest_series over the fragments seen, numbers sorted at etmp.
 __device__ __forceinline__ uint32_t longest_series_of(const SmVec& s, const BlockPlan& B, int n,
                                                       uint32_t type, int etmp) {
   int m = 0;
+#pragma unroll 1
   for (int i = 0; i < n; ++i) {
     const uint32_t tn = s.u(B.tn + i);
-    if (s.f(B.obs + i) > 0.0f && (tn & 0xffu) == type) s.su(etmp + m++, tn >> 8);
+    if (s.f(B.obs + i) > 0.0f && (tn & 0xffu) == type) s.su(etmp + m++, (tn >> 8) & 0xffu);
   }
   return longest_run(s, etmp, m);
 }
 
-// Flags of a kept fragment.
-constexpr uint32_t kFlagNz = 1u;    // profile not all zero
-constexpr uint32_t kFlagTop = 2u;   // among the six highest IDF values
-constexpr int kFlagBand = 2;        // from this bit: intensity rank / 6 (4: rank 24 and on)
+// A kept fragment's word `tn`: type, number << 8, and these flags.  (Quantification has its
+// library offset in `corr` and its observed m/z in `idf`.)
+constexpr uint32_t kFlagNz = 1u << 16;   // profile not all zero
+constexpr uint32_t kFlagTop = 1u << 17;  // among the six highest IDF values
+constexpr int kFlagBand = 18;            // from this bit: intensity rank / 6 (4: rank 24 and on)
 
 template <bool QUANT>
 __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid_constant__ QuantArgs qa,
@@ -238,6 +251,7 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
   __shared__ int sh_max[3];  // of the group: raw fragments, kept fragments, cycles
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const ThreadVec own{thr + tid};
+  const Ln ln{a.ln_tab, LnCoef()};
   const int64_t first = (int64_t)blockIdx.x * group;
 
   // ---- the candidates and their precursors
@@ -319,6 +333,7 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
   if (tid < group) {
     const SmVec s{vec + tid * B.words};
     int nk = 0;
+#pragma unroll 1
     for (int r = 0; r < cand[tid].nraw; ++r) nk += (int)s.u(KEEP + r);
     cand[tid].F = nk;
   }
@@ -332,8 +347,10 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
     if (!s.u(KEEP + r)) continue;
     const float I = s.f(RAWI + r);
     int rank = 0;
+#pragma unroll 1
     for (int j = 0; j < r; ++j)
       if (s.u(KEEP + j)) rank += !(s.f(RAWI + j) < I);
+#pragma unroll 1
     for (int j = r + 1; j < k.nraw; ++j)
       if (s.u(KEEP + j)) rank += s.f(RAWI + j) > I;
     if (rank < top_k) s.su(KEEP + r, 2u);  // (only told from 1 after the barrier)
@@ -349,20 +366,23 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
     if (s.u(KEEP + r) < need) continue;
     const float m = s.f(RAWM + r);
     int pos = 0;
+#pragma unroll 1
     for (int j = 0; j < r; ++j)
       if (s.u(KEEP + j) >= need) pos += !(s.f(RAWM + j) > m);
+#pragma unroll 1
     for (int j = r + 1; j < k.nraw; ++j)
       if (s.u(KEEP + j) >= need) pos += s.f(RAWM + j) < m;
     s.sf(B.fmz + pos, m);
     s.sf(B.fint + pos, s.f(RAWI + r));
     if (QUANT) {
-      s.su(B.tn + pos, (uint32_t)r);
+      s.su(B.tn + pos, 0u);
+      s.su(B.corr + pos, (uint32_t)r);
     } else {
       s.su(B.tn + pos, (uint32_t)a.l_ftype[k.fs + r] | (uint32_t)a.l_fnum[k.fs + r] << 8);
       float idf = 1.0f;
       if (a.idf_total != 0.0f) {
         const uint32_t cnt = a.idf_counts[grid_find_closest(a.g, a.l_fmzl[k.fs + r])];
-        idf = ln_rn(__fdiv_rn(a.idf_total, (float)max(cnt, 1u)));
+        idf = ln(__fdiv_rn(a.idf_total, (float)max(cnt, 1u)));
       }
       s.sf(B.idf + pos, idf);
     }
@@ -386,6 +406,7 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
     gather_one(a, s, X, own, lib, k.cs, C, k.woff, k.wlen);
     s.sf(B.obs + f, ndarray_sum(s, X, C));
     float ws = 0.0f, wsum = 0.0f;
+#pragma unroll 1
     for (int j = 0; j < C; ++j) {
       const float w = s.f(X + j);
       if (w > 0.0f) {
@@ -394,26 +415,30 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
       }
     }
     const float o = wsum > 0.0f ? __fdiv_rn(ws, wsum) : 0.0f;
-    s.sf(B.err + f, o > 0.0f ? __fmul_rn(__fdiv_rn(__fsub_rn(o, lib), lib), 1e6f) : 0.0f);
+    s.sf(B.fmz + f, o > 0.0f ? __fmul_rn(__fdiv_rn(__fsub_rn(o, lib), lib), 1e6f) : 0.0f);
     if (QUANT) s.sf(B.idf + f, o);
     // normalize_profiles(xic, 1) (normalize_rows), in place
     const int cc = C / 2;
     const int c0 = cc > 1 ? cc - 1 : 0, c1 = cc + 2 < C ? cc + 2 : C;
     float sum = 0.0f;
     int count = 0;
+#pragma unroll 1
     for (int j = c0; j < c1; ++j) {
       sum = __fadd_rn(sum, s.f(X + j));
       ++count;
     }
     const float mean = count > 0 ? __fdiv_rn(sum, (float)count) : 0.0f;
     uint32_t nz = 0;
+#pragma unroll 1
     for (int j = 0; j < C; ++j) {
       const float v = mean > 0.0f ? __fdiv_rn(s.f(X + j), mean) : 0.0f;
       s.sf(X + j, v);
       nz |= v != 0.0f;
     }
-    s.su(B.flag + f, nz);
-    if (nz) atomicAdd(&cand[c].nz, 1);
+    if (nz) {
+      s.su(B.tn + f, s.u(B.tn + f) | kFlagNz);
+      atomicAdd(&cand[c].nz, 1);
+    }
   }
   __syncthreads();
 
@@ -427,8 +452,9 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
 #pragma unroll 1
     for (int pass = QUANT || all_nz ? 1 : 0; pass < 2; ++pass) {
       int R = 0;
+#pragma unroll 1
       for (int f = 0; f < k.F; ++f)
-        if (pass == 0 || (s.u(B.flag + f) & kFlagNz)) own.sf(R++, s.f(B.prof + f * B.cs + j));
+        if (pass == 0 || (s.u(B.tn + f) & kFlagNz)) own.sf(R++, s.f(B.prof + f * B.cs + j));
       float med = 0.0f;
       if (R > 0) {
         sort_floats(own, 0, R);
@@ -451,28 +477,31 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
     const float corr = correlation_fixed_x(s, xmed, B.medf, B.prof + f * B.cs, k.C);
     if (QUANT) {
       int slot = 0;
+#pragma unroll 1
       for (int j = 0; j < f; ++j) slot += s.f(B.obs + j) > 0.0f;
       const int64_t o = k.q * a.Fm + slot;
-      qa.o_frow[o] = (uint64_t)k.fs + s.u(B.tn + f);
+      qa.o_frow[o] = (uint64_t)k.fs + s.u(B.corr + f);
       qa.o_int[o] = s.f(B.obs + f);
       qa.o_mzo[o] = s.f(B.idf + f);
-      qa.o_err[o] = s.f(B.err + f);
+      qa.o_err[o] = s.f(B.fmz + f);
       qa.o_corr[o] = corr;
     } else {
       s.sf(B.corr + f, corr);
       // create_ranked_mask: earlier not below plus later above (ties to the lower index)
       const float v = s.f(B.fint + f), w = s.f(B.idf + f);
       int rank = 0, top = 0;
+#pragma unroll 1
       for (int j = 0; j < f; ++j) {
         rank += !(s.f(B.fint + j) < v);
         top += !(s.f(B.idf + j) < w);
       }
+#pragma unroll 1
       for (int j = f + 1; j < k.F; ++j) {
         rank += s.f(B.fint + j) > v;
         top += s.f(B.idf + j) > w;
       }
-      s.su(B.flag + f, s.u(B.flag + f) | (top < 6 ? kFlagTop : 0u) |
-                           (uint32_t)(rank < 24 ? rank / 6 : 4) << kFlagBand);
+      s.su(B.tn + f, s.u(B.tn + f) | (top < 6 ? kFlagTop : 0u) |
+                         (uint32_t)(rank < 24 ? rank / 6 : 4) << kFlagBand);
     }
   }
   __syncthreads();
@@ -482,6 +511,7 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
       const BlockCand& k = cand[tid];
       const SmVec s{vec + tid * B.words};
       int nq = 0;
+#pragma unroll 1
       for (int f = 0; f < k.F; ++f) nq += s.f(B.obs + f) > 0.0f;
       qa.o_nq[k.q] = nq;
       qa.o_prow[k.q] = qa.l_prow[k.prec];
@@ -490,29 +520,63 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
     return;
   }
 
-  // ---- per candidate: a lane each, the features divided among the warps
-  if (lane >= group || cand[lane].q < 0) return;
-  const BlockCand& k = cand[lane];
-  const SmVec s{vec + lane * B.words};
+  // ---- what feature_kernel needs of them
+  for (int t = tid; t < group * B.head; t += kBlockThreads) {
+    const int c = t / B.head, j = t - c * B.head;
+    if (cand[c].q >= 0) a.heads[(first + c) * B.head + j] = vec[c * B.words + j];
+  }
+  if (tid < group && first + tid < a.n) a.cands[first + tid] = cand[tid];
+}
+
+// The features of the candidates that score_block_kernel has been through, from their
+// vectors: 32 candidates a block, a lane each, the features divided among the warps.  On its
+// own because that kernel's blocks are small (few rows wait at each barrier for the one with
+// most entries), where these steps would run on 8 of 32 lanes.
+constexpr int kFeatureGroup = 32;
+constexpr size_t kFeatureSmem = 128 * 1024;
+
+inline size_t feature_smem_bytes(const BlockPlan& b) {
+  return 4 * (size_t)kFeatureGroup * ((b.head + 2 * b.Fm) | 1);
+}
+
+__global__ void __launch_bounds__(128) feature_kernel(const __grid_constant__ QuantArgs qa,
+                                                      const __grid_constant__ BlockPlan B) {
+  const ScoreArgs& a = qa.s;
+  extern __shared__ __align__(16) uint32_t feature_smem[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int64_t first = (int64_t)blockIdx.x * kFeatureGroup;
+  const int here = (int)min((int64_t)kFeatureGroup, a.n - first);
+  const int words = (B.head + 2 * B.Fm) | 1;
+  const Ln ln{a.ln_tab, LnCoef()};
+  for (int t = tid; t < here * B.head; t += 128) {
+    const int c = t / B.head, j = t - c * B.head;
+    feature_smem[c * words + j] = a.heads[(first + c) * B.head + j];
+  }
+  __syncthreads();
+  if (lane >= here) return;
+  const BlockCand k = a.cands[first + lane];
+  if (k.q < 0) return;
+  const SmVec s{feature_smem + lane * words};
   const int F = k.F, C = k.C;
   const int64_t n = a.n, q = k.q;
-  float* o = a.o_feat;
-  const int TMP = B.prof + (warp >> 1) * F;  // (warps 0 and 2; the profiles are no longer needed)
+  float* o = a.o_feat + q;  // feature j at o[j * n]
+  const int TMP = B.head + (warp >> 1) * B.Fm;  // (warps 0 and 2)
   if (warp == 0) {
     const float mean_corr = F > 0 ? __fdiv_rn(rust_sum(s, B.corr, F), (float)F) : 0.0f;
-    o[0 * n + q] = a.c_score[q];
-    o[1 * n + q] = mean_corr;
-    o[2 * n + q] = median_of(s, B.corr, F, TMP);
-    o[3 * n + q] = std_of(s, B.corr, F);
-    o[4 * n + q] = correlation_safe(s, B.obs, B.fint, F);
-    o[5 * n + q] = (float)F;
-    o[6 * n + q] = (float)C;
+    o[0 * n] = a.c_score[q];
+    o[1 * n] = mean_corr;
+    o[2 * n] = median_of(s, B.corr, F, TMP);
+    o[3 * n] = std_of(s, B.corr, F);
+    o[4 * n] = correlation_safe(s, B.obs, B.fint, F);
+    o[5 * n] = (float)F;
+    o[6 * n] = (float)C;
     // count_values_above (src/utils/mod.rs:223-237), all in one pass
     int c95 = 0, c90 = 0, c80 = 0, c50 = 0, c0 = 0, t0 = 0, t50 = 0;
     int b0[4] = {0, 0, 0, 0}, b50[4] = {0, 0, 0, 0};
+#pragma unroll 1
     for (int f = 0; f < F; ++f) {
       const float c = s.f(B.corr + f);
-      const uint32_t flag = s.u(B.flag + f), band = flag >> kFlagBand;
+      const uint32_t flag = s.u(B.tn + f), band = flag >> kFlagBand;
       const bool top = (flag & kFlagTop) != 0u;
       c95 += c > 0.95f;
       c90 += c > 0.90f;
@@ -527,27 +591,28 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
       t0 += top && c > 0.0f;
       t50 += top && c > 0.50f;
     }
-    o[7 * n + q] = (float)c95;
-    o[8 * n + q] = (float)c90;
-    o[9 * n + q] = (float)c80;
-    o[10 * n + q] = (float)c50;
-    o[11 * n + q] = (float)c0;
+    o[7 * n] = (float)c95;
+    o[8 * n] = (float)c90;
+    o[9 * n] = (float)c80;
+    o[10 * n] = (float)c50;
+    o[11 * n] = (float)c0;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      o[(12 + r) * n + q] = (float)b0[r];
-      o[(16 + r) * n + q] = (float)b50[r];
+      o[(12 + r) * n] = (float)b0[r];
+      o[(16 + r) * n] = (float)b50[r];
     }
-    o[39 * n + q] = (float)t0;
-    o[40 * n + q] = (float)t50;
+    o[39 * n] = (float)t0;
+    o[40 * n] = (float)t50;
   } else if (warp == 1) {
-    o[20 * n + q] = hyperscore_of(s, B, B.obs, false, F);
-    o[21 * n + q] = hyperscore_of(s, B, B.fint, false, F);
-    o[22 * n + q] = hyperscore_of(s, B, B.obs, true, F);
-    o[32 * n + q] = hyperscore_of(s, B, B.idf, false, F);
+    o[20 * n] = hyperscore_of(s, B, B.obs, false, F, ln);
+    o[21 * n] = hyperscore_of(s, B, B.fint, false, F, ln);
+    o[22 * n] = hyperscore_of(s, B, B.obs, true, F, ln);
+    o[32 * n] = hyperscore_of(s, B, B.idf, false, F, ln);
   } else if (warp == 2) {
-    o[25 * n + q] = (float)longest_series_of(s, B, F, 98, TMP);
-    o[26 * n + q] = (float)longest_series_of(s, B, F, 121, TMP);
+    o[25 * n] = (float)longest_series_of(s, B, F, 98, TMP);
+    o[26 * n] = (float)longest_series_of(s, B, F, 121, TMP);
     float ib = 0.0f, iy = 0.0f, wmae_s = 0.0f, wmae_w = 0.0f;
+#pragma unroll 1
     for (int f = 0; f < F; ++f) {
       const float v = s.f(B.obs + f);
       if (v > 0.0f) {
@@ -555,15 +620,15 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
         if (type == 98) ib = __fadd_rn(ib, v);
         if (type == 121) iy = __fadd_rn(iy, v);
       }
-      const float w = s.f(B.fint + f), e = s.f(B.err + f);
+      const float w = s.f(B.fint + f), e = s.f(B.fmz + f);
       if (w > 0.0f && e != 0.0f) {
         wmae_s = __fadd_rn(wmae_s, __fmul_rn(fabsf(e), w));
         wmae_w = __fadd_rn(wmae_w, w);
       }
     }
-    o[28 * n + q] = wmae_w > 0.0f ? __fdiv_rn(wmae_s, wmae_w) : 0.0f;
-    o[29 * n + q] = log10_rn(__fadd_rn(ib, 1e-8f));
-    o[30 * n + q] = log10_rn(__fadd_rn(iy, 1e-8f));
+    o[28 * n] = wmae_w > 0.0f ? __fdiv_rn(wmae_s, wmae_w) : 0.0f;
+    o[29 * n] = log10_rn(__fadd_rn(ib, 1e-8f));
+    o[30 * n] = log10_rn(__fadd_rn(iy, 1e-8f));
   } else {
     const float med_sum = rust_sum(s, B.med, C), med_sum_f = rust_sum(s, B.medf, C);
     // calculate_fwhm_rt of the filtered median profile
@@ -571,6 +636,7 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
     if (C > 0) {
       const int half = C / 2;
       const float cen = s.f(B.medf + half);
+#pragma unroll 1
       for (int j = 0; j < half; ++j) {
         const float mean = __fdiv_rn(__fadd_rn(s.f(B.medf + half - j), s.f(B.medf + half + j)), 2.0f);
         if (mean <= __fdiv_rn(cen, 2.0f)) {
@@ -580,22 +646,23 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
       }
     }
     float idf_xic = -0.0f, idf_int = -0.0f;
+#pragma unroll 1
     for (int f = 0; f < F; ++f) {
       idf_xic = __fadd_rn(idf_xic, __fmul_rn(s.f(B.idf + f), s.f(B.corr + f)));
       idf_int = __fadd_rn(idf_int, __fmul_rn(s.f(B.idf + f), s.f(B.obs + f)));
     }
     if (F == 0) idf_xic = idf_int = 0.0f;
     const float rt_obs = a.rt[a.c_center[q]];
-    o[23 * n + q] = rt_obs;
-    o[24 * n + q] = __fsub_rn(rt_obs, a.l_prt[k.prec]);
-    o[27 * n + q] = (float)a.l_naa[k.prec];
-    o[31 * n + q] = fwhm;
-    o[33 * n + q] = idf_xic;
-    o[34 * n + q] = log10_rn(__fadd_rn(idf_int, 1e-8f));
-    o[35 * n + q] = med_sum;
-    o[36 * n + q] = med_sum_f;
-    o[37 * n + q] = (float)F;
-    o[38 * n + q] = (float)k.nz;
+    o[23 * n] = rt_obs;
+    o[24 * n] = __fsub_rn(rt_obs, a.l_prt[k.prec]);
+    o[27 * n] = (float)a.l_naa[k.prec];
+    o[31 * n] = fwhm;
+    o[33 * n] = idf_xic;
+    o[34 * n] = log10_rn(__fadd_rn(idf_int, 1e-8f));
+    o[35 * n] = med_sum;
+    o[36 * n] = med_sum_f;
+    o[37 * n] = (float)F;
+    o[38 * n] = (float)k.nz;
     a.o_pidx[q] = a.c_pidx[q];
     a.o_rank[q] = a.c_rank[q];
     a.o_found[q] = 1;
