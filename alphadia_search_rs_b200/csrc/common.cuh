@@ -158,36 +158,40 @@ std::vector<float> gaussian_kernel(float fwhm_rt, float sigma_scale_rt, int64_t 
 
 __device__ __forceinline__ uint32_t f2bits(float x) { return __float_as_uint(x); }
 
+// The LUT bracket [lo, hi] of the bound of x (g.first < x <= g.last) and a guess inside it: a
+// bucket's floats are evenly spaced and its grid points nearly so, so interpolation is
+// within a point of the bound and its two neighbours load at once, where a binary search
+// took three loads one after the other.
+struct GridGuess {
+  uint32_t lo, hi, at;
+};
+__device__ __forceinline__ GridGuess grid_guess(const GridView& g, float x) {
+  const uint32_t d = f2bits(x) - g.bits0, k = d >> kLutShift;
+  GridGuess r;
+  r.lo = __ldg(g.lut + k);
+  r.hi = __ldg(g.lut + k + 1);
+  r.at = r.lo + (((r.hi - r.lo) * (d & ((1u << kLutShift) - 1u))) >> kLutShift);
+  return r;
+}
+
 // First i with grid[i] >= x (lower_bound), exact for every float x, NaN -> 0.
 __device__ __forceinline__ uint32_t grid_lower_bound(const GridView& g, float x) {
   if (!(x > g.first)) return 0;
   if (x > g.last) return g.n;
-  uint32_t k = (f2bits(x) - g.bits0) >> kLutShift;
-  uint32_t lo = __ldg(g.lut + k), hi = __ldg(g.lut + k + 1);
-  while (lo < hi) {
-    uint32_t mid = (lo + hi) >> 1;
-    if (__ldg(g.grid + mid) < x)
-      lo = mid + 1;
-    else
-      hi = mid;
-  }
-  return lo;
+  GridGuess r = grid_guess(g, x);
+  while (r.at < r.hi && __ldg(g.grid + r.at) < x) ++r.at;
+  while (r.at > r.lo && !(__ldg(g.grid + r.at - 1) < x)) --r.at;
+  return r.at;
 }
 
 // First i with grid[i] > x (upper_bound), exact, NaN -> 0.
 __device__ __forceinline__ uint32_t grid_upper_bound(const GridView& g, float x) {
   if (!(x >= g.first)) return 0;
   if (!(x < g.last)) return g.n;
-  uint32_t k = (f2bits(x) - g.bits0) >> kLutShift;
-  uint32_t lo = __ldg(g.lut + k), hi = __ldg(g.lut + k + 1);
-  while (lo < hi) {
-    uint32_t mid = (lo + hi) >> 1;
-    if (__ldg(g.grid + mid) <= x)
-      lo = mid + 1;
-    else
-      hi = mid;
-  }
-  return lo;
+  GridGuess r = grid_guess(g, x);
+  while (r.at < r.hi && __ldg(g.grid + r.at) <= x) ++r.at;
+  while (r.at > r.lo && !(__ldg(g.grid + r.at - 1) <= x)) --r.at;
+  return r.at;
 }
 
 // MZIndex::find_closest_index (src/mz_index/mod.rs:55-90): nearest grid point,

@@ -7,65 +7,280 @@
 //   intens[base(w) + i]       f32 intensity of entry i
 // Entries are ordered by (bin, cycle), ties in the order the reference visits
 // peaks (spectrum index, then peak index), exactly like its stable sort_by_key.
-#include <cub/cub.cuh>
-
 #include <algorithm>
 #include <cstring>
+#include <memory>
 
 #include "common.cuh"
 
 namespace ads {
 namespace {
 
-constexpr int kBinShift = 16;
-constexpr int kWinShift = 38;  // 22 bits of m/z bin above 16 bits of cycle
+// The entries are put in order by a counting sort, a few observations at a time: the bins
+// are counted in slice_starts itself, scanned in place, and every peak takes the next place
+// of its bin; then each bin's few entries are sorted by (cycle, visit position).  Peaks of
+// a group of observations, their counts and their places fit the L2, so what crosses the
+// memory bus is little more than the peaks once in and the entries once out, and the
+// temporary memory is one group's (64 MB).  A radix sort of (window, bin, cycle) keys with
+// peak indices moved 12 bytes a peak six times through 24 bytes a peak of temporaries:
+// 324 M peaks in 25 ms of kernels and 100 ms of mapping and unmapping that memory.
+constexpr int64_t kGroupItems = int64_t(1) << 23;
+constexpr int kScanTile = 8192;       // bins of one scan block
+constexpr int kScanThreads = 256;
+constexpr int kBinSmall = 8;          // bins of up to this many entries are sorted by a thread
+constexpr int kBinShared = 1024;      // up to this many in shared memory, larger in place
 
-// One block per spectrum: every peak gets its (window, bin, cycle) key and its
-// peak index as value, written at the spectrum's slot in the reference's visit
-// order.
-template <class V>
-__global__ void bin_peaks_kernel(int64_t n_spec, const int64_t* __restrict__ item_off,
-                                 const int64_t* __restrict__ pstart,
-                                 const int64_t* __restrict__ pstop, const int32_t* __restrict__ win,
-                                 const uint16_t* __restrict__ cyc, const float* __restrict__ mz,
-                                 GridView g, uint64_t* __restrict__ keys, V* __restrict__ vals) {
-  for (int64_t s = blockIdx.x; s < n_spec; s += gridDim.x) {
-    const int32_t w = win[s];
-    if (w < 0) continue;
-    const int64_t off = item_off[s], b = pstart[s], e = pstop[s];
-    const uint64_t hi = ((uint64_t)w << kWinShift) | (uint64_t)cyc[s];
-    for (int64_t k = threadIdx.x; k < e - b; k += blockDim.x) {
-      const int64_t i = b + k;
-      const uint32_t bin = grid_find_closest(g, __ldg(mz + i));
-      keys[off + k] = hi | ((uint64_t)bin << kBinShift);
-      vals[off + k] = (V)i;
+// One observation of a group.
+struct BuildWin {
+  int64_t ss;       // element offset of its slice_starts
+  int64_t base;     // its first entry
+};
+
+// One warp per spectrum (listed in window, then visit order): the bin of every peak, kept
+// for place_peaks_kernel, and the bins' counts, each one place up (see place_peaks_kernel).
+__global__ void __launch_bounds__(256) count_peaks_kernel(int64_t n_spec, const int64_t* __restrict__ list,
+                                                          const int64_t* __restrict__ item_off,
+                                                          const int64_t* __restrict__ pstart,
+                                                          const int64_t* __restrict__ pstop,
+                                                          const int32_t* __restrict__ win, int win0,
+                                                          const BuildWin* __restrict__ wins, int64_t item0,
+                                                          const float* __restrict__ mz, GridView g,
+                                                          uint32_t* __restrict__ bins,
+                                                          uint32_t* __restrict__ starts) {
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (warp >= n_spec) return;
+  const int64_t s = list[warp];
+  const int64_t b = pstart[s], n = pstop[s] - b;
+  uint32_t* to = bins + (item_off[s] - item0);
+  uint32_t* count = starts + wins[win[s] - win0].ss + 1;
+  for (int64_t k = lane; k < n; k += 32) {
+    const uint32_t bin = grid_find_closest(g, __ldg(mz + b + k));
+    to[k] = bin;
+    atomicAdd(count + bin, 1u);
+  }
+}
+
+// Exclusive scan of each observation's counts, in place: sums of tiles, their scan, the
+// tiles.  counts[b + 1] becomes the first place of bin b.
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* sh, uint32_t* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (lane == 31) sh[warp] = incl;
+  __syncthreads();
+  if (warp == 0) {
+    const uint32_t w = lane < kScanThreads / 32 ? sh[lane] : 0u;
+    uint32_t wi = w;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, wi, o);
+      if (lane >= o) wi += t;
+    }
+    if (lane < kScanThreads / 32) sh[lane] = wi - w;
+    if (lane == 31) sh[32] = wi;
+  }
+  __syncthreads();
+  const uint32_t r = sh[warp] + incl - v;
+  *total = sh[32];
+  __syncthreads();
+  return r;
+}
+
+__global__ void __launch_bounds__(kScanThreads) tile_sums_kernel(int64_t grid_len, int tiles,
+                                                                 const BuildWin* __restrict__ wins,
+                                                                 const uint32_t* __restrict__ starts,
+                                                                 uint32_t* __restrict__ sums) {
+  __shared__ uint32_t sh[33];
+  const int w = blockIdx.x / tiles, t = blockIdx.x - w * tiles;
+  const uint32_t* c = starts + wins[w].ss + 1;
+  uint32_t v = 0, total;
+  for (int i = threadIdx.x; i < kScanTile; i += kScanThreads) {
+    const int64_t b = (int64_t)t * kScanTile + i;
+    if (b < grid_len) v += c[b];
+  }
+  block_scan(v, sh, &total);
+  if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(kScanThreads) scan_sums_kernel(int tiles, uint32_t* __restrict__ sums) {
+  __shared__ uint32_t sh[33];
+  uint32_t* s = sums + (int64_t)blockIdx.x * tiles;
+  uint32_t carry = 0;
+  for (int t0 = 0; t0 < tiles; t0 += kScanThreads) {
+    const int t = t0 + (int)threadIdx.x;
+    uint32_t total;
+    const uint32_t v = t < tiles ? s[t] : 0u;
+    const uint32_t ex = block_scan(v, sh, &total);
+    if (t < tiles) s[t] = carry + ex;
+    carry += total;
+  }
+}
+
+__global__ void __launch_bounds__(kScanThreads) scan_tiles_kernel(int64_t grid_len, int tiles,
+                                                                  const BuildWin* __restrict__ wins,
+                                                                  const uint32_t* __restrict__ sums,
+                                                                  uint32_t* __restrict__ starts) {
+  __shared__ uint32_t sh[33];
+  __shared__ uint32_t tile[kScanTile + kScanTile / 32];  // (padded: a thread's run is strided)
+  const int w = blockIdx.x / tiles, t = blockIdx.x - w * tiles;
+  uint32_t* c = starts + wins[w].ss + 1;
+  const int64_t b0 = (int64_t)t * kScanTile;
+  constexpr int kRun = kScanTile / kScanThreads;  // 32
+  for (int i = threadIdx.x; i < kScanTile; i += kScanThreads)
+    tile[i + i / 32] = b0 + i < grid_len ? c[b0 + i] : 0u;
+  __syncthreads();
+  uint32_t sum = 0, total;
+  for (int i = 0; i < kRun; ++i) sum += tile[threadIdx.x * (kRun + 1) + i];
+  uint32_t run = sums[blockIdx.x] + block_scan(sum, sh, &total);
+  for (int i = 0; i < kRun; ++i) {
+    const uint32_t v = tile[threadIdx.x * (kRun + 1) + i];
+    tile[threadIdx.x * (kRun + 1) + i] = run;
+    run += v;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kScanTile; i += kScanThreads)
+    if (b0 + i < grid_len) c[b0 + i] = tile[i + i / 32];
+}
+
+// Every peak takes the next place of its bin, counting starts[bin + 1] up from the bin's
+// first place to its end, the next bin's first: what is left is slice_starts.
+__global__ void __launch_bounds__(256) place_peaks_kernel(
+    int64_t n_spec, const int64_t* __restrict__ list, const int64_t* __restrict__ item_off,
+    const int64_t* __restrict__ pstart, const int64_t* __restrict__ pstop, const int32_t* __restrict__ win,
+    const uint16_t* __restrict__ cyc, int win0, const BuildWin* __restrict__ wins, int64_t item0,
+    const float* __restrict__ inten, const uint32_t* __restrict__ bins, uint32_t* __restrict__ starts,
+    uint16_t* __restrict__ o_cyc, float* __restrict__ o_int, uint32_t* __restrict__ o_vis) {
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (warp >= n_spec) return;
+  const int64_t s = list[warp];
+  const BuildWin w = wins[win[s] - win0];
+  const int64_t b = pstart[s], n = pstop[s] - b;
+  const uint32_t* from = bins + (item_off[s] - item0);
+  uint32_t* next = starts + w.ss + 1;
+  const uint16_t c = cyc[s];
+  const uint32_t vis0 = (uint32_t)(item_off[s] - w.base);  // visit position in the observation
+  for (int64_t k = lane; k < n; k += 32) {
+    const uint32_t at = atomicAdd(next + from[k], 1u);
+    o_cyc[w.base + at] = c;
+    o_int[w.base + at] = __ldg(inten + b + k);
+    o_vis[w.base - item0 + at] = vis0 + (uint32_t)k;
+  }
+}
+
+__device__ __forceinline__ uint64_t entry_key(const uint16_t* cyc, const uint32_t* vis, int64_t i) {
+  return (uint64_t)cyc[i] << 32 | vis[i];
+}
+
+// One thread per bin: up to kBinSmall entries by insertion, larger bins listed.
+__global__ void __launch_bounds__(256) order_bins_kernel(int64_t grid_len, int n_win,
+                                                         const BuildWin* __restrict__ wins, int64_t item0,
+                                                         const uint32_t* __restrict__ starts,
+                                                         uint16_t* cyc, float* inten, uint32_t* vis,
+                                                         uint2* __restrict__ large,
+                                                         unsigned int* __restrict__ n_large) {
+  const int64_t total = grid_len * n_win;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int w = (int)(i / grid_len);
+    const int64_t b = i - w * grid_len;
+    const BuildWin bw = wins[w];
+    const uint32_t e0 = starts[bw.ss + b], n = starts[bw.ss + b + 1] - e0;
+    if (n < 2) continue;
+    if (n > kBinSmall) {
+      large[atomicAdd(n_large, 1u)] = make_uint2((unsigned)w, (unsigned)b);
+      continue;
+    }
+    uint16_t* c = cyc + bw.base + e0;
+    float* y = inten + bw.base + e0;
+    uint32_t* v = vis + (bw.base - item0) + e0;
+    for (uint32_t a = 1; a < n; ++a) {
+      const uint64_t key = entry_key(c, v, a);
+      uint32_t j = a;
+      if (entry_key(c, v, j - 1) < key) continue;
+      const float ya = y[a];
+      while (j > 0 && entry_key(c, v, j - 1) > key) {
+        c[j] = c[j - 1];
+        v[j] = v[j - 1];
+        y[j] = y[j - 1];
+        --j;
+      }
+      c[j] = (uint16_t)(key >> 32);
+      v[j] = (uint32_t)key;
+      y[j] = ya;
     }
   }
 }
 
-// counts[slot(w)][bin] += 1 for every sorted entry; cycles/intensities gathered.
-template <class V>
-__global__ void scatter_entries_kernel(int64_t n, const uint64_t* __restrict__ keys,
-                                       const V* __restrict__ vals,
-                                       const float* __restrict__ pint,
-                                       const int64_t* __restrict__ slot_of_win, int64_t stride,
-                                       uint32_t* __restrict__ counts, uint16_t* __restrict__ cycles,
-                                       float* __restrict__ intens) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t k = keys[i];
-    const int64_t w = (int64_t)(k >> kWinShift);
-    const uint32_t bin = (uint32_t)((k >> kBinShift) & ((1u << 22) - 1));
-    cycles[i] = (uint16_t)(k & 0xFFFFu);
-    intens[i] = __ldg(pint + vals[i]);
-    atomicAdd(counts + slot_of_win[w] * stride + bin, 1u);
+// Bitonic sort of n entries by a block, every exchange ascending (the first step of each
+// merge mirrored), so that the missing entries past n count as larger than all.
+__device__ void block_sort(uint16_t* c, float* y, uint32_t* v, uint32_t n) {
+  uint32_t p2 = 1;
+  while (p2 < n) p2 <<= 1;
+  for (uint32_t k = 2; k <= p2; k <<= 1) {
+    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+      const uint32_t flip = j == k >> 1 ? k - 1 : j;
+      for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+        const uint32_t o = i ^ flip;
+        if (o > i && o < n) {
+          const uint64_t a = entry_key(c, v, i), b = entry_key(c, v, o);
+          if (a > b) {
+            const float t = y[i];
+            y[i] = y[o];
+            y[o] = t;
+            c[i] = (uint16_t)(b >> 32);
+            v[i] = (uint32_t)b;
+            c[o] = (uint16_t)(a >> 32);
+            v[o] = (uint32_t)a;
+          }
+        }
+      }
+      __syncthreads();
+    }
   }
 }
 
-struct SegmentOf {
-  int64_t stride;
-  __host__ __device__ int64_t operator()(int64_t i) const { return i / stride; }
-};
+// The bins that order_bins_kernel listed, a block each.
+__global__ void __launch_bounds__(256) order_large_bins_kernel(const unsigned int* __restrict__ n_large,
+                                                               const uint2* __restrict__ large,
+                                                               const BuildWin* __restrict__ wins,
+                                                               int64_t item0,
+                                                               const uint32_t* __restrict__ starts,
+                                                               uint16_t* cyc, float* inten, uint32_t* vis) {
+  __shared__ float sy[kBinShared];
+  __shared__ uint32_t sv[kBinShared];
+  __shared__ uint16_t sc[kBinShared];
+  const unsigned int m = *n_large;
+  for (unsigned int l = blockIdx.x; l < m; l += gridDim.x) {
+    const uint2 id = large[l];
+    const BuildWin bw = wins[id.x];
+    const uint32_t e0 = starts[bw.ss + id.y], n = starts[bw.ss + id.y + 1] - e0;
+    uint16_t* c = cyc + bw.base + e0;
+    float* y = inten + bw.base + e0;
+    uint32_t* v = vis + (bw.base - item0) + e0;
+    if (n <= kBinShared) {
+      for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+        sc[i] = c[i];
+        sy[i] = y[i];
+        sv[i] = v[i];
+      }
+      __syncthreads();
+      block_sort(sc, sy, sv, n);
+      for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+        c[i] = sc[i];
+        y[i] = sy[i];
+      }
+      __syncthreads();
+    } else {
+      block_sort(c, y, v, n);
+    }
+  }
+}
 
 struct SpectrumTable {
   std::vector<int64_t> dsi, start, stop, cyc;
@@ -85,110 +300,110 @@ int fetch(const T* src, int64_t n, int loc, std::vector<T>& dst) {
   return ADS_OK;
 }
 
-template <class V>
+// Uploads the spectrum table (and host peak arrays), and builds cycles, intens and
+// slice_starts.  `list`: the spectra of window w in visit order from first_spec[w].
 int build_entries(AdsDia* d, const AdsRawArrays* raw, const std::vector<int32_t>& win_of_spec,
                   const std::vector<uint16_t>& cyc16, const std::vector<int64_t>& item_off,
-                  int64_t n_items, const std::vector<int64_t>& slot_of_win, int64_t n_slots,
-                  const GridView& g, cudaStream_t st) {
+                  int64_t n_items, const std::vector<int64_t>& list, const std::vector<int64_t>& first_spec,
+                  int64_t n_slots, const GridView& g, cudaStream_t st) {
   const int64_t n_spec = raw->n_spectra;
   const int64_t stride = d->grid_len + 1;
+  if (n_slots == 0 || n_items == 0) return ADS_OK;
   // device copies of the spectrum table and, if needed, the peak arrays
-  DevBuf<int64_t> d_off, d_start, d_stop, d_slot;
+  DevBuf<int64_t> d_off, d_start, d_stop;
   DevBuf<int32_t> d_win;
+  DevBuf<int64_t> d_list;
   DevBuf<uint16_t> d_cyc;
   DevBuf<float> d_mz, d_int;
   const float* mz = raw->peak_mz;
   const float* pint = raw->peak_intensity;
+  const int64_t *pstart = raw->spectrum_peak_start_idx, *pstop = raw->spectrum_peak_stop_idx;
   ADS_TRY(d_off.alloc(n_spec));
   ADS_TRY(d_win.alloc(n_spec));
   ADS_TRY(d_cyc.alloc(n_spec));
-  ADS_TRY(d_slot.alloc(slot_of_win.size()));
+  ADS_TRY(d_list.alloc(list.size()));
   ADS_CUDA(cudaMemcpyAsync(d_off.p, item_off.data(), n_spec * 8, cudaMemcpyHostToDevice, st));
   ADS_CUDA(cudaMemcpyAsync(d_win.p, win_of_spec.data(), n_spec * 4, cudaMemcpyHostToDevice, st));
   ADS_CUDA(cudaMemcpyAsync(d_cyc.p, cyc16.data(), n_spec * 2, cudaMemcpyHostToDevice, st));
-  ADS_CUDA(cudaMemcpyAsync(d_slot.p, slot_of_win.data(), slot_of_win.size() * 8,
-                           cudaMemcpyHostToDevice, st));
-  if (raw->location == ADS_MEM_DEVICE) {
+  ADS_CUDA(cudaMemcpyAsync(d_list.p, list.data(), list.size() * 8, cudaMemcpyHostToDevice, st));
+  if (raw->location != ADS_MEM_DEVICE) {
     ADS_TRY(d_start.alloc(n_spec));
     ADS_TRY(d_stop.alloc(n_spec));
-    ADS_CUDA(cudaMemcpyAsync(d_start.p, raw->spectrum_peak_start_idx, n_spec * 8,
-                             cudaMemcpyDeviceToDevice, st));
-    ADS_CUDA(cudaMemcpyAsync(d_stop.p, raw->spectrum_peak_stop_idx, n_spec * 8,
-                             cudaMemcpyDeviceToDevice, st));
-  } else {
-    ADS_TRY(d_start.alloc(n_spec));
-    ADS_TRY(d_stop.alloc(n_spec));
-    ADS_CUDA(cudaMemcpyAsync(d_start.p, raw->spectrum_peak_start_idx, n_spec * 8,
-                             cudaMemcpyHostToDevice, st));
-    ADS_CUDA(cudaMemcpyAsync(d_stop.p, raw->spectrum_peak_stop_idx, n_spec * 8,
-                             cudaMemcpyHostToDevice, st));
+    ADS_CUDA(cudaMemcpyAsync(d_start.p, pstart, n_spec * 8, cudaMemcpyHostToDevice, st));
+    ADS_CUDA(cudaMemcpyAsync(d_stop.p, pstop, n_spec * 8, cudaMemcpyHostToDevice, st));
     ADS_TRY(d_mz.alloc(raw->n_peaks));
     ADS_TRY(d_int.alloc(raw->n_peaks));
-    if (raw->n_peaks) {
-      ADS_CUDA(cudaMemcpyAsync(d_mz.p, raw->peak_mz, raw->n_peaks * 4, cudaMemcpyHostToDevice, st));
-      ADS_CUDA(cudaMemcpyAsync(d_int.p, raw->peak_intensity, raw->n_peaks * 4,
-                               cudaMemcpyHostToDevice, st));
-    }
+    ADS_CUDA(cudaMemcpyAsync(d_mz.p, raw->peak_mz, raw->n_peaks * 4, cudaMemcpyHostToDevice, st));
+    ADS_CUDA(cudaMemcpyAsync(d_int.p, raw->peak_intensity, raw->n_peaks * 4, cudaMemcpyHostToDevice, st));
+    pstart = d_start.p;
+    pstop = d_stop.p;
     mz = d_mz.p;
     pint = d_int.p;
   }
-
-  DevBuf<uint64_t> keys_a, keys_b;
-  DevBuf<V> vals_a, vals_b;
-  ADS_TRY(keys_a.alloc(n_items));
-  ADS_TRY(keys_b.alloc(n_items));
-  ADS_TRY(vals_a.alloc(n_items));
-  ADS_TRY(vals_b.alloc(n_items));
-  if (n_spec > 0 && n_items > 0) {
-    const int grid = (int)std::min<int64_t>(n_spec, 1 << 20);
-    bin_peaks_kernel<V><<<grid, 128, 0, st>>>(n_spec, d_off.p, d_start.p, d_stop.p, d_win.p,
-                                               d_cyc.p, mz, g, keys_a.p, vals_a.p);
-    ADS_LAUNCH_CHECK();
-  }
-  // stable LSD radix sort on (window, bin, cycle): equal keys keep visit order
-  int n_win_bits = 1;
-  while ((int64_t(1) << n_win_bits) < (int64_t)slot_of_win.size()) ++n_win_bits;
-  const int end_bit = kWinShift + n_win_bits;
-  size_t tmp_bytes = 0;
-  ADS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys_a.p, keys_b.p, vals_a.p,
-                                           vals_b.p, n_items, kBinShift - 16, end_bit, st));
-  DevBuf<unsigned char> tmp;
-  ADS_TRY(tmp.alloc(tmp_bytes + 16));
-  if (n_items > 0)
-    ADS_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tmp_bytes, keys_a.p, keys_b.p, vals_a.p,
-                                             vals_b.p, n_items, 0, end_bit, st));
-  keys_a.release();
-  vals_a.release();
-  tmp.release();
-
-  if (n_items > 0) {  // (16-byte copies may reach past the last entry)
-    ADS_TRY(d->cycles.alloc(n_items + kEntrySlack));
-    ADS_TRY(d->intens.alloc(n_items + kEntrySlack));
-  }
-  DevBuf<uint32_t> counts;
-  ADS_TRY(counts.alloc((size_t)(n_slots * stride)));
+  ADS_TRY(d->cycles.alloc(n_items + kEntrySlack));  // (16-byte copies may reach past the last entry)
+  ADS_TRY(d->intens.alloc(n_items + kEntrySlack));
   ADS_TRY(d->slice_starts.alloc((size_t)(n_slots * stride)));
-  if (n_slots > 0) {
-    ADS_CUDA(cudaMemsetAsync(counts.p, 0, counts.bytes(), st));
-    if (n_items > 0) {
-      scatter_entries_kernel<V><<<4 * 148 * 8, 256, 0, st>>>(n_items, keys_b.p, vals_b.p, pint,
-                                                             d_slot.p, stride, counts.p,
-                                                             d->cycles.p, d->intens.p);
-      ADS_LAUNCH_CHECK();
-    }
-    // per-observation exclusive scan of the bin counts -> slice_starts
-    cub::CountingInputIterator<int64_t> idx(0);
-    cub::TransformInputIterator<int64_t, SegmentOf, cub::CountingInputIterator<int64_t>> seg(
-        idx, SegmentOf{stride});
-    size_t sb = 0;
-    const int64_t total = n_slots * stride;
-    ADS_CUDA(cub::DeviceScan::ExclusiveSumByKey(nullptr, sb, seg, counts.p, d->slice_starts.p,
-                                                total, ::cuda::std::equal_to<>(), st));
-    DevBuf<unsigned char> stmp;
-    ADS_TRY(stmp.alloc(sb + 16));
-    ADS_CUDA(cub::DeviceScan::ExclusiveSumByKey(stmp.p, sb, seg, counts.p, d->slice_starts.p,
-                                                total, ::cuda::std::equal_to<>(), st));
-    ADS_CUDA(cudaStreamSynchronize(st));
+  ADS_CUDA(cudaMemsetAsync(d->slice_starts.p, 0, d->slice_starts.bytes(), st));
+
+  // the observations that hold peaks, in groups of up to kGroupItems peaks (or one)
+  struct Group {
+    int64_t w0, w1, items, specs;
+    int slots;
+  };
+  std::vector<Group> groups;
+  std::vector<BuildWin> wins((size_t)d->n_obs, BuildWin{0, 0});
+  int64_t most_items = 0;
+  int most_slots = 0;
+  for (int64_t w = 0; w < d->n_obs; ++w) {
+    wins[w] = BuildWin{d->win[w].ss_off, d->win[w].base};
+    if (d->num_peaks[w] == 0) continue;
+    if (groups.empty() || groups.back().items + d->num_peaks[w] > kGroupItems || groups.back().w1 != w)
+      groups.push_back(Group{w, w, 0, 0, 0});
+    Group& gr = groups.back();
+    gr.w1 = w + 1;
+    gr.items += d->num_peaks[w];
+    gr.specs += first_spec[w + 1] - first_spec[w];
+    ++gr.slots;
+    most_items = std::max(most_items, gr.items);
+    most_slots = std::max(most_slots, gr.slots);
+  }
+  const int tiles = (int)((d->grid_len + kScanTile - 1) / kScanTile);
+  DevBuf<BuildWin> d_wins;
+  DevBuf<uint32_t> bins, vis, sums;
+  DevBuf<uint2> large;
+  DevBuf<unsigned int> n_large;
+  ADS_TRY(d_wins.alloc(wins.size()));
+  ADS_TRY(bins.alloc((size_t)most_items));
+  ADS_TRY(vis.alloc((size_t)most_items));
+  ADS_TRY(sums.alloc((size_t)most_slots * tiles));
+  ADS_TRY(large.alloc((size_t)(most_items / (kBinSmall + 1) + 1)));
+  ADS_TRY(n_large.alloc(groups.size()));
+  ADS_CUDA(cudaMemcpyAsync(d_wins.p, wins.data(), wins.size() * sizeof(BuildWin), cudaMemcpyHostToDevice, st));
+  ADS_CUDA(cudaMemsetAsync(n_large.p, 0, n_large.bytes(), st));
+  for (size_t k = 0; k < groups.size(); ++k) {
+    const Group& gr = groups[k];
+    const int64_t item0 = d->win[gr.w0].base;
+    const BuildWin* gw = d_wins.p + gr.w0;
+    const int64_t* gl = d_list.p + first_spec[gr.w0];
+    const int sg = (int)((gr.specs + 7) / 8);
+    count_peaks_kernel<<<sg, 256, 0, st>>>(gr.specs, gl, d_off.p, pstart, pstop, d_win.p, (int)gr.w0, gw, item0,
+                                           mz, g, bins.p, d->slice_starts.p);
+    ADS_LAUNCH_CHECK();
+    tile_sums_kernel<<<gr.slots * tiles, kScanThreads, 0, st>>>(d->grid_len, tiles, gw, d->slice_starts.p, sums.p);
+    ADS_LAUNCH_CHECK();
+    scan_sums_kernel<<<gr.slots, kScanThreads, 0, st>>>(tiles, sums.p);
+    ADS_LAUNCH_CHECK();
+    scan_tiles_kernel<<<gr.slots * tiles, kScanThreads, 0, st>>>(d->grid_len, tiles, gw, sums.p, d->slice_starts.p);
+    ADS_LAUNCH_CHECK();
+    place_peaks_kernel<<<sg, 256, 0, st>>>(gr.specs, gl, d_off.p, pstart, pstop, d_win.p, d_cyc.p, (int)gr.w0, gw,
+                                           item0, pint, bins.p, d->slice_starts.p, d->cycles.p, d->intens.p, vis.p);
+    ADS_LAUNCH_CHECK();
+    order_bins_kernel<<<(int)std::min<int64_t>((d->grid_len * gr.slots + 255) / 256, 148 * 16), 256, 0, st>>>(
+        d->grid_len, gr.slots, gw, item0, d->slice_starts.p, d->cycles.p, d->intens.p, vis.p, large.p, n_large.p + k);
+    ADS_LAUNCH_CHECK();
+    order_large_bins_kernel<<<148 * 4, 256, 0, st>>>(n_large.p + k, large.p, gw, item0, d->slice_starts.p,
+                                                     d->cycles.p, d->intens.p, vis.p);
+    ADS_LAUNCH_CHECK();
   }
   ADS_CUDA(cudaStreamSynchronize(st));
   return ADS_OK;
@@ -297,10 +512,11 @@ int dia_create(const AdsRawArrays* raw, int device, AdsDia** out) {
   // per observation: isolation window of the first spectrum, unique cycles,
   // peak counts (src/dia_data_builder/mod.rs:57-91)
   std::vector<char> seen_first((size_t)n_obs, 0);
-  std::vector<std::pair<int64_t, int64_t>> wc;
-  wc.reserve((size_t)n_spec);
   std::vector<int32_t> win_of_spec((size_t)n_spec, -1);
   std::vector<uint16_t> cyc16((size_t)n_spec);
+  std::vector<int64_t> first_spec((size_t)n_obs + 1, 0);
+  std::vector<int64_t> last_cycle((size_t)n_obs, -1);
+  std::vector<char> unsorted((size_t)n_obs, 0);  // cycles that step back: counted below
   for (int64_t s = 0; s < n_spec; ++s) {
     cyc16[s] = (uint16_t)t.cyc[s];
     const int64_t w = t.dsi[s];
@@ -312,14 +528,31 @@ int dia_create(const AdsRawArrays* raw, int device, AdsDia** out) {
       d->win[w].hi = t.hi[s];
     }
     d->num_peaks[w] += t.stop[s] - t.start[s];
-    wc.emplace_back(w, t.cyc[s]);
+    ++first_spec[w + 1];
+    if (t.cyc[s] > last_cycle[w]) {
+      ++d->num_cycles[w];
+      last_cycle[w] = t.cyc[s];
+    } else if (t.cyc[s] < last_cycle[w]) {
+      unsorted[w] = 1;
+    }
   }
-  std::sort(wc.begin(), wc.end());
-  for (size_t i = 0; i < wc.size(); ++i)
-    if (i == 0 || wc[i] != wc[i - 1]) d->num_cycles[wc[i].first]++;
+  // spectra by window, in visit order
+  for (int64_t w = 0; w < n_obs; ++w) first_spec[w + 1] += first_spec[w];
+  std::vector<int64_t> spec_list((size_t)first_spec[n_obs]);
+  {
+    std::vector<int64_t> cursor(first_spec.begin(), first_spec.end() - 1);
+    for (int64_t s = 0; s < n_spec; ++s)
+      if (win_of_spec[s] >= 0) spec_list[cursor[win_of_spec[s]]++] = s;
+  }
+  for (int64_t w = 0; w < n_obs; ++w) {
+    if (!unsorted[w]) continue;
+    std::vector<int64_t> c;
+    for (int64_t k = first_spec[w]; k < first_spec[w + 1]; ++k) c.push_back(t.cyc[spec_list[k]]);
+    std::sort(c.begin(), c.end());
+    d->num_cycles[w] = std::unique(c.begin(), c.end()) - c.begin();
+  }
 
   // entry bases and slice_starts slots (observations without peaks get none)
-  std::vector<int64_t> slot_of_win((size_t)std::max<int64_t>(n_obs, 1), 0);
   int64_t n_slots = 0, n_items = 0;
   for (int64_t w = 0; w < n_obs; ++w) {
     if (d->num_peaks[w] > 0xFFFFFFFFll)
@@ -328,7 +561,7 @@ int dia_create(const AdsRawArrays* raw, int device, AdsDia** out) {
     n_items += d->num_peaks[w];
     if (d->num_peaks[w] > 0) {
       d->win[w].ss_off = n_slots * (d->grid_len + 1);
-      slot_of_win[w] = n_slots++;
+      ++n_slots;
     }
   }
   std::vector<int64_t> item_off((size_t)n_spec, 0);
@@ -375,13 +608,7 @@ int dia_create(const AdsRawArrays* raw, int device, AdsDia** out) {
   ADS_TRY(device_grid(device, &g));
   cudaStream_t st;
   ADS_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-  int rc;
-  if (n_peaks < (int64_t(1) << 32))
-    rc = build_entries<uint32_t>(d, raw, win_of_spec, cyc16, item_off, n_items, slot_of_win,
-                                 n_slots, g, st);
-  else
-    rc = build_entries<uint64_t>(d, raw, win_of_spec, cyc16, item_off, n_items, slot_of_win,
-                                 n_slots, g, st);
+  const int rc = build_entries(d, raw, win_of_spec, cyc16, item_off, n_items, spec_list, first_spec, n_slots, g, st);
   cudaStreamDestroy(st);
   if (rc != ADS_OK) return rc;
 
