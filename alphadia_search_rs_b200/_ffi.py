@@ -175,6 +175,7 @@ SIGNATURES = {
                                       C.c_int, C.c_int, C.POINTER(vp)]),
     "ads_quant_sizes": (C.c_int, [vp, C.POINTER(i64), C.POINTER(i64)]),
     "ads_quant_kernel_ms": (C.c_float, [vp]),
+    "ads_host_gather": (C.c_int, [C.c_int, vp, vp, vp, vp, vp, vp]),
     "ads_quant_copy_out": (C.c_int, [vp] + [vp] * 13),
     "ads_quant_destroy": (C.c_int, [vp]),
     "ads_idf_bins": (i64, []),

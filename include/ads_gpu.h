@@ -384,6 +384,13 @@ int ads_quantify_arrays(const AdsQuantParams* params, const AdsDia* dia, AdsLib*
 int ads_quant_sizes(const AdsQuant* quant, int64_t* n_precursors, int64_t* n_fragments);
 /* Device time of the quantification kernel in ms (an addition). */
 float ads_quant_kernel_ms(const AdsQuant* quant);
+/* Gathers rows of host columns with several host threads (an addition): column c's
+ * dst[c][i] = src[c][rows[c][i]] for i < n[c], elements of elem_size[c] (1, 4 or 8) bytes,
+ * src[c] of src_len[c] elements; rows[c] NULL copies src[c]'s first n[c] elements.  A row
+ * past src_len is ADS_ERR_INVALID_ARGUMENT. */
+int ads_host_gather(int n_cols, const void* const* src, const int64_t* src_len,
+                    const int32_t* elem_size, const uint64_t* const* rows, const int64_t* n,
+                    void* const* dst);
 /* Copies the SpecLibFlatQuantified layout into host arrays (any may be NULL): per
  * precursor (n_precursors, sorted by precursor_idx, ties in candidate order)
  * precursor_idx, the precursor's row in the arrays given to ads_lib_create, rank,
