@@ -17,18 +17,21 @@ namespace ads {
 namespace {
 
 // The entries are put in order by a counting sort, a few observations at a time: the bins
-// are counted in slice_starts itself, scanned in place, and every peak takes the next place
-// of its bin; then each bin's few entries are sorted by (cycle, visit position).  Peaks of
-// a group of observations, their counts and their places fit the L2, so what crosses the
-// memory bus is little more than the peaks once in and the entries once out, and the
-// temporary memory is one group's (64 MB).  A radix sort of (window, bin, cycle) keys with
-// peak indices moved 12 bytes a peak six times through 24 bytes a peak of temporaries:
-// 324 M peaks in 25 ms of kernels and 100 ms of mapping and unmapping that memory.
-constexpr int64_t kGroupItems = int64_t(1) << 23;
+// are counted in slice_starts itself, every peak keeping its number within its bin; the
+// counts are scanned in place; every peak goes to its place as one 16-byte record; and a
+// thread per bin puts its few records in (cycle, visit position) order and writes the
+// entries.  Peaks of a group of observations, their counts and records fit the L2, so what
+// crosses the memory bus is little more than the peaks once in and the entries once out,
+// and the temporary memory is one group's (100 MB).  A radix sort of (window, bin, cycle)
+// keys with peak indices moved 12 bytes a peak six times through 24 bytes a peak of
+// temporaries: 324 M peaks in 25 ms of kernels and 100 ms of mapping and unmapping that
+// memory.
+constexpr int64_t kGroupItems = int64_t(1) << 22;
 constexpr int kScanTile = 8192;       // bins of one scan block
 constexpr int kScanThreads = 256;
-constexpr int kBinSmall = 8;          // bins of up to this many entries are sorted by a thread
-constexpr int kBinShared = 1024;      // up to this many in shared memory, larger in place
+constexpr int kBinRegs = 4;           // bins of up to this many entries are sorted in registers
+constexpr int kBinThread = 24;        // up to this many by one thread in place
+constexpr int kBinShared = 1024;      // up to this many by a block in shared memory, else in place
 
 // One observation of a group.
 struct BuildWin {
@@ -36,8 +39,11 @@ struct BuildWin {
   int64_t base;     // its first entry
 };
 
-// One warp per spectrum (listed in window, then visit order): the bin of every peak, kept
-// for place_peaks_kernel, and the bins' counts, each one place up (see place_peaks_kernel).
+// A peak on its way to its bin: x intensity, y visit position in the observation, z cycle.
+__device__ __forceinline__ uint64_t record_key(const uint4& r) { return (uint64_t)r.z << 32 | r.y; }
+
+// One warp per spectrum (listed in window, then visit order): every peak's bin and its
+// number within the bin (in order of arrival, which is any).
 __global__ void __launch_bounds__(256) count_peaks_kernel(int64_t n_spec, const int64_t* __restrict__ list,
                                                           const int64_t* __restrict__ item_off,
                                                           const int64_t* __restrict__ pstart,
@@ -45,24 +51,24 @@ __global__ void __launch_bounds__(256) count_peaks_kernel(int64_t n_spec, const 
                                                           const int32_t* __restrict__ win, int win0,
                                                           const BuildWin* __restrict__ wins, int64_t item0,
                                                           const float* __restrict__ mz, GridView g,
-                                                          uint32_t* __restrict__ bins,
+                                                          uint2* __restrict__ bins,
                                                           uint32_t* __restrict__ starts) {
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= n_spec) return;
   const int64_t s = list[warp];
   const int64_t b = pstart[s], n = pstop[s] - b;
-  uint32_t* to = bins + (item_off[s] - item0);
+  uint2* to = bins + (item_off[s] - item0);
   uint32_t* count = starts + wins[win[s] - win0].ss + 1;
+#pragma unroll 2
   for (int64_t k = lane; k < n; k += 32) {
     const uint32_t bin = grid_find_closest(g, __ldg(mz + b + k));
-    to[k] = bin;
-    atomicAdd(count + bin, 1u);
+    to[k] = make_uint2(bin, atomicAdd(count + bin, 1u));
   }
 }
 
-// Exclusive scan of each observation's counts, in place: sums of tiles, their scan, the
-// tiles.  counts[b + 1] becomes the first place of bin b.
+// Inclusive scan of each observation's counts, in place: sums of tiles, their scan, the
+// tiles.  counts[b + 1] becomes the end of bin b, which is what slice_starts holds there.
 __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* sh, uint32_t* total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t incl = v;
@@ -139,87 +145,100 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles_kernel(int64_t grid_l
   uint32_t run = sums[blockIdx.x] + block_scan(sum, sh, &total);
   for (int i = 0; i < kRun; ++i) {
     const uint32_t v = tile[threadIdx.x * (kRun + 1) + i];
-    tile[threadIdx.x * (kRun + 1) + i] = run;
     run += v;
+    tile[threadIdx.x * (kRun + 1) + i] = run;
   }
   __syncthreads();
   for (int i = threadIdx.x; i < kScanTile; i += kScanThreads)
     if (b0 + i < grid_len) c[b0 + i] = tile[i + i / 32];
 }
 
-// Every peak takes the next place of its bin, counting starts[bin + 1] up from the bin's
-// first place to its end, the next bin's first: what is left is slice_starts.
+// Every peak to its place, as a record.
 __global__ void __launch_bounds__(256) place_peaks_kernel(
     int64_t n_spec, const int64_t* __restrict__ list, const int64_t* __restrict__ item_off,
     const int64_t* __restrict__ pstart, const int64_t* __restrict__ pstop, const int32_t* __restrict__ win,
     const uint16_t* __restrict__ cyc, int win0, const BuildWin* __restrict__ wins, int64_t item0,
-    const float* __restrict__ inten, const uint32_t* __restrict__ bins, uint32_t* __restrict__ starts,
-    uint16_t* __restrict__ o_cyc, float* __restrict__ o_int, uint32_t* __restrict__ o_vis) {
+    const float* __restrict__ inten, const uint2* __restrict__ bins, const uint32_t* __restrict__ starts,
+    uint4* __restrict__ recs) {
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= n_spec) return;
   const int64_t s = list[warp];
   const BuildWin w = wins[win[s] - win0];
   const int64_t b = pstart[s], n = pstop[s] - b;
-  const uint32_t* from = bins + (item_off[s] - item0);
-  uint32_t* next = starts + w.ss + 1;
-  const uint16_t c = cyc[s];
-  const uint32_t vis0 = (uint32_t)(item_off[s] - w.base);  // visit position in the observation
+  const uint2* from = bins + (item_off[s] - item0);
+  const uint32_t* first = starts + w.ss;
+  uint4* to = recs + (w.base - item0);
+  const uint32_t c = cyc[s];
+  const uint32_t vis0 = (uint32_t)(item_off[s] - w.base);
+#pragma unroll 4
   for (int64_t k = lane; k < n; k += 32) {
-    const uint32_t at = atomicAdd(next + from[k], 1u);
-    o_cyc[w.base + at] = c;
-    o_int[w.base + at] = __ldg(inten + b + k);
-    o_vis[w.base - item0 + at] = vis0 + (uint32_t)k;
+    const uint2 br = from[k];
+    to[__ldg(first + br.x) + br.y] =
+        make_uint4(__float_as_uint(__ldg(inten + b + k)), vis0 + (uint32_t)k, c, 0u);
   }
 }
 
-__device__ __forceinline__ uint64_t entry_key(const uint16_t* cyc, const uint32_t* vis, int64_t i) {
-  return (uint64_t)cyc[i] << 32 | vis[i];
+__device__ __forceinline__ void put_in_order(uint4& a, uint4& b) {
+  if (record_key(a) > record_key(b)) {
+    const uint4 t = a;
+    a = b;
+    b = t;
+  }
 }
 
-// One thread per bin: up to kBinSmall entries by insertion, larger bins listed.
-__global__ void __launch_bounds__(256) order_bins_kernel(int64_t grid_len, int n_win,
-                                                         const BuildWin* __restrict__ wins, int64_t item0,
-                                                         const uint32_t* __restrict__ starts,
-                                                         uint16_t* cyc, float* inten, uint32_t* vis,
-                                                         uint2* __restrict__ large,
+// One thread per bin: its records in order, and its entries.  Larger bins are listed.
+__global__ void __launch_bounds__(256) order_bins_kernel(int64_t grid_len, const BuildWin* __restrict__ wins,
+                                                         int64_t item0, const uint32_t* __restrict__ starts,
+                                                         uint4* recs, uint16_t* __restrict__ cyc,
+                                                         float* __restrict__ inten, uint2* __restrict__ large,
                                                          unsigned int* __restrict__ n_large) {
-  const int64_t total = grid_len * n_win;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int w = (int)(i / grid_len);
-    const int64_t b = i - w * grid_len;
-    const BuildWin bw = wins[w];
-    const uint32_t e0 = starts[bw.ss + b], n = starts[bw.ss + b + 1] - e0;
-    if (n < 2) continue;
-    if (n > kBinSmall) {
-      large[atomicAdd(n_large, 1u)] = make_uint2((unsigned)w, (unsigned)b);
-      continue;
-    }
-    uint16_t* c = cyc + bw.base + e0;
-    float* y = inten + bw.base + e0;
-    uint32_t* v = vis + (bw.base - item0) + e0;
-    for (uint32_t a = 1; a < n; ++a) {
-      const uint64_t key = entry_key(c, v, a);
-      uint32_t j = a;
-      if (entry_key(c, v, j - 1) < key) continue;
-      const float ya = y[a];
-      while (j > 0 && entry_key(c, v, j - 1) > key) {
-        c[j] = c[j - 1];
-        v[j] = v[j - 1];
-        y[j] = y[j - 1];
-        --j;
+  const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (b >= grid_len) return;
+  const BuildWin bw = wins[blockIdx.y];
+  const uint32_t e0 = starts[bw.ss + b], n = starts[bw.ss + b + 1] - e0;
+  if (n == 0) return;
+  if (n > kBinThread) {
+    large[atomicAdd(n_large, 1u)] = make_uint2(blockIdx.y, (unsigned)b);
+    return;
+  }
+  uint4* r = recs + (bw.base - item0) + e0;
+  uint16_t* c = cyc + bw.base + e0;
+  float* y = inten + bw.base + e0;
+  if (n <= kBinRegs) {
+    uint4 v[kBinRegs];
+#pragma unroll
+    for (int i = 0; i < kBinRegs; ++i)
+      v[i] = i < (int)n ? r[i] : make_uint4(0u, 0xffffffffu, 0xffffffffu, 0u);  // past every key
+    put_in_order(v[0], v[1]);
+    put_in_order(v[2], v[3]);
+    put_in_order(v[0], v[2]);
+    put_in_order(v[1], v[3]);
+    put_in_order(v[1], v[2]);
+#pragma unroll
+    for (int i = 0; i < kBinRegs; ++i)
+      if (i < (int)n) {
+        c[i] = (uint16_t)v[i].z;
+        y[i] = __uint_as_float(v[i].x);
       }
-      c[j] = (uint16_t)(key >> 32);
-      v[j] = (uint32_t)key;
-      y[j] = ya;
-    }
+    return;
+  }
+  for (uint32_t a = 1; a < n; ++a) {
+    const uint4 v = r[a];
+    uint32_t j = a;
+    for (; j > 0 && record_key(r[j - 1]) > record_key(v); --j) r[j] = r[j - 1];
+    r[j] = v;
+  }
+  for (uint32_t a = 0; a < n; ++a) {
+    const uint4 v = r[a];
+    c[a] = (uint16_t)v.z;
+    y[a] = __uint_as_float(v.x);
   }
 }
 
-// Bitonic sort of n entries by a block, every exchange ascending (the first step of each
-// merge mirrored), so that the missing entries past n count as larger than all.
-__device__ void block_sort(uint16_t* c, float* y, uint32_t* v, uint32_t n) {
+// Bitonic sort of n records by a block, every exchange ascending (the first step of each
+// merge mirrored), so that the missing records past n count as larger than all.
+__device__ void block_sort(uint4* r, uint32_t n) {
   uint32_t p2 = 1;
   while (p2 < n) p2 <<= 1;
   for (uint32_t k = 2; k <= p2; k <<= 1) {
@@ -228,15 +247,10 @@ __device__ void block_sort(uint16_t* c, float* y, uint32_t* v, uint32_t n) {
       for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
         const uint32_t o = i ^ flip;
         if (o > i && o < n) {
-          const uint64_t a = entry_key(c, v, i), b = entry_key(c, v, o);
-          if (a > b) {
-            const float t = y[i];
-            y[i] = y[o];
-            y[o] = t;
-            c[i] = (uint16_t)(b >> 32);
-            v[i] = (uint32_t)b;
-            c[o] = (uint16_t)(a >> 32);
-            v[o] = (uint32_t)a;
+          uint4 a = r[i], b = r[o];
+          if (record_key(a) > record_key(b)) {
+            r[i] = b;
+            r[o] = a;
           }
         }
       }
@@ -251,34 +265,26 @@ __global__ void __launch_bounds__(256) order_large_bins_kernel(const unsigned in
                                                                const BuildWin* __restrict__ wins,
                                                                int64_t item0,
                                                                const uint32_t* __restrict__ starts,
-                                                               uint16_t* cyc, float* inten, uint32_t* vis) {
-  __shared__ float sy[kBinShared];
-  __shared__ uint32_t sv[kBinShared];
-  __shared__ uint16_t sc[kBinShared];
+                                                               uint4* recs, uint16_t* __restrict__ cyc,
+                                                               float* __restrict__ inten) {
+  __shared__ uint4 tile[kBinShared];
   const unsigned int m = *n_large;
   for (unsigned int l = blockIdx.x; l < m; l += gridDim.x) {
     const uint2 id = large[l];
     const BuildWin bw = wins[id.x];
     const uint32_t e0 = starts[bw.ss + id.y], n = starts[bw.ss + id.y + 1] - e0;
-    uint16_t* c = cyc + bw.base + e0;
-    float* y = inten + bw.base + e0;
-    uint32_t* v = vis + (bw.base - item0) + e0;
+    uint4* r = recs + (bw.base - item0) + e0;
     if (n <= kBinShared) {
-      for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-        sc[i] = c[i];
-        sy[i] = y[i];
-        sv[i] = v[i];
-      }
+      for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) tile[i] = r[i];
       __syncthreads();
-      block_sort(sc, sy, sv, n);
-      for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-        c[i] = sc[i];
-        y[i] = sy[i];
-      }
-      __syncthreads();
-    } else {
-      block_sort(c, y, v, n);
+      r = tile;
     }
+    block_sort(r, n);
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+      cyc[bw.base + e0 + i] = (uint16_t)r[i].z;
+      inten[bw.base + e0 + i] = __uint_as_float(r[i].x);
+    }
+    __syncthreads();
   }
 }
 
@@ -357,7 +363,8 @@ int build_entries(AdsDia* d, const AdsRawArrays* raw, const std::vector<int32_t>
   for (int64_t w = 0; w < d->n_obs; ++w) {
     wins[w] = BuildWin{d->win[w].ss_off, d->win[w].base};
     if (d->num_peaks[w] == 0) continue;
-    if (groups.empty() || groups.back().items + d->num_peaks[w] > kGroupItems || groups.back().w1 != w)
+    if (groups.empty() || groups.back().items + d->num_peaks[w] > kGroupItems || groups.back().w1 != w ||
+        groups.back().slots == 1024)  // (slots are a grid dimension)
       groups.push_back(Group{w, w, 0, 0, 0});
     Group& gr = groups.back();
     gr.w1 = w + 1;
@@ -369,14 +376,15 @@ int build_entries(AdsDia* d, const AdsRawArrays* raw, const std::vector<int32_t>
   }
   const int tiles = (int)((d->grid_len + kScanTile - 1) / kScanTile);
   DevBuf<BuildWin> d_wins;
-  DevBuf<uint32_t> bins, vis, sums;
-  DevBuf<uint2> large;
+  DevBuf<uint32_t> sums;
+  DevBuf<uint2> bins, large;
+  DevBuf<uint4> recs;
   DevBuf<unsigned int> n_large;
   ADS_TRY(d_wins.alloc(wins.size()));
   ADS_TRY(bins.alloc((size_t)most_items));
-  ADS_TRY(vis.alloc((size_t)most_items));
+  ADS_TRY(recs.alloc((size_t)most_items));
   ADS_TRY(sums.alloc((size_t)most_slots * tiles));
-  ADS_TRY(large.alloc((size_t)(most_items / (kBinSmall + 1) + 1)));
+  ADS_TRY(large.alloc((size_t)(most_items / (kBinThread + 1) + 1)));
   ADS_TRY(n_large.alloc(groups.size()));
   ADS_CUDA(cudaMemcpyAsync(d_wins.p, wins.data(), wins.size() * sizeof(BuildWin), cudaMemcpyHostToDevice, st));
   ADS_CUDA(cudaMemsetAsync(n_large.p, 0, n_large.bytes(), st));
@@ -396,13 +404,13 @@ int build_entries(AdsDia* d, const AdsRawArrays* raw, const std::vector<int32_t>
     scan_tiles_kernel<<<gr.slots * tiles, kScanThreads, 0, st>>>(d->grid_len, tiles, gw, sums.p, d->slice_starts.p);
     ADS_LAUNCH_CHECK();
     place_peaks_kernel<<<sg, 256, 0, st>>>(gr.specs, gl, d_off.p, pstart, pstop, d_win.p, d_cyc.p, (int)gr.w0, gw,
-                                           item0, pint, bins.p, d->slice_starts.p, d->cycles.p, d->intens.p, vis.p);
+                                           item0, pint, bins.p, d->slice_starts.p, recs.p);
     ADS_LAUNCH_CHECK();
-    order_bins_kernel<<<(int)std::min<int64_t>((d->grid_len * gr.slots + 255) / 256, 148 * 16), 256, 0, st>>>(
-        d->grid_len, gr.slots, gw, item0, d->slice_starts.p, d->cycles.p, d->intens.p, vis.p, large.p, n_large.p + k);
+    order_bins_kernel<<<dim3((unsigned)((d->grid_len + 255) / 256), (unsigned)gr.slots), 256, 0, st>>>(
+        d->grid_len, gw, item0, d->slice_starts.p, recs.p, d->cycles.p, d->intens.p, large.p, n_large.p + k);
     ADS_LAUNCH_CHECK();
     order_large_bins_kernel<<<148 * 4, 256, 0, st>>>(n_large.p + k, large.p, gw, item0, d->slice_starts.p,
-                                                     d->cycles.p, d->intens.p, vis.p);
+                                                     recs.p, d->cycles.p, d->intens.p);
     ADS_LAUNCH_CHECK();
   }
   ADS_CUDA(cudaStreamSynchronize(st));
