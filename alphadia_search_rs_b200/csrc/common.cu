@@ -92,6 +92,25 @@ int pool_alloc(int device, size_t bytes, void** out) {
   return ADS_OK;
 }
 
+int pool_alloc_async(int device, size_t bytes, cudaStream_t st, void** out) {
+  *out = nullptr;
+  DevicePool dp;
+  ADS_TRY(device_pool(device, &dp));
+  const cudaError_t e = cudaMallocFromPoolAsync(out, bytes, dp.pool, st);
+  if (e != cudaSuccess) {
+    *out = nullptr;
+    return cuda_fail(e, "cudaMallocFromPoolAsync", __FILE__, __LINE__);
+  }
+  update_release_threshold(dp.pool);
+  return ADS_OK;
+}
+
+void pool_free_idle(int device, void* p) {
+  DevicePool dp;
+  if (device_pool(device, &dp) != ADS_OK) return;
+  pool_free_async(device, p, dp.stream);
+}
+
 void pool_free(int device, void* p) {
   DevicePool dp;
   if (device_pool(device, &dp) != ADS_OK) return;

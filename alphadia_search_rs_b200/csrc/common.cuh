@@ -78,6 +78,11 @@ void pool_free(int device, void* p);
 // memory that only `st` uses.
 void pool_free_async(int device, void* p, cudaStream_t st);
 
+// Memory for `st` only, from where it stands: no host synchronisation.
+int pool_alloc_async(int device, size_t bytes, cudaStream_t st, void** out);
+// Frees p, which no work in flight uses: no host synchronisation.
+void pool_free_idle(int device, void* p);
+
 // Owning device buffer (move-only) on the current device's pool.
 template <class T>
 struct DevBuf {
@@ -114,6 +119,25 @@ struct DevBuf {
     p = nullptr;
     n = 0;
   }
+  // release() for a buffer that no work in flight uses.
+  void release_idle() {
+    if (p) pool_free_idle(dev, p);
+    p = nullptr;
+    n = 0;
+  }
+  // alloc() for a buffer that `st` uses first (any other stream after an event of `st`).
+  int alloc_on(size_t count, cudaStream_t st) {
+    release();
+    if (count == 0) return ADS_OK;
+    int d = 0;
+    ADS_CUDA(cudaGetDevice(&d));
+    void* q = nullptr;
+    ADS_TRY(pool_alloc_async(d, count * sizeof(T), st, &q));
+    p = static_cast<T*>(q);
+    n = count;
+    dev = d;
+    return ADS_OK;
+  }
   // Allocates exactly `count` elements on the current device (frees the previous
   // buffer).
   int alloc(size_t count) {
@@ -131,6 +155,20 @@ struct DevBuf {
   // Grows to at least `count` elements, keeping nothing.
   int reserve(size_t count) { return count <= n ? ADS_OK : alloc(count); }
   size_t bytes() const { return n * sizeof(T); }
+};
+
+// A call's temporary memory on one stream: allocated and freed in its order (an allocation
+// with a host synchronisation and a release after a device-wide one took 10 to 15 us each,
+// more than the kernels of a small call between them).
+template <class T>
+struct TmpBuf : DevBuf<T> {
+  cudaStream_t st;
+  explicit TmpBuf(cudaStream_t s) : st(s) {}
+  ~TmpBuf() { this->release_async(st); }
+  int alloc(size_t count) {
+    this->release_async(st);
+    return this->alloc_on(count, st);
+  }
 };
 
 // ---------------------------------------------------------------- m/z grid
@@ -409,8 +447,11 @@ struct AdsCandidates {
   bool pending = false;
   ~AdsCandidates() {
     if (done) {
-      cudaEventSynchronize(done);
+      // the last search into the buffers has ended, and every reader waits for its own
+      // copies or kernels before it returns: nothing uses them any more
+      const bool ended = cudaEventSynchronize(done) == cudaSuccess;
       cudaEventDestroy(done);
+      if (ended) arena.release_idle();
     }
   }
 };

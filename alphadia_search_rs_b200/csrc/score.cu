@@ -40,7 +40,10 @@ struct AdsFeatures {
   uint64_t* rank_p = nullptr;
   float* feat_p = nullptr;  // feature k of row q at k * n + q
   uint8_t* found_p = nullptr;
-  std::vector<uint8_t> found;
+  bool idle = false;  // set once filled: every call that uses the memory ends synchronised
+  ~AdsFeatures() {
+    if (idle) arena.release_idle();
+  }
   float kernel_ms = 0.0f;  // CUDA-event time of score_kernel
 };
 
@@ -65,6 +68,12 @@ struct AdsQuant {
   float* p_rt = nullptr;
   uint64_t *f_row = nullptr, *f_pidx = nullptr, *f_rank = nullptr;
   float* f_val[4] = {nullptr, nullptr, nullptr, nullptr};
+  bool idle = false;  // as in AdsFeatures
+  ~AdsQuant() {
+    if (!idle) return;
+    arena.release_idle();
+    flat.release_idle();
+  }
 };
 
 namespace ads {
@@ -436,7 +445,7 @@ __global__ void work_key_kernel(int64_t n, const uint64_t* c_pidx, int64_t P, co
 
 // The candidates' work order (ScoreArgs::order): indices stably sorted by work_key_kernel's
 // key.  `buf` receives the order and holds the sort's temporaries.
-int work_order(int64_t n, const uint64_t* c_pidx, const AdsLib* l, cudaStream_t st, DevBuf<char>* buf,
+int work_order(int64_t n, const uint64_t* c_pidx, const AdsLib* l, cudaStream_t st, TmpBuf<char>* buf,
                const uint32_t** order) {
   *order = nullptr;
   // nothing to group when every precursor has the same number of library fragments
@@ -1046,7 +1055,7 @@ int quant_assemble(AdsQuant* r, const uint64_t* d_off, const int* d_pos, cudaStr
   r->f_rank = reinterpret_cast<uint64_t*>(take(bF8));
   for (int k = 0; k < 4; ++k) r->f_val[k] = reinterpret_cast<float*>(take(bF4));
   // temporaries: unsorted precursor columns, permutation, sort space
-  DevBuf<char> tmp;
+  TmpBuf<char> tmp(st);
   ADS_TRY(tmp.alloc(6 * bP8 + bP4 + 2 * bP4 + rnd(sort_bytes)));
   b = tmp.p;
   uint64_t* u_idx = reinterpret_cast<uint64_t*>(take(bP8));
@@ -1073,7 +1082,7 @@ int quant_assemble(AdsQuant* r, const uint64_t* d_off, const int* d_pos, cudaStr
       P, perm, u_row, u_rank, u_rt, u_fs, u_fe, r->p_row, r->p_rank, r->p_rt, r->p_fs, r->p_fe);
   ADS_LAUNCH_CHECK();
   ADS_CUDA(cudaStreamSynchronize(st));
-  r->arena.release();  // the per-candidate slots are no longer needed
+  r->arena.release_idle();  // the per-candidate slots are no longer needed
   return ADS_OK;
 }
 
@@ -1113,6 +1122,15 @@ int ensure_idf(AdsLib* l, const GridView& g, cudaStream_t st) {
   return ADS_OK;
 }
 
+__global__ void count_found_kernel(int64_t n, const uint8_t* found, int* out) {
+  int v = 0;
+  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n;
+       q += (int64_t)gridDim.x * blockDim.x)
+    v += found[q];
+  v = (int)__reduce_add_sync(0xffffffffu, (unsigned)v);
+  if ((threadIdx.x & 31) == 0 && v) atomicAdd(out, v);
+}
+
 int score_device(const AdsScoringParams* p, const AdsDia* d, AdsLib* l, int64_t n,
                  const uint64_t* pidx, const uint64_t* rank, const float* score,
                  const uint64_t* center, const uint64_t* start, const uint64_t* stop, int64_t c_max,
@@ -1138,9 +1156,9 @@ int score_device(const AdsScoringParams* p, const AdsDia* d, AdsLib* l, int64_t 
   f->rank_p = reinterpret_cast<uint64_t*>(f->arena.p + b8);
   f->feat_p = reinterpret_cast<float*>(f->arena.p + 2 * b8);
   f->found_p = reinterpret_cast<uint8_t*>(f->arena.p + 2 * b8 + b4);
-  DevBuf<int> err;
-  ADS_TRY(err.alloc(1));
-  ADS_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), st));
+  TmpBuf<int> err(st);  // error word, candidates found
+  ADS_TRY(err.alloc(2));
+  ADS_CUDA(cudaMemsetAsync(err.p, 0, 2 * sizeof(int), st));
   struct Events {
     cudaEvent_t a = nullptr, b = nullptr;
     ~Events() {
@@ -1155,7 +1173,7 @@ int score_device(const AdsScoringParams* p, const AdsDia* d, AdsLib* l, int64_t 
     const BlockPlan plan = block_plan(Fm, Fraw, Cm);
     const int group = block_group(d, plan, c_max);
     int64_t T = 0;
-    DevBuf<uint32_t> scratch;
+    TmpBuf<uint32_t> scratch(st);
     if (group == 0) {
       const int64_t words = scratch_words(Fm, Fraw, Cm);
       int n_sm = 0;
@@ -1204,7 +1222,7 @@ int score_device(const AdsScoringParams* p, const AdsDia* d, AdsLib* l, int64_t 
     a.Fraw = Fraw;
     a.Cm = Cm;
     a.scratch = scratch.p;
-    DevBuf<char> order_buf;  // candidates grouped by work (kept until the kernel is done)
+    TmpBuf<char> order_buf(st);  // candidates grouped by work (kept until the kernel is done)
     ADS_TRY(work_order(n, pidx, l, st, &order_buf, &a.order));
     a.T = T;
     a.o_pidx = f->pidx_p;
@@ -1214,8 +1232,8 @@ int score_device(const AdsScoringParams* p, const AdsDia* d, AdsLib* l, int64_t 
     a.err = err.p;
     ADS_CUDA(cudaEventCreate(&ev.a));
     ADS_CUDA(cudaEventCreate(&ev.b));
-    DevBuf<uint32_t> heads;
-    DevBuf<BlockCand> cands;
+    TmpBuf<uint32_t> heads(st);
+    TmpBuf<BlockCand> cands(st);
     if (group > 0) {
       ADS_TRY(heads.alloc((size_t)n * plan.head));
       ADS_TRY(cands.alloc((size_t)n));
@@ -1235,17 +1253,19 @@ int score_device(const AdsScoringParams* p, const AdsDia* d, AdsLib* l, int64_t 
       score_kernel<false><<<(int)((T + kScoreBlock - 1) / kScoreBlock), kScoreBlock, 0, st>>>(a);
     ADS_LAUNCH_CHECK();
     ADS_CUDA(cudaEventRecord(ev.b, st));
-    f->found.resize((size_t)n);
-    ADS_CUDA(cudaMemcpyAsync(f->found.data(), f->found_p, (size_t)n, cudaMemcpyDeviceToHost, st));
+    count_found_kernel<<<(int)std::min<int64_t>((n + 255) / 256, 592), 256, 0, st>>>(n, f->found_p, err.p + 1);
+    ADS_LAUNCH_CHECK();
   }
-  int herr = 0;
-  ADS_CUDA(cudaMemcpyAsync(&herr, err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+  int h[2] = {0, 0};
+  ADS_CUDA(cudaMemcpyAsync(h, err.p, sizeof(h), cudaMemcpyDeviceToHost, st));
   ADS_CUDA(cudaStreamSynchronize(st));
+  const int herr = h[0];
   if (herr & 1)
     return fail(ADS_ERR_INVALID_ARGUMENT,
                 "candidate cycle range outside the run's RT index (or cycle_start > cycle_stop)");
   if (herr & 2) return fail(ADS_ERR_INTERNAL, "fragment count above the scratch plan");
-  for (uint8_t v : f->found) f->count += v;
+  f->count = (int64_t)(uint32_t)h[1];
+  f->idle = true;
   if (n > 0) ADS_CUDA(cudaEventElapsedTime(&f->kernel_ms, ev.a, ev.b));
   if (verbose && n > 0) {
     // src/peak_group_scoring/mod.rs:91-98
@@ -1273,7 +1293,7 @@ int quant_device(const AdsQuantParams* p, const AdsDia* d, AdsLib* l, int64_t n,
   auto r = std::make_unique<AdsQuant>();
   r->device = d->device;
   r->n = n;
-  DevBuf<int> tmp;
+  TmpBuf<int> tmp(st);
   ADS_TRY(tmp.alloc(2));
   ADS_CUDA(cudaMemsetAsync(tmp.p, 0, 8, st));
   int64_t c_max = 0;
@@ -1320,7 +1340,7 @@ int quant_device(const AdsQuantParams* p, const AdsDia* d, AdsLib* l, int64_t n,
     const BlockPlan plan = block_plan(Fm, Fraw, Cm);
     const int group = block_group(d, plan, c_max);
     int64_t T = 0;
-    DevBuf<uint32_t> scratch;
+    TmpBuf<uint32_t> scratch(st);
     if (group == 0) {
       const int64_t words = scratch_words(Fm, Fraw, Cm);
       int n_sm = 0;
@@ -1364,7 +1384,7 @@ int quant_device(const AdsQuantParams* p, const AdsDia* d, AdsLib* l, int64_t n,
     a.Fraw = Fraw;
     a.Cm = Cm;
     a.scratch = scratch.p;
-    DevBuf<char> order_buf;  // candidates grouped by work (kept until the kernel is done)
+    TmpBuf<char> order_buf(st);  // candidates grouped by work (kept until the kernel is done)
     ADS_TRY(work_order(n, pidx, l, st, &order_buf, &a.order));
     a.T = T;
     a.err = tmp.p + 1;
@@ -1403,7 +1423,7 @@ int quant_device(const AdsQuantParams* p, const AdsDia* d, AdsLib* l, int64_t n,
     ADS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, b1, frag_in, (uint64_t*)nullptr, (int)n, st));
     ADS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, b2, prec_in, (int*)nullptr, (int)n, st));
     const size_t bo = rnd((size_t)n * 8), bpos = rnd((size_t)n * 4);
-    DevBuf<char> scan;
+    TmpBuf<char> scan(st);
     ADS_TRY(scan.alloc(bo + bpos + 256 + rnd(std::max(b1, b2))));
     uint64_t* d_off = reinterpret_cast<uint64_t*>(scan.p);
     int* d_pos = reinterpret_cast<int*>(scan.p + bo);
@@ -1429,6 +1449,8 @@ int quant_device(const AdsQuantParams* p, const AdsDia* d, AdsLib* l, int64_t n,
     if (r->n_prec > INT_MAX) return fail(ADS_ERR_INVALID_ARGUMENT, "too many quantified precursors");
     ADS_TRY(quant_assemble(r.get(), d_off, d_pos, st));
   }
+  ADS_CUDA(cudaStreamSynchronize(st));
+  r->idle = true;
   if (verbose) {
     // src/peak_group_quantification/mod.rs:73-78 (the kernel's device time)
     printf("Peak group quantification completed in %.2fs for %lld precursors\n",
@@ -1465,7 +1487,7 @@ int ads_score(const AdsScoringParams* params, const AdsDia* dia, AdsLib* lib, Ad
     DeviceGuard dg(dia->device);
     int64_t c_max = 0;
     if (n > 0) {
-      DevBuf<int> tmp;
+      TmpBuf<int> tmp(cudaStreamPerThread);
       ADS_TRY(tmp.alloc(2));
       ADS_CUDA(cudaMemsetAsync(tmp.p, 0, 8, cudaStreamPerThread));
       cycle_span_kernel<<<(int)std::min<int64_t>((n + 255) / 256, 4096), 256, 0, cudaStreamPerThread>>>(
@@ -1498,8 +1520,8 @@ int ads_score_arrays(const AdsScoringParams* params, const AdsDia* dia, AdsLib* 
     DeviceGuard dg(dia->device);
     cudaStream_t st = cudaStreamPerThread;
     const size_t n1 = (size_t)std::max<int64_t>(n, 1);
-    DevBuf<uint64_t> cols;
-    DevBuf<float> sc;
+    TmpBuf<uint64_t> cols(st);
+    TmpBuf<float> sc(st);
     ADS_TRY(cols.alloc(5 * n1));
     ADS_TRY(sc.alloc(n1));
     const cudaMemcpyKind kind = location == ADS_MEM_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
@@ -1509,7 +1531,7 @@ int ads_score_arrays(const AdsScoringParams* params, const AdsDia* dia, AdsLib* 
       for (int k = 0; k < 5; ++k)
         ADS_CUDA(cudaMemcpyAsync(cols.p + k * n1, src[k], (size_t)n * 8, kind, st));
       ADS_CUDA(cudaMemcpyAsync(sc.p, score, (size_t)n * 4, kind, st));
-      DevBuf<int> tmp;
+      TmpBuf<int> tmp(st);
       ADS_TRY(tmp.alloc(2));
       ADS_CUDA(cudaMemsetAsync(tmp.p, 0, 8, st));
       cycle_span_kernel<<<(int)std::min<int64_t>((n + 255) / 256, 4096), 256, 0, st>>>(
@@ -1545,13 +1567,15 @@ int ads_features_copy_out(const AdsFeatures* f, uint64_t* precursor_idx, uint64_
     }
     std::vector<uint64_t> p(n), r(n);
     std::vector<float> x(n * kFeatures);
+    std::vector<uint8_t> found(n);
+    ADS_CUDA(cudaMemcpy(found.data(), f->found_p, n, cudaMemcpyDeviceToHost));
     ADS_CUDA(cudaMemcpy(p.data(), f->pidx_p, n * 8, cudaMemcpyDeviceToHost));
     ADS_CUDA(cudaMemcpy(r.data(), f->rank_p, n * 8, cudaMemcpyDeviceToHost));
     ADS_CUDA(cudaMemcpy(x.data(), f->feat_p, n * 4 * kFeatures, cudaMemcpyDeviceToHost));
     const size_t m = (size_t)f->count;
     size_t o = 0;
     for (size_t q = 0; q < n; ++q) {
-      if (!f->found[q]) continue;
+      if (!found[q]) continue;
       if (precursor_idx) precursor_idx[o] = p[q];
       if (rank) rank[o] = r[q];
       if (features)
@@ -1614,7 +1638,7 @@ int ads_quantify_arrays(const AdsQuantParams* params, const AdsDia* dia, AdsLib*
     DeviceGuard dg(dia->device);
     cudaStream_t st = cudaStreamPerThread;
     const size_t n1 = (size_t)std::max<int64_t>(n, 1);
-    DevBuf<uint64_t> cols;
+    TmpBuf<uint64_t> cols(st);
     ADS_TRY(cols.alloc(5 * n1));
     const cudaMemcpyKind kind = location == ADS_MEM_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
     if (n > 0) {

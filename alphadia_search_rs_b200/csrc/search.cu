@@ -759,11 +759,12 @@ int need_f32_intensities(const AdsDia* d, const char* what) {
                                   "intensities only (built with BF16-only storage)");
 }
 
-int reserve_candidates(AdsCandidates* c, int64_t cap) {
+int reserve_candidates(AdsCandidates* c, int64_t cap, cudaStream_t st) {
   if (c->cap >= cap) return ADS_OK;
   const size_t n = (size_t)std::max<int64_t>(cap, 1);
   const size_t col8 = (n * 8 + 255) / 256 * 256, col4 = (n * 4 + 255) / 256 * 256;
-  ADS_TRY(c->arena.alloc(5 * col8 + col4 + 256));
+  // (readers on other streams wait for the search's event)
+  ADS_TRY(c->arena.alloc_on(5 * col8 + col4 + 256, st));
   char* q = c->arena.p;
   c->pidx_p = reinterpret_cast<uint64_t*>(q);
   c->rank_p = reinterpret_cast<uint64_t*>(q + col8);
@@ -815,7 +816,7 @@ int enqueue_search(AdsSelection* s, const AdsDia* d, const AdsLib* l, AdsCandida
   const int kf = (int)std::max<int64_t>(1, std::min<int64_t>(prm.top_k_fragments, l->max_frag));
   const int maxw = std::max(1, d->max_overlap);
 
-  ADS_TRY(reserve_candidates(c, P * (int64_t)k_out));
+  ADS_TRY(reserve_candidates(c, P * (int64_t)k_out, st));
   ADS_CUDA(cudaMemsetAsync(c->count_p, 0, 16, st));  // and err_p behind it
   c->pending = true;
   c->count = 0;
