@@ -157,7 +157,8 @@ const std::vector<float>& host_grid() {
 namespace {
 struct DeviceGridStore {
   float* grid = nullptr;
-  uint32_t* lut = nullptr;
+  GridRun* runs = nullptr;
+  uint8_t* run_of = nullptr;
   GridView view;
 };
 std::mutex g_grid_mu;
@@ -168,10 +169,30 @@ uint32_t bits_of(float x) {
   std::memcpy(&u, &x, 4);
   return u;
 }
-float float_of(uint32_t u) {
-  float x;
-  std::memcpy(&x, &u, 4);
-  return x;
+
+// The runs of equal steps of the grid's bit patterns, and the run of every 2^kRunShift-th
+// pattern; false if the grid is not made that way (it is, whatever libm: it is built from
+// products and sums alone).
+bool grid_runs(const std::vector<float>& g, std::vector<GridRun>* runs, std::vector<uint8_t>* run_of) {
+  for (size_t i = 0; i + 1 < g.size();) {
+    const uint32_t b = bits_of(g[i]), step = bits_of(g[i + 1]) - b;
+    size_t j = i + 1;
+    while (j + 1 < g.size() && bits_of(g[j + 1]) - bits_of(g[j]) == step) ++j;
+    if (step < 2 || step > 255 || i >= (1u << 24)) return false;
+    runs->push_back(GridRun{b, bits_of(g[j]), (uint32_t)((uint64_t(1) << 32) / step) + 1,
+                            (uint32_t)i | step << 24});
+    if ((uint64_t)(bits_of(g[j]) - b) * step >> 32) return false;
+    i = j;
+  }
+  // the last point starts a run of its own, which no lookup leaves
+  runs->push_back(GridRun{bits_of(g.back()), 0xffffffffu, uint32_t(1) << 31, (uint32_t)(g.size() - 1) | 2u << 24});
+  if (runs->size() > 255) return false;
+  size_t k = 0;
+  for (uint64_t p = bits_of(g[0]); p <= bits_of(g.back()); p += 1u << kRunShift) {
+    while ((*runs)[k].next <= p) ++k;
+    run_of->push_back((uint8_t)k);
+  }
+  return true;
 }
 }  // namespace
 
@@ -184,29 +205,25 @@ int device_grid(int device, GridView* out) {
   }
   const auto& g = host_grid();
   const uint32_t n = (uint32_t)g.size();
-  const uint32_t b0 = bits_of(g[0]);
-  const uint32_t n_lut = ((bits_of(g[n - 1]) - b0) >> kLutShift) + 2;
-  std::vector<uint32_t> lut(n_lut);
-  size_t pos = 0;
-  for (uint32_t k = 0; k < n_lut; ++k) {
-    float t = float_of(b0 + (k << kLutShift));
-    while (pos < n && g[pos] < t) ++pos;  // lower_bound, monotone in k
-    lut[k] = (uint32_t)pos;
-  }
+  std::vector<GridRun> runs;
+  std::vector<uint8_t> run_of;
+  if (!grid_runs(g, &runs, &run_of)) return fail(ADS_ERR_INTERNAL, "the m/z grid is not made of runs of equal steps");
   DeviceGuard dg(device);
   DeviceGridStore st;
   ADS_CUDA(cudaMalloc(&st.grid, n * sizeof(float)));
-  ADS_CUDA(cudaMalloc(&st.lut, n_lut * sizeof(uint32_t)));
+  ADS_CUDA(cudaMalloc(&st.runs, runs.size() * sizeof(GridRun)));
+  ADS_CUDA(cudaMalloc(&st.run_of, run_of.size()));
   ADS_CUDA(cudaMemcpy(st.grid, g.data(), n * sizeof(float), cudaMemcpyHostToDevice));
-  ADS_CUDA(cudaMemcpy(st.lut, lut.data(), n_lut * sizeof(uint32_t), cudaMemcpyHostToDevice));
+  ADS_CUDA(cudaMemcpy(st.runs, runs.data(), runs.size() * sizeof(GridRun), cudaMemcpyHostToDevice));
+  ADS_CUDA(cudaMemcpy(st.run_of, run_of.data(), run_of.size(), cudaMemcpyHostToDevice));
   // copies from pageable memory may return before their DMA ends, and the kernels
   // that read the grid run on non-blocking streams
   ADS_CUDA(cudaDeviceSynchronize());
   st.view.grid = st.grid;
-  st.view.lut = st.lut;
+  st.view.runs = st.runs;
+  st.view.run_of = st.run_of;
   st.view.n = n;
-  st.view.n_lut = n_lut;
-  st.view.bits0 = b0;
+  st.view.bits0 = bits_of(g[0]);
   st.view.first = g[0];
   st.view.last = g[n - 1];
   g_grids[device] = st;

@@ -172,16 +172,25 @@ struct TmpBuf : DevBuf<T> {
 };
 
 // ---------------------------------------------------------------- m/z grid
-// The global 1-ppm grid (src/mz_index/mod.rs:4-25) and a coarse lookup table
-// over the grid's float bit patterns that brackets any lower/upper bound to a
-// handful of grid points.
-constexpr int kLutShift = 6;
+// The global 1-ppm grid (src/mz_index/mod.rs:4-25).  Each of its steps, cur * 1e-6 rounded
+// to cur's last place, is a whole number of such places (8 to 17), and the number changes
+// only 39 times between 150 and 2000 m/z: the float bit patterns of the 2.6 M points are 40
+// arithmetic sequences.  A bound is found from its sequence by one division, without
+// reading the grid (a bracket by a table of the bit patterns and a search of the grid inside
+// it were 5 dependent loads from 12 MB).
+struct GridRun {
+  uint32_t bits;   // bit pattern of the first point
+  uint32_t next;   // of the next run's first point
+  uint32_t magic;  // floor(2^32 / step) + 1: x * magic >> 32 = x / step for x * step < 2^32
+  uint32_t at;     // index of the first point; the step in the top 8 bits
+};
+constexpr int kRunShift = 16;  // bit patterns per entry of run_of (runs are longer, but three)
 
 struct GridView {
   const float* grid = nullptr;
-  const uint32_t* lut = nullptr;
+  const GridRun* runs = nullptr;
+  const uint8_t* run_of = nullptr;  // run of the first bit pattern of each 2^kRunShift
   uint32_t n = 0;       // grid length
-  uint32_t n_lut = 0;   // lut length
   uint32_t bits0 = 0;   // bit pattern of grid[0]
   float first = 0.0f;
   float last = 0.0f;
@@ -196,53 +205,45 @@ std::vector<float> gaussian_kernel(float fwhm_rt, float sigma_scale_rt, int64_t 
 
 __device__ __forceinline__ uint32_t f2bits(float x) { return __float_as_uint(x); }
 
-// The LUT bracket [lo, hi] of the bound of x (g.first < x <= g.last) and a guess inside it: a
-// bucket's floats are evenly spaced and its grid points nearly so, so interpolation is
-// within a point of the bound and its two neighbours load at once, where a binary search
-// took three loads one after the other.
-struct GridGuess {
-  uint32_t lo, hi, at;
+// The last grid point at or below x (g.first <= x <= g.last): its index, its bit pattern, the
+// step to the next point and how far above it x is (in bit patterns).
+struct GridPoint {
+  uint32_t at, bits, step, above;
 };
-__device__ __forceinline__ GridGuess grid_guess(const GridView& g, float x) {
-  const uint32_t d = f2bits(x) - g.bits0, k = d >> kLutShift;
-  GridGuess r;
-  r.lo = __ldg(g.lut + k);
-  r.hi = __ldg(g.lut + k + 1);
-  r.at = r.lo + (((r.hi - r.lo) * (d & ((1u << kLutShift) - 1u))) >> kLutShift);
-  return r;
+__device__ __forceinline__ GridPoint grid_point(const GridView& g, float x) {
+  const uint32_t bx = f2bits(x);
+  uint32_t k = __ldg(g.run_of + ((bx - g.bits0) >> kRunShift));
+  uint4 r = __ldg(reinterpret_cast<const uint4*>(g.runs) + k);
+  while (bx >= r.y) r = __ldg(reinterpret_cast<const uint4*>(g.runs) + ++k);
+  const uint32_t d = bx - r.x, step = r.w >> 24, q = __umulhi(d, r.z);
+  return GridPoint{(r.w & 0xFFFFFFu) + q, r.x + q * step, step, d - q * step};
 }
 
 // First i with grid[i] >= x (lower_bound), exact for every float x, NaN -> 0.
 __device__ __forceinline__ uint32_t grid_lower_bound(const GridView& g, float x) {
   if (!(x > g.first)) return 0;
   if (x > g.last) return g.n;
-  GridGuess r = grid_guess(g, x);
-  while (r.at < r.hi && __ldg(g.grid + r.at) < x) ++r.at;
-  while (r.at > r.lo && !(__ldg(g.grid + r.at - 1) < x)) --r.at;
-  return r.at;
+  const GridPoint p = grid_point(g, x);
+  return p.at + (p.above ? 1u : 0u);
 }
 
 // First i with grid[i] > x (upper_bound), exact, NaN -> 0.
 __device__ __forceinline__ uint32_t grid_upper_bound(const GridView& g, float x) {
   if (!(x >= g.first)) return 0;
   if (!(x < g.last)) return g.n;
-  GridGuess r = grid_guess(g, x);
-  while (r.at < r.hi && __ldg(g.grid + r.at) <= x) ++r.at;
-  while (r.at > r.lo && !(__ldg(g.grid + r.at - 1) <= x)) --r.at;
-  return r.at;
+  return grid_point(g, x).at + 1u;
 }
 
 // MZIndex::find_closest_index (src/mz_index/mod.rs:55-90): nearest grid point,
 // ties to the lower index, clamped to the ends.
 __device__ __forceinline__ uint32_t grid_find_closest(const GridView& g, float mz) {
-  uint32_t left = grid_lower_bound(g, mz);
-  if (left == 0) return 0;
-  if (left == g.n) return g.n - 1;
-  float a = __ldg(g.grid + left);
-  if (a == mz) return left;
-  float ld = fabsf(__fsub_rn(a, mz));
-  float rd = fabsf(__fsub_rn(__ldg(g.grid + left - 1), mz));
-  return ld < rd ? left : left - 1;
+  if (!(mz > g.first)) return 0;
+  if (!(mz < g.last)) return g.n - 1;
+  const GridPoint p = grid_point(g, mz);
+  if (p.above == 0) return p.at;
+  const float ld = fabsf(__fsub_rn(__uint_as_float(p.bits + p.step), mz));
+  const float rd = fabsf(__fsub_rn(__uint_as_float(p.bits), mz));
+  return ld < rd ? p.at + 1u : p.at;
 }
 
 // ln(x) of a float rounded to the nearest float: evaluated in double and rounded
