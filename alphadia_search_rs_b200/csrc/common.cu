@@ -78,10 +78,31 @@ void update_release_threshold(cudaMemPool_t pool) {
 }
 }  // namespace
 
+namespace {
+// The pool maps new memory kPoolGrowBytes at a time: mapping costs tens of milliseconds
+// however little it is.  (Of an allocation that the pool's free memory cannot hold, this
+// much is allocated and freed first, which leaves it mapped.)
+constexpr uint64_t kPoolGrowBytes = uint64_t(1) << 30;
+void grow_pool(const DevicePool& dp, size_t bytes, cudaStream_t st) {
+  uint64_t used = 0, held = 0;
+  if (bytes >= kPoolGrowBytes / 2 ||
+      cudaMemPoolGetAttribute(dp.pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess ||
+      cudaMemPoolGetAttribute(dp.pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+      used + bytes <= held) {
+    cudaGetLastError();
+    return;
+  }
+  void* p = nullptr;
+  if (cudaMallocFromPoolAsync(&p, kPoolGrowBytes, dp.pool, st) == cudaSuccess) cudaFreeAsync(p, st);
+  cudaGetLastError();
+}
+}  // namespace
+
 int pool_alloc(int device, size_t bytes, void** out) {
   *out = nullptr;
   DevicePool dp;
   ADS_TRY(device_pool(device, &dp));
+  grow_pool(dp, bytes, dp.stream);
   cudaError_t e = cudaMallocFromPoolAsync(out, bytes, dp.pool, dp.stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(dp.stream);  // usable on every stream
   if (e != cudaSuccess) {
@@ -96,6 +117,7 @@ int pool_alloc_async(int device, size_t bytes, cudaStream_t st, void** out) {
   *out = nullptr;
   DevicePool dp;
   ADS_TRY(device_pool(device, &dp));
+  grow_pool(dp, bytes, st);
   const cudaError_t e = cudaMallocFromPoolAsync(out, bytes, dp.pool, st);
   if (e != cudaSuccess) {
     *out = nullptr;

@@ -141,7 +141,8 @@ __device__ __forceinline__ void gather_one(const ScoreArgs& a, const X& x, int x
     const uint4* c8 = reinterpret_cast<const uint4*>(a.cyc + (q0 - skip));
     const uint16_t* cy = a.cyc + q0;
     const float* iy = a.inten + q0;
-    uint32_t b = b0;
+    uint32_t b = b0, b_end = 0;  // bin of the last entry and the bin's end
+    float actual = 0.0f;
     for (uint32_t j = 0; j < skip + n; j += 8) {
       const uint4 v = __ldg(c8 + (j >> 3));
       // most groups of 8 hold none: a half of a word is in the window where clamping it
@@ -161,46 +162,26 @@ __device__ __forceinline__ void gather_one(const ScoreArgs& a, const X& x, int x
       if (j < skip) in &= 0xffu << skip;
       if (j + 8 > skip + n) in &= 0xffu >> (j + 8 - skip - n);
       while (in) {
-        // kBatch entries at once, whose loads do not wait for one another (4: 4 % slower)
-        constexpr int kBatch = 2;
-        uint32_t at[kBatch], bin[kBatch];
-        float y[kBatch];
-        int k = 0;
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u) {
-          at[u] = 0xffffffffu;
-          if (in) {
-            at[u] = j + (uint32_t)__ffs(in) - 1u - skip;
-            in &= in - 1;
-            ++k;
-          }
+        const uint32_t at = j + (uint32_t)__ffs(in) - 1u - skip;
+        in &= in - 1;
+        const float y = __ldg(iy + at);
+        const int c = (int)__ldg(cy + at) - cs;
+        if (r0 + at >= b_end) {  // (entries of one ion mostly share a bin)
+          b = bin_of(ssw, b, b1, r0 + at);
+          b_end = __ldg(ssw + b + 1);
+          actual = __ldg(a.g.grid + b);
         }
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u)
-          if (u < k) {
-            y[u] = __ldg(iy + at[u]);
-            bin[u] = bin_of(ssw, b, b1, r0 + at[u]);
-          }
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u)
-          if (u < k) {
-            const int c = (int)__ldg(cy + at[u]) - cs;
-            const float actual = __ldg(a.g.grid + bin[u]);
-            b = bin[u];
-            // Rust's binary_search lands on the last of a bin's entries at the first cycle
-            if (c == 0 && at[u] + 1 < n && r0 + at[u] + 1 < __ldg(ssw + b + 1) &&
-                (int)__ldg(cy + at[u] + 1) == cs)
-              continue;
-            const float xs = __fadd_rn(x.f(x0 + c), y[u]);
-            x.sf(x0 + c, xs);
-            if (y[u] > 0.0f) {
-              const float prev = __fsub_rn(xs, y[u]);
-              if (prev == 0.0f)
-                z.sf(c, actual);
-              else
-                z.sf(c, __fdiv_rn(__fadd_rn(__fmul_rn(z.f(c), prev), __fmul_rn(actual, y[u])), xs));
-            }
-          }
+        // Rust's binary_search lands on the last of a bin's entries at the first cycle
+        if (c == 0 && r0 + at + 1 < b_end && (int)__ldg(cy + at + 1) == cs) continue;
+        const float xs = __fadd_rn(x.f(x0 + c), y);
+        x.sf(x0 + c, xs);
+        if (y > 0.0f) {
+          const float prev = __fsub_rn(xs, y);
+          if (prev == 0.0f)
+            z.sf(c, actual);
+          else
+            z.sf(c, __fdiv_rn(__fadd_rn(__fmul_rn(z.f(c), prev), __fmul_rn(actual, y)), xs));
+        }
       }
     }
   }
