@@ -418,8 +418,9 @@ int build_entries(AdsDia* d, const AdsRawArrays* raw, const std::vector<int32_t>
 }
 
 // The run's WinIndex on the device.  Left out (windows are then scanned) where its lists
-// would exceed kWinIndexMax entries: thousands of windows all over one another.
-constexpr size_t kWinIndexMax = size_t(1) << 22;
+// would exceed kWinIndexMax entries: hundreds of windows all over one another (a run of 300
+// windows that meet at their limits has 1500).
+constexpr size_t kWinIndexMax = size_t(1) << 16;
 
 int build_win_index(AdsDia* d) {
   std::vector<float> v;

@@ -1,7 +1,7 @@
 // PeakGroupScoring.score on the device (src/peak_group_scoring/mod.rs:42-340).
 //
-// One thread per candidate walks the reference's per-candidate steps in their
-// order, so every f32 operation rounds as the reference's does:
+// The reference's per-candidate steps in their order, so every f32 operation rounds as
+// the reference's does:
 //   1. the precursor by binary search of its precursor_idx, its fragments filtered
 //      (non-zero, no y1), the top-k by intensity and sorted by m/z
 //      (src/speclib_flat/mod.rs:240-345, 458-474);
@@ -15,9 +15,12 @@
 // correlation that comes out NaN or infinite, where the reference panics
 // (src/peak_group_scoring/utils.rs:164-166), is 0 here.
 //
-// A thread's matrices (F x C dense XIC, m/z and normalised profiles) and vectors
-// live in a global scratch interleaved across threads (element e of thread t at
-// e * T + t), so threads working on the same element read consecutive words.
+// score_block_kernel (score_block.cuh) takes a few candidates per block through the
+// steps in shared memory.  Candidates whose matrices do not fit there, or a run without a
+// window index, go to score_kernel / quant_kernel: a thread per candidate, its matrices
+// (F x C dense XIC, m/z and normalised profiles) and vectors in a global scratch
+// interleaved across threads (element e of thread t at e * T + t), so threads working on
+// the same element read consecutive words.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -44,7 +47,7 @@ struct AdsFeatures {
   ~AdsFeatures() {
     if (idle) arena.release_idle();
   }
-  float kernel_ms = 0.0f;  // CUDA-event time of score_kernel
+  float kernel_ms = 0.0f;  // CUDA-event time of the scoring kernels
 };
 
 // Quantified candidates (SpecLibFlatQuantified, src/speclib_flat_quantified/mod.rs:19-64),

@@ -1,4 +1,4 @@
-// The block kernel of scoring and quantification: a block of 4 warps takes kGroup
+// The block kernel of scoring and quantification: a block of 2 warps takes up to kGroup
 // candidates through the steps of score_kernel / quant_kernel with one thread per
 // (candidate, fragment), per (candidate, cycle) or per candidate, whatever the step is
 // made of, and everything in shared memory.  Included by score.cu inside namespace

@@ -4,7 +4,8 @@
 //   1. prep_kernel      one warp per precursor: RT cycle limits, quadrupole
 //                       windows, fragment filter / top-k / m/z sort, m/z bin
 //                       range of every kept fragment.
-//   2. classify_kernel  precursors into RT-window length classes.
+//   2. classify_kernel  precursors into RT-window length classes (class_scatter_kernel:
+//                       and by fragment count), where there are several.
 //   3. search_kernel    one instance per class, one warp per precursor
 //                       (persistent warps pulling from an atomic counter): XIC
 //                       gather into shared memory, Gaussian convolution,
@@ -356,7 +357,7 @@ __global__ void __launch_bounds__(kPrepThreads, 8) prep_kernel(PrepArgs a) {
 // all RT windows up to kSmemMaxCycles.
 constexpr int kLaneCycles[] = {4, 8, 10, 12, 16};
 // Global working sets of one long-window launch: at most this many bytes (the grid
-// is trimmed to fit; a warp's set is about 15 bytes per cycle of the longest window).
+// is trimmed to fit; a warp's set is about 11 bytes per cycle of the longest window).
 constexpr int64_t kGrowBudgetBytes = int64_t(1) << 30;
 constexpr int kDefaultWarpsPerBlock = 4;
 constexpr int kMaxClasses = 10;
@@ -803,7 +804,7 @@ int enqueue_search(AdsSelection* s, const AdsDia* d, const AdsLib* l, AdsCandida
 
   const float tol_max = l->has_tol ? std::max(l->max_tol, 0.0f) : prm.rt_tolerance;
   const int64_t c_max = std::max<int64_t>(1, max_cycle_span(d->rt, d->delta_t, tol_max, prm.kernel_size));
-  // length classes and their cycles per lane (a fixed cycles_per_lane: one class)
+  // length classes (a fixed cycles_per_lane: one class)
   const int S_fixed = s->o.cycles_per_lane;
   if (S_fixed != 0 &&
       std::find(std::begin(kLaneCycles), std::end(kLaneCycles), S_fixed) == std::end(kLaneCycles))
@@ -1056,8 +1057,8 @@ int enqueue_search(AdsSelection* s, const AdsDia* d, const AdsLib* l, AdsCandida
 
 // ------------------------------------------------------------------ autotuner
 // Launch shapes of the search kernel: warps per block (precursors in flight per
-// CTA) and cycles per lane (0 = length classes, else one fixed width), timed on the
-// caller's run and library; the fastest is kept in the selection's options and
+// CTA) and cycles_per_lane (0 = length classes, 16 = one class), timed on the caller's
+// run and library; the fastest is kept in the selection's options and
 // cached per workload shape for the rest of the process.
 struct TuneKey {
   int device, precision, h;
@@ -1068,7 +1069,7 @@ struct TuneKey {
   }
 };
 std::mutex g_tune_mu;
-std::map<TuneKey, std::array<float, 3>> g_tune_cache;  // warps, cycles per lane, ms
+std::map<TuneKey, std::array<float, 3>> g_tune_cache;  // warps, cycles_per_lane, ms
 
 int autotune(AdsSelection* s, const AdsDia* d, const AdsLib* l, int32_t repeats,
              int32_t* out_warps, int32_t* out_cycles, float* out_ms) {
@@ -1099,8 +1100,7 @@ int autotune(AdsSelection* s, const AdsDia* d, const AdsLib* l, int32_t repeats,
     AdsCandidates scratch;
     scratch.device = s->device;
     int rc = ADS_OK;
-    for (int nw : {2, 4, 8}) {
-      if (nw > max_warps_per_block(false)) continue;
+    for (int nw : {2, 4}) {  // up to max_warps_per_block(false)
       for (int S : {0, 16}) {  // length classes, or one class
         s->o.warps_per_block = nw;
         s->o.cycles_per_lane = S;

@@ -183,13 +183,14 @@ typedef struct {
                           (src/peak_group_selection/mod.rs:123-125) */
   int32_t use_graph;   /* 1: capture the search pipeline in a CUDA graph and replay it */
   int32_t warps_per_block; /* 0 = default (4); else 1..8 warps, one precursor each
-                              (FP32 searches: at most 4) */
+                              (RT windows up to 2048 cycles: at most 4) */
   int32_t blocks_per_sm;   /* 0 = autotuned/default */
   int32_t gather_mode;     /* 0 = automatic, 1 = always scan bin ranges, 2 = always
                               binary-search each bin (both are exact; for testing) */
   int32_t time_stages;     /* 1: record CUDA events around each stage of a search */
-  int32_t cycles_per_lane; /* 0 = chosen from the longest RT window; else 4, 8, 10, 12
-                              or 16 consecutive cycles per lane of the search kernel */
+  int32_t cycles_per_lane; /* 0 = RT-window length classes, launched one after the other;
+                              4, 8, 10, 12 or 16 = one launch for all windows up to 2048
+                              cycles (every lane convolves 4 cycles at a time either way) */
   int64_t stream;          /* cudaStream_t to run on, 0 = the handle's own stream */
 } AdsEngineOptions;
 
@@ -243,8 +244,8 @@ int ads_select_async(AdsSelection* sel, const AdsDia* dia, const AdsLib* lib,
  * Working memory is a fixed device array of ADS_NOALLOC_SCRATCH_BYTES that every
  * GPU context loading this library holds until the process exits; a search that
  * needs more (about 200 bytes per precursor with 12 fragments and 3 candidates;
- * RT windows longer than 2048 cycles also need about 60 KB per 1000 cycles for each
- * of at least four warps) fails with ADS_ERR_INVALID_ARGUMENT and should be split
+ * RT windows longer than 2048 cycles also need about 45 KB per 1000 cycles for at
+ * least four warps) fails with ADS_ERR_INVALID_ARGUMENT and should be split
  * over smaller libraries.  The first call on a device sets the array up (looks up its
  * device address and copies a 4 KiB table into it, then synchronises the device);
  * make that first call before any stream capture.  A cudaDeviceReset after it is
@@ -277,12 +278,10 @@ int ads_selection_last_stats(AdsSelection* sel, int64_t* out, int64_t cap);
 int ads_selection_stage_times(AdsSelection* sel, float* ms, int64_t cap);
 /* Autotuner (an engine addition; the reference has no launch shapes to tune).
  * Times the search of `dia` x `lib` (`repeats` timed searches per shape, after
- * one warm-up) for warps per block 2, 4, 8 (precursors in flight per CTA; 2 and 4 for
- * FP32) and cycles
- * per lane 0 (length classes), 4, 8, 10, 12, 16 (cycles per tile = 32 x that),
- * keeps the fastest in the selection's options and caches it per workload shape
- * (device, precision, kernel half width, longest RT window, precursors, fragments)
- * for the process.  Writes the choice and its mean ms where the pointers are not
+ * one warm-up) for warps per block 2 and 4 (precursors in flight per CTA) and
+ * cycles_per_lane 0 (length classes) and 16 (one class), keeps the fastest in the
+ * selection's options and caches it per workload shape (device, precision, kernel half
+ * width, longest RT window, precursors, fragments) for the process.  Writes the choice and its mean ms where the pointers are not
  * NULL.  Blocks until done. */
 int ads_selection_autotune(AdsSelection* sel, const AdsDia* dia, const AdsLib* lib,
                            int32_t repeats, int32_t* warps_per_block, int32_t* cycles_per_lane,

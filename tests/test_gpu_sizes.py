@@ -192,3 +192,32 @@ def test_scoring_and_quantification_blocks(candidates, n, span):
     assert_features_equal(got, oracle.score(od, ol, c, log_mode=oracle.LOG_RN), exact=True, where=f"{n}x{span}")
     q = PeakGroupQuantification(QuantificationParameters(), verbose=False).quantify(dia, slib, cc)
     assert_quant_equal(q, oracle.quantify(od, ol, c, la), where=f"{n}x{span}")
+
+
+@pytest.mark.parametrize("n_windows", [179, 184])
+def test_windows_all_over_one_another(n_windows):
+    """Nested windows: as many as the window index lists, and a few more, where windows are
+    scanned and the per-candidate kernels score."""
+    rng = np.random.default_rng(n_windows)
+    n_cyc, P, F = 60, 5, 3
+    fmz = rng.uniform(200, 1700, (P, F))
+    spectra, lo, hi = [], [], []
+    for c in range(n_cyc):
+        for w in range(n_windows + 1):
+            mz = np.sort(rng.choice(fmz.reshape(-1), 2 if w else 0))
+            spectra.append((w, c, mz, rng.lognormal(6, 1, len(mz))))
+            lo.append(-1.0 if w == 0 else 500.0 - w)
+            hi.append(-1.0 if w == 0 else 500.0 + w)
+    run = run_of(spectra, n_windows)
+    run["isolation_lower_mz"], run["isolation_upper_mz"] = np.float32(lo), np.float32(hi)
+    la = library_of(500.0, np.full(P, 30.0), fmz, rng.uniform(0.1, 1.0, (P, F)))
+    la["precursor_mz"] = np.array([500.0, 400.0, 500.0 - n_windows, 620.5, 321.0], np.float32)
+    got, ref = search_both(run, la, dict(PARAMS, kernel_size=14, fwhm_rt=2.0, rt_tolerance=30.0))
+    assert len(ref["rank"]) > 0
+    assert_candidates_equal(got, ref, exact_scores=True, where=f"{n_windows} windows")
+    dia, slib, od, ol = build(run, la)
+    cc = CandidateCollection.from_arrays(*(ref[k] for k in COLS))
+    feats = PeakGroupScoring(ScoringParameters(), verbose=False).score(dia, slib, cc).to_dict_arrays()
+    assert_features_equal(feats, oracle.score(od, ol, ref, log_mode=oracle.LOG_RN), exact=True, where="nested")
+    q = PeakGroupQuantification(QuantificationParameters(), verbose=False).quantify(dia, slib, cc)
+    assert_quant_equal(q, oracle.quantify(od, ol, ref, la), where="nested")
