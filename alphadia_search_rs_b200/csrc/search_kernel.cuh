@@ -791,6 +791,39 @@ __device__ __forceinline__ void flush_counters(const SearchArgs& a, const Counte
   }
 }
 
+// A warp's next precursor: its place in the work queue, its row and its header.  The place
+// is taken before the last row of the precursor before is convolved and the header read
+// before its maxima are picked: the two round trips, about 2 of the 50 us that a warp spends
+// on 12 rows of 301 cycles, are no longer waited for (200,000 uneven precursors FP32 3.80 ->
+// 3.77 ms, 500,000 BF16 7.88 -> 7.79).  Taken earlier, a place would be held by a warp that
+// is still busy when others have run out.
+struct Work {
+  unsigned pw;
+  int64_t p;
+  int nf, cs, ce, nwin;
+};
+// (lane 0 holds the place, which load_work gives to every lane)
+__device__ __forceinline__ unsigned take_index(const SearchArgs& a, int lane) {
+  return lane == 0 ? (unsigned)min(atomicAdd(a.work, 1ull), 0xffffffffull) : 0u;
+}
+__device__ __forceinline__ Work load_work(const SearchArgs& a, unsigned taken, unsigned n_work) {
+  Work w;
+  w.pw = __reduce_max_sync(kFull, taken);
+  w.p = 0;
+  w.nf = w.cs = w.ce = w.nwin = 0;
+  if (w.pw < n_work) {
+    w.p = a.list ? (int64_t)uniform(a.list[w.pw]) : (int64_t)w.pw;
+    w.nf = a.nf[w.p];
+    w.cs = a.cs[w.p];
+    w.ce = a.ce[w.p];
+    w.nwin = a.nwin[w.p];
+  }
+  return w;
+}
+__device__ __forceinline__ Work take_work(const SearchArgs& a, int lane, unsigned n_work) {
+  return load_work(a, take_index(a, lane), n_work);
+}
+
 // GROW: the warp's working set (row, bitmaps, scores, lists, maxima) lives in
 // a global buffer of P.total words per warp (`a.grow`) instead of shared memory, for
 // RT windows longer than kSmemMaxCycles; the code and every operation are the same.
@@ -839,29 +872,24 @@ __global__ void __launch_bounds__(LaunchShape<GROW>::threads, LaunchShape<GROW>:
   const unsigned lt = (1u << lane) - 1u;
 
   const unsigned n_work = a.list ? (unsigned)uniform((int)*a.list_len) : (unsigned)a.n_prec;
+  Work next_p = take_work(a, lane, n_work);
 #pragma unroll 1
-  for (;;) {
-    unsigned pw = 0;
-    if (lane == 0) pw = (unsigned)min(atomicAdd(a.work, 1ull), 0xffffffffull);
-    pw = __reduce_max_sync(kFull, pw);
-    if (pw >= n_work) break;
-    const int64_t p = a.list ? (int64_t)uniform(a.list[pw]) : (int64_t)pw;
-    const int F = uniform(a.nf[p]);
-    const int cs = uniform(a.cs[p]);
-    const int C = uniform(a.ce[p]) - cs;
-    if (F == 0 || C <= 0) {
-      if (lane == 0) a.cand_n[p] = 0;
-      continue;
-    }
-    if (C > a.c_max) {
+  while (next_p.pw < n_work) {
+    const int64_t p = next_p.p;
+    const int F = uniform(next_p.nf);
+    const int cs = uniform(next_p.cs);
+    const int C = uniform(next_p.ce) - cs;
+    const int nwin = uniform(next_p.nwin);
+    if (F == 0 || C <= 0 || C > a.c_max) {
       if (lane == 0) {
         a.cand_n[p] = 0;
-        atomicOr(a.err, 2);
+        if (F != 0 && C > a.c_max) atomicOr(a.err, 2);
       }
+      next_p = take_work(a, lane, n_work);
       continue;
     }
-    const int nwin = uniform(a.nwin[p]);
     const int npairs = F * nwin;
+    unsigned taken = npairs == 0 ? take_index(a, lane) : 0u;  // else with the last pair
     k.frag += F;
     // fragment weights, lane f holding fragment f's (fetched once per precursor)
     const float wf_lane = lane < F ? __ldg(a.fw + p * a.kf + lane) : 0.0f;
@@ -892,6 +920,8 @@ __global__ void __launch_bounds__(LaunchShape<GROW>::threads, LaunchShape<GROW>:
         if (pi + 1 >= pc.pb + 32) load_pairs(a, p, pi + 1, nwin, npairs, lane, pc);
         next = pair_of(pc, pi + 1 - pc.pb, lane);
         staged = stage_pair<FAST>(a, next, lane, stage);
+      } else {
+        taken = take_index(a, lane);
       }
       if (++wi < nwin) continue;  // more windows hold this fragment
       wi = 0;
@@ -1001,7 +1031,9 @@ __global__ void __launch_bounds__(LaunchShape<GROW>::threads, LaunchShape<GROW>:
       clear_row(r, row, P, lane);
     }
     __syncwarp();
-
+    // the next precursor was taken before the last row's convolution; its header arrives
+    // while this one's maxima are picked
+    next_p = load_work(a, taken, n_work);
     pick_top_k(a, p, cs, C, score, mval, midx, P.mx, lane);
   }
   flush_counters<STATS>(a, k, lane);
