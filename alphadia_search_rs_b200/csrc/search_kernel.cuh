@@ -73,6 +73,11 @@ constexpr int kTouchCap = 256;        // accepted cells a row records for cleari
                                       // row is zeroed whole
 // Listed outputs: up to 31 left over, 4 per lane of one round, a warp of idle ones.
 constexpr int kOutCap = 31 + 32 * kSeg + 32;
+// Listed outputs that a lane takes the logarithm of at a time: the logarithm is a chain of
+// dependent double operations, and 20 warps per SM do not hide it (1, 2, 3, 4 at a time:
+// 200,000 uneven precursors FP32 3.77, 3.65, 3.60, 3.78 ms; 500,000 BF16 7.79, 7.71, 7.70,
+// 7.82; windows of 4000 cycles 0.987, 0.903, 0.872, 0.909).
+constexpr int kTerms = 3;
 
 __host__ __device__ inline int maxima_cap(int c_max) { return c_max / 4 + 8; }
 
@@ -589,18 +594,42 @@ __device__ __forceinline__ float ln1p_fast(float c) {
   return fabsf(c) < 0.0625f ? series : __logf(__fadd_rn(c, 1.0f));
 }
 
-// s + ln(c + 1) * w (src/score/scalar.rs:16-22): one rounded operation at a time with the
-// exact ln; FAST (BF16 storage) takes the hardware log2 and a fused multiply-add.  Called
-// by whole warps: the slow path of the exact ln is behind one vote.
-template <bool FAST>
-__device__ __forceinline__ float score_term(float s, float c, float w, const double2* lnt,
-                                            const LnCoef& k) {
-  if (FAST) return __fmaf_rn(ln1p_fast(c), w, s);
-  const float x = __fadd_rn(c, 1.0f);
-  float y;
-  const bool slow = ln_table(x, lnt, k, &y);
-  if (__any_sync(kFull, slow)) y = slow ? ln_rn_slow(x) : y;
-  return __fadd_rn(s, __fmul_rn(y, w));
+// The score terms s + ln(c + 1) * w (src/score/scalar.rs:16-22) of the 32 * U listed outputs
+// from lst[0]: one rounded operation at a time with the exact ln; FAST (BF16 storage) takes
+// the hardware log2 and a fused multiply-add.  The slow path of the exact ln is behind one
+// vote.
+template <int U, bool FAST>
+__device__ __forceinline__ void score_terms(const float2* lst, float* score, float w,
+                                            const double2* lnt, const LnCoef& k, int lane) {
+  float* at[U];
+  float s[U], x[U], y[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const float2 e = lst[32 * u + lane];
+    at[u] = score + __float_as_int(e.y);
+    s[u] = *at[u];
+    x[u] = e.x;
+  }
+  if (FAST) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) s[u] = __fmaf_rn(ln1p_fast(x[u]), w, s[u]);
+  } else {
+    bool slow[U], any = false;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      x[u] = __fadd_rn(x[u], 1.0f);
+      slow[u] = ln_table(x[u], lnt, k, &y[u]);
+      any = any || slow[u];
+    }
+    if (__any_sync(kFull, any)) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) y[u] = slow[u] ? ln_rn_slow(x[u]) : y[u];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) s[u] = __fadd_rn(s[u], __fmul_rn(y[u], w));
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) *at[u] = s[u];
 }
 
 // Stores the pair (v, at) where `on`, predicated (a branch around each store cost three
@@ -1020,11 +1049,14 @@ __global__ void __launch_bounds__(LaunchShape<GROW>::threads, LaunchShape<GROW>:
         }
         __syncwarp();
 #pragma unroll 1
+        while (listed >= 32 * kTerms) {
+          listed -= 32 * kTerms;
+          score_terms<kTerms, FAST>(lst + listed, score, wf, lnt, a.ln, lane);
+        }
+#pragma unroll 1
         while (listed >= 32) {
           listed -= 32;
-          const float2 e = lst[listed + lane];
-          float* sp = score + __float_as_int(e.y);
-          *sp = score_term<FAST>(*sp, e.x, wf, lnt, a.ln);
+          score_terms<1, FAST>(lst + listed, score, wf, lnt, a.ln, lane);
         }
         __syncwarp();
       }
