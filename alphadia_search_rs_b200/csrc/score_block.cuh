@@ -5,11 +5,16 @@
 // ads::{anonymous}; every f32 operation is that of the per-candidate kernels, in their
 // order, through the same helpers.
 //
-// What bounds it: instruction issue.  A thread per candidate (score_kernel) ran 8 of 32
-// lanes per instruction on matrices in a global scratch, and walked every bin of every
-// fragment with a binary search.  Here a row's whole range of entries is read 8 cycle
-// indices at a time, and only an entry inside the window looks up its bin.
+// What bounds it: the gather's loads and the waits between steps (31 warps per SM issue on
+// 48 % of the cycles with 15 of 32 lanes; 4.4 warps wait for memory and 4.4 at a barrier per
+// issue).  A thread per candidate (score_kernel) ran 8 of 32 lanes per instruction on matrices
+// in a global scratch, and walked every bin of every fragment with a binary search.  Here a
+// row's whole range of entries is read 8 cycle indices at a time, and only an entry inside
+// the window looks up its bin: 1.48 M candidates of 4-24 fragments scored 41.0 -> 10.5 ms,
+// quantified 29.0 -> 8.0 ms.
 constexpr int kGroup = 4;        // candidates of a block (at most)
+// 2 warps for 4 candidates; for 2: scored 3.06 ms against 2.51 (295,000 candidates); 1 warp
+// for 4: 2.76; 1 for 2: 2.47, but quantified 1.19 against 1.18.
 constexpr int kBlockWarps = 2;
 constexpr int kBlockThreads = 32 * kBlockWarps;
 // A candidate's shared memory grows with fragments x cycles; beyond this many bytes a block
@@ -220,6 +225,30 @@ constexpr uint32_t kFlagNz = 1u << 16;   // profile not all zero
 constexpr uint32_t kFlagTop = 1u << 17;  // among the six highest IDF values
 constexpr int kFlagBand = 18;            // from this bit: intensity rank / 6 (4: rank 24 and on)
 
+// Where the reference's binary search of the sorted precursor_idx ends: the last row at or
+// below `pidx` (0 where there is none).  kRowLanes lanes of the warp per search, each
+// testing the end of one of as many parts: 5 dependent loads in 500,000 rows instead of 19,
+// which a block's other threads waited for (295,000 candidates of 4-24 fragments scored
+// 2.55 -> 2.51 ms, 6000 of them 80.5 -> 78.8 us).  Whole warps call it, those without a search
+// with no rows.
+constexpr int kRowLanes = kBlockThreads / kGroup;
+static_assert(kRowLanes <= 32 && 32 % kRowLanes == 0, "a search stays within a warp");
+__device__ __forceinline__ int64_t find_row(const uint64_t* idx, int64_t n, uint64_t pidx, int lane) {
+  const int sub = lane % kRowLanes;
+  int64_t lo = 0;
+  while (__any_sync(0xffffffffu, n > 0)) {
+    const int64_t part = (n + kRowLanes - 1) / kRowLanes;
+    const int64_t end = min((sub + 1) * part, n);
+    const bool below = n > 0 && idx[lo + end - 1] <= pidx;
+    const unsigned all = __ballot_sync(0xffffffffu, below) >> (lane - sub);
+    const int parts = __popc(all & (unsigned)((1ull << kRowLanes) - 1ull));
+    const int64_t from = min(parts * part, n);
+    lo += from;
+    n = max(min((parts + 1) * part, n) - 1 - from, (int64_t)0);
+  }
+  return max(lo - 1, (int64_t)0);
+}
+
 template <bool QUANT>
 __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid_constant__ QuantArgs qa,
                                                                     const __grid_constant__ BlockPlan B,
@@ -236,7 +265,15 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
   const int64_t first = (int64_t)blockIdx.x * group;
 
   // ---- the candidates and their precursors
+  __shared__ int64_t sh_row[kGroup];
   if (tid < 3) sh_max[tid] = 0;
+  {
+    const int c = tid / kRowLanes;
+    const bool on = c < group && first + c < a.n;
+    const int64_t q = on ? (a.order ? (int64_t)a.order[first + c] : first + c) : 0;
+    const int64_t row = find_row(a.l_pidx, on ? a.P : 0, on ? a.c_pidx[q] : 0, lane);
+    if (on && tid % kRowLanes == 0) sh_row[c] = row;
+  }
   __syncthreads();
   if (tid < group) {
     BlockCand k;
@@ -266,12 +303,7 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
       }
       if (take && a.P > 0) {
         // SpecLibFlat::get_precursor_by_idx_filtered: binary search of the sorted idx
-        int64_t size = a.P, base = 0;
-        while (size > 1) {
-          const int64_t half = size / 2, mid = base + half;
-          base = a.l_pidx[mid] > pidx ? base : mid;
-          size -= half;
-        }
+        const int64_t base = sh_row[tid];
         if (a.l_pidx[base] == pidx) {  // else skipped, as in the reference
           const int64_t fs = (int64_t)a.l_fs[base], nraw = (int64_t)a.l_fe[base] - fs;
           if (nraw > B.Fraw) {
