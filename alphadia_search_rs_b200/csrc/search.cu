@@ -42,6 +42,10 @@ constexpr int kScanBlock = 1024;
 // Up to so many blocks of precursors, the compaction is one launch whose blocks count what
 // precedes them (64 values a thread at most) instead of three (21 -> 8 us at 2000 precursors).
 constexpr int64_t kFusedScatterBlocks = 64;
+// Up to so many, its blocks have a quarter of the threads, which spreads the stores over
+// more SMs: 2000 precursors 14 -> 9 us.  But a thread then counts four times the values:
+// 23,457 precursors 28 us against 15.5; the two meet near 7000.
+constexpr int64_t kSmallScatter = 4096;
 
 // Rust 1.88 slice::binary_search (Ok: the LAST equal element; Err: insertion
 // point) on a sorted array, for the u16 cycle lists of fill_xic_slice
@@ -512,16 +516,17 @@ struct ScatterArgs {
 
 // Candidate::new (src/candidate/entry.rs:19-38) as assembled in
 // src/peak_group_selection/mod.rs:172-192, written in precursor then rank order.
-__global__ void __launch_bounds__(kScanBlock) scatter_kernel(ScatterArgs a) {
+template <int T>
+__global__ void __launch_bounds__(T) scatter_kernel(ScatterArgs a) {
   __shared__ int64_t sh[33];
-  const int64_t p = (int64_t)blockIdx.x * kScanBlock + threadIdx.x;
+  const int64_t p = (int64_t)blockIdx.x * T + threadIdx.x;
   const int n = p < a.n_prec ? a.cand_n[p] : 0;
   int64_t total, before = 0;
   if (a.block_off) {
     before = a.block_off[blockIdx.x];
   } else {
     int64_t v = 0;
-    for (int64_t i = threadIdx.x; i < (int64_t)blockIdx.x * kScanBlock; i += kScanBlock) v += a.cand_n[i];
+    for (int64_t i = threadIdx.x; i < (int64_t)blockIdx.x * T; i += T) v += a.cand_n[i];
     block_exclusive_scan(v, sh, &before);
   }
   const int64_t off = before + block_exclusive_scan(n, sh, &total);
@@ -1044,7 +1049,10 @@ int enqueue_search(AdsSelection* s, const AdsDia* d, const AdsLib* l, AdsCandida
   ca.o_center = c->center_p;
   ca.o_start = c->start_p;
   ca.o_stop = c->stop_p;
-  scatter_kernel<<<(int)nb, kScanBlock, 0, st>>>(ca);
+  if (P <= kSmallScatter)
+    scatter_kernel<kScanBlock / 4><<<(int)((P + kScanBlock / 4 - 1) / (kScanBlock / 4)), kScanBlock / 4, 0, st>>>(ca);
+  else
+    scatter_kernel<kScanBlock><<<(int)nb, kScanBlock, 0, st>>>(ca);
   ADS_LAUNCH_CHECK();
   launches += 1;
   if (timed) {
@@ -1755,7 +1763,7 @@ int select_noalloc(const AdsDia* d, const AdsLib* l, const AdsSelectionParams* p
   ca.o_center = o_center;
   ca.o_start = o_start;
   ca.o_stop = o_stop;
-  scatter_kernel<<<(int)nb, kScanBlock, 0, st>>>(ca);
+  scatter_kernel<kScanBlock><<<(int)nb, kScanBlock, 0, st>>>(ca);
   ADS_LAUNCH_CHECK();
   return ADS_OK;
 }

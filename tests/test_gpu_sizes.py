@@ -194,6 +194,38 @@ def test_scoring_and_quantification_blocks(candidates, n, span):
     assert_quant_equal(q, oracle.quantify(od, ol, c, la), where=f"{n}x{span}")
 
 
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 1024, 4096, 4097, 5000, 65536, 65537, 70000])
+def test_candidates_of_many_precursors_in_order(n):
+    """Eleven precursors over and over: the candidates of each are the oracle's, in order,
+    whichever way they are brought together (small blocks, one launch, three launches)."""
+    rng = np.random.default_rng(5)
+    n_cyc, P, F = 200, 11, 3
+    fmz = rng.uniform(200, 1700, (P, F))
+    spectra = []
+    for c in range(n_cyc):
+        mz = np.sort(rng.choice(fmz.reshape(-1), 4))
+        spectra.append((0, c, np.zeros(0), np.zeros(0)))
+        spectra.append((1, c, mz, rng.lognormal(6, 2, len(mz))))
+    run = run_of(spectra, 1)
+    prt, fint = rng.uniform(20, 180, P), rng.uniform(0.1, 1.0, (P, F))
+    pmz = np.where(np.arange(P) % 4 == 3, 300.0, 405.0)  # every fourth in no window
+    params = dict(PARAMS, rt_tolerance=60.0)
+    la = library_of(405.0, prt, fmz, fint)
+    la["precursor_mz"] = pmz.astype(np.float32)
+    od, ol, tol = oracle_inputs(run, la)
+    ref = oracle_search(run, la, params, oracle.LOG_RN, od, ol, tol)
+    rows = [np.flatnonzero(ref["precursor_idx"] == k) for k in range(P)]
+    assert len({len(r) for r in rows}) > 1 and max(len(r) for r in rows) == 3
+    base = np.arange(n) % P
+    la = library_of(405.0, prt[base], fmz[base], fint[base])
+    la["precursor_mz"] = pmz[base].astype(np.float32)
+    got, *_ = product_search(run, la, params)
+    at = np.concatenate([rows[k] for k in base])
+    want = {k: ref[k][at] for k in COLS}
+    want["precursor_idx"] = np.repeat(np.arange(n), [len(rows[k]) for k in base]).astype(np.uint64)
+    assert_candidates_equal(got, want, exact_scores=True, where=f"{n} precursors")
+
+
 @pytest.mark.parametrize("n_windows", [179, 184])
 def test_windows_all_over_one_another(n_windows):
     """Nested windows: as many as the window index lists, and a few more, where windows are
