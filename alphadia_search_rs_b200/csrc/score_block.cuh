@@ -128,12 +128,13 @@ __device__ __forceinline__ void gather_one(const ScoreArgs& a, const X& x, int x
     x.sf(x0 + j, 0.0f);
     z.sf(j, 0.0f);
   }
-  if (C <= 0) return;
+  if (C <= 0 || cs > 0xffff) return;
   const float delta = __fmul_rn(__fmul_rn(mz, a.tol), 1e-6f);
   const uint32_t b0 = grid_lower_bound(a.g, __fsub_rn(mz, delta));
   const uint32_t b1 = max(b0, grid_upper_bound(a.g, __fadd_rn(mz, delta)));
   if (b1 <= b0) return;
-  const uint32_t first2 = (uint32_t)cs * 0x10001u, last2 = (uint32_t)(cs + C - 1) * 0x10001u;
+  // (entries' cycles end at 65,535, a range may not: the RT index counts MS1 spectra)
+  const uint32_t first2 = (uint32_t)cs * 0x10001u, last2 = (uint32_t)min(cs + C - 1, 0xffff) * 0x10001u;
   for (int w = 0; w < wlen; ++w) {
     const WinInfo wi = a.win[__ldg(a.wi.list + woff + w)];
     const uint32_t* ssw = a.ss + wi.ss_off;
