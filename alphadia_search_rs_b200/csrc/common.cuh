@@ -68,9 +68,10 @@ struct DeviceGuard {
 // Every device buffer of the engine comes from one memory pool per device that
 // keeps up to kPoolKeepBytes of freed memory for reuse, so that building a
 // library or a candidate collection per call does not map and unmap device pages
-// each time.  Allocation and release are ordered on a private stream of the pool;
-// a release first waits for the device to go idle (the guarantee cudaFree gives),
-// so no kernel still in flight can see its memory handed out again.
+// each time.  pool_alloc and pool_free are ordered on a private stream of the pool, and
+// pool_free first waits for the device to go idle (the guarantee cudaFree gives), so no
+// kernel still in flight can see its memory handed out again; the forms below leave the
+// waits out where the caller knows the order.
 constexpr uint64_t kPoolKeepBytes = uint64_t(4) << 30;
 int pool_alloc(int device, size_t bytes, void** out);
 void pool_free(int device, void* p);
@@ -446,11 +447,15 @@ struct AdsCandidates {
   int* err_p = nullptr;
   int64_t count = 0;
   bool pending = false;
+  // `done` was recorded behind everything that a search has enqueued on the buffers, in
+  // part or whole (false while one is being enqueued)
+  bool covered = false;
   ~AdsCandidates() {
     if (done) {
-      // the last search into the buffers has ended, and every reader waits for its own
-      // copies or kernels before it returns: nothing uses them any more
-      const bool ended = cudaEventSynchronize(done) == cudaSuccess;
+      // what searches have enqueued on the buffers has ended, and every reader waits for its
+      // own copies or kernels before it returns: nothing uses them any more (else the arena
+      // goes by the release that waits for the device)
+      const bool ended = covered && cudaEventSynchronize(done) == cudaSuccess;
       cudaEventDestroy(done);
       if (ended) arena.release_idle();
     }

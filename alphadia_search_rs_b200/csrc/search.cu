@@ -823,14 +823,31 @@ int enqueue_search(AdsSelection* s, const AdsDia* d, const AdsLib* l, AdsCandida
   const int kf = (int)std::max<int64_t>(1, std::min<int64_t>(prm.top_k_fragments, l->max_frag));
   const int maxw = std::max(1, d->max_overlap);
 
+  // `done` is recorded behind what has been enqueued by then, also when the search fails
+  // half way: the buffers may be read or freed once it has passed
+  struct Cover {
+    AdsCandidates* c;
+    cudaStream_t st;
+    bool on;
+    int end() {
+      if (!on) return ADS_OK;
+      on = false;
+      const cudaError_t e = cudaEventRecord(c->done, st);
+      c->covered = e == cudaSuccess;
+      return e == cudaSuccess ? ADS_OK : cuda_fail(e, "cudaEventRecord", __FILE__, __LINE__);
+    }
+    ~Cover() {
+      if (on) c->covered = cudaEventRecord(c->done, st) == cudaSuccess;
+    }
+  } cover{c, st, !capturing};
+  if (!capturing) c->covered = false;
   ADS_TRY(reserve_candidates(c, P * (int64_t)k_out, st));
   ADS_CUDA(cudaMemsetAsync(c->count_p, 0, 16, st));  // and err_p behind it
   c->pending = true;
   c->count = 0;
   if (P == 0 || k_out == 0) {
     s->last_launches = 0;
-    if (!capturing) ADS_CUDA(cudaEventRecord(c->done, st));
-    return ADS_OK;
+    return cover.end();
   }
 
   const size_t Pn = (size_t)P;
@@ -1060,8 +1077,7 @@ int enqueue_search(AdsSelection* s, const AdsDia* d, const AdsLib* l, AdsCandida
     ++s->stage_used;
   }
   s->last_launches = launches;
-  if (!capturing) ADS_CUDA(cudaEventRecord(c->done, st));
-  return ADS_OK;
+  return cover.end();
 }
 
 // ------------------------------------------------------------------ autotuner
@@ -1180,9 +1196,11 @@ int launch_search(AdsSelection* s, const AdsDia* d, const AdsLib* l, AdsCandidat
     ADS_CUDA(cudaStreamWaitEvent(st, c->done, 0));
     c->pending = true;
     c->count = 0;
+    c->covered = false;
     ADS_CUDA(cudaGraphLaunch(s->graph, st));
     s->last_launches = s->graph_launches;
     ADS_CUDA(cudaEventRecord(c->done, st));
+    c->covered = true;
     return ADS_OK;
   }
   ADS_TRY(enqueue_search(s, d, l, c, false));

@@ -5,10 +5,11 @@ import numpy as np
 import pytest
 
 import oracle
-from alphadia_search_rs_b200 import (CandidateCollection, PeakGroupQuantification, PeakGroupScoring,
-                                     QuantificationParameters, ScoringParameters)
+from alphadia_search_rs_b200 import (CandidateCollection, DIAData, PeakGroupQuantification,
+                                     PeakGroupScoring, PeakGroupSelection, QuantificationParameters,
+                                     ScoringParameters, SpecLibFlat, synth)
 
-from _util import COLS
+from _util import COLS, RUN_KEYS, params_from
 from test_gpu_quant import assert_quant_equal
 from test_gpu_scoring import assert_features_equal, build
 from test_gpu_sizes import library_of, run_of
@@ -54,3 +55,50 @@ def test_cycle_ranges_past_the_last_cycle_index(start, stop):
     la = library_of(405.0, np.full(P, float(start)), fmz, rng.uniform(0.1, 1.0, (P, F)))
     c = candidates_at(np.arange(P), np.full(P, start), np.full(P, stop))
     assert_scored_and_quantified(run, la, c, f"{start}-{stop}")
+
+
+def empty_library(n, frags_of_first):
+    """n precursors without fragments, but for the first."""
+    la = library_of(405.0, [100.0], np.linspace(200, 1700, frags_of_first)[None], np.ones((1, frags_of_first)))
+    for k in list(la):
+        if k.startswith("precursor"):
+            la[k] = np.arange(n, dtype=np.uint64) if k == "precursor_idx" else np.repeat(la[k], n)
+    la["flat_frag_start_idx"] = np.where(np.arange(n) == 0, 0, frags_of_first).astype(np.uint64)
+    la["flat_frag_stop_idx"] = np.full(n, frags_of_first, np.uint64)
+    return la
+
+
+def small_workload():
+    cfg, lib, run = synth.make_workload("tiny", "numpy")
+    return cfg, DIAData.from_arrays(*(run[k] for k in RUN_KEYS), run["cycle"]), synth.library_arrays(lib)
+
+
+@pytest.mark.parametrize("into", [False, True])
+def test_failed_search_leaves_nothing_behind(into):
+    """A search whose workspace does not fit the device (320 GB of fragment weights) fails
+    after it has queued work on its candidate buffers, here behind other work of its stream.
+    Buffers that are freed with the failure have been waited for; those that stay serve the
+    next search."""
+    import torch
+
+    cfg, dia, la = small_workload()
+    big = SpecLibFlat.from_arrays(**empty_library(200_000, 400_000))
+    lib = SpecLibFlat.from_arrays(**la)
+    params = params_from(dict(cfg.params_dict(), top_k_fragments=10**6))
+    stream = torch.cuda.Stream()
+    sel = PeakGroupSelection(params, verbose=False, stream=stream.cuda_stream)
+    want = sel.search(dia, lib).to_arrays()
+    cand = sel.new_candidates()
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(10**9)  # about half a second
+    with pytest.raises(MemoryError):
+        sel.search_into(dia, big, cand) if into else sel.search(dia, big)
+    if into:
+        assert cand.size() == 0
+    assert stream.query()
+    sel.search_into(dia, lib, cand)
+    n = len(want[0])
+    out = {c: np.zeros(n, w.dtype) for c, w in zip(COLS, want)}
+    assert cand.copy_out(out) == n
+    for c, w in zip(COLS, want):
+        assert np.array_equal(out[c].view(np.uint8), w.view(np.uint8)), c
