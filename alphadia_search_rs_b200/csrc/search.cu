@@ -770,6 +770,10 @@ int reserve_candidates(AdsCandidates* c, int64_t cap, cudaStream_t st) {
   if (c->cap >= cap) return ADS_OK;
   const size_t n = (size_t)std::max<int64_t>(cap, 1);
   const size_t col8 = (n * 8 + 255) / 256 * 256, col4 = (n * 4 + 255) / 256 * 256;
+  // the old arena goes first: nothing may use it, or what it held, when the new one does not fit
+  c->cap = -1;
+  c->count = 0;
+  c->pending = false;
   // (readers on other streams wait for the search's event)
   ADS_TRY(c->arena.alloc_on(5 * col8 + col4 + 256, st));
   char* q = c->arena.p;

@@ -102,3 +102,29 @@ def test_failed_search_leaves_nothing_behind(into):
     assert cand.copy_out(out) == n
     for c, w in zip(COLS, want):
         assert np.array_equal(out[c].view(np.uint8), w.view(np.uint8)), c
+
+
+def test_candidate_buffers_that_cannot_grow():
+    """Candidate buffers that would have to grow past the device's memory (214 GB) are gone
+    with the failure, and come back with the next search."""
+    cfg, dia, la = small_workload()
+    lib = SpecLibFlat.from_arrays(**la)
+    sel = PeakGroupSelection(params_from(cfg.params_dict()), verbose=False)
+    want = sel.search(dia, lib).to_arrays()
+    n = len(want[0])
+    out = {c: np.zeros(n, w.dtype) for c, w in zip(COLS, want)}
+    cand = sel.new_candidates()
+    sel.search_into(dia, lib, cand)
+    none = np.zeros(0)
+    run = run_of([(0, c, none, none) for c in range(65_000)] + [(1, 5, [500.0], [1.0])], 1)
+    long_run = DIAData.from_arrays(*(run[k] for k in RUN_KEYS), run["cycle"])
+    big = SpecLibFlat.from_arrays(**empty_library(300_000, 2))
+    many = PeakGroupSelection(params_from(dict(cfg.params_dict(), candidate_count=20_000,
+                                               rt_tolerance=65_000.0)), verbose=False)
+    with pytest.raises(MemoryError):
+        many.search_into(long_run, big, cand)
+    assert cand.size() == 0
+    sel.search_into(dia, lib, cand)
+    assert cand.copy_out(out) == n
+    for c, w in zip(COLS, want):
+        assert np.array_equal(out[c].view(np.uint8), w.view(np.uint8)), c
