@@ -30,6 +30,11 @@ int cuda_fail(cudaError_t e, const char* what, const char* file, int line) {
   return e == cudaErrorMemoryAllocation ? ADS_ERR_OUT_OF_MEMORY : ADS_ERR_CUDA;
 }
 
+uint64_t new_id() {
+  static std::atomic<uint64_t> last{0};
+  return ++last;
+}
+
 // ------------------------------------------------------------ device memory
 
 namespace {

@@ -354,7 +354,13 @@ namespace ads {
 constexpr int kEntrySlack = 8;
 }
 
+// A number that no other run of the process has or had (an address may come again).
+namespace ads {
+uint64_t new_id();
+}
+
 struct AdsDia {
+  const uint64_t id = ads::new_id();
   int device = 0;
   int64_t n_obs = 0;
   int64_t grid_len = 0;

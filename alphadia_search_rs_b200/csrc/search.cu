@@ -581,7 +581,7 @@ struct AdsSelection {
   // use_graph: the pipeline captured for one (run, library, collection) and the
   // buffers it was captured with
   cudaGraphExec_t graph = nullptr;
-  std::vector<const void*> graph_key;
+  std::vector<uint64_t> graph_key;
   int64_t graph_launches = 0;
 };
 
@@ -1167,25 +1167,23 @@ int autotune(AdsSelection* s, const AdsDia* d, const AdsLib* l, int32_t repeats,
   return ADS_OK;
 }
 
-// Everything a captured search depends on: the handles and every buffer address.
-// Everything a captured pipeline bakes in: the handles, every buffer it reads or
-// writes, and the run- and library-derived sizes its launch plan depends on (a handle
-// released and another created at the same address must not replay a stale graph).
-std::vector<const void*> graph_key(const AdsSelection* s, const AdsDia* d, const AdsLib* l,
-                                   const AdsCandidates* c) {
-  auto v = [](int64_t x) { return reinterpret_cast<const void*>(static_cast<intptr_t>(x)); };
+// Everything a captured pipeline bakes in: the run, by its number (its cycle time and longest
+// RT window are in the launch plan, and another run may come to the same addresses), the
+// library's values in the plan, and every buffer that it reads or writes, with the capacity
+// that the candidate columns' places in their arena follow from.
+std::vector<uint64_t> graph_key(const AdsSelection* s, const AdsDia* d, const AdsLib* l,
+                                const AdsCandidates* c) {
+  auto v = [](const void* x) { return (uint64_t)reinterpret_cast<uintptr_t>(x); };
   uint32_t tol_bits = 0;
   std::memcpy(&tol_bits, &l->max_tol, sizeof(tol_bits));
-  return {d, l, c, c->arena.p, s->nf.p, s->cs.p, s->ce.p, s->nwin.p, s->wins.p, s->fw.p,
-          s->blo.p, s->bhi.p, s->keep.p, s->cand_n.p, s->cand_score.p, s->cand_center.p,
-          s->work.p, s->class_lists.p, s->class_hist.p, s->block_sums.p,
-          s->stats_on ? s->stats.p : nullptr,
-          d->intens_bf16.p, s->grow.p, s->taps.p,
-          d->slice_starts.p, d->cycles.p, d->intens.p, d->win_dev.p, d->rt_dev.p, d->win_index_dev.p,
-          v(d->win_index_m), v(d->win_index_ok), v(d->n_obs),
-          v((int64_t)d->rt.size()), v(d->max_overlap),
-          l->arena.p, v(l->n_prec), v(l->n_frag), v(l->max_frag), v(l->min_frag), v(l->has_tol),
-          v(tol_bits)};
+  return {d->id, v(d->intens.p), v(d->intens_bf16.p),
+          v(l->arena.p), (uint64_t)l->n_prec, (uint64_t)l->n_frag, (uint64_t)l->max_frag,
+          (uint64_t)l->min_frag, l->has_tol, tol_bits,
+          v(c->arena.p), (uint64_t)c->cap,
+          v(s->nf.p), v(s->cs.p), v(s->ce.p), v(s->nwin.p), v(s->wins.p), v(s->fw.p),
+          v(s->blo.p), v(s->bhi.p), v(s->keep.p), v(s->cand_n.p), v(s->cand_score.p),
+          v(s->cand_center.p), v(s->work.p), v(s->class_lists.p), v(s->class_hist.p),
+          v(s->block_sums.p), v(s->stats_on ? s->stats.p : nullptr), v(s->grow.p), v(s->taps.p)};
 }
 
 // A search, with use_graph: the first search of a (run, library, collection) runs

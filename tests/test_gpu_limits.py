@@ -128,3 +128,27 @@ def test_candidate_buffers_that_cannot_grow():
     assert cand.copy_out(out) == n
     for c, w in zip(COLS, want):
         assert np.array_equal(out[c].view(np.uint8), w.view(np.uint8)), c
+
+
+def test_replayed_graph_belongs_to_its_run():
+    """Runs of equal shape and different cycle time, each in the place of the one before (its
+    memory is freed first): a captured search of one is not replayed for the next."""
+    cfg, lib, run = synth.make_workload("tiny_uneven", "numpy")
+    la = synth.library_arrays(lib)
+    slib = SpecLibFlat.from_arrays(**la)
+    params = params_from(cfg.params_dict())
+    sel = PeakGroupSelection(params, verbose=False, use_graph=True)
+    cand = sel.new_candidates()
+    for cycle_time in (1.0, 0.5, 2.0, 0.25):
+        r = dict(run, spectrum_rt=(run["spectrum_rt"] * np.float32(cycle_time)).astype(np.float32))
+        dia = DIAData.from_arrays(*(r[k] for k in RUN_KEYS), r["cycle"])
+        want = PeakGroupSelection(params, verbose=False).search(dia, slib).to_arrays()
+        for again in range(2):  # captured, replayed
+            sel.search_into(dia, slib, cand)
+            n = len(want[0])
+            assert cand.size() == n, cycle_time
+            out = {c: np.zeros(n, w.dtype) for c, w in zip(COLS, want)}
+            cand.copy_out(out)
+            for c, w in zip(COLS, want):
+                assert np.array_equal(out[c].view(np.uint8), w.view(np.uint8)), (cycle_time, again, c)
+        del dia
