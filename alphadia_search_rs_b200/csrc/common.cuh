@@ -247,6 +247,10 @@ __device__ __forceinline__ uint32_t grid_find_closest(const GridView& g, float m
   return ld < rd ? p.at + 1u : p.at;
 }
 
+// Fragment m/z ordering key: NaN sorts after every number (ties by library
+// position), so the output positions always form a permutation.
+__device__ __forceinline__ float mz_key(float m) { return m != m ? INFINITY : m; }
+
 // ln(x) of a float rounded to the nearest float: evaluated in double and rounded
 // once.  (The reference calls glibc logf, which is not correctly rounded for
 // about 1e-3 of its inputs: there the two differ by one ulp.)

@@ -524,12 +524,12 @@ __device__ __forceinline__ int64_t select_fragments(const ScoreArgs& a, const Sc
   const uint32_t need = topk ? 2u : 1u;
   for (int64_t r = 0; r < nraw; ++r) {
     if (s.u(KEEP + r) < need) continue;
-    const float m = a.l_fmz[fs + r];
+    const float m = a.l_fmz[fs + r], key = mz_key(m);
     int64_t pos = 0;  // stable: ties keep their library order
     for (int64_t j = 0; j < r; ++j)
-      if (s.u(KEEP + j) >= need) pos += !(a.l_fmz[fs + j] > m);
+      if (s.u(KEEP + j) >= need) pos += mz_key(a.l_fmz[fs + j]) <= key;
     for (int64_t j = r + 1; j < nraw; ++j)
-      if (s.u(KEEP + j) >= need) pos += a.l_fmz[fs + j] < m;
+      if (s.u(KEEP + j) >= need) pos += mz_key(a.l_fmz[fs + j]) < key;
     s.sf(FMZ + pos, m);
     s.su(FRAW + pos, (uint32_t)r);
   }

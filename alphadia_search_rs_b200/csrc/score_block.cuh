@@ -378,14 +378,14 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
     const SmVec s{vec + c * B.words};
     const uint32_t need = k.F > top_k ? 2u : 1u;
     if (s.u(KEEP + r) < need) continue;
-    const float m = s.f(RAWM + r);
+    const float m = s.f(RAWM + r), key = mz_key(m);
     int pos = 0;
 #pragma unroll 1
     for (int j = 0; j < r; ++j)
-      if (s.u(KEEP + j) >= need) pos += !(s.f(RAWM + j) > m);
+      if (s.u(KEEP + j) >= need) pos += mz_key(s.f(RAWM + j)) <= key;
 #pragma unroll 1
     for (int j = r + 1; j < k.nraw; ++j)
-      if (s.u(KEEP + j) >= need) pos += s.f(RAWM + j) < m;
+      if (s.u(KEEP + j) >= need) pos += mz_key(s.f(RAWM + j)) < key;
     s.sf(B.fmz + pos, m);
     s.sf(B.fint + pos, s.f(RAWI + r));
     if (QUANT) {

@@ -178,10 +178,6 @@ size_t plan_prep(PrepArgs* a, const AdsDia* d) {
   return a->rt_in_smem ? rb : 0;
 }
 
-// Fragment m/z ordering key: NaN sorts after every number (ties by library
-// position), so the output positions always form a permutation.
-__device__ __forceinline__ float mz_key(float m) { return m != m ? INFINITY : m; }
-
 // The ppm bin range of one kept fragment (src/quadrupole_observation/mod.rs:79-83,
 // src/mz_index/mod.rs:95-127), stored at its position in m/z order.
 __device__ __forceinline__ void write_fragment(const PrepArgs& a, int64_t p, int pos, float mz,

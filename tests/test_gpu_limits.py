@@ -152,3 +152,25 @@ def test_replayed_graph_belongs_to_its_run():
             for c, w in zip(COLS, want):
                 assert np.array_equal(out[c].view(np.uint8), w.view(np.uint8)), (cycle_time, again, c)
         del dia
+
+
+@pytest.mark.parametrize("span", [11, 400])
+def test_fragments_without_an_mz(span):
+    """NaN fragment m/z in scoring and quantification (in blocks, and the per-candidate
+    kernels of whole-run ranges): last in m/z order, ties in library order, as in the search
+    and the oracle."""
+    rng = np.random.default_rng(span)
+    P, F, n_cyc = 9, 7, 400
+    fmz = rng.uniform(200, 1700, (P, F))
+    none = np.zeros(0)
+    spectra = []
+    for c in range(n_cyc):
+        mz = np.sort(np.concatenate([rng.choice(fmz.reshape(-1), 30), rng.uniform(200, 1700, 20)]))
+        spectra += [(0, c, none, none), (1, c, mz, rng.lognormal(6, 1, len(mz)))]
+    run = run_of(spectra, 1)
+    for p in range(P):  # none to all of a precursor's fragments
+        fmz[p, rng.permutation(F)[:p % 8]] = np.nan
+    la = library_of(405.0, np.full(P, 200.0), fmz, rng.uniform(0.1, 1.0, (P, F)))
+    la["fragment_position"] = rng.integers(0, 200, P * F).astype(np.uint8)
+    start = rng.integers(0, n_cyc - span + 1, P)
+    assert_scored_and_quantified(run, la, candidates_at(np.arange(P), start, start + span), f"span {span}")
