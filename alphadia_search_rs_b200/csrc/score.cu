@@ -1102,8 +1102,10 @@ int block_group(const AdsDia* d, const BlockPlan& b, int64_t C) {
 template <bool QUANT>
 int launch_block(const QuantArgs& qa, const BlockPlan& b, int group, cudaStream_t st) {
   const size_t smem = block_smem_bytes(b, group);
+  // (the attribute is the process's: always the most, so that no thread's launch meets a
+  // smaller one of another's)
   ADS_CUDA(cudaFuncSetAttribute(score_block_kernel<QUANT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem));
+                                (int)kBlockSmem));
   score_block_kernel<QUANT><<<(int)((qa.s.n + group - 1) / group), kBlockThreads, smem, st>>>(qa, b, group);
   ADS_LAUNCH_CHECK();
   return ADS_OK;
@@ -1247,7 +1249,7 @@ int score_device(const AdsScoringParams* p, const AdsDia* d, AdsLib* l, int64_t 
     if (group > 0) {
       ADS_TRY(launch_block<false>(qa, plan, group, st));
       const size_t fs = feature_smem_bytes(plan);
-      ADS_CUDA(cudaFuncSetAttribute(feature_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fs));
+      ADS_CUDA(cudaFuncSetAttribute(feature_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFeatureSmem));
       feature_kernel<<<(int)((n + kFeatureGroup - 1) / kFeatureGroup), 128, fs, st>>>(qa, plan);
       ADS_LAUNCH_CHECK();
     } else if (a.order)

@@ -1018,7 +1018,9 @@ int enqueue_search(AdsSelection* s, const AdsDia* d, const AdsLib* l, AdsCandida
       return fail(ADS_ERR_INTERNAL, "search kernel plan exceeds shared memory (" +
                                         std::to_string(cmax_b) + " cycles)");
     void (*kern)(SearchArgs) = pick_search_kernel(s->h, bf16, grow, s->stats_on);
-    ADS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // (the attribute is the process's: always the most, so that no thread's launch meets a
+    // smaller one of another's)
+    ADS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
     int occ = 0;
     ADS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, nw * 32, smem));
     if (occ <= 0) return fail(ADS_ERR_INTERNAL, "search kernel cannot be resident");
@@ -1714,7 +1716,7 @@ int select_noalloc(const AdsDia* d, const AdsLib* l, const AdsSelectionParams* p
     return fail(ADS_ERR_INTERNAL, "search kernel plan exceeds shared memory (" +
                                       std::to_string(c_max) + " cycles)");
   void (*kern)(SearchArgs) = pick_search_kernel(h, false, grow, false);
-  ADS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  ADS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
   int occ = 0;
   ADS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, nw * 32, smem));
   if (occ <= 0) return fail(ADS_ERR_INTERNAL, "search kernel cannot be resident");

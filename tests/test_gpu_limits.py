@@ -174,3 +174,50 @@ def test_fragments_without_an_mz(span):
     la["fragment_position"] = rng.integers(0, 200, P * F).astype(np.uint8)
     start = rng.integers(0, n_cyc - span + 1, P)
     assert_scored_and_quantified(run, la, candidates_at(np.arange(P), start, start + span), f"span {span}")
+
+
+@pytest.mark.parametrize("what", ["score", "search"])
+def test_threads_with_different_plans(what):
+    """Threads whose calls of the same kernels take different amounts of shared memory (a
+    thread's candidates have 3 cycles or 60, its RT windows 80 or 1200): every call
+    succeeds, with its own thread's result."""
+    import threading
+
+    cfg = synth.get_config("tiny_uneven", n_cycles=1200, n_precursors=60, rt_half_window=(40.0, 40.0),
+                           frag_min=20, frag_max=24)
+    lib = synth.make_library(cfg, "numpy")
+    run = synth.make_run(cfg, lib, "numpy")
+    la = synth.library_arrays(lib)
+    dia = DIAData.from_arrays(*(run[k] for k in RUN_KEYS), run["cycle"])
+    slib = SpecLibFlat.from_arrays(**la)
+    scoring = PeakGroupScoring(ScoringParameters(), verbose=False)
+
+    def call_of(i):
+        if what == "search":
+            sel = PeakGroupSelection(params_from(dict(cfg.params_dict(), rt_tolerance=(40.0, 900.0)[i % 2])),
+                                     verbose=False)
+            return lambda: sel.search(dia, slib).to_arrays()
+        span = (3, 60)[i % 2]
+        c = candidates_at(la["precursor_idx"][:2], [100 * i, 50 + 100 * i], [100 * i + span, 50 + 100 * i + span])
+        cc = CandidateCollection.from_arrays(*(c[k] for k in COLS))
+        return lambda: list(scoring.score(dia, slib, cc).to_dict_arrays().values())
+
+    calls = [call_of(i) for i in range(8)]
+    want = [f() for f in calls]
+    faults = []
+
+    def work(i):
+        try:
+            for _ in range(1000):
+                got = calls[i]()
+            for a, b in zip(got, want[i]):
+                assert np.array_equal(a.view(np.uint8), b.view(np.uint8))
+        except Exception as e:  # noqa: BLE001 (told by the main thread)
+            faults.append((i, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not faults, faults
