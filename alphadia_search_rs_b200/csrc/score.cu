@@ -131,7 +131,9 @@ struct ScoreArgs {
   uint64_t* o_pidx;
   uint64_t* o_rank;
   float* o_feat;
-  uint32_t* heads;          // (block kernel) the candidates' vectors for feature_kernel, by work order
+  // (block kernels) a launch takes the candidates at .. at + take of the work order
+  int64_t at, take;
+  uint32_t* heads;   // their vectors for feature_kernel
   BlockCand* cands;  // and what the block knows of each
   uint8_t* o_found;
   int* err;
@@ -1099,6 +1101,11 @@ int block_group(const AdsDia* d, const BlockPlan& b, int64_t C) {
   return block_smem_bytes(b, group) <= kBlockSmem && feature_smem_bytes(b) <= kFeatureSmem ? group : 0;
 }
 
+// The vectors of so many bytes of candidates lie between score_block_kernel and
+// feature_kernel; calls of more candidates (360,000 of 24 fragments and 11 cycles) take
+// them in parts.
+constexpr size_t kHeadBytes = size_t(256) << 20;
+
 template <bool QUANT>
 int launch_block(const QuantArgs& qa, const BlockPlan& b, int group, cudaStream_t st) {
   const size_t smem = block_smem_bytes(b, group);
@@ -1106,7 +1113,7 @@ int launch_block(const QuantArgs& qa, const BlockPlan& b, int group, cudaStream_
   // smaller one of another's)
   ADS_CUDA(cudaFuncSetAttribute(score_block_kernel<QUANT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)kBlockSmem));
-  score_block_kernel<QUANT><<<(int)((qa.s.n + group - 1) / group), kBlockThreads, smem, st>>>(qa, b, group);
+  score_block_kernel<QUANT><<<(int)((qa.s.take + group - 1) / group), kBlockThreads, smem, st>>>(qa, b, group);
   ADS_LAUNCH_CHECK();
   return ADS_OK;
 }
@@ -1239,19 +1246,25 @@ int score_device(const AdsScoringParams* p, const AdsDia* d, AdsLib* l, int64_t 
     ADS_CUDA(cudaEventCreate(&ev.b));
     TmpBuf<uint32_t> heads(st);
     TmpBuf<BlockCand> cands(st);
+    int64_t part = n;  // candidates of a launch
     if (group > 0) {
-      ADS_TRY(heads.alloc((size_t)n * plan.head));
-      ADS_TRY(cands.alloc((size_t)n));
+      const size_t each = (size_t)plan.head * 4 + sizeof(BlockCand);
+      part = std::min<int64_t>(n, std::max<int64_t>(1, (int64_t)(kHeadBytes / each / kFeatureGroup)) * kFeatureGroup);
+      ADS_TRY(heads.alloc((size_t)part * plan.head));
+      ADS_TRY(cands.alloc((size_t)part));
       a.heads = heads.p;
       a.cands = cands.p;
     }
     ADS_CUDA(cudaEventRecord(ev.a, st));
     if (group > 0) {
-      ADS_TRY(launch_block<false>(qa, plan, group, st));
       const size_t fs = feature_smem_bytes(plan);
       ADS_CUDA(cudaFuncSetAttribute(feature_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFeatureSmem));
-      feature_kernel<<<(int)((n + kFeatureGroup - 1) / kFeatureGroup), 128, fs, st>>>(qa, plan);
-      ADS_LAUNCH_CHECK();
+      for (a.at = 0; a.at < n; a.at += part) {
+        a.take = std::min(part, n - a.at);
+        ADS_TRY(launch_block<false>(qa, plan, group, st));
+        feature_kernel<<<(int)((a.take + kFeatureGroup - 1) / kFeatureGroup), 128, fs, st>>>(qa, plan);
+        ADS_LAUNCH_CHECK();
+      }
     } else if (a.order)
       score_kernel<true><<<(int)((T + kScoreBlock - 1) / kScoreBlock), kScoreBlock, 0, st>>>(a);
     else
@@ -1412,6 +1425,7 @@ int quant_device(const AdsQuantParams* p, const AdsDia* d, AdsLib* l, int64_t n,
     ADS_CUDA(cudaEventCreate(&ev.a));
     ADS_CUDA(cudaEventCreate(&ev.b));
     ADS_CUDA(cudaEventRecord(ev.a, st));
+    a.take = n;
     if (group > 0)
       ADS_TRY(launch_block<true>(qa, plan, group, st));
     else if (qa.s.order)

@@ -260,17 +260,17 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
   uint32_t* vec = reinterpret_cast<uint32_t*>(cand + group);
   uint32_t* thr = vec + (size_t)group * B.words;
   __shared__ int sh_max[3];  // of the group: raw fragments, kept fragments, cycles
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
   const ThreadVec own{thr + tid};
   const Ln ln{a.ln_tab, LnCoef()};
-  const int64_t first = (int64_t)blockIdx.x * group;
+  const int64_t first = a.at + (int64_t)blockIdx.x * group, end = a.at + a.take;
 
   // ---- the candidates and their precursors
   __shared__ int64_t sh_row[kGroup];
   if (tid < 3) sh_max[tid] = 0;
   {
     const int c = tid / kRowLanes;
-    const bool on = c < group && first + c < a.n;
+    const bool on = c < group && first + c < end;
     const int64_t q = on ? (a.order ? (int64_t)a.order[first + c] : first + c) : 0;
     const int64_t row = find_row(a.l_pidx, on ? a.P : 0, on ? a.c_pidx[q] : 0, lane);
     if (on && tid % kRowLanes == 0) sh_row[c] = row;
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
     k.fs = k.prec = 0;
     k.nraw = k.F = k.cs = k.C = k.woff = k.wlen = k.nz = 0;
     k.pmz = 0.0f;
-    if (first + tid < a.n) {
+    if (first + tid < end) {
       const int64_t q = a.order ? (int64_t)a.order[first + tid] : first + tid;
       const uint64_t pidx = a.c_pidx[q], cs64 = a.c_start[q], ce64 = a.c_stop[q], center = a.c_center[q];
       bool take = true;
@@ -537,9 +537,9 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
   // ---- what feature_kernel needs of them
   for (int t = tid; t < group * B.head; t += kBlockThreads) {
     const int c = t / B.head, j = t - c * B.head;
-    if (cand[c].q >= 0) a.heads[(first + c) * B.head + j] = vec[c * B.words + j];
+    if (cand[c].q >= 0) a.heads[(first - a.at + c) * B.head + j] = vec[c * B.words + j];
   }
-  if (tid < group && first + tid < a.n) a.cands[first + tid] = cand[tid];
+  if (tid < group && first + tid < end) a.cands[first - a.at + tid] = cand[tid];
 }
 
 // The features of the candidates that score_block_kernel has been through, from their
@@ -558,8 +558,8 @@ __global__ void __launch_bounds__(128) feature_kernel(const __grid_constant__ Qu
   const ScoreArgs& a = qa.s;
   extern __shared__ __align__(16) uint32_t feature_smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int64_t first = (int64_t)blockIdx.x * kFeatureGroup;
-  const int here = (int)min((int64_t)kFeatureGroup, a.n - first);
+  const int64_t first = (int64_t)blockIdx.x * kFeatureGroup;  // of the launch's candidates
+  const int here = (int)min((int64_t)kFeatureGroup, a.take - first);
   const int words = (B.head + 2 * B.Fm) | 1;
   const Ln ln{a.ln_tab, LnCoef()};
   for (int t = tid; t < here * B.head; t += 128) {

@@ -10,7 +10,7 @@ from alphadia_search_rs_b200 import (CandidateCollection, DIAData, PeakGroupQuan
                                      ScoringParameters, SpecLibFlat, synth)
 
 from _util import COLS, RUN_KEYS, params_from
-from test_gpu_quant import assert_quant_equal
+from test_gpu_quant import assert_quant_equal, quant_library
 from test_gpu_scoring import assert_features_equal, build
 from test_gpu_sizes import library_of, run_of
 
@@ -221,3 +221,26 @@ def test_threads_with_different_plans(what):
     for t in threads:
         t.join()
     assert not faults, faults
+
+
+def test_scoring_in_parts():
+    """More candidates than one pair of launches takes (360,000 here): every copy of a
+    candidate has the oracle's features, in its own row, also where the work order mixes
+    precursors of few and many fragments; and the device holds little besides the results
+    (all candidates' vectors at once would be 2.9 GB)."""
+    import torch
+
+    cfg, lib, run = synth.make_workload("tiny_uneven", "numpy")
+    la = quant_library(synth.library_arrays(lib), seed=4)
+    dia, slib, od, ol = build(run, la)
+    rng = np.random.default_rng(4)
+    m, n = 500, 4_000_000
+    start = rng.integers(0, cfg.n_cycles - 11, m)
+    few = candidates_at(la["precursor_idx"][rng.integers(0, cfg.n_precursors, m)], start, start + 11)
+    ref = oracle.score(od, ol, few, log_mode=oracle.LOG_RN)
+    at = rng.integers(0, m, n)
+    cc = CandidateCollection.from_arrays(*(few[k][at] for k in COLS))
+    free = torch.cuda.mem_get_info()[0]
+    feats = PeakGroupScoring(ScoringParameters(), verbose=False).score(dia, slib, cc)
+    assert free - torch.cuda.mem_get_info()[0] < n * (41 * 4 + 17) + 1.75 * 2**30
+    assert_features_equal(feats.to_dict_arrays(), {k: v[at] for k, v in ref.items()}, exact=True, where="in parts")
