@@ -34,6 +34,24 @@ constexpr int kBinRegs = 4;           // bins of up to this many entries are sor
 constexpr int kBinThread = 24;        // up to this many by one thread in place
 constexpr int kBinShared = 1024;      // up to this many by a block in shared memory, else in place
 
+// A warp takes up to so many peaks of one spectrum: spectra of 150,000 peaks, a warp each,
+// left most of the GPU idle (400 of them, 60 M peaks, 123 ms).
+constexpr int kPiecePeaks = 2048;
+constexpr int kPieceShift = 40;  // a piece: its spectrum, and above it its number in the spectrum
+
+struct PeakPiece {
+  int64_t s;      // spectrum
+  int64_t first;  // its first peak, counted in the spectrum
+  int64_t n;      // peaks
+};
+__device__ __forceinline__ PeakPiece peak_piece(int64_t id, const int64_t* pstart, const int64_t* pstop) {
+  PeakPiece p;
+  p.s = id & ((int64_t(1) << kPieceShift) - 1);
+  p.first = (id >> kPieceShift) * kPiecePeaks;
+  p.n = min(pstop[p.s] - pstart[p.s] - p.first, (int64_t)kPiecePeaks);
+  return p;
+}
+
 // One observation of a group.
 struct BuildWin {
   int64_t ss;       // element offset of its slice_starts
@@ -43,9 +61,9 @@ struct BuildWin {
 // A peak on its way to its bin: x intensity, y visit position in the observation, z cycle.
 __device__ __forceinline__ uint64_t record_key(const uint4& r) { return (uint64_t)r.z << 32 | r.y; }
 
-// One warp per spectrum (listed in window, then visit order): every peak's bin and its
-// number within the bin (in order of arrival, which is any).
-__global__ void __launch_bounds__(256) count_peaks_kernel(int64_t n_spec, const int64_t* __restrict__ list,
+// One warp per piece of a spectrum (listed in window, then visit order): every peak's bin and
+// its number within the bin (in order of arrival, which is any).
+__global__ void __launch_bounds__(256) count_peaks_kernel(int64_t n_pieces, const int64_t* __restrict__ list,
                                                           const int64_t* __restrict__ item_off,
                                                           const int64_t* __restrict__ pstart,
                                                           const int64_t* __restrict__ pstop,
@@ -56,11 +74,11 @@ __global__ void __launch_bounds__(256) count_peaks_kernel(int64_t n_spec, const 
                                                           uint32_t* __restrict__ starts) {
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (warp >= n_spec) return;
-  const int64_t s = list[warp];
-  const int64_t b = pstart[s], n = pstop[s] - b;
-  uint2* to = bins + (item_off[s] - item0);
-  uint32_t* count = starts + wins[win[s] - win0].ss + 1;
+  if (warp >= n_pieces) return;
+  const PeakPiece p = peak_piece(list[warp], pstart, pstop);
+  const int64_t b = pstart[p.s] + p.first, n = p.n;
+  uint2* to = bins + (item_off[p.s] + p.first - item0);
+  uint32_t* count = starts + wins[win[p.s] - win0].ss + 1;
 #pragma unroll 2
   for (int64_t k = lane; k < n; k += 32) {
     const uint32_t bin = grid_find_closest(g, __ldg(mz + b + k));
@@ -156,22 +174,22 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles_kernel(int64_t grid_l
 
 // Every peak to its place, as a record.
 __global__ void __launch_bounds__(256) place_peaks_kernel(
-    int64_t n_spec, const int64_t* __restrict__ list, const int64_t* __restrict__ item_off,
+    int64_t n_pieces, const int64_t* __restrict__ list, const int64_t* __restrict__ item_off,
     const int64_t* __restrict__ pstart, const int64_t* __restrict__ pstop, const int32_t* __restrict__ win,
     const uint16_t* __restrict__ cyc, int win0, const BuildWin* __restrict__ wins, int64_t item0,
     const float* __restrict__ inten, const uint2* __restrict__ bins, const uint32_t* __restrict__ starts,
     uint4* __restrict__ recs) {
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (warp >= n_spec) return;
-  const int64_t s = list[warp];
-  const BuildWin w = wins[win[s] - win0];
-  const int64_t b = pstart[s], n = pstop[s] - b;
-  const uint2* from = bins + (item_off[s] - item0);
+  if (warp >= n_pieces) return;
+  const PeakPiece p = peak_piece(list[warp], pstart, pstop);
+  const BuildWin w = wins[win[p.s] - win0];
+  const int64_t b = pstart[p.s] + p.first, n = p.n, at = item_off[p.s] + p.first;
+  const uint2* from = bins + (at - item0);
   const uint32_t* first = starts + w.ss;
   uint4* to = recs + (w.base - item0);
-  const uint32_t c = cyc[s];
-  const uint32_t vis0 = (uint32_t)(item_off[s] - w.base);
+  const uint32_t c = cyc[p.s];
+  const uint32_t vis0 = (uint32_t)(at - w.base);
 #pragma unroll 4
   for (int64_t k = lane; k < n; k += 32) {
     const uint2 br = from[k];
@@ -308,14 +326,24 @@ int fetch(const T* src, int64_t n, int loc, std::vector<T>& dst) {
 }
 
 // Uploads the spectrum table (and host peak arrays), and builds cycles, intens and
-// slice_starts.  `list`: the spectra of window w in visit order from first_spec[w].
-int build_entries(AdsDia* d, const AdsRawArrays* raw, const std::vector<int32_t>& win_of_spec,
+// slice_starts.  `spec_list`: the spectra of window w in visit order from first_spec[w].
+int build_entries(AdsDia* d, const AdsRawArrays* raw, const SpectrumTable& t, const std::vector<int32_t>& win_of_spec,
                   const std::vector<uint16_t>& cyc16, const std::vector<int64_t>& item_off,
-                  int64_t n_items, const std::vector<int64_t>& list, const std::vector<int64_t>& first_spec,
+                  int64_t n_items, const std::vector<int64_t>& spec_list, const std::vector<int64_t>& first_spec,
                   int64_t n_slots, const GridView& g, cudaStream_t st) {
   const int64_t n_spec = raw->n_spectra;
   const int64_t stride = d->grid_len + 1;
   if (n_slots == 0 || n_items == 0) return ADS_OK;
+  // the pieces of the spectra, in the same order
+  std::vector<int64_t> list, first_piece((size_t)d->n_obs + 1, 0);
+  list.reserve(spec_list.size());
+  for (int64_t w = 0; w < d->n_obs; ++w) {
+    for (int64_t k = first_spec[w]; k < first_spec[w + 1]; ++k) {
+      const int64_t s = spec_list[k], n = t.stop[s] - t.start[s];
+      for (int64_t i = 0; i * kPiecePeaks < n; ++i) list.push_back(s | i << kPieceShift);
+    }
+    first_piece[w + 1] = (int64_t)list.size();
+  }
   // device copies of the spectrum table and, if needed, the peak arrays
   DevBuf<int64_t> d_off, d_start, d_stop;
   DevBuf<int32_t> d_win;
@@ -354,7 +382,7 @@ int build_entries(AdsDia* d, const AdsRawArrays* raw, const std::vector<int32_t>
 
   // the observations that hold peaks, in groups of up to kGroupItems peaks (or one)
   struct Group {
-    int64_t w0, w1, items, specs;
+    int64_t w0, w1, items, pieces;
     int slots;
   };
   std::vector<Group> groups;
@@ -370,7 +398,7 @@ int build_entries(AdsDia* d, const AdsRawArrays* raw, const std::vector<int32_t>
     Group& gr = groups.back();
     gr.w1 = w + 1;
     gr.items += d->num_peaks[w];
-    gr.specs += first_spec[w + 1] - first_spec[w];
+    gr.pieces += first_piece[w + 1] - first_piece[w];
     ++gr.slots;
     most_items = std::max(most_items, gr.items);
     most_slots = std::max(most_slots, gr.slots);
@@ -393,9 +421,9 @@ int build_entries(AdsDia* d, const AdsRawArrays* raw, const std::vector<int32_t>
     const Group& gr = groups[k];
     const int64_t item0 = d->win[gr.w0].base;
     const BuildWin* gw = d_wins.p + gr.w0;
-    const int64_t* gl = d_list.p + first_spec[gr.w0];
-    const int sg = (int)((gr.specs + 7) / 8);
-    count_peaks_kernel<<<sg, 256, 0, st>>>(gr.specs, gl, d_off.p, pstart, pstop, d_win.p, (int)gr.w0, gw, item0,
+    const int64_t* gl = d_list.p + first_piece[gr.w0];
+    const int sg = (int)((gr.pieces + 7) / 8);
+    count_peaks_kernel<<<sg, 256, 0, st>>>(gr.pieces, gl, d_off.p, pstart, pstop, d_win.p, (int)gr.w0, gw, item0,
                                            mz, g, bins.p, d->slice_starts.p);
     ADS_LAUNCH_CHECK();
     tile_sums_kernel<<<gr.slots * tiles, kScanThreads, 0, st>>>(d->grid_len, tiles, gw, d->slice_starts.p, sums.p);
@@ -404,7 +432,7 @@ int build_entries(AdsDia* d, const AdsRawArrays* raw, const std::vector<int32_t>
     ADS_LAUNCH_CHECK();
     scan_tiles_kernel<<<gr.slots * tiles, kScanThreads, 0, st>>>(d->grid_len, tiles, gw, sums.p, d->slice_starts.p);
     ADS_LAUNCH_CHECK();
-    place_peaks_kernel<<<sg, 256, 0, st>>>(gr.specs, gl, d_off.p, pstart, pstop, d_win.p, d_cyc.p, (int)gr.w0, gw,
+    place_peaks_kernel<<<sg, 256, 0, st>>>(gr.pieces, gl, d_off.p, pstart, pstop, d_win.p, d_cyc.p, (int)gr.w0, gw,
                                            item0, pint, bins.p, d->slice_starts.p, recs.p);
     ADS_LAUNCH_CHECK();
     order_bins_kernel<<<dim3((unsigned)((d->grid_len + 255) / 256), (unsigned)gr.slots), 256, 0, st>>>(
@@ -618,7 +646,8 @@ int dia_create(const AdsRawArrays* raw, int device, AdsDia** out) {
   ADS_TRY(device_grid(device, &g));
   cudaStream_t st;
   ADS_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-  const int rc = build_entries(d, raw, win_of_spec, cyc16, item_off, n_items, spec_list, first_spec, n_slots, g, st);
+  const int rc = build_entries(d, raw, t, win_of_spec, cyc16, item_off, n_items, spec_list, first_spec,
+                               n_slots, g, st);
   cudaStreamDestroy(st);
   if (rc != ADS_OK) return rc;
 

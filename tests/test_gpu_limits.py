@@ -7,12 +7,12 @@ import pytest
 import oracle
 from alphadia_search_rs_b200 import (CandidateCollection, DIAData, PeakGroupQuantification,
                                      PeakGroupScoring, PeakGroupSelection, QuantificationParameters,
-                                     ScoringParameters, SpecLibFlat, synth)
+                                     ScoringParameters, SpecLibFlat, mz_grid, synth)
 
 from _util import COLS, RUN_KEYS, params_from
 from test_gpu_quant import assert_quant_equal, quant_library
 from test_gpu_scoring import assert_features_equal, build
-from test_gpu_sizes import library_of, run_of
+from test_gpu_sizes import closest_bins, library_of, run_of
 
 pytestmark = pytest.mark.gpu
 
@@ -244,3 +244,78 @@ def test_scoring_in_parts():
     feats = PeakGroupScoring(ScoringParameters(), verbose=False).score(dia, slib, cc)
     assert free - torch.cuda.mem_get_info()[0] < n * (41 * 4 + 17) + 1.75 * 2**30
     assert_features_equal(feats.to_dict_arrays(), {k: v[at] for k, v in ref.items()}, exact=True, where="in parts")
+
+
+def assert_entries_in_order(dia, spectra, n_windows, where):
+    """Entries by (bin, cycle), ties in visit order."""
+    grid = mz_grid()
+    for w in range(1, n_windows + 1):
+        rows = [s for s in spectra if s[0] == w]
+        mz = np.concatenate([s[2] for s in rows]).astype(np.float32)
+        cyc = np.concatenate([np.full(len(s[2]), s[1]) for s in rows])
+        inten = np.concatenate([s[3] for s in rows]).astype(np.float32)
+        bins = closest_bins(grid, mz)
+        order = np.lexsort((np.arange(len(mz)), cyc, bins))
+        got = dia.observation(w)
+        starts = np.concatenate([[0], np.cumsum(np.bincount(bins, minlength=len(grid)))])
+        assert np.array_equal(got["slice_starts"], starts.astype(np.uint32)), (where, w)
+        assert np.array_equal(got["cycle_indices"], cyc[order].astype(np.uint16)), (where, w)
+        assert np.array_equal(got["intensities"].view(np.uint32), inten[order].view(np.uint32)), (where, w)
+
+
+@pytest.mark.parametrize("peaks", [2047, 2048, 2049, 4096, 10_001])
+def test_build_of_long_spectra(peaks):
+    """Spectra around the multiples of the 2048 peaks that a warp takes."""
+    rng = np.random.default_rng(peaks)
+    none = np.zeros(0)
+    spectra = []
+    for c in range(7):
+        spectra.append((0, c, none, none))
+        for w in (1, 2):
+            n = peaks + (w - 1) * int(rng.integers(0, 3000))
+            spectra.append((w, c, rng.uniform(150, 2000, n), rng.lognormal(5, 2, n)))
+    run = run_of(spectra, 2)
+    dia = DIAData.from_arrays(*(run[k] for k in RUN_KEYS), run["cycle"])
+    assert_entries_in_order(dia, spectra, 2, peaks)
+
+
+def device_run(cycles, windows, peaks, mz):
+    """A run of device arrays: `mz(n)` gives the peaks' m/z."""
+    import torch
+
+    dsi = torch.arange(windows + 1, device="cuda").repeat(cycles)
+    cyc = torch.arange(cycles, device="cuda").repeat_interleave(windows + 1)
+    stop = torch.cumsum(torch.where(dsi == 0, 0, peaks), 0)
+    lo = torch.where(dsi == 0, -1.0, 390.0 + 10.0 * dsi).float()
+    n = cycles * windows * peaks
+    return dict(spectrum_delta_scan_idx=dsi, isolation_lower_mz=lo, isolation_upper_mz=(lo + 10.0).float(),
+                spectrum_peak_start_idx=stop - torch.where(dsi == 0, 0, peaks), spectrum_peak_stop_idx=stop,
+                spectrum_cycle_idx=cyc, spectrum_rt=cyc.float(), peak_mz=mz(n).float(),
+                peak_intensity=torch.rand(n, device="cuda") + 1.0,
+                cycle=np.zeros((windows + 1, 1, 1, 1), np.float32))
+
+
+def build_ms(run):
+    import time
+
+    import torch
+
+    best = 1e9
+    for _ in range(6):
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        dia = DIAData.from_arrays(**run)
+        torch.cuda.synchronize()
+        best = min(best, time.perf_counter() - t0)
+        del dia
+    return best * 1e3
+
+
+def test_build_time_of_long_spectra():
+    """24 M peaks in 160 spectra take no more than 4 times as long as in 24,000 (a warp for
+    each of the 160: 20 times)."""
+    import torch
+
+    mz = lambda n: torch.rand(n, device="cuda") * 1650 + 150
+    few, many = build_ms(device_run(20, 8, 150_000, mz)), build_ms(device_run(3000, 8, 1000, mz))
+    assert few < 4 * many, (few, many)
