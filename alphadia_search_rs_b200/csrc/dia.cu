@@ -7,6 +7,8 @@
 //   intens[base(w) + i]       f32 intensity of entry i
 // Entries are ordered by (bin, cycle), ties in the order the reference visits
 // peaks (spectrum index, then peak index), exactly like its stable sort_by_key.
+#include <cub/cub.cuh>
+
 #include <algorithm>
 #include <cstring>
 #include <memory>
@@ -23,7 +25,7 @@ namespace {
 // entries.  Peaks of a group of observations, their counts and records fit the L2, so what
 // crosses the memory bus is little more than the peaks once in and the entries once out,
 // and the temporary memory is one group's (100 MB).  A radix sort of (window, bin, cycle)
-// keys with peak indices moved 12 bytes a peak six times through 24 bytes a peak of
+// keys with peak indices for all moved 12 bytes a peak six times through 24 bytes a peak of
 // temporaries: 324 M peaks in 25 ms of kernels and 100 ms of mapping and unmapping that
 // memory; now 18 ms of kernels and none.  What bounds it: the counting's atomics in the L2
 // (5 ms) and the records' scattered writes and reads there (10 ms).
@@ -32,7 +34,26 @@ constexpr int kScanTile = 8192;       // bins of one scan block
 constexpr int kScanThreads = 256;
 constexpr int kBinRegs = 4;           // bins of up to this many entries are sorted in registers
 constexpr int kBinThread = 24;        // up to this many by one thread in place
-constexpr int kBinShared = 1024;      // up to this many by a block in shared memory, else in place
+constexpr int kBinShared = 1024;      // up to this many by a block in shared memory
+// Bins of many peaks undo that: a block sorts one, and peaks outside the grid all lie in its
+// first and last bin.  A group with a bin of more than kBinShared peaks, or with more than
+// 1 / kCrowdedShare of its peaks in bins of more than kBinThread, is told by its counts
+// before any peak is placed, and sorted whole by a stable radix sort of (window, bin, cycle)
+// keys afterwards, whose time does not depend on the bins.  60 M peaks, 10 % of them below the
+// grid: 1166 -> 9.3 ms; 1 %: 88 -> 9.3; in 2000 bins: 20 -> 9.1; none crowded: 4.9.  The line:
+// 12 M peaks of 16, 20 and 30 a bin in the mean 2.56, 3.12 and 3.95 ms counted, 2.32 sorted;
+// a quarter of them in bins of 40, 200 and 700 2.13, 1.79 and 1.96, half 2.71, 2.15 and 2.38,
+// against 2.26.
+constexpr int kCrowdedShare = 8;
+
+struct GroupCounts {
+  unsigned int crowded;  // peaks in bins of more than kBinThread
+  unsigned int widest;   // peaks of the widest of those bins
+  unsigned int listed;   // of those bins, for order_large_bins_kernel
+};
+__host__ __device__ inline bool sorted_whole(const GroupCounts& c, int64_t items) {
+  return c.widest > (unsigned)kBinShared || (int64_t)c.crowded * kCrowdedShare > items;
+}
 
 // A warp takes up to so many peaks of one spectrum: spectra of 150,000 peaks, a warp each,
 // left most of the GPU idle (400 of them, 60 M peaks, 123 ms).
@@ -61,6 +82,20 @@ struct BuildWin {
 // A peak on its way to its bin: x intensity, y visit position in the observation, z cycle.
 __device__ __forceinline__ uint64_t record_key(const uint4& r) { return (uint64_t)r.z << 32 | r.y; }
 
+// The grid's first and last bin take every peak outside it: a warp's of them are numbered by
+// one atomic (60 M peaks, 10 % of them below the grid: 14.9 -> 9.5 ms).  Whole warps call it.
+__device__ __forceinline__ bool at_end(const GridView& g, uint32_t bin) { return bin == 0u || bin == g.n - 1u; }
+__device__ __noinline__ uint32_t number_peak(uint32_t* count, const GridView& g, uint32_t bin, bool on, int lane) {
+  const bool end = on && at_end(g, bin);
+  const unsigned lo = __ballot_sync(0xffffffffu, end && bin == 0u), hi = __ballot_sync(0xffffffffu, end && bin != 0u);
+  const unsigned own = bin == 0u ? lo : hi;
+  const int first = __ffs(own) - 1;  // (of lanes at an end: the first of their bin)
+  uint32_t number = 0;
+  if (on && (!end || lane == first)) number = atomicAdd(count + bin, end ? (uint32_t)__popc(own) : 1u);
+  const uint32_t base = __shfl_sync(0xffffffffu, number, end ? first : lane);
+  return end ? base + (uint32_t)__popc(own & ((1u << lane) - 1u)) : number;
+}
+
 // One warp per piece of a spectrum (listed in window, then visit order): every peak's bin and
 // its number within the bin (in order of arrival, which is any).
 __global__ void __launch_bounds__(256) count_peaks_kernel(int64_t n_pieces, const int64_t* __restrict__ list,
@@ -79,10 +114,22 @@ __global__ void __launch_bounds__(256) count_peaks_kernel(int64_t n_pieces, cons
   const int64_t b = pstart[p.s] + p.first, n = p.n;
   uint2* to = bins + (item_off[p.s] + p.first - item0);
   uint32_t* count = starts + wins[win[p.s] - win0].ss + 1;
-#pragma unroll 2
-  for (int64_t k = lane; k < n; k += 32) {
-    const uint32_t bin = grid_find_closest(g, __ldg(mz + b + k));
-    to[k] = make_uint2(bin, atomicAdd(count + bin, 1u));
+  // two peaks a lane at a time: their loads and atomics overlap
+  for (int64_t k0 = 0; k0 < n; k0 += 64) {
+    const int64_t k = k0 + lane;
+    const bool on_a = k < n, on_b = k + 32 < n;
+    const uint32_t bin_a = on_a ? grid_find_closest(g, __ldg(mz + b + k)) : 1u;
+    const uint32_t bin_b = on_b ? grid_find_closest(g, __ldg(mz + b + k + 32)) : 1u;
+    uint32_t number_a = 0, number_b = 0;
+    if (__any_sync(0xffffffffu, at_end(g, bin_a) || at_end(g, bin_b))) {
+      number_a = number_peak(count, g, bin_a, on_a, lane);
+      number_b = number_peak(count, g, bin_b, on_b, lane);
+    } else {
+      if (on_a) number_a = atomicAdd(count + bin_a, 1u);
+      if (on_b) number_b = atomicAdd(count + bin_b, 1u);
+    }
+    if (on_a) to[k] = make_uint2(bin_a, number_a);
+    if (on_b) to[k + 32] = make_uint2(bin_b, number_b);
   }
 }
 
@@ -119,14 +166,31 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* sh, uint32_
 __global__ void __launch_bounds__(kScanThreads) tile_sums_kernel(int64_t grid_len, int tiles,
                                                                  const BuildWin* __restrict__ wins,
                                                                  const uint32_t* __restrict__ starts,
-                                                                 uint32_t* __restrict__ sums) {
+                                                                 uint32_t* __restrict__ sums,
+                                                                 GroupCounts* __restrict__ counts) {
   __shared__ uint32_t sh[33];
   const int w = blockIdx.x / tiles, t = blockIdx.x - w * tiles;
   const uint32_t* c = starts + wins[w].ss + 1;
-  uint32_t v = 0, total;
-  for (int i = threadIdx.x; i < kScanTile; i += kScanThreads) {
-    const int64_t b = (int64_t)t * kScanTile + i;
-    if (b < grid_len) v += c[b];
+  uint32_t v = 0, total, crowded = 0, widest = 0;
+  c += (int64_t)t * kScanTile;
+  const int here = (int)min(grid_len - (int64_t)t * kScanTile, (int64_t)kScanTile);
+#pragma unroll 8
+  for (int i = threadIdx.x; i < here; i += kScanThreads) {
+    const uint32_t n = c[i];
+    v += n;
+    if (n > (uint32_t)kBinThread) {
+      crowded += n;
+      widest = max(widest, n);
+    }
+  }
+  __syncwarp();
+  crowded = __reduce_add_sync(0xffffffffu, crowded);
+  if (crowded) {
+    widest = __reduce_max_sync(0xffffffffu, widest);
+    if ((threadIdx.x & 31) == 0) {
+      atomicAdd(&counts->crowded, crowded);
+      atomicMax(&counts->widest, widest);
+    }
   }
   block_scan(v, sh, &total);
   if (threadIdx.x == 0) sums[blockIdx.x] = total;
@@ -178,7 +242,8 @@ __global__ void __launch_bounds__(256) place_peaks_kernel(
     const int64_t* __restrict__ pstart, const int64_t* __restrict__ pstop, const int32_t* __restrict__ win,
     const uint16_t* __restrict__ cyc, int win0, const BuildWin* __restrict__ wins, int64_t item0,
     const float* __restrict__ inten, const uint2* __restrict__ bins, const uint32_t* __restrict__ starts,
-    uint4* __restrict__ recs) {
+    uint4* __restrict__ recs, const GroupCounts* __restrict__ counts, int64_t items) {
+  if (sorted_whole(*counts, items)) return;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= n_pieces) return;
@@ -211,14 +276,15 @@ __global__ void __launch_bounds__(256) order_bins_kernel(int64_t grid_len, const
                                                          int64_t item0, const uint32_t* __restrict__ starts,
                                                          uint4* recs, uint16_t* __restrict__ cyc,
                                                          float* __restrict__ inten, uint2* __restrict__ large,
-                                                         unsigned int* __restrict__ n_large) {
+                                                         GroupCounts* counts, int64_t items) {
+  if (sorted_whole(*counts, items)) return;
   const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (b >= grid_len) return;
   const BuildWin bw = wins[blockIdx.y];
   const uint32_t e0 = starts[bw.ss + b], n = starts[bw.ss + b + 1] - e0;
   if (n == 0) return;
   if (n > kBinThread) {
-    large[atomicAdd(n_large, 1u)] = make_uint2(blockIdx.y, (unsigned)b);
+    large[atomicAdd(&counts->listed, 1u)] = make_uint2(blockIdx.y, (unsigned)b);
     return;
   }
   uint4* r = recs + (bw.base - item0) + e0;
@@ -278,33 +344,63 @@ __device__ void block_sort(uint4* r, uint32_t n) {
   }
 }
 
-// The bins that order_bins_kernel listed, a block each.
-__global__ void __launch_bounds__(256) order_large_bins_kernel(const unsigned int* __restrict__ n_large,
+// The bins that order_bins_kernel listed (none of a group that is sorted whole), a block each.
+__global__ void __launch_bounds__(256) order_large_bins_kernel(const GroupCounts* __restrict__ counts,
                                                                const uint2* __restrict__ large,
                                                                const BuildWin* __restrict__ wins,
                                                                int64_t item0,
                                                                const uint32_t* __restrict__ starts,
-                                                               uint4* recs, uint16_t* __restrict__ cyc,
+                                                               const uint4* __restrict__ recs,
+                                                               uint16_t* __restrict__ cyc,
                                                                float* __restrict__ inten) {
   __shared__ uint4 tile[kBinShared];
-  const unsigned int m = *n_large;
+  const unsigned int m = counts->listed;
   for (unsigned int l = blockIdx.x; l < m; l += gridDim.x) {
     const uint2 id = large[l];
     const BuildWin bw = wins[id.x];
     const uint32_t e0 = starts[bw.ss + id.y], n = starts[bw.ss + id.y + 1] - e0;
-    uint4* r = recs + (bw.base - item0) + e0;
-    if (n <= kBinShared) {
-      for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) tile[i] = r[i];
-      __syncthreads();
-      r = tile;
-    }
-    block_sort(r, n);
+    const uint4* r = recs + (bw.base - item0) + e0;
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) tile[i] = r[i];
+    __syncthreads();
+    block_sort(tile, n);
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-      cyc[bw.base + e0 + i] = (uint16_t)r[i].z;
-      inten[bw.base + e0 + i] = __uint_as_float(r[i].x);
+      cyc[bw.base + e0 + i] = (uint16_t)tile[i].z;
+      inten[bw.base + e0 + i] = __uint_as_float(tile[i].x);
     }
     __syncthreads();
   }
+}
+
+// ---- groups that are sorted whole: every peak's key and intensity in visit order, a stable
+// radix sort of the keys (window of the group, bin, cycle), the entries
+constexpr int kKeyBinShift = 16;
+constexpr int kKeyWinShift = 38;  // 22 bits of bin
+
+__global__ void __launch_bounds__(256) key_peaks_kernel(
+    int64_t n_pieces, const int64_t* __restrict__ list, const int64_t* __restrict__ item_off,
+    const int64_t* __restrict__ pstart, const int64_t* __restrict__ pstop, const int32_t* __restrict__ win,
+    const uint16_t* __restrict__ cyc, int win0, int64_t item0, const float* __restrict__ mz,
+    const float* __restrict__ inten, GridView g, uint64_t* __restrict__ keys, float* __restrict__ vals) {
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (warp >= n_pieces) return;
+  const PeakPiece p = peak_piece(list[warp], pstart, pstop);
+  const int64_t b = pstart[p.s] + p.first, to = item_off[p.s] + p.first - item0;
+  const uint64_t rest = (uint64_t)(win[p.s] - win0) << kKeyWinShift | cyc[p.s];
+  for (int64_t k = lane; k < p.n; k += 32) {
+    keys[to + k] = rest | (uint64_t)grid_find_closest(g, __ldg(mz + b + k)) << kKeyBinShift;
+    vals[to + k] = __ldg(inten + b + k);
+  }
+}
+
+__global__ void __launch_bounds__(256) sorted_entries_kernel(int64_t n, const uint64_t* __restrict__ keys,
+                                                             const float* __restrict__ vals,
+                                                             uint16_t* __restrict__ cyc,
+                                                             float* __restrict__ inten) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  cyc[i] = (uint16_t)keys[i];
+  inten[i] = vals[i];
 }
 
 struct SpectrumTable {
@@ -326,24 +422,14 @@ int fetch(const T* src, int64_t n, int loc, std::vector<T>& dst) {
 }
 
 // Uploads the spectrum table (and host peak arrays), and builds cycles, intens and
-// slice_starts.  `spec_list`: the spectra of window w in visit order from first_spec[w].
-int build_entries(AdsDia* d, const AdsRawArrays* raw, const SpectrumTable& t, const std::vector<int32_t>& win_of_spec,
+// slice_starts.  `list`: the pieces of window w's spectra in visit order from first_piece[w].
+int build_entries(AdsDia* d, const AdsRawArrays* raw, const std::vector<int32_t>& win_of_spec,
                   const std::vector<uint16_t>& cyc16, const std::vector<int64_t>& item_off,
-                  int64_t n_items, const std::vector<int64_t>& spec_list, const std::vector<int64_t>& first_spec,
+                  int64_t n_items, const std::vector<int64_t>& list, const std::vector<int64_t>& first_piece,
                   int64_t n_slots, const GridView& g, cudaStream_t st) {
   const int64_t n_spec = raw->n_spectra;
   const int64_t stride = d->grid_len + 1;
   if (n_slots == 0 || n_items == 0) return ADS_OK;
-  // the pieces of the spectra, in the same order
-  std::vector<int64_t> list, first_piece((size_t)d->n_obs + 1, 0);
-  list.reserve(spec_list.size());
-  for (int64_t w = 0; w < d->n_obs; ++w) {
-    for (int64_t k = first_spec[w]; k < first_spec[w + 1]; ++k) {
-      const int64_t s = spec_list[k], n = t.stop[s] - t.start[s];
-      for (int64_t i = 0; i * kPiecePeaks < n; ++i) list.push_back(s | i << kPieceShift);
-    }
-    first_piece[w + 1] = (int64_t)list.size();
-  }
   // device copies of the spectrum table and, if needed, the peak arrays
   DevBuf<int64_t> d_off, d_start, d_stop;
   DevBuf<int32_t> d_win;
@@ -408,15 +494,18 @@ int build_entries(AdsDia* d, const AdsRawArrays* raw, const SpectrumTable& t, co
   DevBuf<uint32_t> sums;
   DevBuf<uint2> bins, large;
   DevBuf<uint4> recs;
-  DevBuf<unsigned int> n_large;
+  DevBuf<GroupCounts> counts;
   ADS_TRY(d_wins.alloc(wins.size()));
-  ADS_TRY(bins.alloc((size_t)most_items));
-  ADS_TRY(recs.alloc((size_t)most_items));
+  // (a group that is sorted whole has its keys in `bins` and the rest of the sort's buffers
+  // in `recs`, in four multiples of 64 peaks)
+  const size_t most_up = ((size_t)most_items + 63) / 64 * 64;
+  ADS_TRY(bins.alloc(most_up));
+  ADS_TRY(recs.alloc(most_up));
   ADS_TRY(sums.alloc((size_t)most_slots * tiles));
   ADS_TRY(large.alloc((size_t)(most_items / (kBinThread + 1) + 1)));
-  ADS_TRY(n_large.alloc(groups.size()));
+  ADS_TRY(counts.alloc(groups.size()));
   ADS_CUDA(cudaMemcpyAsync(d_wins.p, wins.data(), wins.size() * sizeof(BuildWin), cudaMemcpyHostToDevice, st));
-  ADS_CUDA(cudaMemsetAsync(n_large.p, 0, n_large.bytes(), st));
+  ADS_CUDA(cudaMemsetAsync(counts.p, 0, counts.bytes(), st));
   for (size_t k = 0; k < groups.size(); ++k) {
     const Group& gr = groups[k];
     const int64_t item0 = d->win[gr.w0].base;
@@ -426,20 +515,49 @@ int build_entries(AdsDia* d, const AdsRawArrays* raw, const SpectrumTable& t, co
     count_peaks_kernel<<<sg, 256, 0, st>>>(gr.pieces, gl, d_off.p, pstart, pstop, d_win.p, (int)gr.w0, gw, item0,
                                            mz, g, bins.p, d->slice_starts.p);
     ADS_LAUNCH_CHECK();
-    tile_sums_kernel<<<gr.slots * tiles, kScanThreads, 0, st>>>(d->grid_len, tiles, gw, d->slice_starts.p, sums.p);
+    tile_sums_kernel<<<gr.slots * tiles, kScanThreads, 0, st>>>(d->grid_len, tiles, gw, d->slice_starts.p, sums.p,
+                                                                counts.p + k);
     ADS_LAUNCH_CHECK();
     scan_sums_kernel<<<gr.slots, kScanThreads, 0, st>>>(tiles, sums.p);
     ADS_LAUNCH_CHECK();
     scan_tiles_kernel<<<gr.slots * tiles, kScanThreads, 0, st>>>(d->grid_len, tiles, gw, sums.p, d->slice_starts.p);
     ADS_LAUNCH_CHECK();
     place_peaks_kernel<<<sg, 256, 0, st>>>(gr.pieces, gl, d_off.p, pstart, pstop, d_win.p, d_cyc.p, (int)gr.w0, gw,
-                                           item0, pint, bins.p, d->slice_starts.p, recs.p);
+                                           item0, pint, bins.p, d->slice_starts.p, recs.p, counts.p + k, gr.items);
     ADS_LAUNCH_CHECK();
     order_bins_kernel<<<dim3((unsigned)((d->grid_len + 255) / 256), (unsigned)gr.slots), 256, 0, st>>>(
-        d->grid_len, gw, item0, d->slice_starts.p, recs.p, d->cycles.p, d->intens.p, large.p, n_large.p + k);
+        d->grid_len, gw, item0, d->slice_starts.p, recs.p, d->cycles.p, d->intens.p, large.p, counts.p + k,
+        gr.items);
     ADS_LAUNCH_CHECK();
-    order_large_bins_kernel<<<148 * 4, 256, 0, st>>>(n_large.p + k, large.p, gw, item0, d->slice_starts.p,
+    order_large_bins_kernel<<<148 * 4, 256, 0, st>>>(counts.p + k, large.p, gw, item0, d->slice_starts.p,
                                                      recs.p, d->cycles.p, d->intens.p);
+    ADS_LAUNCH_CHECK();
+  }
+  // the groups whose bins are too full for that
+  std::vector<GroupCounts> told(groups.size());
+  ADS_CUDA(cudaMemcpyAsync(told.data(), counts.p, counts.bytes(), cudaMemcpyDeviceToHost, st));
+  ADS_CUDA(cudaStreamSynchronize(st));
+  DevBuf<unsigned char> tmp;
+  for (size_t k = 0; k < groups.size(); ++k) {
+    const Group& gr = groups[k];
+    if (!sorted_whole(told[k], gr.items)) continue;
+    const int64_t item0 = d->win[gr.w0].base;
+    uint64_t* keys_b = reinterpret_cast<uint64_t*>(recs.p);
+    float* vals_a = reinterpret_cast<float*>(keys_b + most_up);
+    cub::DoubleBuffer<uint64_t> keys(reinterpret_cast<uint64_t*>(bins.p), keys_b);
+    cub::DoubleBuffer<float> vals(vals_a, vals_a + most_up);
+    int end_bit = kKeyWinShift;
+    while ((gr.slots - 1) >> (end_bit - kKeyWinShift)) ++end_bit;
+    size_t need = 0;
+    ADS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, need, keys, vals, gr.items, 0, end_bit, st));
+    ADS_TRY(tmp.reserve(need + 16));
+    key_peaks_kernel<<<(int)((gr.pieces + 7) / 8), 256, 0, st>>>(
+        gr.pieces, d_list.p + first_piece[gr.w0], d_off.p, pstart, pstop, d_win.p, d_cyc.p, (int)gr.w0, item0, mz,
+        pint, g, keys.Current(), vals.Current());
+    ADS_LAUNCH_CHECK();
+    ADS_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, need, keys, vals, gr.items, 0, end_bit, st));
+    sorted_entries_kernel<<<(unsigned)((gr.items + 255) / 256), 256, 0, st>>>(
+        gr.items, keys.Current(), vals.Current(), d->cycles.p + item0, d->intens.p + item0);
     ADS_LAUNCH_CHECK();
   }
   ADS_CUDA(cudaStreamSynchronize(st));
@@ -552,7 +670,7 @@ int dia_create(const AdsRawArrays* raw, int device, AdsDia** out) {
   std::vector<char> seen_first((size_t)n_obs, 0);
   std::vector<int32_t> win_of_spec((size_t)n_spec, -1);
   std::vector<uint16_t> cyc16((size_t)n_spec);
-  std::vector<int64_t> first_spec((size_t)n_obs + 1, 0);
+  std::vector<int64_t> first_piece((size_t)n_obs + 1, 0);
   std::vector<int64_t> last_cycle((size_t)n_obs, -1);
   std::vector<char> unsorted((size_t)n_obs, 0);  // cycles that step back: counted below
   for (int64_t s = 0; s < n_spec; ++s) {
@@ -566,7 +684,7 @@ int dia_create(const AdsRawArrays* raw, int device, AdsDia** out) {
       d->win[w].hi = t.hi[s];
     }
     d->num_peaks[w] += t.stop[s] - t.start[s];
-    ++first_spec[w + 1];
+    first_piece[w + 1] += (t.stop[s] - t.start[s] + kPiecePeaks - 1) / kPiecePeaks;
     if (t.cyc[s] > last_cycle[w]) {
       ++d->num_cycles[w];
       last_cycle[w] = t.cyc[s];
@@ -574,20 +692,24 @@ int dia_create(const AdsRawArrays* raw, int device, AdsDia** out) {
       unsorted[w] = 1;
     }
   }
-  // spectra by window, in visit order
-  for (int64_t w = 0; w < n_obs; ++w) first_spec[w + 1] += first_spec[w];
-  std::vector<int64_t> spec_list((size_t)first_spec[n_obs]);
+  // the pieces of the spectra by window, in visit order
+  for (int64_t w = 0; w < n_obs; ++w) first_piece[w + 1] += first_piece[w];
+  std::vector<int64_t> pieces((size_t)first_piece[n_obs]);
   {
-    std::vector<int64_t> cursor(first_spec.begin(), first_spec.end() - 1);
+    std::vector<int64_t> cursor(first_piece.begin(), first_piece.end() - 1);
     for (int64_t s = 0; s < n_spec; ++s)
-      if (win_of_spec[s] >= 0) spec_list[cursor[win_of_spec[s]]++] = s;
+      for (int64_t i = 0; win_of_spec[s] >= 0 && i * kPiecePeaks < t.stop[s] - t.start[s]; ++i)
+        pieces[cursor[win_of_spec[s]]++] = s | i << kPieceShift;
   }
-  for (int64_t w = 0; w < n_obs; ++w) {
-    if (!unsorted[w]) continue;
-    std::vector<int64_t> c;
-    for (int64_t k = first_spec[w]; k < first_spec[w + 1]; ++k) c.push_back(t.cyc[spec_list[k]]);
-    std::sort(c.begin(), c.end());
-    d->num_cycles[w] = std::unique(c.begin(), c.end()) - c.begin();
+  if (std::find(unsorted.begin(), unsorted.end(), 1) != unsorted.end()) {
+    std::vector<std::vector<int64_t>> c((size_t)n_obs);
+    for (int64_t s = 0; s < n_spec; ++s)
+      if (t.dsi[s] >= 0 && unsorted[t.dsi[s]]) c[t.dsi[s]].push_back(t.cyc[s]);
+    for (int64_t w = 0; w < n_obs; ++w) {
+      if (!unsorted[w]) continue;
+      std::sort(c[w].begin(), c[w].end());
+      d->num_cycles[w] = std::unique(c[w].begin(), c[w].end()) - c[w].begin();
+    }
   }
 
   // entry bases and slice_starts slots (observations without peaks get none)
@@ -646,8 +768,7 @@ int dia_create(const AdsRawArrays* raw, int device, AdsDia** out) {
   ADS_TRY(device_grid(device, &g));
   cudaStream_t st;
   ADS_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-  const int rc = build_entries(d, raw, t, win_of_spec, cyc16, item_off, n_items, spec_list, first_spec,
-                               n_slots, g, st);
+  const int rc = build_entries(d, raw, win_of_spec, cyc16, item_off, n_items, pieces, first_piece, n_slots, g, st);
   cudaStreamDestroy(st);
   if (rc != ADS_OK) return rc;
 

@@ -319,3 +319,47 @@ def test_build_time_of_long_spectra():
     mz = lambda n: torch.rand(n, device="cuda") * 1650 + 150
     few, many = build_ms(device_run(20, 8, 150_000, mz)), build_ms(device_run(3000, 8, 1000, mz))
     assert few < 4 * many, (few, many)
+
+
+@pytest.mark.parametrize("in_cycle_order", [True, False])
+@pytest.mark.parametrize("widths,background", [
+    ((25, 26, 64, 500), 9000),   # up to an eighth of the peaks in bins of more than 24: counted
+    ((1023, 1024), 16_500),      # ... in the widest bins that a block sorts
+    ((1025,), 16_500),           # wider, or more of them: sorted whole
+    ((40,) * 60, 3000),
+    ((3000, 7), 100),
+])
+def test_build_of_crowded_bins(widths, background, in_cycle_order):
+    """Bins of many peaks, with peaks outside the grid at both ends, three windows to a group:
+    the order is the same whichever way a group is put in order."""
+    rng = np.random.default_rng(len(widths) + background)
+    grid = mz_grid()
+    centres = grid[rng.choice(len(grid) - 2, len(widths), replace=False) + 1]
+    cycles = np.arange(40) if in_cycle_order else rng.permutation(40)
+    none = np.zeros(0)
+    spectra = []
+    for c in cycles:
+        spectra.append((0, c, none, none))
+        for w in (1, 2, 3):
+            k = [v // 40 + (1 if c < v % 40 else 0) for v in widths]
+            mz = np.concatenate([np.repeat(centres, k), rng.uniform(150, 2000, background // 40),
+                                 [90.0, 149.99, 2000.5][:int(rng.integers(0, 3))]])
+            mz = mz[rng.permutation(len(mz))]
+            spectra.append((w, c, mz, rng.lognormal(5, 2, len(mz))))
+    run = run_of(spectra, 3)
+    dia = DIAData.from_arrays(*(run[k] for k in RUN_KEYS), run["cycle"])
+    assert_entries_in_order(dia, spectra, 3, widths)
+
+
+@pytest.mark.parametrize("share", [0.01, 0.3])
+def test_build_time_of_peaks_outside_the_grid(share):
+    """A run with peaks below m/z 150, which all share a bin, is loaded in no more than 5
+    times the time of one without (a block to the bin: 18 times at 1 %)."""
+    import torch
+
+    def mz(n):
+        inside = torch.rand(n, device="cuda") * 1650 + 150
+        return torch.where(torch.rand(n, device="cuda") < share, inside * 0.05 + 50, inside)
+    some = build_ms(device_run(3000, 8, 1000, mz))
+    none = build_ms(device_run(3000, 8, 1000, lambda n: torch.rand(n, device="cuda") * 1650 + 150))
+    assert some < 5 * none, (some, none)
