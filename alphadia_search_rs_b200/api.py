@@ -10,6 +10,7 @@ behaviour.
 from __future__ import annotations
 
 import ctypes as C
+import threading
 from typing import Any
 
 import numpy as np
@@ -73,6 +74,63 @@ def _host_empty(n: int, dtype) -> np.ndarray:
     tdt = {np.dtype(np.uint64): t.uint64, np.dtype(np.float32): t.float32,
            np.dtype(np.uint8): t.uint8, np.dtype(np.int64): t.int64}[np.dtype(dtype)]
     return t.empty(n, dtype=tdt, pin_memory=True).numpy()
+
+
+class _HostBlocks:
+    """Host memory of tables that their caller has let go, kept for the next tables: fresh
+    pages cost a quantified library of 100,000 precursors 2.5 of 10.5 ms.  At most LIMIT bytes
+    are kept; what does not fit goes back to the system."""
+
+    LIMIT = 256 << 20
+    SMALL = 64 << 10  # arrays below are numpy's own
+
+    class _Block:
+        def __init__(self, home, buf):
+            self._home, self._buf = home, buf
+            self.__array_interface__ = buf.__array_interface__
+
+        def __del__(self):  # no array refers to the block any more
+            try:
+                self._home._give(self._buf)
+            except Exception:  # interpreter shutdown
+                pass
+
+    def __init__(self):
+        self._lock = threading.Lock()
+        self._free = {}
+        self.held = 0
+
+    def empty(self, n: int, dtype) -> np.ndarray:
+        """An uninitialised array of n elements."""
+        dtype = np.dtype(dtype)
+        need = n * dtype.itemsize
+        if need < self.SMALL:
+            return np.empty(n, dtype)
+        step = 1 << (need.bit_length() - 4)  # sizes in steps of an eighth or less
+        size = -(-need // step) * step
+        buf = None
+        with self._lock:
+            if self._free.get(size):
+                buf = self._free[size].pop()
+                self.held -= size
+        block = self._Block(self, np.empty(size, np.uint8) if buf is None else buf)
+        return np.asarray(block)[:need].view(dtype)
+
+    def _give(self, buf) -> None:
+        if not self._lock.acquire(blocking=False):
+            return  # busy, perhaps in this very thread (a collection inside empty())
+        try:
+            if self.held + buf.size > self.LIMIT:  # sizes that were not asked for again
+                self._free.clear()
+                self.held = 0
+            if buf.size <= self.LIMIT:
+                self._free.setdefault(buf.size, []).append(buf)
+                self.held += buf.size
+        finally:
+            self._lock.release()
+
+
+_HOST_BLOCKS = _HostBlocks()
 
 
 def _dev_ptr(name: str, t: Any, dtype, device: int) -> int:
@@ -905,13 +963,13 @@ class SpecLibFlatQuantified:
 
 def _gather_columns(cols) -> list:
     """Fresh host arrays src[rows] for (src, rows) pairs of contiguous numpy arrays (rows
-    None: a copy), gathered by native threads into page-locked memory that is reused (numpy
-    gathered and copied 100 MB of a quantified library with one thread into fresh pages:
-    25 of a call's 30 ms)."""
+    None: a copy), gathered by native threads (numpy gathered and copied 100 MB of a quantified
+    library with one thread into fresh pages: 25 of a call's 30 ms).  Not page-locked memory:
+    its allocator would keep all that a caller ever held at once."""
     if sum((len(s) if r is None else len(r)) * s.itemsize for s, r in cols) < 1 << 18:
         return [s.copy() if r is None else s[r] for s, r in cols]
     n = [len(s) if r is None else len(r) for s, r in cols]
-    out = [_host_empty(max(k, 1), s.dtype)[:k] for k, (s, _) in zip(n, cols)]
+    out = [_HOST_BLOCKS.empty(k, s.dtype) for k, (s, _) in zip(n, cols)]
     k = len(cols)
     ptrs = lambda xs: (C.c_void_p * k)(*[None if x is None else x.ctypes.data for x in xs])
     F.check(_lib().ads_host_gather(
