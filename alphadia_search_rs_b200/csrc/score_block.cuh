@@ -86,6 +86,7 @@ inline size_t block_smem_bytes(const BlockPlan& b, int group) {
 // Words of one candidate, for the shared helpers.
 struct SmVec {
   typedef int I;
+  static constexpr int kUnroll = 1;
   uint32_t* base;
   __device__ float f(int e) const { return __uint_as_float(base[e]); }
   __device__ void sf(int e, float v) const { base[e] = __float_as_uint(v); }
@@ -95,6 +96,7 @@ struct SmVec {
 // One thread's buffer, interleaved across the block's threads.
 struct ThreadVec {
   typedef int I;
+  static constexpr int kUnroll = 1;
   uint32_t* base;  // of the thread
   __device__ float f(int e) const { return __uint_as_float(base[e * kBlockThreads]); }
   __device__ void sf(int e, float v) const { base[e * kBlockThreads] = __float_as_uint(v); }
