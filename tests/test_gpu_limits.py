@@ -9,10 +9,10 @@ from alphadia_search_rs_b200 import (CandidateCollection, DIAData, PeakGroupQuan
                                      PeakGroupScoring, PeakGroupSelection, QuantificationParameters,
                                      ScoringParameters, SpecLibFlat, mz_grid, synth)
 
-from _util import COLS, RUN_KEYS, params_from
+from _util import COLS, RUN_KEYS, assert_candidates_equal, params_from
 from test_gpu_quant import assert_quant_equal, quant_library
 from test_gpu_scoring import assert_features_equal, build
-from test_gpu_sizes import closest_bins, library_of, run_of
+from test_gpu_sizes import PARAMS, closest_bins, library_of, run_of, search_both
 
 pytestmark = pytest.mark.gpu
 
@@ -363,3 +363,36 @@ def test_build_time_of_peaks_outside_the_grid(share):
     some = build_ms(device_run(3000, 8, 1000, mz))
     none = build_ms(device_run(3000, 8, 1000, lambda n: torch.rand(n, device="cuda") * 1650 + 150))
     assert some < 5 * none, (some, none)
+
+
+@pytest.mark.parametrize("kernel_size,half", [(14, 7), (20, 10), (21, 11), (31, 16), (40, 20)])
+def test_search_shortest_windows(kernel_size, half):
+    """RT windows that the run's ends cut to so many cycles: from the longest that hold no
+    candidate (the kernel's length) over the shortest that may hold one to 4 half widths and
+    more, at both ends."""
+    rng = np.random.default_rng(kernel_size)
+    n_cyc, F = 300, 5
+    lengths = np.arange(2 * half - 1, 4 * half + 6)
+    pad = 10.0 + kernel_size  # the least tolerance, at a cycle a second
+    prt = np.concatenate([lengths - 0.5 - pad, n_cyc - lengths - 0.5 + pad])
+    spans = [oracle.rt_limits(np.arange(n_cyc, dtype=np.float32), 1.0, t, 1.0, kernel_size)
+             for t in prt.astype(np.float32)]
+    assert [b - a for a, b in spans] == [*lengths, *lengths]
+    P = len(prt)
+    fmz = rng.uniform(200, 1700, (P, F))
+    mz = [[] for _ in range(n_cyc)]
+    for (a, b), row in zip(spans, fmz):
+        for f in row:
+            for c in rng.integers(a, b, 12):
+                mz[c].append(f * (1 + rng.uniform(-9e-6, 9e-6)))
+    none = np.zeros(0)
+    spectra = []
+    for c in range(n_cyc):
+        spectra += [(0, c, none, none), (1, c, np.sort(mz[c]), rng.lognormal(6, 2, len(mz[c])))]
+    run = run_of(spectra, 1)
+    la = library_of(405.0, prt, fmz, rng.uniform(0.1, 1.0, (P, F)))
+    params = dict(PARAMS, kernel_size=kernel_size, rt_tolerance=1.0, fwhm_rt=1.5 if half == 7 else 3.0)
+    for mode in (1, 2):
+        got, ref = search_both(run, la, params, gather_mode=mode)
+        assert len(set(ref["precursor_idx"])) > P // 3
+        assert_candidates_equal(got, ref, exact_scores=True, where=f"kernel {kernel_size} mode {mode}")
