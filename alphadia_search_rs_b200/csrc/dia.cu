@@ -832,7 +832,8 @@ int64_t ads_dia_memory_footprint_bytes(const AdsDia* dia) {
 int64_t ads_dia_device_bytes(const AdsDia* dia) {
   if (!dia) return 0;
   return (int64_t)(dia->slice_starts.bytes() + dia->cycles.bytes() + dia->intens.bytes() +
-                   dia->intens_bf16.bytes() + dia->win_dev.bytes() + dia->rt_dev.bytes());
+                   dia->intens_bf16.bytes() + dia->win_dev.bytes() + dia->win_index_dev.bytes() +
+                   dia->rt_dev.bytes());
 }
 
 int ads_dia_rt_values(const AdsDia* dia, float* out, int64_t cap, int64_t* n) {

@@ -396,3 +396,16 @@ def test_search_shortest_windows(kernel_size, half):
         got, ref = search_both(run, la, params, gather_mode=mode)
         assert len(set(ref["precursor_idx"])) > P // 3
         assert_candidates_equal(got, ref, exact_scores=True, where=f"kernel {kernel_size} mode {mode}")
+
+
+def test_device_bytes_count_the_window_index():
+    """Windows all over one another have a longer index than windows side by side."""
+    none = np.zeros(0)
+    spectra = [(0, 0, none, none)] + [(w, 0, [300.0 + w], [1.0]) for w in range(1, 101)]
+    run = run_of(spectra, 100)
+    nested = dict(run)
+    w = run["spectrum_delta_scan_idx"]
+    nested["isolation_lower_mz"] = np.where(w == 0, -1, 600 - w).astype(np.float32)
+    nested["isolation_upper_mz"] = np.where(w == 0, -1, 600 + w).astype(np.float32)
+    held = [DIAData.from_arrays(*(r[k] for k in RUN_KEYS), r["cycle"]).device_bytes() for r in (run, nested)]
+    assert held[1] - held[0] > 4 * 90 * 100
