@@ -9,6 +9,7 @@ behaviour.
 """
 from __future__ import annotations
 
+import collections
 import ctypes as C
 import threading
 from typing import Any
@@ -77,28 +78,38 @@ def _host_empty(n: int, dtype) -> np.ndarray:
 
 
 class _HostBlocks:
-    """Host memory of tables that their caller has let go, kept for the next tables: fresh
-    pages cost a quantified library of 100,000 precursors 2.5 of 10.5 ms.  At most LIMIT bytes
-    are kept; what does not fit goes back to the system."""
+    """Host memory for tables that callers hold, by whose size it must not grow for good.
+    The first LOCKED bytes that are out at a time are page-locked (_host_empty; its allocator
+    keeps all that was ever out at once), the others ordinary memory, of which up to KEPT
+    bytes are kept for the next tables when callers let them go, since fresh pages cost: two
+    sets of tables of 100,000 quantified precursors in turn 8.0 ms a call from page-locked
+    memory, 8.6 from kept, 10.5 from fresh (the copies from the device into memory that the
+    host has just read are the slower ones)."""
 
-    LIMIT = 256 << 20
+    LOCKED = 512 << 20
+    KEPT = 256 << 20
     SMALL = 64 << 10  # arrays below are numpy's own
 
     class _Block:
-        def __init__(self, home, buf):
-            self._home, self._buf = home, buf
+        def __init__(self, home, buf, locked):
+            self._home, self._buf, self._locked = home, buf, locked
             self.__array_interface__ = buf.__array_interface__
 
         def __del__(self):  # no array refers to the block any more
             try:
-                self._home._give(self._buf)
+                if self._locked:
+                    self._home._unlocked.append(self._locked)
+                else:
+                    self._home._give(self._buf)
             except Exception:  # interpreter shutdown
                 pass
 
     def __init__(self):
         self._lock = threading.Lock()
         self._free = {}
-        self.held = 0
+        self.kept = 0
+        self._unlocked = collections.deque()  # sizes no longer out, counted by the next empty()
+        self.locked = 0
 
     def empty(self, n: int, dtype) -> np.ndarray:
         """An uninitialised array of n elements."""
@@ -106,26 +117,39 @@ class _HostBlocks:
         need = n * dtype.itemsize
         if need < self.SMALL:
             return np.empty(n, dtype)
-        step = 1 << (need.bit_length() - 4)  # sizes in steps of an eighth or less
-        size = -(-need // step) * step
+        whole = 1 << (need - 1).bit_length()  # what the page-locked memory's allocator takes
+        step = whole >> 4
+        size = -(-need // step) * step  # kept memory in steps of an eighth or less
         buf = None
         with self._lock:
-            if self._free.get(size):
+            while self._unlocked:
+                self.locked -= self._unlocked.popleft()
+            lock = self.locked + whole <= self.LOCKED
+            if lock:
+                self.locked += whole
+            elif self._free.get(size):
                 buf = self._free[size].pop()
-                self.held -= size
-        block = self._Block(self, np.empty(size, np.uint8) if buf is None else buf)
+                self.kept -= size
+        if lock:
+            try:
+                block = self._Block(self, _host_empty(n, dtype), whole)
+            except BaseException:
+                self._unlocked.append(whole)
+                raise
+            return np.asarray(block)
+        block = self._Block(self, np.empty(size, np.uint8) if buf is None else buf, 0)
         return np.asarray(block)[:need].view(dtype)
 
     def _give(self, buf) -> None:
         if not self._lock.acquire(blocking=False):
             return  # busy, perhaps in this very thread (a collection inside empty())
         try:
-            if self.held + buf.size > self.LIMIT:  # sizes that were not asked for again
+            if self.kept + buf.size > self.KEPT:  # sizes that were not asked for again
                 self._free.clear()
-                self.held = 0
-            if buf.size <= self.LIMIT:
+                self.kept = 0
+            if buf.size <= self.KEPT:
                 self._free.setdefault(buf.size, []).append(buf)
-                self.held += buf.size
+                self.kept += buf.size
         finally:
             self._lock.release()
 
@@ -964,8 +988,7 @@ class SpecLibFlatQuantified:
 def _gather_columns(cols) -> list:
     """Fresh host arrays src[rows] for (src, rows) pairs of contiguous numpy arrays (rows
     None: a copy), gathered by native threads (numpy gathered and copied 100 MB of a quantified
-    library with one thread into fresh pages: 25 of a call's 30 ms).  Not page-locked memory:
-    its allocator would keep all that a caller ever held at once."""
+    library with one thread into fresh pages: 25 of a call's 30 ms)."""
     if sum((len(s) if r is None else len(r)) * s.itemsize for s, r in cols) < 1 << 18:
         return [s.copy() if r is None else s[r] for s, r in cols]
     n = [len(s) if r is None else len(r) for s, r in cols]

@@ -52,28 +52,30 @@ def test_memory_of_tables_still_held_is_not_reused():
 
 def test_kept_memory_is_bounded_and_given_back():
     blocks = api._HostBlocks()
+    blocks.LOCKED = 0  # ordinary memory alone
     assert blocks.empty(10, np.float32).base is None  # small ones are numpy's own
     a = blocks.empty(10**6, np.float32)
     b = blocks.empty(10**6, np.float32)
     first = a.ctypes.data
     del a
     gc.collect()
-    assert 4 * 10**6 <= blocks.held <= 4.6 * 10**6
+    assert 4 * 10**6 <= blocks.kept <= 4.6 * 10**6
     a = blocks.empty(10**6 - 7, np.uint32)
-    assert a.ctypes.data == first and blocks.held == 0 and len(a) == 10**6 - 7
+    assert a.ctypes.data == first and blocks.kept == 0 and len(a) == 10**6 - 7
     del a, b
     many = [blocks.empty(40_000_000 + i * 6_000_000, np.uint8) for i in range(40)]  # 6.3 GB, untouched
     del many
     gc.collect()
-    assert blocks.held <= blocks.LIMIT
-    big = blocks.empty(blocks.LIMIT + 1, np.uint8)
+    assert blocks.kept <= blocks.KEPT
+    big = blocks.empty(blocks.KEPT + 1, np.uint8)
     del big
     gc.collect()
-    assert blocks.held <= blocks.LIMIT
+    assert blocks.kept <= blocks.KEPT
 
 
 def test_blocks_of_several_threads():
     blocks = api._HostBlocks()
+    blocks.LOCKED = 600_000  # of both kinds
     faults = []
 
     def work(t):
@@ -96,14 +98,38 @@ def test_blocks_of_several_threads():
         t.start()
     for t in threads:
         t.join()
-    assert not faults and blocks.held <= blocks.LIMIT
+    assert not faults and blocks.kept <= blocks.KEPT and blocks.locked <= blocks.LOCKED
 
 
-def test_gathered_columns_are_not_page_locked(monkeypatch):
-    """Tables that callers hold are ordinary memory: page-locked memory (_host_empty) is for
-    the copies from the device."""
-    def page_locked(*_):
-        raise AssertionError("page-locked memory for a gathered column")
+def test_page_locked_memory_is_bounded(monkeypatch):
+    """However many tables a caller holds, at most LOCKED bytes of them are page-locked
+    (_host_empty, whose allocator takes powers of two and keeps them)."""
+    out = {}  # address -> bytes, of the page-locked arrays that are out
+    most = [0]
+
+    class Locked(np.ndarray):
+        def __del__(self):
+            out.pop(self.__dict__.get("key"), None)
+
+    def page_locked(n, dtype):
+        a = np.empty(n, dtype).view(Locked)
+        a.key = (a.ctypes.data, a.nbytes)
+        out[a.key] = 1 << (a.nbytes - 1).bit_length()
+        most[0] = max(most[0], sum(out.values()))
+        return a
 
     monkeypatch.setattr(api, "_host_empty", page_locked)
-    api._gather_columns(columns(np.random.default_rng(1), 70_000, 200_000))
+    monkeypatch.setattr(api, "_HOST_BLOCKS", api._HostBlocks())
+    limit = 16 << 20
+    monkeypatch.setattr(api._HostBlocks, "LOCKED", limit)
+    cols = columns(np.random.default_rng(1), 70_000, 200_000)  # 5.2 MB of tables
+    held = [api._gather_columns(cols) for _ in range(8)]
+    assert limit // 2 < most[0] <= limit
+    for tables in held:
+        for got, (s, r) in zip(tables, cols):
+            assert np.array_equal(got, s if r is None else s[r])
+    del held, tables, got
+    gc.collect()
+    most[0] = 0
+    api._gather_columns(cols)
+    assert 0 < most[0] <= limit  # those let go are page-locked memory's again
