@@ -1105,9 +1105,10 @@ int block_group(const AdsDia* d, const BlockPlan& b, int64_t C) {
 }
 
 // The vectors of so many bytes of candidates lie between score_block_kernel and
-// feature_kernel; calls of more candidates (360,000 of 24 fragments and 11 cycles) take
-// them in parts.
-constexpr size_t kHeadBytes = size_t(256) << 20;
+// feature_kernel; calls of more candidates (730,000 of 24 fragments and 11 cycles) take
+// them in parts.  (Each part ends on a last wave of its own: 1.48 M candidates in parts of
+// 256 MB 10.58 ms, in one 10.15.)
+constexpr size_t kHeadBytes = size_t(512) << 20;
 
 template <bool QUANT>
 int launch_block(const QuantArgs& qa, const BlockPlan& b, int group, cudaStream_t st) {

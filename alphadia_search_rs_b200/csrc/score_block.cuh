@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
   }
   __syncthreads();
 
-  // ---- filter_sort_fragments (select_fragments): raw m/z, intensity and keep mark ...
+  // ---- filter_sort_fragments (select_fragments): m/z key, intensity and keep mark ...
   const int RAWM = B.prof, RAWI = B.prof + B.Fraw, KEEP = B.prof + 2 * B.Fraw;
   const int nraw_max = sh_max[0];
   for (int t = tid; t < group * nraw_max; t += kBlockThreads) {
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
     if (r >= k.nraw) continue;
     const SmVec s{vec + c * B.words};
     const float I = a.l_fint[k.fs + r];
-    s.sf(RAWM + r, a.l_fmz[k.fs + r]);
+    s.sf(RAWM + r, mz_key(a.l_fmz[k.fs + r]));
     s.sf(RAWI + r, I);
     s.su(KEEP + r, I > 0.0f && !(a.l_ftype[k.fs + r] == 121 && a.l_fnum[k.fs + r] == 1) ? 1u : 0u);
   }
@@ -380,14 +380,14 @@ __global__ void __launch_bounds__(kBlockThreads) score_block_kernel(const __grid
     const SmVec s{vec + c * B.words};
     const uint32_t need = k.F > top_k ? 2u : 1u;
     if (s.u(KEEP + r) < need) continue;
-    const float m = s.f(RAWM + r), key = mz_key(m);
+    const float key = s.f(RAWM + r), m = key < INFINITY ? key : a.l_fmz[k.fs + r];
     int pos = 0;
 #pragma unroll 1
     for (int j = 0; j < r; ++j)
-      if (s.u(KEEP + j) >= need) pos += mz_key(s.f(RAWM + j)) <= key;
+      if (s.u(KEEP + j) >= need) pos += s.f(RAWM + j) <= key;
 #pragma unroll 1
     for (int j = r + 1; j < k.nraw; ++j)
-      if (s.u(KEEP + j) >= need) pos += mz_key(s.f(RAWM + j)) < key;
+      if (s.u(KEEP + j) >= need) pos += s.f(RAWM + j) < key;
     s.sf(B.fmz + pos, m);
     s.sf(B.fint + pos, s.f(RAWI + r));
     if (QUANT) {

@@ -224,7 +224,7 @@ def test_threads_with_different_plans(what):
 
 
 def test_scoring_in_parts():
-    """More candidates than one pair of launches takes (360,000 here): every copy of a
+    """More candidates than one pair of launches takes (730,000 here): every copy of a
     candidate has the oracle's features, in its own row, also where the work order mixes
     precursors of few and many fragments; and the device holds little besides the results
     (all candidates' vectors at once would be 2.9 GB)."""
