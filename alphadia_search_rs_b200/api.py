@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import collections
 import ctypes as C
+import os
 import threading
 from typing import Any
 
@@ -77,6 +78,15 @@ def _host_empty(n: int, dtype) -> np.ndarray:
     return t.empty(n, dtype=tdt, pin_memory=True).numpy()
 
 
+def _share_of_memory() -> int:
+    """A 64th of the machine's memory, at least 256 MB."""
+    try:
+        whole = os.sysconf("SC_PAGE_SIZE") * os.sysconf("SC_PHYS_PAGES")
+    except (AttributeError, OSError, ValueError):
+        whole = 0
+    return max(whole // 64, 256 << 20)
+
+
 class _HostBlocks:
     """Host memory for tables that callers hold, by whose size it must not grow for good.
     The first LOCKED bytes that are out at a time are page-locked (_host_empty; its allocator
@@ -84,10 +94,11 @@ class _HostBlocks:
     bytes are kept for the next tables when callers let them go, since fresh pages cost: two
     sets of tables of 100,000 quantified precursors in turn 8.0 ms a call from page-locked
     memory, 8.6 from kept, 10.5 from fresh (the copies from the device into memory that the
-    host has just read are the slower ones)."""
+    host has just read are the slower ones); quantify of 9.2 M precursors 146 ms from
+    page-locked memory, 225 from fresh."""
 
-    LOCKED = 512 << 20
-    KEPT = 256 << 20
+    LOCKED = _share_of_memory()
+    KEPT = _share_of_memory()
     SMALL = 64 << 10  # arrays below are numpy's own
 
     class _Block:

@@ -52,7 +52,7 @@ def test_memory_of_tables_still_held_is_not_reused():
 
 def test_kept_memory_is_bounded_and_given_back():
     blocks = api._HostBlocks()
-    blocks.LOCKED = 0  # ordinary memory alone
+    blocks.LOCKED, blocks.KEPT = 0, 256 << 20  # ordinary memory alone
     assert blocks.empty(10, np.float32).base is None  # small ones are numpy's own
     a = blocks.empty(10**6, np.float32)
     b = blocks.empty(10**6, np.float32)
