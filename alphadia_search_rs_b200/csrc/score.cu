@@ -16,8 +16,9 @@
 // (src/peak_group_scoring/utils.rs:164-166), is 0 here.
 //
 // score_block_kernel (score_block.cuh) takes a few candidates per block through the
-// steps in shared memory.  Candidates whose matrices do not fit there, or a run without a
-// window index, go to score_kernel / quant_kernel: a thread per candidate, its matrices
+// steps in shared memory.  A call whose longest cycle range and longest fragment list do not
+// fit there, or one on a run without a window index, goes to score_kernel / quant_kernel
+// whole: a thread per candidate, its matrices
 // (F x C dense XIC, m/z and normalised profiles) and vectors in a global scratch
 // interleaved across threads (element e of thread t at e * T + t), so threads working on
 // the same element read consecutive words.
@@ -1095,8 +1096,8 @@ int quant_assemble(AdsQuant* r, const uint64_t* d_off, const int* d_pos, cudaStr
 }
 
 // The candidates a block of score_block_kernel takes, or 0 where the per-candidate kernels
-// run: candidates of so many fragments or cycles that fewer than 2 fit a block's shared
-// memory (whole-run cycle ranges), or a run without a window index.
+// run: so many fragments or cycles that fewer than 2 candidates fit a block's shared memory
+// (whole-run cycle ranges; the most of the call count), or a run without a window index.
 int block_group(const AdsDia* d, const BlockPlan& b, int64_t C) {
   if (!d->win_index_ok || C > 4096) return 0;
   int group = kGroup;

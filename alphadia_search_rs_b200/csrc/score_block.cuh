@@ -10,8 +10,8 @@
 // issue).  A thread per candidate (score_kernel) ran 8 of 32 lanes per instruction on matrices
 // in a global scratch, and walked every bin of every fragment with a binary search.  Here a
 // row's whole range of entries is read 8 cycle indices at a time, and only an entry inside
-// the window looks up its bin: 1.48 M candidates of 4-24 fragments scored 41.0 -> 10.5 ms,
-// quantified 29.0 -> 8.0 ms.
+// the window looks up its bin: 1.48 M candidates of 4-24 fragments scored 41.0 -> 10.2 ms,
+// quantified 29.0 -> 7.8 ms.
 constexpr int kGroup = 4;        // candidates of a block (at most)
 // 2 warps for 4 candidates; for 2: scored 3.06 ms against 2.51 (295,000 candidates); 1 warp
 // for 4: 2.76; 1 for 2: 2.47, but quantified 1.19 against 1.18.

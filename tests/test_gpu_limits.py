@@ -328,6 +328,7 @@ def test_build_time_of_long_spectra():
     ((1025,), 16_500),           # wider, or more of them: sorted whole
     ((40,) * 60, 3000),
     ((3000, 7), 100),
+    ((30_000, 1), 2000),
 ])
 def test_build_of_crowded_bins(widths, background, in_cycle_order):
     """Bins of many peaks, with peaks outside the grid at both ends, three windows to a group:
