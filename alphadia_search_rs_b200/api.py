@@ -13,6 +13,7 @@ import collections
 import ctypes as C
 import os
 import threading
+import weakref
 from typing import Any
 
 import numpy as np
@@ -102,16 +103,15 @@ class _HostBlocks:
     SMALL = 64 << 10  # arrays below are numpy's own
 
     class _Block:
-        def __init__(self, home, buf, locked):
-            self._home, self._buf, self._locked = home, buf, locked
+        """Ordinary memory that comes back once no array refers to it."""
+
+        def __init__(self, home, buf):
+            self._home, self._buf = home, buf
             self.__array_interface__ = buf.__array_interface__
 
-        def __del__(self):  # no array refers to the block any more
+        def __del__(self):
             try:
-                if self._locked:
-                    self._home._unlocked.append(self._locked)
-                else:
-                    self._home._give(self._buf)
+                self._home._give(self._buf)
             except Exception:  # interpreter shutdown
                 pass
 
@@ -119,13 +119,13 @@ class _HostBlocks:
         self._lock = threading.Lock()
         self._free = {}
         self.kept = 0
-        self._unlocked = collections.deque()  # sizes no longer out, counted by the next empty()
+        self._out = {}  # page-locked arrays that are out: their owners' weak references, bytes
+        self._back = collections.deque()  # bytes no longer out, counted by the next empty()
         self.locked = 0
 
     def empty(self, n: int, dtype) -> np.ndarray:
         """An uninitialised array of n elements."""
-        dtype = np.dtype(dtype)
-        need = n * dtype.itemsize
+        need = n * np.dtype(dtype).itemsize
         if need < self.SMALL:
             return np.empty(n, dtype)
         whole = 1 << (need - 1).bit_length()  # what the page-locked memory's allocator takes
@@ -133,8 +133,8 @@ class _HostBlocks:
         size = -(-need // step) * step  # kept memory in steps of an eighth or less
         buf = None
         with self._lock:
-            while self._unlocked:
-                self.locked -= self._unlocked.popleft()
+            while self._back:
+                self.locked -= self._back.popleft()
             lock = self.locked + whole <= self.LOCKED
             if lock:
                 self.locked += whole
@@ -143,13 +143,18 @@ class _HostBlocks:
                 self.kept -= size
         if lock:
             try:
-                block = self._Block(self, _host_empty(n, dtype), whole)
+                a = _host_empty(n, dtype)
             except BaseException:
-                self._unlocked.append(whole)
+                self._back.append(whole)
                 raise
-            return np.asarray(block)
-        block = self._Block(self, np.empty(size, np.uint8) if buf is None else buf, 0)
-        return np.asarray(block)[:need].view(dtype)
+            # (views of `a` refer to the owner of its memory, not to `a`)
+            ref = weakref.ref(a if a.base is None else a.base, self._unlocked)
+            self._out[id(ref)] = ref, whole
+            return a
+        return np.asarray(self._Block(self, np.empty(size, np.uint8) if buf is None else buf))[:need].view(dtype)
+
+    def _unlocked(self, ref) -> None:
+        self._back.append(self._out.pop(id(ref))[1])
 
     def _give(self, buf) -> None:
         if not self._lock.acquire(blocking=False):

@@ -410,3 +410,22 @@ def test_device_bytes_count_the_window_index():
     nested["isolation_upper_mz"] = np.where(w == 0, -1, 600 + w).astype(np.float32)
     held = [DIAData.from_arrays(*(r[k] for k in RUN_KEYS), r["cycle"]).device_bytes() for r in (run, nested)]
     assert held[1] - held[0] > 4 * 90 * 100
+
+
+def test_page_locked_tables_are_counted_while_any_view_lives():
+    import gc
+
+    from alphadia_search_rs_b200 import api
+
+    blocks = api._HostBlocks()
+    a = blocks.empty(10**6, np.float32)
+    assert blocks.locked == 1 << 22
+    part = a[7:9].view(np.uint8)
+    del a
+    gc.collect()
+    b = blocks.empty(10**6, np.uint8)  # counts those that are gone: none
+    assert blocks.locked == (1 << 22) + (1 << 20)
+    del part, b
+    gc.collect()
+    blocks.empty(70_000, np.uint8)
+    assert blocks.locked == 1 << 17
